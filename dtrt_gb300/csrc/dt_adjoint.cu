@@ -1,9 +1,10 @@
 // dtrt_gb300 — host orchestration of the reverse-mode density adjoint (k_adjoint).
 //
-// The replay runs with derivative width 1 whatever the scene's nder: the adjoint needs the
+// The replay runs with derivative width 0 whatever the scene's nder: the adjoint needs the
 // path values only, and the per-voxel gradient replaces the derivative slots. The scene
-// copy given to the kernel drops every velocity input so the dual slot stays zero and the
-// no-derivative fast paths apply; values and random decisions are those of dtrt_render_fwd.
+// copy given to the kernel drops every velocity input; values and random decisions are
+// those of dtrt_render_fwd. (At width 1, with a slot that was always zero, an AdjState took
+// 208 B instead of 144 B.)
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -28,12 +29,12 @@ cudaError_t launch_adjoint(const DevScene &sc, const RenderParams &rp, const flo
                            unsigned long long *ctr, long long stride, cudaStream_t st) {
     const long long n = (rp.path_count + stride - 1) / stride;
     if (n <= 0) return cudaSuccess;
-    k_adjoint<1><<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(sc, rp, dimg, grad, img_acc, ctr, stride);
+    k_adjoint<0><<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(sc, rp, dimg, grad, img_acc, ctr, stride);
     return cudaGetLastError();
 }
 
 size_t AdjWave::bytes(long long cap, int levels) {
-    return (size_t)cap * (sizeof(AdjState<1>) + sizeof(VertexIn<1>) + 4 * sizeof(int) + sizeof(float3) +
+    return (size_t)cap * (sizeof(AdjState<0>) + sizeof(VertexIn<0>) + 4 * sizeof(int) + sizeof(float3) +
                           kReplayEvents * sizeof(float3)) +
            (size_t)6 * (levels + 1) * sizeof(unsigned long long) + 2048;  // + 256-byte alignment of 6 arrays
 }
@@ -47,8 +48,8 @@ void AdjWave::carve(void *base, long long capacity, int lv) {
     };
     cap = capacity;
     levels = lv;
-    states = take((size_t)cap * sizeof(AdjState<1>));
-    vins = take((size_t)cap * sizeof(VertexIn<1>));
+    states = take((size_t)cap * sizeof(AdjState<0>));
+    vins = take((size_t)cap * sizeof(VertexIn<0>));
     q = (int *)take((size_t)4 * cap * sizeof(int));
     tots = (float3 *)take((size_t)cap * sizeof(float3));
     ev = (float3 *)take((size_t)cap * kReplayEvents * sizeof(float3));
@@ -64,8 +65,8 @@ cudaError_t launch_adjoint_wave(const DevScene &sc, const RenderParams &range, c
     const int levels = range.max_bounces + 1;
     if (levels > w.levels) return cudaErrorInvalidValue;
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
-    AdjState<1> *states = (AdjState<1> *)w.states;
-    VertexIn<1> *vins = (VertexIn<1> *)w.vins;
+    AdjState<0> *states = (AdjState<0> *)w.states;
+    VertexIn<0> *vins = (VertexIn<0> *)w.vins;
     int *qa = w.q, *qb = qa + w.cap, *qv = qb + w.cap, *qs = qv + w.cap;
     const bool pass_b = grad != nullptr && dimg != nullptr;
     RenderParams rp = range;
@@ -82,19 +83,19 @@ cudaError_t launch_adjoint_wave(const DevScene &sc, const RenderParams &range, c
             unsigned long long *vc = w.cnt + pass * 3 * (levels + 1), *sc_ = vc + (levels + 1);
             const QueueEnds qx{w.cap, levels + 1};
             // volume / interface queues of level L: (qa, qb) for even L, (qv, qs) for odd L
-            k_adj_start<1><<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, states, vins, qa, vc, qv, vc + 1, qs,
+            k_adj_start<0><<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, states, vins, qa, vc, qv, vc + 1, qs,
                                                                     sc_ + 1, dimg, grad, w.tots, w.ev, qx, b, ctr);
             for (int L = 0; L < levels; ++L) {
                 int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
                 int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
-                k_adj_vertex<1, true><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vc + L, qvn, vc + L + 1, qsn,
+                k_adj_vertex<0, true><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vc + L, qvn, vc + L + 1, qsn,
                                                             sc_ + L + 1, dimg, grad, w.tots, w.ev, qx, b, ctr);
                 if (L > 0)  // level 0's interface vertices ran in k_adj_start
-                    k_adj_vertex<1, false><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qsl, sc_ + L, qvn, vc + L + 1,
+                    k_adj_vertex<0, false><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qsl, sc_ + L, qvn, vc + L + 1,
                                                                  qsn, sc_ + L + 1, dimg, grad, w.tots, w.ev, qx, b,
                                                                  ctr);
             }
-            if (pass == 0) k_adj_totals<1><<<blocks(rp.path_count), kBlock, 0, st>>>(rp, states, w.tots, img_acc);
+            if (pass == 0) k_adj_totals<0><<<blocks(rp.path_count), kBlock, 0, st>>>(rp, states, w.tots, img_acc);
             if (launches) *launches += 2 * levels + (pass == 0 ? 1 : 0);  // start, 2 per level (1 at level 0), totals in pass A
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

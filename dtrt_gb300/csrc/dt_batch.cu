@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kBlock) k_batch(const BatchItemDev *items, con
         const long long base = ((long long)c - cbeg[lo]) * chunk;
         Ctr ctr;
         for (int k = lane; k < chunk; k += 32)  // sample_stride > 1 (tuning): every stride-th path
-            adjoint_one<1>(s_sc[warp], s_rp[warp], stack, base + k, dimg, grad, img_acc, ctr, sample_stride);
+            adjoint_one<0>(s_sc[warp], s_rp[warp], stack, base + k, dimg, grad, img_acc, ctr, sample_stride);
     }
 }
 
@@ -283,8 +283,8 @@ int upload_wave_layout(dtrt_batch *b, const std::vector<int> &order, long long s
 int enqueue_chunk(dtrt_batch *b, const AdjWave &w, BatchWave bw, cudaStream_t st) {
     const int levels = b->max_levels;
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
-    AdjState<1> *states = (AdjState<1> *)w.states;
-    VertexIn<1> *vins = (VertexIn<1> *)w.vins;
+    AdjState<0> *states = (AdjState<0> *)w.states;
+    VertexIn<0> *vins = (VertexIn<0> *)w.vins;
     int *qa = w.q, *qb = qa + w.cap, *qv = qb + w.cap, *qs = qv + w.cap;
     {
         const unsigned gw = std::min<unsigned>(blocks(bw.count), (unsigned)std::max(1, b->sms) * 16u);
@@ -294,18 +294,18 @@ int enqueue_chunk(dtrt_batch *b, const AdjWave &w, BatchWave bw, cudaStream_t st
             // per level: volume, interface front-end and back-end counts (as launch_adjoint_wave)
             unsigned long long *vc = w.cnt + pass * 3 * (levels + 1), *scn = vc + (levels + 1);
             const QueueEnds qx{w.cap, levels + 1};
-            k_badj_start<1><<<blocks(bw.count), kBlock, 0, st>>>(bw, states, vins, qa, vc, qv, vc + 1, qs, scn + 1,
+            k_badj_start<0><<<blocks(bw.count), kBlock, 0, st>>>(bw, states, vins, qa, vc, qv, vc + 1, qs, scn + 1,
                                                                 w.tots, w.ev, qx, pb);
             for (int L = 0; L < levels; ++L) {
                 int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
                 int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
-                k_badj_vertex<1, true><<<gw, kBlock, 0, st>>>(bw, states, vins, qvl, vc + L, qvn, vc + L + 1, qsn,
+                k_badj_vertex<0, true><<<gw, kBlock, 0, st>>>(bw, states, vins, qvl, vc + L, qvn, vc + L + 1, qsn,
                                                              scn + L + 1, w.tots, w.ev, qx, pb);
                 if (L > 0)
-                    k_badj_vertex<1, false><<<gw, kBlock, 0, st>>>(bw, states, vins, qsl, scn + L, qvn, vc + L + 1,
+                    k_badj_vertex<0, false><<<gw, kBlock, 0, st>>>(bw, states, vins, qsl, scn + L, qvn, vc + L + 1,
                                                                   qsn, scn + L + 1, w.tots, w.ev, qx, pb);
             }
-            if (pass == 0) k_badj_totals<1><<<blocks(bw.count), kBlock, 0, st>>>(bw, states, w.tots);
+            if (pass == 0) k_badj_totals<0><<<blocks(bw.count), kBlock, 0, st>>>(bw, states, w.tots);
         }
         DT_BCK(cudaGetLastError());
     }

@@ -1,0 +1,7 @@
+// dtrt_gb300 — camera stage of scenes without ray derivatives (static_rays) for nder = 1.
+#define DT_CAMERA_STATIC_UNIT
+#include "dt_render.cuh"
+
+namespace dt {
+template struct CameraStage<1, 0>;
+}

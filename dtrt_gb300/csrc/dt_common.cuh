@@ -179,7 +179,9 @@ struct Frame {
     DT_D Frame() {}
     DT_D explicit Frame(float3 nn) : n(nn) {
         const float R[9] = DT_PREROT_INIT;
-        float3 q = rot_apply(R, nn);
+        from_rotated(R, rot_apply(R, nn));
+    }
+    DT_D void from_rotated(const float *R, float3 q) {
         float3 tt;
         if (fabsf(q.x) > fabsf(q.y)) {
             float il = 1.0f / sqrtf(q.x * q.x + q.z * q.z);
@@ -195,6 +197,40 @@ struct Frame {
     DT_D float3 to_local(float3 v) const { return mk(dot(v, s), dot(v, t), dot(v, n)); }
     DT_D float3 to_world(float3 v) const { return s * v.x + t * v.y + n * v.z; }
 };
+
+// Sums of products with the fused operations written out: a b + c d and a b - c d with the
+// first product fused. Left to the compiler, which product of a sum is rounded and which is
+// fused depends on the code around it (a negated argument folds into a constant, a product
+// that has a second use is kept), and two kernels that run the same path then differ in the
+// last bit of a direction. Behind a dielectric of alpha 1e-4 that is a change of 1e-3.
+DT_D float sum2(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+DT_D float diff2(float a, float b, float c, float d) { return fmaf(a, b, -__fmul_rn(c, d)); }
+
+// Frame(n).to_world(l) for a sampled local direction l, with every rounding written out.
+// kNeg: n is the negation of a ray direction whose sign the compiler folds into the rotation.
+template <bool kNeg>
+DT_D float3 frame_to_world(float3 n, float3 l) {
+    const float R[9] = DT_PREROT_INIT;
+    const float3 q = mk(fmaf(R[2], n.z, kNeg ? sum2(R[1], n.y, R[0], n.x) : sum2(R[0], n.x, R[1], n.y)),
+                        fmaf(R[5], n.z, sum2(R[3], n.x, R[4], n.y)),
+                        fmaf(R[8], n.z, kNeg ? sum2(R[6], n.x, R[7], n.y) : sum2(R[7], n.y, R[6], n.x)));
+    float3 tt;
+    if (fabsf(q.x) > fabsf(q.y)) {
+        const float il = 1.0f / sqrtf(sum2(q.x, q.x, q.z, q.z));
+        tt = mk(__fmul_rn(q.z, il), 0.f, __fmul_rn(-q.x, il));
+    } else {
+        const float il = 1.0f / sqrtf(sum2(q.y, q.y, q.z, q.z));
+        tt = mk(0.f, __fmul_rn(q.z, il), __fmul_rn(-q.y, il));
+    }
+    const float3 ss = mk(diff2(tt.y, q.z, tt.z, q.y), diff2(tt.z, q.x, tt.x, q.z), diff2(tt.x, q.y, tt.y, q.x));
+    auto rot_t = [&](float3 v) {
+        return mk(fmaf(R[6], v.z, sum2(R[0], v.x, R[3], v.y)), fmaf(R[7], v.z, sum2(R[4], v.y, R[1], v.x)),
+                  fmaf(R[8], v.z, sum2(R[2], v.x, R[5], v.y)));
+    };
+    const float3 s = rot_t(ss), t = rot_t(tt);
+    return mk(fmaf(n.x, l.z, sum2(t.x, l.y, s.x, l.x)), fmaf(n.y, l.z, sum2(t.y, l.y, s.y, l.x)),
+              fmaf(n.z, l.z, sum2(t.z, l.y, s.z, l.x)));
+}
 
 template <int N>
 struct FrameAD {

@@ -33,6 +33,15 @@ template <int N> DT_HD DV<N> make_vec(const Df<N> &a, const Df<N> &b, const Df<N
 DT_HD float3 vval(float3 a) { return a; }
 template <int N> DT_HD float3 vval(const DV<N> &a) { return a.val(); }
 
+// A dual of width G as one of width N: G is N, or 0 (a quantity whose derivative slots are
+// zero by construction: rays and hits of static geometry under a static camera).
+template <int N, int G> DT_HD Df<N> lift(const Df<G> &a) {
+    static_assert(G == N || G == 0, "a dual is lifted from width 0 or kept");
+    if constexpr (G == N) return a;
+    else return Df<N>(a.v);
+}
+template <int N, int G> DT_HD DV<N> lift(const DV<G> &a) { return DV<N>(lift<N>(a.x), lift<N>(a.y), lift<N>(a.z)); }
+
 template <int N> DT_D Df<N> load_dual(float v, const float *d) {
     Df<N> r(v);
 #pragma unroll
@@ -214,7 +223,7 @@ struct RayAD {
 // utils.cpp:237-254 and shape.cpp:210-252
 template <int N>
 DT_HEAVY void shape_intersect_ad(const DevScene &sc, int prim, const RayAD<N> &ray, ItsAD<N> &its) {
-    if (!sc.vert_der && !sc.face_n_der && !sc.normal_der && ray.o.der_zero(0.f) && ray.d.der_zero(0.f)) {
+    if (N == 0 || (!sc.vert_der && !sc.face_n_der && !sc.normal_der && ray.o.der_zero(0.f) && ray.d.der_zero(0.f))) {
         // static geometry hit by a ray without derivatives: every slot is zero; the values
         // below follow the dual expressions operation for operation
         const int4 tri = __ldg(sc.tris + prim);
@@ -462,10 +471,11 @@ DT_D float3 bsdf_eval(const DevBsdf &b, float3 wi, float3 wo) {
     }
 }
 
-template <int N>
-DT_D DV<N> bsdf_eval_ad(const DevBsdf &b, const DV<N> &wi, const DV<N> &wo) {
+template <int N, int G>
+DT_D DV<N> bsdf_eval_ad(const DevBsdf &b, const DV<G> &wi_g, const DV<G> &wo_g) {
     // no parameter slots and fixed directions: the plain evaluation, lifted (all slots zero)
-    if (!b.has_der && wi.der_zero(0.f) && wo.der_zero(0.f)) return DV<N>(bsdf_eval(b, wi.val(), wo.val()));
+    if (!b.has_der && wi_g.der_zero(0.f) && wo_g.der_zero(0.f)) return DV<N>(bsdf_eval(b, wi_g.val(), wo_g.val()));
+    const DV<N> wi = lift<N>(wi_g), wo = lift<N>(wo_g);
     switch (b.type) {
         case BSDF_NULL: return DV<N>(mk(1.f, 1.f, 1.f));
         case BSDF_DIFFUSE:  // diffuse.cpp:15-20
@@ -584,9 +594,9 @@ DT_HEAVY float3 bsdf_sample(const DevBsdf &b, float3 wi, float r0, float r1, flo
 }
 
 // bsdf.cpp:11-21 (null.cpp:20-25 for the null BSDF)
-template <int N>
-DT_D DV<N> bsdf_sample_ad(const DevBsdf &b, const ItsAD<N> &its, const FrameAD<N> &fr, const Its &its0, float r0,
-                          float r1, float r2, DV<N> &wo, float &pdf, float &eta) {
+template <int N, int G>
+DT_D DV<N> bsdf_sample_ad(const DevBsdf &b, const ItsAD<G> &its, const FrameAD<G> &fr, const Its &its0, float r0,
+                          float r1, float r2, DV<G> &wo, float &pdf, float &eta) {
     if (b.type == BSDF_NULL) {
         wo = -its.wi;
         pdf = 1.f;
@@ -600,7 +610,7 @@ DT_D DV<N> bsdf_sample_ad(const DevBsdf &b, const ItsAD<N> &its, const FrameAD<N
         if (pdf > kEps) {
             if (fixed) {  // no slot can become non-zero: plain evaluation, lifted
                 const float3 w = fr.plain().to_local(its0.to_world(wo0));
-                wo = DV<N>(w);
+                wo = DV<G>(w);
                 ret = DV<N>(bsdf_eval(b, its.wi.val(), w) / pdf);
             } else {
                 wo = fr.to_local(its0.to_world(wo0));
@@ -616,15 +626,18 @@ DT_D float phase_eval(const DevPhase &p, float3 wi, float3 wo) {
     float g = p.g, tmp = 1.f + g * g + 2.f * g * dot(wi, wo);
     return kInvFourPi * (1.f - g * g) / (tmp * sqrtf(tmp));
 }
-template <int N>
-DT_D Df<N> phase_eval_ad(const DevPhase &p, const DV<N> &wi, const DV<N> &wo) {
+template <int N, int G>
+DT_D Df<N> phase_eval_ad(const DevPhase &p, const DV<G> &wi, const DV<G> &wo) {
     if (p.type == PHASE_ISOTROPIC) return Df<N>(kInvFourPi);
     if (!p.has_der && wi.der_zero(0.f) && wo.der_zero(0.f)) return Df<N>(phase_eval(p, wi.val(), wo.val()));
     Df<N> g = load_dual<N>(p.g, p.d_g);
-    Df<N> tmp = 1.f + g * g + 2.f * g * dot(wi, wo);
+    Df<N> tmp = 1.f + g * g + 2.f * g * lift<N>(dot(wi, wo));
     return kInvFourPi * (1.f - g * g) / dpow(tmp, 1.5f);
 }
 // phase.h:40-51: the HG local frame is built around wi (the reference's convention, kept)
+// kMode 1, 2: the sampled direction with every rounding written out (frame_to_world), as the
+// kernels with derivatives of width up to 1 and above 1 round it
+template <int kMode = 0>
 DT_D float phase_sample(const DevPhase &p, float3 wi, float u, float v, float3 &wo) {
     if (p.type == PHASE_ISOTROPIC) {
         wo = square_to_uniform_sphere(u, v);
@@ -640,14 +653,16 @@ DT_D float phase_sample(const DevPhase &p, float3 wi, float u, float v, float3 &
     float st = sqrtf(fmaxf(0.f, 1.f - ct * ct));
     float sp, cp;
     sincosf(2.f * kPi * v, &sp, &cp);
-    wo = Frame(wi).to_world(mk(st * cp, st * sp, ct));
+    const float3 l = mk(st * cp, st * sp, ct);
+    if constexpr (kMode == 0) wo = Frame(wi).to_world(l);
+    else wo = frame_to_world<kMode == 1>(wi, l);
     return 1.f;
 }
-template <int N>
-DT_D Df<N> phase_sample_ad(const DevPhase &p, const DV<N> &wi, float u, float v, DV<N> &wo) {
+template <int N, int G>
+DT_D Df<N> phase_sample_ad(const DevPhase &p, const DV<G> &wi, float u, float v, DV<G> &wo) {
     float3 w;
-    phase_sample(p, wi.val(), u, v, w);
-    wo = DV<N>(w);
+    phase_sample<G == 0 ? (N <= 1 ? 1 : 2) : 0>(p, wi.val(), u, v, w);
+    wo = DV<G>(w);
     if (p.type == PHASE_ISOTROPIC) return Df<N>(1.f);  // phase.h:14-19 with evalAD == pdf
     Df<N> tmp = phase_eval_ad<N>(p, wi, wo);           // phase.h:53-58
     return tmp.v > kEps ? tmp / tmp.v : Df<N>(0.f);
@@ -664,12 +679,12 @@ DT_D float3 le(const DevScene &sc, const Its &its, float3 w) {
     const DevEmitter &e = sc.emitters[sc.shapes[its.shape].light_id];
     return le_normal(e, e.type == EMITTER_AREA ? its.ng : its.fr.n, w);
 }
-template <int N>
-DT_D DV<N> le_ad(const DevScene &sc, const ItsAD<N> &its, const DV<N> &w) {
+template <int N, int G>
+DT_D DV<N> le_ad(const DevScene &sc, const ItsAD<G> &its, const DV<G> &w) {
     const DevEmitter &e = sc.emitters[sc.shapes[its.shape].light_id];
     if (e.type == EMITTER_AREA)
         return (e.two_sided || dot(its.ng, w.val()) > 0.f) ? DV<N>(f3(e.intensity)) : DV<N>();
-    Df<N> t = dot(its.ns, w);
+    Df<N> t = lift<N>(dot(its.ns, w));
     if (t.v > kEps) {
         Df<N> k = load_dual<N>(e.kappa, e.d_kappa);
         return load_dual3<N>(e.intensity, e.d_intensity) * (dexp(k * (t - 1.f)) * k * kInvTwoPi);
@@ -713,9 +728,10 @@ DT_D float3 grid_point(const DevGrid &g, float3 pw) {  // worldToVolume + volume
                   m[8] * pw.x + m[9] * pw.y + m[10] * pw.z + m[11]);
     return mk((p.x - g.mn[0]) * g.to_grid[0], (p.y - g.mn[1]) * g.to_grid[1], (p.z - g.mn[2]) * g.to_grid[2]);
 }
-template <int N>
-DT_D DV<N> grid_point_ad(const DevGrid &g, const DV<N> &pw) {  // gridvolume.h:301-326
+template <int N, int G>
+DT_D DV<N> grid_point_ad(const DevGrid &g, const DV<G> &pw_g) {  // gridvolume.h:301-326
     const float *m = g.w2v;
+    const DV<N> pw = lift<N>(pw_g);
     const float3 pv = pw.val();
     DV<N> p(grid_point(g, pv));
     const float3 q = pv - f3(g.center);
@@ -754,12 +770,47 @@ DT_D float grid_lookup(const DevGrid &g, float3 pw, Ctr &c) {  // gridvolume.h:1
     return ((d000 * gx + d001 * fx) * gy + (d010 * gx + d011 * fx) * fy) * gz +
            ((d100 * gx + d101 * fx) * gy + (d110 * gx + d111 * fx) * fy) * fz;
 }
-template <int N>
-DT_D Df<N> grid_lookup_ad(const DevGrid &g, const DV<N> &pw, Ctr &c) {  // gridvolume.h:174-201
+// Density value and its gradient in world space at a point (zero outside the grid). With a
+// point that carries no derivative, slot j of a moving grid's density is the gradient times
+// the point's velocity in the grid, h . -(rot_j x q + trans_j) = -(rot_j . (q x h) +
+// trans_j . h) with q = p - centre (gridvolume.h:301-326): one gradient serves every slot,
+// and its sums over the samples of a line integral do as well.
+DT_D float grid_lookup_grad(const DevGrid &g, float3 pw, float3 &h, Ctr &c) {
+    c.lookups++;
+    h = mk(0.f, 0.f, 0.f);
+    const float3 p = grid_point(g, pw);
+    int x1, y1, z1;
+    if (!grid_cell(g, p, x1, y1, z1)) return 0.f;
+    const float fx = p.x - x1, fy = p.y - y1, fz = p.z - z1, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
+    const int sx = 1, sy = g.res[0], sz = g.res[0] * g.res[1];
+    const float *d = g.data + (size_t)z1 * sz + (size_t)y1 * sy + x1;
+    const float d000 = __ldg(d), d001 = __ldg(d + sx), d010 = __ldg(d + sy), d011 = __ldg(d + sy + sx);
+    const float d100 = __ldg(d + sz), d101 = __ldg(d + sz + sx), d110 = __ldg(d + sz + sy), d111 = __ldg(d + sz + sy + sx);
+    const float a00 = d000 * gx + d001 * fx, a01 = d010 * gx + d011 * fx, a10 = d100 * gx + d101 * fx,
+                a11 = d110 * gx + d111 * fx;
+    const float3 u = mk((((d001 - d000) * gy + (d011 - d010) * fy) * gz + ((d101 - d100) * gy + (d111 - d110) * fy) * fz) * g.to_grid[0],
+                        ((a01 - a00) * gz + (a11 - a10) * fz) * g.to_grid[1],
+                        ((a10 - a00) * gy + (a11 - a01) * fy) * g.to_grid[2]);
+    const float *m = g.w2v;
+    h = mk(m[0] * u.x + m[4] * u.y + m[8] * u.z, m[1] * u.x + m[5] * u.y + m[9] * u.z, m[2] * u.x + m[6] * u.y + m[10] * u.z);
+    return (a00 * gy + a01 * fy) * gz + (a10 * gy + a11 * fy) * fz;
+}
+template <int N, int G>
+DT_D Df<N> grid_lookup_ad(const DevGrid &g, const DV<G> &pw, Ctr &c) {  // gridvolume.h:174-201
     const bool voxel_dirs = g.dgrid != nullptr && g.dgrid_n == N;
     // A static grid sampled at a point without derivatives has none either: the plain
     // lookup gives the same dual exactly (all slots zero) at a fraction of the cost.
-    if (!g.moving && !voxel_dirs && pw.der_zero(0.f)) return Df<N>(grid_lookup(g, pw.val(), c));
+    if (N == 0 || (!g.moving && !voxel_dirs && pw.der_zero(0.f))) return Df<N>(grid_lookup(g, pw.val(), c));
+    if constexpr (G == 0) {
+        if (!voxel_dirs) {
+            float3 h;
+            Df<N> r(grid_lookup_grad(g, pw.val(), h, c));
+            const float3 qh = cross(pw.val() - f3(g.center), h);
+#pragma unroll
+            for (int j = 0; j < N; ++j) r.d[j] = -(dot(f3(g.rot_vel[j]), qh) + dot(f3(g.trans_vel[j]), h));
+            return r;
+        }
+    }
     c.lookups++;
     const DV<N> p = grid_point_ad<N>(g, pw);
     int x1, y1, z1;
@@ -830,8 +881,8 @@ DT_D float3 grid_lookup3(const DevGrid &g, float3 pw) {  // gridvolume.h:204-232
     }
     return mk(r[0], r[1], r[2]);
 }
-template <int N>
-DT_D DV<N> grid_lookup3_ad(const DevGrid &g, const DV<N> &pw) {  // gridvolume.h:235-263
+template <int N, int G>
+DT_D DV<N> grid_lookup3_ad(const DevGrid &g, const DV<G> &pw) {  // gridvolume.h:235-263
     const DV<N> p = grid_point_ad<N>(g, pw);
     int x1, y1, z1;
     if (!grid_cell(g, p.val(), x1, y1, z1)) return DV<N>();
@@ -913,16 +964,17 @@ DT_HEAVY bool sample_distance(const DevScene &sc, const DevMedium &m, float3 &o,
 // heterogeneous.cpp:121-141: -d/dtheta of the optical depth over [tmin, tmax]
 // With `adj`, each sample also scatters adj->w * (-scale * len / 10) into the gradient:
 // the factor exp(-optical depth) has log-derivative -(this integral).
-template <int N>
-DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<N> &ray, const Df<N> &tmin, const Df<N> &tmax,
-                    Rng &rng, float out[N], Ctr &c, const AdjCtx *adj = nullptr) {
+template <int N, int G>
+DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &ray, const Df<G> &tmin, const Df<G> &tmax,
+                    Rng &rng, float *out, Ctr &c, const AdjCtx *adj = nullptr) {
     const Df<N> scale = load_dual<N>(m.scale, m.d_scale);
 #pragma unroll
     for (int j = 0; j < N; ++j) out[j] = 0.f;
     const float len = tmax.v - tmin.v;
     const bool scatter = adj != nullptr && m.grad_off >= 0 && adj->w != 0.f;
-    if (scale.der_zero(0.f) && !m.density.moving && !(m.density.dgrid && m.density.dgrid_n == N) &&
-        ray.o.der_zero(0.f) && ray.d.der_zero(0.f) && tmin.der_zero(1e-6f) && tmax.der_zero(1e-6f)) {
+    if (N == 0 ||
+        (scale.der_zero(0.f) && !m.density.moving && !(m.density.dgrid && m.density.dgrid_n == N) &&
+         ray.o.der_zero(0.f) && ray.d.der_zero(0.f) && tmin.der_zero(1e-6f) && tmax.der_zero(1e-6f))) {
         // nothing in the integral carries a derivative: every slot is zero. Draw the same
         // random numbers; the scatter pass only needs the sample positions.
         const float3 o = ray.o.val(), d = ray.d.val();
@@ -948,11 +1000,30 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<N> &
         }
 #pragma unroll
         for (int j = 0; j < N; ++j) out[j] = scale.d[j] * sum * (len * 0.1f);
+    } else if (G == 0 && !(m.density.dgrid && m.density.dgrid_n == N) && !scatter) {
+        // a moving grid under a fixed ray: the sums of the density, of its gradient h and of
+        // q x h over the samples give every slot (grid_lookup_grad): 6 multiply-adds per slot
+        // after the loop instead of a dual lookup per sample
+        const float3 o = ray.o.val(), d = ray.d.val(), ctr = f3(m.density.center);
+        float sum = 0.f;
+        float3 sh = mk(0.f, 0.f, 0.f), sqh = sh;
+        for (int i = 0; i < 10; ++i) {
+            const float r = ((float)i + rng.next1()) * 0.1f;
+            const float3 p = o + d * (tmin.v + len * r);
+            float3 h;
+            sum += grid_lookup_grad(m.density, p, h, c);
+            sh += h;
+            sqh += cross(p - ctr, h);
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            out[j] = (scale.d[j] * sum - scale.v * (dot(f3(m.density.rot_vel[j]), sqh) + dot(f3(m.density.trans_vel[j]), sh))) *
+                     (len * 0.1f);
     } else {
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
-            const Df<N> tt = tmin + len * r;
-            const DV<N> pt = ray.o + ray.d * tt;
+            const Df<G> tt = tmin + len * r;
+            const DV<G> pt = ray.o + ray.d * tt;
             const Df<N> s = scale * grid_lookup_ad<N>(m.density, pt, c);
 #pragma unroll
             for (int j = 0; j < N; ++j) out[j] += s.d[j];
@@ -961,23 +1032,25 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<N> &
 #pragma unroll
         for (int j = 0; j < N; ++j) out[j] *= len * 0.1f;
     }
-    const float3 o = ray.o.val(), d = ray.d.val();
-    if (!tmax.der_zero(1e-6f)) {
-        const float dv = m.scale * grid_lookup(m.density, o + d * (tmax.v - kEps), c);
+    if constexpr (G > 0) {
+        const float3 o = ray.o.val(), d = ray.d.val();
+        if (!tmax.der_zero(1e-6f)) {
+            const float dv = m.scale * grid_lookup(m.density, o + d * (tmax.v - kEps), c);
 #pragma unroll
-        for (int j = 0; j < N; ++j) out[j] += tmax.d[j] * dv;
-    }
-    if (!tmin.der_zero(1e-6f)) {
-        const float dv = m.scale * grid_lookup(m.density, o + d * (tmin.v + kEps), c);
+            for (int j = 0; j < N; ++j) out[j] += tmax.d[j] * dv;
+        }
+        if (!tmin.der_zero(1e-6f)) {
+            const float dv = m.scale * grid_lookup(m.density, o + d * (tmin.v + kEps), c);
 #pragma unroll
-        for (int j = 0; j < N; ++j) out[j] -= tmin.d[j] * dv;
+            for (int j = 0; j < N; ++j) out[j] -= tmin.d[j] * dv;
+        }
     }
 }
 
 // homogeneous.cpp:27-49 / heterogeneous.cpp:40-75; moves ray.o to the scatter point
 // With `adj`, the factor applied to `thr` scatters adj->w times its log-derivative.
-template <int N>
-DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<N> &ray, const Df<N> &tmax, float r0,
+template <int N, int G>
+DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<G> &ray, const Df<G> &tmax, float r0,
                              float r1, Rng &rng, DV<N> &thr, Ctr &c, const AdjCtx *adj = nullptr) {
     if (m.type == MEDIUM_HOMOGENEOUS) {
         const Df<N> sig = load_dual<N>(m.sigma_t, m.d_sigma_t);
@@ -994,11 +1067,11 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<N
                 }
                 return true;
             }
-            Df<N> tmp = dexp(-(tmax * sig));
+            Df<N> tmp = dexp(-(lift<N>(tmax) * sig));
             thr = thr * (tmp / tmp.v);
             return false;
         }
-        thr = thr * dexp(-(tmax * sig));
+        thr = thr * dexp(-(lift<N>(tmax) * sig));
         return false;
     }
     float tn, tf;
@@ -1016,7 +1089,7 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<N
         }
         // the acceptance test needs the density value only; a null collision discards the
         // derivative slots, so the dual lookup runs at an accepted collision (same point)
-        const DV<N> p = ray.o + ray.d * t;
+        const DV<G> p = ray.o + ray.d * t;
         const float dv = grid_lookup(m.density, p.val(), c);
         if (rng.next1() * m.density.max_value < dv) {
             Ctr again;  // the lookup just counted, repeated with its derivative slots
@@ -1024,14 +1097,14 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<N
             // The reference aliases p_scatter with ray.org (volpathAD.cpp:164), so the
             // line integral below runs from the scatter point forward over [0, t].
             // EST_SCATTER_FROM_ORIGIN integrates the segment actually travelled instead.
-            const RayAD<N> ray0 = ray;
+            const RayAD<G> ray0 = ray;
             ray.o = p;
             const DV<N> alb = m.albedo_vol.valid ? grid_lookup3_ad<N>(m.albedo_vol, p) : load_dual3<N>(m.albedo, m.d_albedo);
             const Df<N> sig = load_dual<N>(m.scale, m.d_scale) * dens;
             if (adj != nullptr && m.grad_off >= 0)  // d log(sigma_t(p)) = d density / density
                 grid_scatter(m.density, adj->grad + m.grad_off, p.val(), adj->w / dens.v);
-            float ist[N];
-            int_sig_t<N>(sc, m, (sc.est_flags & EST_SCATTER_FROM_ORIGIN) ? ray0 : ray, Df<N>(0.f), Df<N>(t), rng, ist,
+            float ist[N > 0 ? N : 1];
+            int_sig_t<N>(sc, m, (sc.est_flags & EST_SCATTER_FROM_ORIGIN) ? ray0 : ray, Df<G>(0.f), Df<G>(t), rng, ist,
                          c, adj);
             Df<N> tmp(1.f);
 #pragma unroll
@@ -1040,8 +1113,8 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<N
             return true;
         }
     }
-    float ist[N];
-    int_sig_t<N>(sc, m, ray, Df<N>(0.f), tmax, rng, ist, c, adj);
+    float ist[N > 0 ? N : 1];
+    int_sig_t<N>(sc, m, ray, Df<G>(0.f), tmax, rng, ist, c, adj);
     Df<N> tmp(1.f);
 #pragma unroll
     for (int j = 0; j < N; ++j) tmp.d[j] = -ist[j];
@@ -1066,13 +1139,13 @@ DT_HEAVY float medium_transmittance(const DevScene &sc, const DevMedium &m, floa
     }
     return ret;
 }
-template <int N>
-DT_HEAVY Df<N> medium_transmittance_ad(const DevScene &sc, const DevMedium &m, const RayAD<N> &ray, float tmin,
-                                   const Df<N> &tmax, Rng &rng, Ctr &c, const AdjCtx *adj = nullptr) {
-    if (m.type == MEDIUM_HOMOGENEOUS) return dexp((tmin - tmax) * load_dual<N>(m.sigma_t, m.d_sigma_t));
+template <int N, int G>
+DT_HEAVY Df<N> medium_transmittance_ad(const DevScene &sc, const DevMedium &m, const RayAD<G> &ray, float tmin,
+                                   const Df<G> &tmax, Rng &rng, Ctr &c, const AdjCtx *adj = nullptr) {
+    if (m.type == MEDIUM_HOMOGENEOUS) return dexp(lift<N>(tmin - tmax) * load_dual<N>(m.sigma_t, m.d_sigma_t));
     Df<N> ret(medium_transmittance(sc, m, ray.o.val(), ray.d.val(), tmin, tmax.v, rng, c));  // heterogeneous.cpp:113-118
-    float ist[N];
-    int_sig_t<N>(sc, m, ray, Df<N>(tmin), tmax, rng, ist, c, adj);
+    float ist[N > 0 ? N : 1];
+    int_sig_t<N>(sc, m, ray, Df<G>(tmin), tmax, rng, ist, c, adj);
 #pragma unroll
     for (int j = 0; j < N; ++j) ret.d[j] = -ret.v * ist[j];
     return ret;
@@ -1192,31 +1265,31 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, int *stack, float3 o, float
 }
 
 // scene.cpp:703-793
-template <int N>
-DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<N> ray, bool on_surface, Rng &rng, int med,
-                               int max_inter, ItsAD<N> &its, float &pdf_nee, int *far_shape, float *far_t, Ctr &c,
+template <int N, int G>
+DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray, bool on_surface, Rng &rng, int med,
+                               int max_inter, ItsAD<G> &its, float &pdf_nee, int *far_shape, float *far_t, Ctr &c,
                                const AdjCtx *adj = nullptr) {
     float tmin = on_surface ? kShadowEps : 0.f, th;
     const float3 scatter = ray.o.val();
     int prim = closest_hit(sc, stack, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
     if (prim < 0) {
         its.shape = -1;
-        its.t = Df<N>(INFINITY);
+        its.t = Df<G>(INFINITY);
         return DV<N>();
     }
-    shape_intersect_ad<N>(sc, prim, ray, its);
+    shape_intersect_ad<G>(sc, prim, ray, its);
     if (sc.has_grid_media) {
         // Geometry first: follow null interfaces to the surface that ends the chain. A chain
         // that does not end at an emitter contributes nothing, so its transmittance (a
         // tracking estimate through the grid, with random numbers) is never evaluated. The
         // reference evaluates it segment by segment before the emitter test
         // (scene.cpp:660-690); the contribution is the same, its random numbers are not drawn.
-        RayAD<N> r1 = ray;
-        ItsAD<N> n1 = its;
+        RayAD<G> r1 = ray;
+        ItsAD<G> n1 = its;
         int p1 = prim;
         bool emitter = false;
         for (int inter = 0; inter < kMaxInteractions; ++inter) {
-            if (inter > 0) shape_intersect_ad<N>(sc, p1, r1, n1);
+            if (inter > 0) shape_intersect_ad<G>(sc, p1, r1, n1);
             const DevShape &s = sc.shapes[n1.shape];
             if (s.light_id >= 0) {
                 emitter = true;
@@ -1229,12 +1302,13 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<N> ray,
         }
         if (!emitter) return DV<N>();
     }
-    Df<N> tr(1.f), dist(0.f);
-    ItsAD<N> ni = its;
+    Df<N> tr(1.f);
+    float dist = 0.f;
+    ItsAD<G> ni = its;
     for (int inter = 0; inter < kMaxInteractions; ++inter) {
-        if (inter > 0) shape_intersect_ad<N>(sc, prim, ray, ni);
-        const Df<N> tmax = ni.t;
-        dist += ni.t;
+        if (inter > 0) shape_intersect_ad<G>(sc, prim, ray, ni);
+        const Df<G> tmax = ni.t;
+        dist += ni.t.v;
         if (med >= 0) tr *= medium_transmittance_ad<N>(sc, sc.media[med], ray, tmin, tmax, rng, c, adj);
         const DevShape &s = sc.shapes[ni.shape];
         if (s.light_id >= 0) {
@@ -1243,7 +1317,7 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<N> ray,
             pdf_nee = sc.light_pmf[s.light_id] / (sc.light_area[s.light_id] * G);
             if (far_shape) {
                 *far_shape = ni.shape;
-                *far_t = dist.v;
+                *far_t = dist;
             }
             return le_ad<N>(sc, ni, -ray.d) * tr;
         }
@@ -1307,9 +1381,9 @@ DT_HEAVY float3 nee_surface(const DevScene &sc, int *stack, const Its &its, cons
 }
 
 // scene.cpp:428-454 (AD, from a point; the light sample carries no derivative)
-template <int N>
-DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<N> &p, const float rnd[4], Rng &rng, int med,
-                        int max_inter, DV<N> &wo, float &pdf, Ctr &c, const AdjCtx *adj = nullptr) {
+template <int N, int G>
+DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<G> &p, const float rnd[4], Rng &rng, int med,
+                        int max_inter, DV<G> &wo, float &pdf, Ctr &c, const AdjCtx *adj = nullptr) {
     float3 lp, ln;
     float pdf0;
     const int l = sample_light(sc, rnd, lp, ln, pdf0);
@@ -1319,14 +1393,14 @@ DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<N> &p, cons
     if (dot(dir, ln) < 0.f) {
         const float dist = length(dir);
         dir = dir / dist;
-        ItsAD<N> near_its;
+        ItsAD<G> near_its;
         int far_shape = -1;
         float far_t = 0.f;
-        RayAD<N> r{p, DV<N>(dir)};
+        RayAD<G> r{p, DV<G>(dir)};
         DV<N> v = look_for_emitter_ad<N>(sc, stack, r, false, rng, med, max_inter, near_its, pdf, &far_shape, &far_t, c,
                                          adj);
         if (!v.is_zero() && pdf > kEps && far_shape == sc.emitters[l].shape_id && fabsf(far_t - dist) < kShadowEps) {
-            wo = DV<N>(dir);
+            wo = DV<G>(dir);
             return v / pdf;
         }
     }
@@ -1334,13 +1408,13 @@ DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<N> &p, cons
 }
 
 // scene.cpp:493-524 (AD, from a surface; wo in the dual shading frame)
-template <int N>
 // With `bsdf` (a BSDF without derivative slots, whose value the caller multiplies in), a
 // light sample where that value is exactly zero returns zero before its visibility chain is
 // traced: the contribution is zero either way (a near-specular dielectric is zero for almost
 // every light sample). Random numbers such a chain would have drawn are not drawn.
-DT_HEAVY DV<N> nee_surface_ad(const DevScene &sc, int *stack, const ItsAD<N> &its, const FrameAD<N> &fr, const float rnd[4],
-                          Rng &rng, int med, int max_inter, DV<N> &wo, float &pdf, Ctr &c, const AdjCtx *adj = nullptr,
+template <int N, int G>
+DT_HEAVY DV<N> nee_surface_ad(const DevScene &sc, int *stack, const ItsAD<G> &its, const FrameAD<G> &fr, const float rnd[4],
+                          Rng &rng, int med, int max_inter, DV<G> &wo, float &pdf, Ctr &c, const AdjCtx *adj = nullptr,
                           const DevBsdf *bsdf = nullptr) {
     float3 lp, ln;
     float pdf0;
@@ -1357,10 +1431,10 @@ DT_HEAVY DV<N> nee_surface_ad(const DevScene &sc, int *stack, const ItsAD<N> &it
         dir = dir / dist;
         if (bsdf && !bsdf->has_der && is_zero3(bsdf_eval(*bsdf, its.wi.val(), fr.plain().to_local(dir)), 0.f))
             return DV<N>();
-        ItsAD<N> near_its;
+        ItsAD<G> near_its;
         int far_shape = -1;
         float far_t = 0.f;
-        RayAD<N> r{its.p, DV<N>(dir)};
+        RayAD<G> r{its.p, DV<G>(dir)};
         DV<N> v = look_for_emitter_ad<N>(sc, stack, r, true, rng, med, max_inter, near_its, pdf, &far_shape, &far_t, c,
                                          adj);
         if (!v.is_zero() && pdf > kEps && far_shape == sc.emitters[l].shape_id && fabsf(far_t - dist) < kShadowEps) {

@@ -78,6 +78,34 @@ inline const int *sort_primary_samples(const RenderParams &rp, Scratch &sb, uint
 }
 
 
+// Rays and hits of the scene carry no derivatives: nothing moves but materials and media
+// (vertex, normal and camera velocities all absent or exactly zero). Continuation rays then
+// have none either: a scatter point lies on its ray, a new direction is sampled from values.
+inline bool static_rays(const DevScene &sc) {
+    if (sc.vert_der || sc.face_n_der || sc.normal_der || sc.moving_geometry) return false;
+    for (int j = 0; j < sc.nder; ++j)
+        for (int a = 0; a < 3; ++a) {
+            if (sc.cam.d_cpos[j][a] != 0.f) return false;
+            for (int k = 0; k < 3; ++k)
+                if (sc.cam.d_cframe[j][a][k] != 0.f) return false;
+        }
+    return true;
+}
+
+// Camera paths per batch of a scene of static_rays(): its batches hold no records, only path
+// states (2 GB at nder 8)
+constexpr long long kStaticBatchPaths = 1ll << 22;
+
+// Buffers of the camera wavefront for `cap` paths: path states, vertex inputs, four
+// path-index queues, level counts
+struct CamWave {
+    void *states, *vins;
+    int *q;
+    unsigned long long *cnt;
+    long long cap;
+    int levels;
+};
+
 // Connectivity kept from the last build, so that a rebuild from a description with the
 // same triangles (an optimisation step that moves vertices) skips the edge search and
 // refits the BVH instead of building it again.

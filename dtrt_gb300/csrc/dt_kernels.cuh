@@ -171,18 +171,25 @@ DT_D RayAD<N> camera_ray_ad(const DevCamera &cam, double x, double y) {
 // ====================================================================== camera AD paths
 // State of one camera path between vertices (volpathAD.cpp:145-620 as a loop): the
 // megakernel keeps it in registers, the wavefront schedule in HBM between launches.
-template <int N>
+// G is the width of the ray's and hit's derivatives: N, or 0 where they are zero by
+// construction (static geometry under a static camera: static_rays()). Then they take no
+// registers, no path state and no local-memory call frames; only the throughput and the
+// sums carry slots. At nder 8 a state is 336 B instead of 848 B and a call frame 1.1 KB
+// instead of 4.7 KB. The kernels wait on L1/L2 (local frames, path state, voxels) at 8
+// resident warps, so the traffic is time: C3 forward (512^2, 128 spp, nder 8) 328 -> 112 ms,
+// C1 forward (512^2, 64 spp, nder 3) 34.5 -> 17.4 ms.
+template <int N, int G>
 struct alignas(16) CamState {  // 16-byte aligned: whole-state copies compile to 128-bit loads and stores
     Rng rng;
-    RayAD<N> ray;
-    ItsAD<N> its;
+    RayAD<G> ray;
+    ItsAD<G> its;
     DV<N> P, acc;
     int med, depth, mode, level;
 };
 
 // Path start: jittered primary ray and first intersection. False: nothing was hit.
-template <int N>
-DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N> &st, Ctr &c) {
+template <int N, int G>
+DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st, Ctr &c) {
     const int pixel = (int)(g / rp.spp);
     const int ix = rp.crop_x + pixel % rp.out_w, iy = rp.crop_y + pixel / rp.out_w;
     st.rng.init(rp.seed, (uint64_t)g);
@@ -191,15 +198,15 @@ DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, int *stack, l
         jx = st.rng.next1d();
         jy = st.rng.next1d();
     }
-    st.ray = camera_ray_ad<N>(sc.cam, ix + jx, iy + jy);
-    st.its = ItsAD<N>();
+    st.ray = camera_ray_ad<G>(sc.cam, ix + jx, iy + jy);
+    st.its = ItsAD<G>();
     st.med = sc.cam.med_id;
     st.depth = rp.max_bounces;
     st.mode = rp.mode;
     st.level = 0;
     st.P = DV<N>(mk(1.f, 1.f, 1.f));
     st.acc = DV<N>();
-    return ray_intersect_ad<N>(sc, stack, st.ray, false, st.its, c);
+    return ray_intersect_ad<G>(sc, stack, st.ray, false, st.its, c);
 }
 
 // Random numbers of a vertex drawn before its branch, the distance-sampling throughput and
@@ -214,8 +221,8 @@ struct alignas(16) VertexIn {
 // First part of a vertex of camera path g (volpathAD.cpp:160-164, 306-308): the vertex's
 // random numbers and distance sampling. 0: the path ends here, 1: volume vertex, 2:
 // interface vertex.
-template <int N>
-DT_D int camera_decide(const DevScene &sc, CamState<N> &st, VertexIn<N> &vin, Ctr &c) {
+template <int N, int G>
+DT_D int camera_decide(const DevScene &sc, CamState<N, G> &st, VertexIn<N> &vin, Ctr &c) {
     Rng &rng = st.rng;
     const float r1a = rng.next1(), r1b = rng.next1();
     vin.r2[0] = rng.next1(); vin.r2[1] = rng.next1(); vin.r2[2] = rng.next1(); vin.r2[3] = rng.next1();
@@ -229,12 +236,12 @@ DT_D int camera_decide(const DevScene &sc, CamState<N> &st, VertexIn<N> &vin, Ct
 
 // Volume vertex (volpathAD.cpp:164-305): NEE, volume edge record, phase sampling and the
 // emitter lookup along the new direction. Returns whether the path continues.
-template <int N>
-DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N> &st,
+template <int N, int G>
+DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
                         const VertexIn<N> &vin, const Queue &qe, Ctr &c) {
     Rng &rng = st.rng;
-    RayAD<N> &ray = st.ray;
-    ItsAD<N> &its = st.its;
+    RayAD<G> &ray = st.ray;
+    ItsAD<G> &its = st.its;
     DV<N> &P = st.P, &acc = st.acc;
     int &med = st.med, &depth = st.depth, &mode = st.mode;
     const int level = st.level;
@@ -248,7 +255,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     // ------------------------------------------------ volumetric vertex, volpathAD.cpp:164-305
     const DevPhase &ph = sc.phases[sc.media[med].phase_id];
     const DV<N> Q = cmul(P, thr);
-    DV<N> wo;
+    DV<G> wo;
     float pdf_nee;
     if (mode & MODE_VOLUME_MAIN) {
         DV<N> v = nee_point_ad<N>(sc, stack, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c);
@@ -258,7 +265,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
         }
     }
     // edge record before the continuation overwrites the vertex state
-    if (rp.sppse > 0 && (mode & MODE_VOLUME_BOUNDARY2) && sc.has_edges &&
+    if (G > 0 && rp.sppse > 0 && (mode & MODE_VOLUME_BOUNDARY2) && sc.has_edges &&
         (sc.moving_geometry || !ray.o.der_zero(0.f))) {
         const long long slot = queue_reserve(sc, qe);
         if (slot >= 0) {
@@ -266,7 +273,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
             const float3 x = ray.o.val(), w = cmul(P.val(), thr.val()) * rp.inv_spp, wi = -dir_in;
             r.x0[0] = x.x; r.x0[1] = x.y; r.x0[2] = x.z;
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
+            for (int j = 0; j < G; ++j) {
                 const float3 gj = ray.o.grad(j);
                 r.x0d[j][0] = gj.x; r.x0d[j][1] = gj.y; r.x0d[j][2] = gj.z;
             }
@@ -280,7 +287,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     if (pvs.v > kEps) {
         const DV<N> thr1 = thr * pvs;
         ray.d = wo;
-        ItsAD<N> its1;
+        ItsAD<G> its1;
         DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, false, rng, med, depth - 1, its1, pdf_nee, nullptr,
                                            nullptr, c);
         if (!att.is_zero() && (mode & MODE_VOLUME_MAIN))
@@ -297,12 +304,12 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
 // Interface vertex (volpathAD.cpp:306-617): emission, Lins and surface edge records, NEE,
 // BSDF sampling and the emitter lookup (or null-interface crossing). Returns whether the
 // path continues.
-template <int N>
-DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N> &st,
+template <int N, int G>
+DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
                          const VertexIn<N> &vin, const Queue &qe, const Queue &ql, Ctr &c) {
     Rng &rng = st.rng;
-    RayAD<N> &ray = st.ray;
-    ItsAD<N> &its = st.its;
+    RayAD<G> &ray = st.ray;
+    ItsAD<G> &its = st.its;
     DV<N> &P = st.P, &acc = st.acc;
     int &med = st.med, &depth = st.depth, &mode = st.mode;
     const int level = st.level;
@@ -321,10 +328,10 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
     if (depth == 0) return false;
     const DevBsdf &b = sc.bsdfs[sh.bsdf_id];
     const bool is_null = b.type == BSDF_NULL;
-    const FrameAD<N> fr = its.frame();
+    const FrameAD<G> fr = its.frame();
     const Its its0 = its.plain();
     // Lins boundary term, volpathAD.cpp:321-467
-    if (med >= 0 && !its.t.der_zero(kDerZeroEps) && (mode & MODE_VOLUME_BOUNDARY1)) {
+    if (G > 0 && med >= 0 && !its.t.der_zero(kDerZeroEps) && (mode & MODE_VOLUME_BOUNDARY1)) {
         const long long slot = queue_reserve(sc, ql);
         if (slot >= 0) {
             LinsRec<N> &r = reinterpret_cast<LinsRec<N> *>(ql.data)[slot];
@@ -338,13 +345,13 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
             for (int k = 0; k < 8; ++k) { dst[k][0] = src[k]->x; dst[k][1] = src[k]->y; dst[k][2] = src[k]->z; }
             r.w[0] = w.x; r.w[1] = w.y; r.w[2] = w.z;
 #pragma unroll
-            for (int j = 0; j < N; ++j) r.s[j] = its.t.d[j];
+            for (int j = 0; j < G; ++j) r.s[j] = its.t.d[j];
             r.shape = its.shape; r.med = med; r.phase = sc.media[med].phase_id; r.depth = depth;
             r.pixel = pixel; r.ns = ns; r.key = child_key(key, 2u, (uint32_t)level);
         }
     }
     // interface edge record, volpathAD.cpp:513-616
-    if (!is_null && rp.sppse > 0 && (mode & MODE_SURFACE_BOUNDARY) && sc.has_edges &&
+    if (G > 0 && !is_null && rp.sppse > 0 && (mode & MODE_SURFACE_BOUNDARY) && sc.has_edges &&
         (sc.moving_geometry || !its.p.der_zero(0.f))) {
         const long long slot = queue_reserve(sc, qe);
         if (slot >= 0) {
@@ -352,7 +359,7 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
             const float3 x = its0.p, w = cmul(P.val(), thr.val()) * rp.inv_spp;
             r.x0[0] = x.x; r.x0[1] = x.y; r.x0[2] = x.z;
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
+            for (int j = 0; j < G; ++j) {
                 const float3 gj = its.p.grad(j);
                 r.x0d[j][0] = gj.x; r.x0d[j][1] = gj.y; r.x0d[j][2] = gj.z;
             }
@@ -367,7 +374,7 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         }
     }
     // area sampling, volpathAD.cpp:469-511
-    DV<N> wo;
+    DV<G> wo;
     float pdf_nee;
     if (!is_null && (mode & MODE_SURFACE_MAIN)) {
         DV<N> v = nee_surface_ad<N>(sc, stack, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c, nullptr, &b);
@@ -386,9 +393,9 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         ray.d = wo;
         const int med1 = is_transition(sh) ? target_medium(sc, its.shape, its.ng, wo.val()) : med;
         DV<N> thr1 = thr;
-        ItsAD<N> its1;
+        ItsAD<G> its1;
         if (is_null) {
-            ray_intersect_ad<N>(sc, stack, ray, true, its1, c);
+            ray_intersect_ad<G>(sc, stack, ray, true, its1, c);
         } else {
             DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, true, rng, med1, depth - 1, its1, pdf_nee,
                                                nullptr, nullptr, c);
@@ -408,13 +415,13 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
 
 // One vertex of camera path g. Returns whether the path continues; st.level is advanced
 // by the caller.
-template <int N>
-DT_D bool camera_step(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N> &st,
+template <int N, int G>
+DT_D bool camera_step(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
                       const Queue &qe, const Queue &ql, Ctr &c) {
     VertexIn<N> vin;
-    const int kind = camera_decide<N>(sc, st, vin, c);
-    if (kind == 1) return camera_volume<N>(sc, rp, stack, g, st, vin, qe, c);
-    if (kind == 2) return camera_surface<N>(sc, rp, stack, g, st, vin, qe, ql, c);
+    const int kind = camera_decide<N, G>(sc, st, vin, c);
+    if (kind == 1) return camera_volume<N, G>(sc, rp, stack, g, st, vin, qe, c);
+    if (kind == 2) return camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
     return false;
 }
 
@@ -450,7 +457,7 @@ DT_D void accumulate_path(const RenderParams &rp, bool active, int pixel, const 
 }
 
 // Megakernel schedule: one thread runs its camera path to the end.
-template <int N>
+template <int N, int G>
 __global__ void __launch_bounds__(kBlock) k_camera(DevScene sc, RenderParams rp, Queue qe, Queue ql, double *acc1,
                                                    unsigned long long *ctr) {
     __shared__ int s_stack[kStackDepth * kBlock];
@@ -461,10 +468,10 @@ __global__ void __launch_bounds__(kBlock) k_camera(DevScene sc, RenderParams rp,
     Ctr c;
     DV<N> acc;
     if (active) {
-        CamState<N> st;
-        bool alive = camera_start<N>(sc, rp, stack, g, st, c);
+        CamState<N, G> st;
+        bool alive = camera_start<N, G>(sc, rp, stack, g, st, c);
         while (alive && st.mode != 0) {
-            alive = camera_step<N>(sc, rp, stack, g, st, qe, ql, c);
+            alive = camera_step<N, G>(sc, rp, stack, g, st, qe, ql, c);
             ++st.level;
         }
         acc = st.acc * rp.inv_spp;
@@ -520,14 +527,14 @@ DT_D bool interface_back(const DevScene &sc, int shape) {
 
 // After a vertex of level L: a continuing path draws the random numbers and samples the
 // distance of level L+1 right away and is queued as a volume or interface vertex of L+1.
-template <int N>
-DT_D int camera_next(const DevScene &sc, CamState<N> &st, bool alive, VertexIn<N> *vins, int id, int *qv,
+template <int N, int G>
+DT_D int camera_next(const DevScene &sc, CamState<N, G> &st, bool alive, VertexIn<N> *vins, int id, int *qv,
                      unsigned long long *cnt_v, int *qs, unsigned long long *cnt_s, unsigned long long *cnt_s_back,
                      long long cap, Ctr &c) {
     int kind = 0;
     if (alive && st.mode != 0) {
         VertexIn<N> vin;
-        kind = camera_decide<N>(sc, st, vin, c);
+        kind = camera_decide<N, G>(sc, st, vin, c);
         if (kind) vins[id] = vin;
     }
     const bool back = kind == 2 && interface_back(sc, st.its.shape);
@@ -540,9 +547,9 @@ DT_D int camera_next(const DevScene &sc, CamState<N> &st, bool alive, VertexIn<N
 // The path state its next launch reads: all of it before an interface vertex; all but the
 // hit record before a volume vertex (which writes the record without reading it); the sums
 // alone when the path has ended (k_cam_accum reads nothing else).
-template <int N>
-DT_D void store_state(CamState<N> *states, int id, const CamState<N> &st, int next_kind) {
-    CamState<N> &d = states[id];
+template <int N, int G>
+DT_D void store_state(CamState<N, G> *states, int id, const CamState<N, G> &st, int next_kind) {
+    CamState<N, G> &d = states[id];
     if (next_kind == 2) {
         d = st;
         return;
@@ -561,8 +568,8 @@ DT_D void store_state(CamState<N> *states, int id, const CamState<N> &st, int ne
 // Path start and level 0: primary ray, first hit, the level's random numbers and distance
 // sampling. An interface vertex (every path from a camera outside media) runs here too and
 // the path goes on to level 1's distance sampling; a volume vertex is queued for level 0.
-template <int N>
-__global__ void __launch_bounds__(kBlock) k_cam_start(DevScene sc, RenderParams rp, CamState<N> *states,
+template <int N, int G>
+__global__ void __launch_bounds__(kBlock) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                       VertexIn<N> *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, unsigned long long *cnt_s1_back,
@@ -572,30 +579,30 @@ __global__ void __launch_bounds__(kBlock) k_cam_start(DevScene sc, RenderParams 
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     int kind = 0;
-    CamState<N> st;
+    CamState<N, G> st;
     bool next = false;
     if (gi < rp.path_count) {
         const long long g = rp.path_begin + gi;
-        if (camera_start<N>(sc, rp, stack, g, st, c) && st.mode != 0) {
+        if (camera_start<N, G>(sc, rp, stack, g, st, c) && st.mode != 0) {
             VertexIn<N> vin;
-            kind = camera_decide<N>(sc, st, vin, c);
+            kind = camera_decide<N, G>(sc, st, vin, c);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
-                next = camera_surface<N>(sc, rp, stack, g, st, vin, qe, ql, c);
+                next = camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
                 ++st.level;
             }
         }
     }
     push_path(qv0, cnt_v0, (int)gi, kind == 1);
-    const int nk = camera_next<N>(sc, st, next, vins, (int)gi, qv1, cnt_v1, qs1, cnt_s1, cnt_s1_back, cap, c);
-    if (gi < rp.path_count) store_state<N>(states, (int)gi, st, kind == 1 ? 1 : nk);
+    const int nk = camera_next<N, G>(sc, st, next, vins, (int)gi, qv1, cnt_v1, qs1, cnt_s1, cnt_s1_back, cap, c);
+    if (gi < rp.path_count) store_state<N, G>(states, (int)gi, st, kind == 1 ? 1 : nk);
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
 // Vertex level L, one launch per kind: the volume (kVolume) or interface vertices of the
 // level; a continuing path then runs level L+1's distance sampling (camera_next).
-template <int N, bool kVolume>
-__global__ void __launch_bounds__(kBlock) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N> *states,
+template <int N, int G, bool kVolume>
+__global__ void __launch_bounds__(kBlock) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                        VertexIn<N> *vins, const int *q_in,
                                                        const unsigned long long *cnt_in,
                                                        const unsigned long long *cnt_in_back, int *qv_next,
@@ -609,11 +616,11 @@ __global__ void __launch_bounds__(kBlock) k_cam_vertex(DevScene sc, RenderParams
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
         const int id = i < nf ? q_in[i] : q_in[cap - 1 - (i - nf)];
-        CamState<N> st;
+        CamState<N, G> st;
         if (kVolume) {
             // a volume vertex writes the hit record (of its continuation) without reading it:
             // the record stays in HBM (380 B of 848 at nder 8)
-            const CamState<N> &s0 = states[id];
+            const CamState<N, G> &s0 = states[id];
             st.rng = s0.rng;
             st.ray = s0.ray;
             st.P = s0.P;
@@ -627,18 +634,18 @@ __global__ void __launch_bounds__(kBlock) k_cam_vertex(DevScene sc, RenderParams
         }
         const VertexIn<N> vin = vins[id];
         const long long g = rp.path_begin + id;
-        const bool alive = kVolume ? camera_volume<N>(sc, rp, stack, g, st, vin, qe, c)
-                                   : camera_surface<N>(sc, rp, stack, g, st, vin, qe, ql, c);
+        const bool alive = kVolume ? camera_volume<N, G>(sc, rp, stack, g, st, vin, qe, c)
+                                   : camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
         ++st.level;
-        const int nk = camera_next<N>(sc, st, alive, vins, id, qv_next, cnt_v_next, qs_next, cnt_s_next,
+        const int nk = camera_next<N, G>(sc, st, alive, vins, id, qv_next, cnt_v_next, qs_next, cnt_s_next,
                                       cnt_s_next_back, cap, c);
-        store_state<N>(states, id, st, nk);
+        store_state<N, G>(states, id, st, nk);
     }
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
-template <int N>
-__global__ void __launch_bounds__(kBlock) k_cam_accum(RenderParams rp, const CamState<N> *states, double *acc1) {
+template <int N, int G>
+__global__ void __launch_bounds__(kBlock) k_cam_accum(RenderParams rp, const CamState<N, G> *states, double *acc1) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < rp.path_count;
     DV<N> acc;

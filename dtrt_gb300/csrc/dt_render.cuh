@@ -27,6 +27,63 @@ namespace dt {
         }                                                                            \
     } while (0)
 
+// The camera stage of one batch of paths, with ray and hit derivatives of width G (N, or 0
+// for scenes of static_rays()). The width-0 kernels are compiled in units of their own
+// (dt_camera_n*.cu).
+template <int N, int G>
+struct CameraStage {
+    static constexpr size_t state_bytes = sizeof(CamState<N, G>), vertex_bytes = sizeof(VertexIn<N>),
+                            hit_bytes = sizeof(ItsAD<G>);
+    static void wave(const DevScene &sc, const RenderParams &rp, const CamWave &w, int sms, const Queue &qe,
+                     const Queue &ql, double *acc1, unsigned long long *ctr, cudaStream_t st);
+    static void mega(const DevScene &sc, const RenderParams &rp, const Queue &qe, const Queue &ql, double *acc1,
+                     unsigned long long *ctr, cudaStream_t st);
+};
+
+inline unsigned path_blocks(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
+
+// Wavefront schedule: start, two launches per vertex level (one at level 0), pixel sums
+template <int N, int G>
+void CameraStage<N, G>::wave(const DevScene &sc, const RenderParams &rp, const CamWave &w, int sms, const Queue &qe,
+                             const Queue &ql, double *acc1, unsigned long long *ctr, cudaStream_t st) {
+    CamState<N, G> *states = (CamState<N, G> *)w.states;
+    VertexIn<N> *vins = (VertexIn<N> *)w.vins;
+    int *qa = w.q, *qb = qa + w.cap, *qv = qb + w.cap, *qs = qv + w.cap;
+    // volume and interface vertices queued per level [0, levels] (interface: pushed from the
+    // front of the queue, scnt, and from its back, sbk)
+    unsigned long long *vcnt = w.cnt, *scnt = vcnt + (w.levels + 1), *sbk = scnt + (w.levels + 1);
+    // grid-stride launches of a few waves: late levels hold few live paths
+    const unsigned gw = std::min<unsigned>(path_blocks(rp.path_count), (unsigned)std::max(1, sms) * 16u);
+    cudaMemsetAsync(vcnt, 0, (size_t)3 * (w.levels + 1) * sizeof(unsigned long long), st);
+    // volume / interface queues of level L: (qa, qb) for even L, (qv, qs) for odd L
+    k_cam_start<N, G><<<path_blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, states, vins, qa, vcnt, qv, vcnt + 1, qs,
+                                                                     scnt + 1, sbk + 1, w.cap, qe, ql, ctr);
+    for (int L = 0; L < w.levels; ++L) {
+        int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
+        int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
+        k_cam_vertex<N, G, true><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vcnt + L, nullptr, qvn, vcnt + L + 1,
+                                                        qsn, scnt + L + 1, sbk + L + 1, w.cap, qe, ql, ctr);
+        if (L > 0)  // level 0's interface vertices ran in k_cam_start
+            k_cam_vertex<N, G, false><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qsl, scnt + L, sbk + L, qvn,
+                                                             vcnt + L + 1, qsn, scnt + L + 1, sbk + L + 1, w.cap, qe,
+                                                             ql, ctr);
+    }
+    k_cam_accum<N, G><<<path_blocks(rp.path_count), kBlock, 0, st>>>(rp, states, acc1);
+}
+
+template <int N, int G>
+void CameraStage<N, G>::mega(const DevScene &sc, const RenderParams &rp, const Queue &qe, const Queue &ql, double *acc1,
+                             unsigned long long *ctr, cudaStream_t st) {
+    k_camera<N, G><<<path_blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, qe, ql, acc1, ctr);
+}
+
+#ifndef DT_CAMERA_STATIC_UNIT
+extern template struct CameraStage<1, 0>;
+extern template struct CameraStage<3, 0>;
+extern template struct CameraStage<4, 0>;
+extern template struct CameraStage<8, 0>;
+#endif
+
 template <int N>
 int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on_device, cudaStream_t st) {
     using clk = std::chrono::steady_clock;
@@ -64,9 +121,13 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     // 16 Mi records bound a camera batch at 16Mi/(max_bounces+1) paths (1.5 M at depth 10):
     // few launches, so the partial last wave of each batch costs little
     const uint64_t rec_cap = s->queue_cap ? s->queue_cap : (uint64_t)16 << 20;
-    if (!ensure_buffer(&sb.qli, &sb.qli_bytes, li_cap * sizeof(LiTask<N>)) ||
-        !ensure_buffer(&sb.qe, &sb.qe_bytes, rec_cap * sizeof(EdgeRec<N>)) ||
-        !ensure_buffer(&sb.ql, &sb.ql_bytes, rec_cap * sizeof(LinsRec<N>)))
+    // Rays and hits without derivatives spawn no boundary records and move no primary edge:
+    // no queues, and the camera stage without ray derivatives (C1, C3 and every density or
+    // material optimisation)
+    const bool fixed_rays = static_rays(sc);
+    if (!fixed_rays && (!ensure_buffer(&sb.qli, &sb.qli_bytes, li_cap * sizeof(LiTask<N>)) ||
+                        !ensure_buffer(&sb.qe, &sb.qe_bytes, rec_cap * sizeof(EdgeRec<N>)) ||
+                        !ensure_buffer(&sb.ql, &sb.ql_bytes, rec_cap * sizeof(LinsRec<N>))))
         return DTRT_ERR_CUDA;
     if (!sb.counts) DT_CK(cudaMalloc(&sb.counts, kCountSlots * sizeof(unsigned long long)));
     if (!sb.err) DT_CK(cudaMalloc(&sb.err, sizeof(unsigned int)));
@@ -111,7 +172,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     bool used_wavefront = false;
     int rc = DTRT_OK;
     // Li sub-path pairs sorted by origin and direction before k_li (needs a tree)
-    const bool li_sorted = sc.num_nodes > 0 && ensure_li_sort(sb, li_cap);
+    const bool li_sorted = !fixed_rays && sc.num_nodes > 0 && ensure_li_sort(sb, li_cap);
     // Li tasks are drained chunk by chunk so that the queue never exceeds li_cap
     auto drain_li = [&]() -> int {
         if ((rc = read_counts())) return rc;
@@ -133,7 +194,9 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     const long long total = (long long)npix * std::max(0, o->spp);
     if (total > 0) {
         const long long unit = std::max<long long>(128, (long long)rp.spp % 32 == 0 ? std::max(rp.spp, 128) : 128);
-        long long B = (long long)(rec_cap / (uint64_t)std::max(1, o->max_bounces + 1));
+        // without records a batch is bounded by the path states alone
+        long long B = fixed_rays && !s->queue_cap ? kStaticBatchPaths
+                                                  : (long long)(rec_cap / (uint64_t)std::max(1, o->max_bounces + 1));
         B = std::max<long long>(unit, (B / unit) * unit);
         const long long per_chunk = std::max<long long>(1, (long long)(li_cap / (uint64_t)std::max(1, 2 * rp.sppse)));
         // camera schedule: the wavefront keeps CamState and VertexIn per path of a batch in device memory
@@ -141,7 +204,9 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         const int levels = o->max_bounces + 1;  // a continuing vertex always spends one bounce
         bool wavefront = s->camera_schedule == DTRT_CAMERA_WAVEFRONT ||
                          (s->camera_schedule == DTRT_CAMERA_AUTO && Bw >= kWavefrontMinPaths);
-        const size_t state_bytes = ((size_t)Bw * sizeof(CamState<N>) + 255) & ~(size_t)255;
+        const size_t state_size = fixed_rays ? CameraStage<N, 0>::state_bytes : CameraStage<N, N>::state_bytes,
+                     hit_size = fixed_rays ? CameraStage<N, 0>::hit_bytes : CameraStage<N, N>::hit_bytes;
+        const size_t state_bytes = ((size_t)Bw * state_size + 255) & ~(size_t)255;
         if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, state_bytes + (size_t)Bw * sizeof(VertexIn<N>)) &&
                            ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * Bw * sizeof(int)) &&
                            ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * (levels + 1) * sizeof(unsigned long long)))) {
@@ -152,39 +217,17 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         int sms = 0;
         DT_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
         used_wavefront = wavefront;
-        CamState<N> *states = (CamState<N> *)sb.cam_state;
-        VertexIn<N> *vins = (VertexIn<N> *)((char *)sb.cam_state + state_bytes);
-        int *qa = (int *)sb.cam_q, *qb = qa + Bw, *qv = qb + Bw, *qs = qv + Bw;
-        // volume and interface vertices queued per level [0, levels] (interface: pushed from the
-        // front of the queue, scnt, and from its back, sbk)
-        unsigned long long *vcnt = (unsigned long long *)sb.cam_cnt, *scnt = vcnt + (levels + 1),
-                           *sbk = scnt + (levels + 1);
+        const CamWave w{sb.cam_state, (char *)sb.cam_state + state_bytes, (int *)sb.cam_q,
+                        (unsigned long long *)sb.cam_cnt, Bw, levels};
         for (long long b0 = 0; b0 < total; b0 += B) {
             ++batches;
             rp.path_begin = b0;
             rp.path_count = std::min(B, total - b0);
             DT_CK(cudaMemsetAsync(sb.counts, 0, 3 * sizeof(unsigned long long), st));
             if (wavefront) {
-                // grid-stride launches of a few waves: late levels hold few live paths
-                const unsigned gw = std::min<unsigned>(blocks(rp.path_count), (unsigned)std::max(1, sms) * 16u);
                 if ((rc = timed(ms_camera, [&] {
-                         cudaMemsetAsync(vcnt, 0, (size_t)3 * (levels + 1) * sizeof(unsigned long long), st);
-                         // volume / interface queues of level L: (qa, qb) for even L, (qv, qs) for odd L
-                         k_cam_start<N><<<blocks(rp.path_count), kBlock, 0, st>>>(
-                             sc, rp, states, vins, qa, vcnt, qv, vcnt + 1, qs, scnt + 1, sbk + 1, Bw, qe, ql, ctr);
-                         for (int L = 0; L < levels; ++L) {
-                             int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
-                             int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
-                             k_cam_vertex<N, true><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vcnt + L, nullptr,
-                                                                          qvn, vcnt + L + 1, qsn, scnt + L + 1,
-                                                                          sbk + L + 1, Bw, qe, ql, ctr);
-                             if (L > 0)  // level 0's interface vertices ran in k_cam_start
-                                 k_cam_vertex<N, false><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qsl, scnt + L,
-                                                                               sbk + L, qvn, vcnt + L + 1, qsn,
-                                                                               scnt + L + 1, sbk + L + 1, Bw, qe, ql,
-                                                                               ctr);
-                         }
-                         k_cam_accum<N><<<blocks(rp.path_count), kBlock, 0, st>>>(rp, states, sb.acc1);
+                         if (fixed_rays) CameraStage<N, 0>::wave(sc, rp, w, sms, qe, ql, sb.acc1, ctr, st);
+                         else CameraStage<N, N>::wave(sc, rp, w, sms, qe, ql, sb.acc1, ctr, st);
                      })))
                     return rc;
                 launches += 2 * levels + 1;  // start, 2 per level (1 at level 0), accumulation
@@ -192,13 +235,13 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                     // every launched vertex reads and writes its path's state and vertex inputs;
                     // the start writes them once per path, the accumulation reads the sums
                     std::vector<unsigned long long> lc((size_t)3 * (levels + 1));
-                    DT_CK(cudaMemcpyAsync(lc.data(), vcnt, lc.size() * sizeof(unsigned long long),
+                    DT_CK(cudaMemcpyAsync(lc.data(), w.cnt, lc.size() * sizeof(unsigned long long),
                                           cudaMemcpyDeviceToHost, st));
                     DT_CK(cudaStreamSynchronize(st));
                     // each queued vertex's state and inputs are written once and read once (a
                     // volume vertex's without the hit record); an ended path writes its sums,
                     // which k_cam_accum reads
-                    const uint64_t sv = sizeof(CamState<N>) + sizeof(VertexIn<N>), si = sizeof(ItsAD<N>);
+                    const uint64_t sv = state_size + sizeof(VertexIn<N>), si = hit_size;
                     uint64_t vol = 0, itf = 0;
                     for (int L = 0; L < levels; ++L) {
                         vol += lc[L];
@@ -207,10 +250,12 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                     state_traffic += 2 * ((sv - si) * vol + sv * itf) + 2 * sizeof(DV<N>) * (uint64_t)rp.path_count;
                 }
             } else if ((rc = timed(ms_camera, [&] {
-                            k_camera<N><<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, qe, ql, sb.acc1, ctr);
+                            if (fixed_rays) CameraStage<N, 0>::mega(sc, rp, qe, ql, sb.acc1, ctr, st);
+                            else CameraStage<N, N>::mega(sc, rp, qe, ql, sb.acc1, ctr, st);
                         }))) {
                 return rc;
             }
+            if (fixed_rays) continue;  // no records
             if ((rc = read_counts())) return rc;
             const unsigned long long ne = std::min<unsigned long long>(hcnt[0], rec_cap);
             const unsigned long long nl = std::min<unsigned long long>(hcnt[1], rec_cap);
@@ -237,7 +282,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         prim_samples = (uint64_t)ns;
         rp.prim_weight = sc.pedge_sum / (double)ns;
         const long long chunk = std::max<long long>(1, (long long)(li_cap / 2));
-        for (long long k0 = 0; k0 < ns; k0 += chunk) {
+        for (long long k0 = 0; k0 < ns && !fixed_rays; k0 += chunk) {  // no edge moves on the screen under fixed rays
             rp.prim_begin = k0;
             rp.prim_count = std::min(chunk, ns - k0);
             if ((rc = timed(ms_primary, [&] {
@@ -418,6 +463,7 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
     if (total > 0) {
         // 128-path units keep every warp inside one pixel whenever spp is a multiple of 32
         const long long unit = 128;
+        const bool fixed_rays = static_rays(sc);
         long long B = (long long)(kNoallocRecCap / (uint64_t)(o->max_bounces + 1));
         B = std::max<long long>(unit, (B / unit) * unit);
         const long long per_chunk = std::max<long long>(1, (long long)(kNoallocLiCap / (uint64_t)std::max(1, 2 * rp.sppse)));
@@ -426,7 +472,8 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
             rp.path_begin = b0;
             rp.path_count = std::min(B, total - b0);
             DT_CK(cudaMemsetAsync(counts, 0, 3 * sizeof(unsigned long long), st));
-            k_camera<N><<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, qe, ql, acc1, nullptr);
+            if (fixed_rays) CameraStage<N, 0>::mega(sc, rp, qe, ql, acc1, nullptr, st);
+            else CameraStage<N, N>::mega(sc, rp, qe, ql, acc1, nullptr, st);
             if ((rc = launched())) return rc;
             if ((rc = read_counts())) return rc;
             const unsigned long long ne = std::min<unsigned long long>(hcnt[0], kNoallocRecCap);
