@@ -186,7 +186,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
                      (s->camera_schedule == DTRT_CAMERA_AUTO && total >= kWavefrontMinPaths);
     AdjWave w{};
     if (wavefront) {
-        const long long cap = std::min<long long>(1ll << 22, std::max<long long>(total, 1));
+        const long long cap = std::min<long long>(1ll << 24, std::max<long long>(total, 1));
         if (ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, AdjWave::bytes(cap, o->max_bounces + 1))) {
             w.carve(sb.cam_state, cap, o->max_bounces + 1);
         } else {

@@ -388,7 +388,7 @@ DT_D void replay_next(const DevScene &sc, const RenderParams &rp, AdjState<N> &s
 // the path goes on to level 1's distance sampling, a volume vertex is queued for level 0.
 // Pass B starts only paths with a value whose pixel has a non-zero dL/dI.
 template <int N>
-__global__ void __launch_bounds__(kBlock) k_adj_start(DevScene sc, RenderParams rp, AdjState<N> *states,
+__global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderParams rp, AdjState<N> *states,
                                                       VertexIn<N> *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, const float *dimg, float *grad,
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_start(DevScene sc, RenderParams 
 // Vertex level of one pass: the volume (kVolume) or interface vertices, each continuing path
 // then running level L+1's distance sampling (replay_next).
 template <int N, bool kVolume>
-__global__ void __launch_bounds__(kBlock) k_adj_vertex(DevScene sc, RenderParams rp, AdjState<N> *states,
+__global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderParams rp, AdjState<N> *states,
                                                        VertexIn<N> *vins, const int *q_in,
                                                        const unsigned long long *cnt_in, int *qv_next,
                                                        unsigned long long *cnt_v_next, int *qs_next,

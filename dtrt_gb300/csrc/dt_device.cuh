@@ -978,6 +978,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
         // nothing in the integral carries a derivative: every slot is zero. Draw the same
         // random numbers; the scatter pass only needs the sample positions.
         const float3 o = ray.o.val(), d = ray.d.val();
+#pragma unroll 1
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
             if (scatter) {
@@ -993,7 +994,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
         // d_scale[j] * density(p), so the integral needs only the sum of ten plain lookups
         const float3 o = ray.o.val(), d = ray.d.val();
         float sum = 0.f;
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
             sum += grid_lookup(m.density, o + d * (tmin.v + len * r), c);
@@ -1007,6 +1008,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
         const float3 o = ray.o.val(), d = ray.d.val(), ctr = f3(m.density.center);
         float sum = 0.f;
         float3 sh = mk(0.f, 0.f, 0.f), sqh = sh;
+#pragma unroll 1
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
             const float3 p = o + d * (tmin.v + len * r);
@@ -1020,6 +1022,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
             out[j] = (scale.d[j] * sum - scale.v * (dot(f3(m.density.rot_vel[j]), sqh) + dot(f3(m.density.trans_vel[j]), sh))) *
                      (len * 0.1f);
     } else {
+#pragma unroll 1
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
             const Df<G> tt = tmin + len * r;
@@ -1264,6 +1267,21 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, int *stack, float3 o, float
     return zero;
 }
 
+// Triangles hit along a null-interface chain after its first, up to two: the walk that finds out
+// whether a chain ends at an emitter keeps them for the transmittance pass, which would trace
+// the same rays again (a chain through a medium's boundary to the light is two).
+struct Chain {
+    static constexpr int kMax = 2;
+    int p0 = -1, p1 = -1, n = 0;
+    DT_D void add(int prim) {
+        if (n == 0) p0 = prim;
+        else if (n == 1) p1 = prim;
+        ++n;
+    }
+    DT_D bool has(int i) const { return i < n && i < kMax; }
+    DT_D int get(int i) const { return i == 0 ? p0 : p1; }
+};
+
 // scene.cpp:703-793
 template <int N, int G>
 DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray, bool on_surface, Rng &rng, int med,
@@ -1278,6 +1296,7 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray,
         return DV<N>();
     }
     shape_intersect_ad<G>(sc, prim, ray, its);
+    Chain chain;
     if (sc.has_grid_media) {
         // Geometry first: follow null interfaces to the surface that ends the chain. A chain
         // that does not end at an emitter contributes nothing, so its transmittance (a
@@ -1289,7 +1308,10 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray,
         int p1 = prim;
         bool emitter = false;
         for (int inter = 0; inter < kMaxInteractions; ++inter) {
-            if (inter > 0) shape_intersect_ad<G>(sc, p1, r1, n1);
+            if (inter > 0) {
+                chain.add(p1);
+                shape_intersect_ad<G>(sc, p1, r1, n1);
+            }
             const DevShape &s = sc.shapes[n1.shape];
             if (s.light_id >= 0) {
                 emitter = true;
@@ -1313,8 +1335,8 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray,
         const DevShape &s = sc.shapes[ni.shape];
         if (s.light_id >= 0) {
             const float3 dp = ni.p.val() - scatter;
-            const float G = ni.wi.z.v / dot(dp, dp);
-            pdf_nee = sc.light_pmf[s.light_id] / (sc.light_area[s.light_id] * G);
+            const float geom = ni.wi.z.v / dot(dp, dp);
+            pdf_nee = sc.light_pmf[s.light_id] / (sc.light_area[s.light_id] * geom);
             if (far_shape) {
                 *far_shape = ni.shape;
                 *far_t = dist;
@@ -1325,7 +1347,8 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray,
         if (is_transition(s)) med = dot(ni.ng, ray.d.val()) > 0.f ? s.med_ext : s.med_int;
         ray.o = ray.o + ray.d * tmax;
         tmin = kShadowEps;
-        prim = closest_hit(sc, stack, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
+        prim = chain.has(inter) ? chain.get(inter)
+                                : closest_hit(sc, stack, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
         if (prim < 0) return DV<N>();
     }
     return DV<N>();

@@ -94,7 +94,7 @@ inline bool static_rays(const DevScene &sc) {
 
 // Camera paths per batch of a scene of static_rays(): its batches hold no records, only path
 // states (2 GB at nder 8)
-constexpr long long kStaticBatchPaths = 1ll << 22;
+constexpr long long kStaticBatchPaths = 1ll << 23;
 
 // Buffers of the camera wavefront for `cap` paths: path states, vertex inputs, four
 // path-index queues, level counts

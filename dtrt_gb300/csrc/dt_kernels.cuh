@@ -569,7 +569,7 @@ DT_D void store_state(CamState<N, G> *states, int id, const CamState<N, G> &st, 
 // sampling. An interface vertex (every path from a camera outside media) runs here too and
 // the path goes on to level 1's distance sampling; a volume vertex is queued for level 0.
 template <int N, int G>
-__global__ void __launch_bounds__(kBlock) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
+__global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                       VertexIn<N> *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, unsigned long long *cnt_s1_back,
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(kBlock) k_cam_start(DevScene sc, RenderParams 
 // Vertex level L, one launch per kind: the volume (kVolume) or interface vertices of the
 // level; a continuing path then runs level L+1's distance sampling (camera_next).
 template <int N, int G, bool kVolume>
-__global__ void __launch_bounds__(kBlock) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
+__global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                        VertexIn<N> *vins, const int *q_in,
                                                        const unsigned long long *cnt_in,
                                                        const unsigned long long *cnt_in_back, int *qv_next,
