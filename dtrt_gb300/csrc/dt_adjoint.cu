@@ -34,7 +34,7 @@ cudaError_t launch_adjoint(const DevScene &sc, const RenderParams &rp, const flo
 }
 
 size_t AdjWave::bytes(long long cap, int levels) {
-    return (size_t)cap * (sizeof(AdjState<0>) + sizeof(VertexIn<0>) + 4 * sizeof(int) + sizeof(float3) +
+    return (size_t)cap * (sizeof(AdjState<0>) + sizeof(VertexIn) + 4 * sizeof(int) + sizeof(float3) +
                           kReplayEvents * sizeof(float3)) +
            (size_t)6 * (levels + 1) * sizeof(unsigned long long) + 2048;  // + 256-byte alignment of 6 arrays
 }
@@ -49,7 +49,7 @@ void AdjWave::carve(void *base, long long capacity, int lv) {
     cap = capacity;
     levels = lv;
     states = take((size_t)cap * sizeof(AdjState<0>));
-    vins = take((size_t)cap * sizeof(VertexIn<0>));
+    vins = take((size_t)cap * sizeof(VertexIn));
     q = (int *)take((size_t)4 * cap * sizeof(int));
     tots = (float3 *)take((size_t)cap * sizeof(float3));
     ev = (float3 *)take((size_t)cap * kReplayEvents * sizeof(float3));
@@ -66,7 +66,7 @@ cudaError_t launch_adjoint_wave(const DevScene &sc, const RenderParams &range, c
     if (levels > w.levels) return cudaErrorInvalidValue;
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
     AdjState<0> *states = (AdjState<0> *)w.states;
-    VertexIn<0> *vins = (VertexIn<0> *)w.vins;
+    VertexIn *vins = (VertexIn *)w.vins;
     int *qa = w.q, *qb = qa + w.cap, *qv = qb + w.cap, *qs = qv + w.cap;
     const bool pass_b = grad != nullptr && dimg != nullptr;
     RenderParams rp = range;
@@ -179,6 +179,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     uint64_t launches = 0;
     float ms_replay = 0.f;
     DT_ACK(cudaEventRecord(e0, st));
+    launches += (uint64_t)prepare_cells(s, sc, total, grad != nullptr && dimg != nullptr, st);
     // schedule: the wavefront (pass A and pass B each one launch per vertex over the live
     // paths) for large renders, as dtrt_render_fwd's camera schedule
     const long long B = 1ll << 24;  // paths per megakernel launch
@@ -209,6 +210,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
             ++launches;
         }
     }
+    if (grad) launches += (uint64_t)gather_cells(s, sc, grad, st);
     DT_ACK(cudaEventRecord(e1, st));
     if (image) {
         float *dst = image;

@@ -75,23 +75,26 @@ DT_D bool replay_start(const DevScene &sc, const RenderParams &rp, int *stack, l
 // then replay_volume or replay_surface.
 template <int N>
 DT_D int replay_decide(const DevScene &sc, const RenderParams &rp, bool pass_b, float3 total, float3 gpix, AdjCtx &adj,
-                       Ctr &c, AdjState<N> &st, VertexIn<N> &vin) {
+                       Ctr &c, AdjState<N> &st, VertexIn &vin) {
     Rng &rng = st.rng;
     const float r1a = rng.next1(), r1b = rng.next1();
     vin.r2[0] = rng.next1(); vin.r2[1] = rng.next1(); vin.r2[2] = rng.next1(); vin.r2[3] = rng.next1();
     vin.r3a = rng.next1(); vin.r3b = rng.next1(); vin.r3c = rng.next1();
-    vin.thr = DV<N>(mk(1.f, 1.f, 1.f));
-    vin.dir_in = st.ray.d.val();
     if (pass_b) adj.w = dot(gpix, total - st.acc) * rp.inv_spp;  // suffix radiance of this factor
-    if (st.med >= 0 && sample_distance_ad<N>(sc, sc.media[st.med], st.ray, st.its.t, r1a, r1b, rng, vin.thr, c,
-                                             pass_b ? &adj : nullptr))
-        return (st.depth == 0 || vin.thr.is_zero()) ? 0 : 1;
-    return (!st.its.valid() || vin.thr.is_zero()) ? 0 : 2;
+    bool zero = false, scatter = false;
+    if (st.med >= 0) {
+        DV<N> P(st.P);
+        scatter = medium_step<N>(sc, sc.media[st.med], st.ray, st.its.t, r1a, r1b, rng, P, zero, c,
+                                 pass_b ? &adj : nullptr);
+        st.P = P.val();
+    }
+    if (scatter) return (st.depth == 0 || zero) ? 0 : 1;
+    return (!st.its.valid() || zero) ? 0 : 2;
 }
 
 template <int N>
 DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, bool pass_b, float3 gpix, AdjCtx &adj,
-                        Ctr &c, float3 *ev, AdjState<N> &st, const VertexIn<N> &vin) {
+                        Ctr &c, float3 *ev, AdjState<N> &st, const VertexIn &vin) {
     Rng &rng = st.rng;
     RayAD<N> &ray = st.ray;
     ItsAD<N> &its = st.its;
@@ -101,12 +104,10 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     const AdjCtx *hook = pass_b ? &adj : nullptr;
     const float *r2 = vin.r2;
     const float r3a = vin.r3a, r3b = vin.r3b;
-    const DV<N> &thr = vin.thr;
-    const float3 dir_in = vin.dir_in;
+    const float3 dir_in = ray.d.val();
     bool alive = false;
     // ------------------------------------------------ volumetric vertex
     const DevPhase &ph = sc.phases[sc.media[med].phase_id];
-    const float3 Q = cmul(P, thr.val());
     DV<N> wo;
     float pdf_nee;
     if (mode & MODE_VOLUME_MAIN) {
@@ -124,7 +125,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
             if (!v.is_zero()) {
                 const Df<N> pv = phase_eval_ad<N>(ph, -ray.d, wo);
                 if (pv.v > kEps)
-                    e = cmul(Q, v.val()) * (pv.v * mis_weight(pdf_nee, phase_eval(ph, -dir_in, wo.val())));
+                    e = cmul(P, v.val()) * (pv.v * mis_weight(pdf_nee, phase_eval(ph, -dir_in, wo.val())));
             }
             if (pass_b && !is_zero3(e, 0.f)) {
                 const Rng after = rng;
@@ -141,7 +142,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     }
     const Df<N> pvs = phase_sample_ad<N>(ph, -ray.d, r3a, r3b, wo);
     if (pvs.v > kEps) {
-        const float3 thr1 = thr.val() * pvs.v;
+        P = P * pvs.v;
         ray.d = wo;
         ItsAD<N> its1;
         const int k = ne++;
@@ -157,7 +158,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
                                                nullptr, nullptr, c);
             float3 e = zero;
             if (!att.is_zero() && (mode & MODE_VOLUME_MAIN))
-                e = cmul(cmul(P, thr1), att.val()) * mis_weight(phase_eval(ph, -wo.val(), wo.val()), pdf_nee);
+                e = cmul(P, att.val()) * mis_weight(phase_eval(ph, -wo.val(), wo.val()), pdf_nee);
             if (pass_b && !is_zero3(e, 0.f)) {
                 const Rng after = rng;
                 rng = saved;
@@ -172,7 +173,6 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
             acc = acc + e;
         }
         its = its1;
-        P = cmul(P, thr1);
         depth -= 1;
         mode &= ~MODE_EMISSION;
         alive = true;
@@ -182,7 +182,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
 
 template <int N>
 DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack, bool pass_b, float3 gpix,
-                         AdjCtx &adj, Ctr &c, float3 *ev, AdjState<N> &st, const VertexIn<N> &vin) {
+                         AdjCtx &adj, Ctr &c, float3 *ev, AdjState<N> &st, const VertexIn &vin) {
     Rng &rng = st.rng;
     RayAD<N> &ray = st.ray;
     ItsAD<N> &its = st.its;
@@ -192,14 +192,12 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
     const AdjCtx *hook = pass_b ? &adj : nullptr;
     const float *r2 = vin.r2;
     const float r3a = vin.r3a, r3b = vin.r3b, r3c = vin.r3c;
-    const DV<N> &thr = vin.thr;
-    const float3 dir_in = vin.dir_in;
+    const float3 dir_in = ray.d.val();
     bool alive = false;
     // ---------------------------------------------------- interface vertex
     const DevShape &sh = sc.shapes[its.shape];
     if (is_transition(sh) && target_medium(sc, its.shape, its.ng, -dir_in) != med) return false;
-    const float3 Q = cmul(P, thr.val());
-    if (sh.light_id >= 0 && (mode & MODE_EMISSION)) acc = acc + cmul(Q, le_ad<N>(sc, its, -ray.d).val());
+    if (sh.light_id >= 0 && (mode & MODE_EMISSION)) acc = acc + cmul(P, le_ad<N>(sc, its, -ray.d).val());
     if (depth == 0) return false;
     const DevBsdf &b = sc.bsdfs[sh.bsdf_id];
     const bool is_null = b.type == BSDF_NULL;
@@ -222,7 +220,7 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
             if (!v.is_zero()) {
                 const DV<N> bv = bsdf_eval_ad<N>(b, its.wi, wo);
                 const float bp = bsdf_pdf(b, its0.wi, wo.val());
-                e = cmul(cmul(Q, v.val()), bv.val()) * mis_weight(pdf_nee, bp);
+                e = cmul(cmul(P, v.val()), bv.val()) * mis_weight(pdf_nee, bp);
             }
             if (pass_b && !is_zero3(e, 0.f)) {
                 const Rng after = rng;
@@ -245,12 +243,11 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         ray.o = its.p;
         ray.d = wo;
         const int med1 = is_transition(sh) ? target_medium(sc, its.shape, its.ng, wo.val()) : med;
-        float3 thr1 = thr.val();
         ItsAD<N> its1;
         if (is_null) {
             ray_intersect_ad<N>(sc, stack, ray, true, its1, c);
         } else {
-            thr1 = cmul(thr1, bw.val());
+            P = cmul(P, bw.val());
             const int k = ne++;
             if (pass_b && k < kReplayEvents) {
                 const float3 e = ev[k];
@@ -264,7 +261,7 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
                                                    nullptr, nullptr, c);
                 float3 e = zero;
                 if (!att.is_zero() && (mode & MODE_SURFACE_MAIN))
-                    e = cmul(cmul(P, thr1), att.val()) * mis_weight(bpdf, pdf_nee);
+                    e = cmul(P, att.val()) * mis_weight(bpdf, pdf_nee);
                 if (pass_b && !is_zero3(e, 0.f)) {
                     const Rng after = rng;
                     rng = saved;
@@ -281,7 +278,6 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
             mode &= ~MODE_EMISSION;
         }
         its = its1;
-        P = cmul(P, thr1);
         med = med1;
         depth -= 1;
         alive = true;
@@ -292,7 +288,7 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
 template <int N>
 DT_D bool replay_step(const DevScene &sc, const RenderParams &rp, int *stack, bool pass_b, float3 total, float3 gpix,
                       AdjCtx &adj, Ctr &c, float3 *ev, AdjState<N> &st) {
-    VertexIn<N> vin;
+    VertexIn vin;
     const int kind = replay_decide<N>(sc, rp, pass_b, total, gpix, adj, c, st, vin);
     if (kind == 1) return replay_volume<N>(sc, rp, stack, pass_b, gpix, adj, c, ev, st, vin);
     if (kind == 2) return replay_surface<N>(sc, rp, stack, pass_b, gpix, adj, c, ev, st, vin);
@@ -369,11 +365,11 @@ DT_D float3 pixel_dldi(const RenderParams &rp, const float *dimg, long long g) {
 // interface vertex of L+1 (as camera_next).
 template <int N>
 DT_D void replay_next(const DevScene &sc, const RenderParams &rp, AdjState<N> &st, bool alive, bool pass_b,
-                      float3 total, float3 gp, AdjCtx &adj, VertexIn<N> *vins, int id, int *qv,
+                      float3 total, float3 gp, AdjCtx &adj, VertexIn *vins, int id, int *qv,
                       unsigned long long *cnt_v, int *qs, unsigned long long *cnt_s, const QueueEnds &qx, Ctr &c) {
     int kind = 0;
     if (alive && st.mode != 0) {
-        VertexIn<N> vin;
+        VertexIn vin;
         kind = replay_decide<N>(sc, rp, pass_b, total, gp, adj, c, st, vin);
         if (kind) vins[id] = vin;
     }
@@ -389,7 +385,7 @@ DT_D void replay_next(const DevScene &sc, const RenderParams &rp, AdjState<N> &s
 // Pass B starts only paths with a value whose pixel has a non-zero dL/dI.
 template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderParams rp, AdjState<N> *states,
-                                                      VertexIn<N> *vins, int *qv0, unsigned long long *cnt_v0,
+                                                      VertexIn *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, const float *dimg, float *grad,
                                                       const float3 *totals, float3 *evbuf, QueueEnds qx, bool pass_b,
@@ -412,7 +408,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderPara
         }
         run = !pass_b || (!is_zero3(total, 0.f) && !is_zero3(gp, 0.f));
         if (run && replay_start<N>(sc, rp, stack, g, st, c) && st.mode != 0) {
-            VertexIn<N> vin;
+            VertexIn vin;
             kind = replay_decide<N>(sc, rp, pass_b, total, gp, adj, c, st, vin);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
@@ -431,7 +427,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderPara
 // then running level L+1's distance sampling (replay_next).
 template <int N, bool kVolume>
 __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderParams rp, AdjState<N> *states,
-                                                       VertexIn<N> *vins, const int *q_in,
+                                                       VertexIn *vins, const int *q_in,
                                                        const unsigned long long *cnt_in, int *qv_next,
                                                        unsigned long long *cnt_v_next, int *qs_next,
                                                        unsigned long long *cnt_s_next, const float *dimg, float *grad,
@@ -444,7 +440,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderPar
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
         const int id = i < nf ? q_in[i] : q_in[qx.cap - 1 - (i - nf)];
         AdjState<N> st = states[id];
-        const VertexIn<N> vin = vins[id];
+        const VertexIn vin = vins[id];
         const float3 zero = mk(0.f, 0.f, 0.f);
         const float3 total = pass_b ? totals[id] : zero, gp = pass_b ? pixel_dldi(rp, dimg, rp.path_begin + id) : zero;
         AdjCtx adj{grad, 0.f};
@@ -534,7 +530,7 @@ DT_D const BatchItemDev &batch_item(const BatchWave &bw, long long i, long long 
 }
 
 template <int N>
-__global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N> *states, VertexIn<N> *vins, int *qv0,
+__global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N> *states, VertexIn *vins, int *qv0,
                                                        unsigned long long *cnt_v0, int *qv1,
                                                        unsigned long long *cnt_v1, int *qs1,
                                                        unsigned long long *cnt_s1, const float3 *totals,
@@ -559,7 +555,7 @@ __global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N>
         }
         run = !pass_b || (it.grad && !is_zero3(total, 0.f) && !is_zero3(gp, 0.f));
         if (run && replay_start<N>(it.sc, it.rp, stack, g, st, c) && st.mode != 0) {
-            VertexIn<N> vin;
+            VertexIn vin;
             kind = replay_decide<N>(it.sc, it.rp, pass_b, total, gp, adj, c, st, vin);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
@@ -576,7 +572,7 @@ __global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N>
 }
 
 template <int N, bool kVolume>
-__global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N> *states, VertexIn<N> *vins,
+__global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N> *states, VertexIn *vins,
                                                         const int *q_in, const unsigned long long *cnt_in,
                                                         int *qv_next, unsigned long long *cnt_v_next, int *qs_next,
                                                         unsigned long long *cnt_s_next, const float3 *totals,
@@ -590,7 +586,7 @@ __global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N
         long long g;
         const BatchItemDev &it = batch_item(bw, id, g);
         AdjState<N> st = states[id];
-        const VertexIn<N> vin = vins[id];
+        const VertexIn vin = vins[id];
         const float3 zero = mk(0.f, 0.f, 0.f);
         const float3 total = pass_b ? totals[id] : zero, gp = pass_b ? pixel_dldi(it.rp, it.dimg, g) : zero;
         AdjCtx adj{it.grad, 0.f};

@@ -27,6 +27,75 @@ namespace dt {
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
 
+// Density cells: voxel v's record holds the 8 corners of the cell whose lower corner it is
+// (corners past the last voxel read as the border voxel; no lookup uses them).
+__global__ void k_grid_cells(const float *data, int rx, int ry, int rz, float4 *cells) {
+    const size_t n = (size_t)rx * ry * rz, v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const int x = (int)(v % rx), y = (int)(v / rx % ry), z = (int)(v / ((size_t)rx * ry));
+    const size_t sx = x + 1 < rx ? 1 : 0, sy = y + 1 < ry ? rx : 0, sz = z + 1 < rz ? (size_t)rx * ry : 0;
+    const float *d = data + v;
+    cells[2 * v] = make_float4(__ldg(d), __ldg(d + sx), __ldg(d + sy), __ldg(d + sy + sx));
+    cells[2 * v + 1] = make_float4(__ldg(d + sz), __ldg(d + sz + sx), __ldg(d + sz + sy), __ldg(d + sz + sy + sx));
+}
+
+// grad[v] = the corners of the 8 cells around voxel v (cells of the border were never written)
+__global__ void k_cells_gather(const float4 *cells, int rx, int ry, int rz, float *grad) {
+    const size_t n = (size_t)rx * ry * rz, v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    const int x = (int)(v % rx), y = (int)(v / rx % ry), z = (int)(v / ((size_t)rx * ry));
+    const float *c = reinterpret_cast<const float *>(cells);
+    float sum = 0.f;
+    for (int k = 0; k < 8; ++k) {
+        const int dx = k & 1, dy = (k >> 1) & 1, dz = k >> 2;
+        if (x < dx || y < dy || z < dz) continue;
+        sum += c[8 * (v - dx - (size_t)dy * rx - (size_t)dz * rx * ry) + k];
+    }
+    grad[v] = sum;
+}
+
+int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, bool with_grad, cudaStream_t st) {
+    sc.cells = nullptr;
+    sc.grad_cells = nullptr;
+    const long long n = s->density_voxels;
+    // The copy costs 40 B of traffic per voxel, 14 us for 128^3; a path makes some tens of
+    // lookups. At most 2^27 voxels (4 GiB each copy).
+    if (n <= 0 || paths < n / 16 || n > (1ll << 27)) return 0;
+    Scratch &sb = s->scratch;
+    if (!ensure_buffer(&sb.cells, &sb.cells_bytes, (size_t)n * 32 * (with_grad ? 2 : 1))) {
+        cudaGetLastError();  // no room: the kernels read the voxels
+        return 0;
+    }
+    float4 *cells = (float4 *)sb.cells;
+    int launches = 0;
+    for (const DevMedium &m : s->media_host) {
+        if (m.type != MEDIUM_HETEROGENEOUS) continue;
+        const int *r = m.density.res;
+        k_grid_cells<<<(unsigned)(((size_t)r[0] * r[1] * r[2] + 255) / 256), 256, 0, st>>>(m.density.data, r[0], r[1], r[2],
+                                                                                         cells + 2 * m.grad_off);
+        ++launches;
+    }
+    if (with_grad) {
+        sc.grad_cells = cells + 2 * n;
+        if (cudaMemsetAsync(sc.grad_cells, 0, (size_t)n * 32, st) != cudaSuccess) sc.grad_cells = nullptr;
+    }
+    sc.cells = cells;
+    return launches;
+}
+
+int gather_cells(const dtrt_scene *s, const DevScene &sc, float *grad, cudaStream_t st) {
+    if (!sc.grad_cells) return 0;
+    int launches = 0;
+    for (const DevMedium &m : s->media_host) {
+        if (m.type != MEDIUM_HETEROGENEOUS) continue;
+        const int *r = m.density.res;
+        k_cells_gather<<<(unsigned)(((size_t)r[0] * r[1] * r[2] + 255) / 256), 256, 0, st>>>(
+            sc.grad_cells + 2 * m.grad_off, r[0], r[1], r[2], grad + m.grad_off);
+        ++launches;
+    }
+    return launches;
+}
+
 bool ensure_buffer(void **ptr, size_t *have, size_t need) {
     if (*have >= need && *ptr) return true;
     if (*ptr) cudaFree(*ptr);
@@ -1067,7 +1136,7 @@ int set_edge_weights(dtrt_scene *s, const float *w) {
 
 void free_scratch(Scratch &b) {
     void *ptrs[] = {b.acc1,     b.acc2,     b.out,     b.qe,     b.ql,      b.qli,       b.counts,   b.err,
-                    b.adj_dimg, b.adj_grad, b.adj_out, b.adj_img, b.cam_state, b.cam_q, b.cam_cnt, b.li_sort};
+                    b.adj_dimg, b.adj_grad, b.adj_out, b.adj_img, b.cam_state, b.cam_q, b.cam_cnt, b.li_sort, b.cells};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     b = Scratch();
@@ -1075,7 +1144,7 @@ void free_scratch(Scratch &b) {
 
 size_t scratch_bytes(const Scratch &b) {
     return b.acc1_n + b.acc2_n + b.out_n + b.qe_bytes + b.ql_bytes + b.qli_bytes + b.adj_dimg_n + b.adj_grad_n +
-           b.adj_out_n + b.adj_img_n + b.cam_state_bytes + b.cam_q_bytes + b.cam_cnt_bytes + b.li_sort_bytes;
+           b.adj_out_n + b.adj_img_n + b.cam_state_bytes + b.cam_q_bytes + b.cam_cnt_bytes + b.li_sort_bytes + b.cells_bytes;
 }
 
 // Render work buffers (queues of 16-24 Mi records, path states, accumulators: GBs) of the

@@ -284,7 +284,7 @@ int enqueue_chunk(dtrt_batch *b, const AdjWave &w, BatchWave bw, cudaStream_t st
     const int levels = b->max_levels;
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
     AdjState<0> *states = (AdjState<0> *)w.states;
-    VertexIn<0> *vins = (VertexIn<0> *)w.vins;
+    VertexIn *vins = (VertexIn *)w.vins;
     int *qa = w.q, *qb = qa + w.cap, *qv = qb + w.cap, *qs = qv + w.cap;
     {
         const unsigned gw = std::min<unsigned>(blocks(bw.count), (unsigned)std::max(1, b->sms) * 16u);

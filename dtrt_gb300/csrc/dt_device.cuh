@@ -757,54 +757,70 @@ DT_D bool grid_cell(const DevGrid &g, float3 p, int &x1, int &y1, int &z1) {
     z1 = (int)floorf(p.z);
     return true;
 }
-DT_D float grid_lookup(const DevGrid &g, float3 pw, Ctr &c) {  // gridvolume.h:144-171
+// The 8 corners of a medium's density cell, y then x fastest: lo at z1, hi at z1 + 1. Large
+// renders read them from a copy of the grid with the corners of each cell together
+// (DevScene::cells: two 128-bit loads of one sector instead of 8 loads of 4 or 5).
+struct Corners {
+    float4 lo, hi;
+};
+DT_D Corners grid_corners(const DevScene &sc, const DevMedium &m, int x1, int y1, int z1) {
+    const DevGrid &g = m.density;
+    const int sy = g.res[0], sz = g.res[0] * g.res[1];
+    const size_t base = (size_t)z1 * sz + (size_t)y1 * sy + x1;
+    if (sc.cells) {
+        const float4 *q = sc.cells + 2 * ((size_t)m.grad_off + base);
+        return {__ldg(q), __ldg(q + 1)};
+    }
+    const float *d = g.data + base;
+    return {make_float4(__ldg(d), __ldg(d + 1), __ldg(d + sy), __ldg(d + sy + 1)),
+            make_float4(__ldg(d + sz), __ldg(d + sz + 1), __ldg(d + sz + sy), __ldg(d + sz + sy + 1))};
+}
+DT_D float grid_lookup(const DevScene &sc, const DevMedium &m, float3 pw, Ctr &c) {  // gridvolume.h:144-171
     c.lookups++;
-    const float3 p = grid_point(g, pw);
+    const float3 p = grid_point(m.density, pw);
     int x1, y1, z1;
-    if (!grid_cell(g, p, x1, y1, z1)) return 0.f;
+    if (!grid_cell(m.density, p, x1, y1, z1)) return 0.f;
     const float fx = p.x - x1, fy = p.y - y1, fz = p.z - z1, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    const int sx = 1, sy = g.res[0], sz = g.res[0] * g.res[1];
-    const float *d = g.data + (size_t)z1 * sz + (size_t)y1 * sy + x1;
-    const float d000 = __ldg(d), d001 = __ldg(d + sx), d010 = __ldg(d + sy), d011 = __ldg(d + sy + sx);
-    const float d100 = __ldg(d + sz), d101 = __ldg(d + sz + sx), d110 = __ldg(d + sz + sy), d111 = __ldg(d + sz + sy + sx);
-    return ((d000 * gx + d001 * fx) * gy + (d010 * gx + d011 * fx) * fy) * gz +
-           ((d100 * gx + d101 * fx) * gy + (d110 * gx + d111 * fx) * fy) * fz;
+    const Corners q = grid_corners(sc, m, x1, y1, z1);
+    return ((q.lo.x * gx + q.lo.y * fx) * gy + (q.lo.z * gx + q.lo.w * fx) * fy) * gz +
+           ((q.hi.x * gx + q.hi.y * fx) * gy + (q.hi.z * gx + q.hi.w * fx) * fy) * fz;
 }
 // Density value and its gradient in world space at a point (zero outside the grid). With a
 // point that carries no derivative, slot j of a moving grid's density is the gradient times
 // the point's velocity in the grid, h . -(rot_j x q + trans_j) = -(rot_j . (q x h) +
 // trans_j . h) with q = p - centre (gridvolume.h:301-326): one gradient serves every slot,
 // and its sums over the samples of a line integral do as well.
-DT_D float grid_lookup_grad(const DevGrid &g, float3 pw, float3 &h, Ctr &c) {
+DT_D float grid_lookup_grad(const DevScene &sc, const DevMedium &m, float3 pw, float3 &h, Ctr &c) {
+    const DevGrid &g = m.density;
     c.lookups++;
     h = mk(0.f, 0.f, 0.f);
     const float3 p = grid_point(g, pw);
     int x1, y1, z1;
     if (!grid_cell(g, p, x1, y1, z1)) return 0.f;
     const float fx = p.x - x1, fy = p.y - y1, fz = p.z - z1, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    const int sx = 1, sy = g.res[0], sz = g.res[0] * g.res[1];
-    const float *d = g.data + (size_t)z1 * sz + (size_t)y1 * sy + x1;
-    const float d000 = __ldg(d), d001 = __ldg(d + sx), d010 = __ldg(d + sy), d011 = __ldg(d + sy + sx);
-    const float d100 = __ldg(d + sz), d101 = __ldg(d + sz + sx), d110 = __ldg(d + sz + sy), d111 = __ldg(d + sz + sy + sx);
+    const Corners k = grid_corners(sc, m, x1, y1, z1);
+    const float d000 = k.lo.x, d001 = k.lo.y, d010 = k.lo.z, d011 = k.lo.w;
+    const float d100 = k.hi.x, d101 = k.hi.y, d110 = k.hi.z, d111 = k.hi.w;
     const float a00 = d000 * gx + d001 * fx, a01 = d010 * gx + d011 * fx, a10 = d100 * gx + d101 * fx,
                 a11 = d110 * gx + d111 * fx;
     const float3 u = mk((((d001 - d000) * gy + (d011 - d010) * fy) * gz + ((d101 - d100) * gy + (d111 - d110) * fy) * fz) * g.to_grid[0],
                         ((a01 - a00) * gz + (a11 - a10) * fz) * g.to_grid[1],
                         ((a10 - a00) * gy + (a11 - a01) * fy) * g.to_grid[2]);
-    const float *m = g.w2v;
-    h = mk(m[0] * u.x + m[4] * u.y + m[8] * u.z, m[1] * u.x + m[5] * u.y + m[9] * u.z, m[2] * u.x + m[6] * u.y + m[10] * u.z);
+    const float *w = g.w2v;
+    h = mk(w[0] * u.x + w[4] * u.y + w[8] * u.z, w[1] * u.x + w[5] * u.y + w[9] * u.z, w[2] * u.x + w[6] * u.y + w[10] * u.z);
     return (a00 * gy + a01 * fy) * gz + (a10 * gy + a11 * fy) * fz;
 }
 template <int N, int G>
-DT_D Df<N> grid_lookup_ad(const DevGrid &g, const DV<G> &pw, Ctr &c) {  // gridvolume.h:174-201
+DT_D Df<N> grid_lookup_ad(const DevScene &sc, const DevMedium &m, const DV<G> &pw, Ctr &c) {  // gridvolume.h:174-201
+    const DevGrid &g = m.density;
     const bool voxel_dirs = g.dgrid != nullptr && g.dgrid_n == N;
     // A static grid sampled at a point without derivatives has none either: the plain
     // lookup gives the same dual exactly (all slots zero) at a fraction of the cost.
-    if (N == 0 || (!g.moving && !voxel_dirs && pw.der_zero(0.f))) return Df<N>(grid_lookup(g, pw.val(), c));
+    if (N == 0 || (!g.moving && !voxel_dirs && pw.der_zero(0.f))) return Df<N>(grid_lookup(sc, m, pw.val(), c));
     if constexpr (G == 0) {
         if (!voxel_dirs) {
             float3 h;
-            Df<N> r(grid_lookup_grad(g, pw.val(), h, c));
+            Df<N> r(grid_lookup_grad(sc, m, pw.val(), h, c));
             const float3 qh = cross(pw.val() - f3(g.center), h);
 #pragma unroll
             for (int j = 0; j < N; ++j) r.d[j] = -(dot(f3(g.rot_vel[j]), qh) + dot(f3(g.trans_vel[j]), h));
@@ -848,7 +864,8 @@ struct AdjCtx {
     float *grad;  // density gradient of all heterogeneous media (DevMedium::grad_off)
     float w;
 };
-DT_D void grid_scatter(const DevGrid &g, float *grad, float3 pw, float w) {
+DT_D void grid_scatter(const DevScene &sc, const DevMedium &m, float *grad, float3 pw, float w) {
+    const DevGrid &g = m.density;
     // a zero weight adds nothing; a non-finite one (a factor whose suffix is zero times an
     // unbounded segment) would poison the gradient, as a non-finite pixel derivative is
     // dropped by the forward write rule
@@ -858,7 +875,14 @@ DT_D void grid_scatter(const DevGrid &g, float *grad, float3 pw, float w) {
     if (!grid_cell(g, p, x1, y1, z1)) return;
     const float fx = p.x - x1, fy = p.y - y1, fz = p.z - z1, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
     const int sy = g.res[0], sz = g.res[0] * g.res[1];
-    float *q = grad + (size_t)z1 * sz + (size_t)y1 * sy + x1;
+    const size_t base = (size_t)m.grad_off + (size_t)z1 * sz + (size_t)y1 * sy + x1;
+    if (sc.grad_cells) {  // the cell's corners together: two vector atomics instead of 8
+        float4 *q = sc.grad_cells + 2 * base;
+        atomicAdd(q, make_float4(w * gx * gy * gz, w * fx * gy * gz, w * gx * fy * gz, w * fx * fy * gz));
+        atomicAdd(q + 1, make_float4(w * gx * gy * fz, w * fx * gy * fz, w * gx * fy * fz, w * fx * fy * fz));
+        return;
+    }
+    float *q = grad + base;
     atomicAdd(q, w * gx * gy * gz);
     atomicAdd(q + 1, w * fx * gy * gz);
     atomicAdd(q + sy, w * gx * fy * gz);
@@ -916,9 +940,9 @@ DT_D bool aabb_hit(const DevGrid &g, float3 o, float3 d, float &tn, float &tf) {
 }
 
 // ------------------------------------------------------------------ media
-DT_D float3 sig_s(const DevMedium &m, float3 x, Ctr &c) {  // homogeneous.h:57, heterogeneous.h:88-90
+DT_D float3 sig_s(const DevScene &sc, const DevMedium &m, float3 x, Ctr &c) {  // homogeneous.h:57, heterogeneous.h:88-90
     if (m.type == MEDIUM_HOMOGENEOUS) return f3(m.sigma_s);
-    return f3(m.albedo) * (m.scale * grid_lookup(m.density, x, c));
+    return f3(m.albedo) * (m.scale * grid_lookup(sc, m, x, c));
 }
 
 // homogeneous.cpp:6-24 / heterogeneous.cpp:9-37; moves `o` to the scatter point
@@ -951,7 +975,7 @@ DT_HEAVY bool sample_distance(const DevScene &sc, const DevMedium &m, float3 &o,
             break;
         }
         const float3 p = o + d * t;
-        const float dens = grid_lookup(m.density, p, c);
+        const float dens = grid_lookup(sc, m, p, c);
         if (rng.next1() * m.density.max_value < dens) {
             o = p;
             thr = cmul(thr, m.albedo_vol.valid ? grid_lookup3(m.albedo_vol, p) : f3(m.albedo));
@@ -983,7 +1007,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
             const float r = ((float)i + rng.next1()) * 0.1f;
             if (scatter) {
                 const float tt = tmin.v + len * r;
-                grid_scatter(m.density, adj->grad + m.grad_off, o + d * tt, -adj->w * m.scale * len * 0.1f);
+                grid_scatter(sc, m, adj->grad, o + d * tt, -adj->w * m.scale * len * 0.1f);
             }
         }
         return;
@@ -997,7 +1021,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
 #pragma unroll 1
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
-            sum += grid_lookup(m.density, o + d * (tmin.v + len * r), c);
+            sum += grid_lookup(sc, m, o + d * (tmin.v + len * r), c);
         }
 #pragma unroll
         for (int j = 0; j < N; ++j) out[j] = scale.d[j] * sum * (len * 0.1f);
@@ -1013,7 +1037,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
             const float r = ((float)i + rng.next1()) * 0.1f;
             const float3 p = o + d * (tmin.v + len * r);
             float3 h;
-            sum += grid_lookup_grad(m.density, p, h, c);
+            sum += grid_lookup_grad(sc, m, p, h, c);
             sh += h;
             sqh += cross(p - ctr, h);
         }
@@ -1027,10 +1051,10 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
             const float r = ((float)i + rng.next1()) * 0.1f;
             const Df<G> tt = tmin + len * r;
             const DV<G> pt = ray.o + ray.d * tt;
-            const Df<N> s = scale * grid_lookup_ad<N>(m.density, pt, c);
+            const Df<N> s = scale * grid_lookup_ad<N>(sc, m, pt, c);
 #pragma unroll
             for (int j = 0; j < N; ++j) out[j] += s.d[j];
-            if (scatter) grid_scatter(m.density, adj->grad + m.grad_off, pt.val(), -adj->w * m.scale * len * 0.1f);
+            if (scatter) grid_scatter(sc, m, adj->grad, pt.val(), -adj->w * m.scale * len * 0.1f);
         }
 #pragma unroll
         for (int j = 0; j < N; ++j) out[j] *= len * 0.1f;
@@ -1038,23 +1062,25 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
     if constexpr (G > 0) {
         const float3 o = ray.o.val(), d = ray.d.val();
         if (!tmax.der_zero(1e-6f)) {
-            const float dv = m.scale * grid_lookup(m.density, o + d * (tmax.v - kEps), c);
+            const float dv = m.scale * grid_lookup(sc, m, o + d * (tmax.v - kEps), c);
 #pragma unroll
             for (int j = 0; j < N; ++j) out[j] += tmax.d[j] * dv;
         }
         if (!tmin.der_zero(1e-6f)) {
-            const float dv = m.scale * grid_lookup(m.density, o + d * (tmin.v + kEps), c);
+            const float dv = m.scale * grid_lookup(sc, m, o + d * (tmin.v + kEps), c);
 #pragma unroll
             for (int j = 0; j < N; ++j) out[j] -= tmin.d[j] * dv;
         }
     }
 }
 
-// homogeneous.cpp:27-49 / heterogeneous.cpp:40-75; moves ray.o to the scatter point
-// With `adj`, the factor applied to `thr` scatters adj->w times its log-derivative.
+// homogeneous.cpp:27-49 / heterogeneous.cpp:40-75; moves ray.o to the scatter point. The
+// throughput changes by the scalar k, and by the albedo at a scatter point (true).
+// With `adj`, that factor scatters adj->w times its log-derivative.
 template <int N, int G>
 DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<G> &ray, const Df<G> &tmax, float r0,
-                             float r1, Rng &rng, DV<N> &thr, Ctr &c, const AdjCtx *adj = nullptr) {
+                             float r1, Rng &rng, Df<N> &k, Ctr &c, const AdjCtx *adj = nullptr) {
+    k = Df<N>(1.f);
     if (m.type == MEDIUM_HOMOGENEOUS) {
         const Df<N> sig = load_dual<N>(m.sigma_t, m.d_sigma_t);
         if (m.sampling_weight > kEps) {
@@ -1063,18 +1089,17 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<G
                 ray.o = ray.o + ray.d * t;
                 if (r1 < m.sampling_weight) {
                     Df<N> tmp = sig * dexp(-t * sig);
-                    Df<N> k = tmp / (tmp.v * m.sampling_weight);
-                    thr = cmul(thr, load_dual3<N>(m.albedo, m.d_albedo) * k);
+                    k = tmp / (tmp.v * m.sampling_weight);
                 } else {
-                    thr = DV<N>();
+                    k = Df<N>(0.f);
                 }
                 return true;
             }
             Df<N> tmp = dexp(-(lift<N>(tmax) * sig));
-            thr = thr * (tmp / tmp.v);
+            k = tmp / tmp.v;
             return false;
         }
-        thr = thr * dexp(-(lift<N>(tmax) * sig));
+        k = dexp(-(lift<N>(tmax) * sig));
         return false;
     }
     float tn, tf;
@@ -1093,36 +1118,50 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<G
         // the acceptance test needs the density value only; a null collision discards the
         // derivative slots, so the dual lookup runs at an accepted collision (same point)
         const DV<G> p = ray.o + ray.d * t;
-        const float dv = grid_lookup(m.density, p.val(), c);
+        const float dv = grid_lookup(sc, m, p.val(), c);
         if (rng.next1() * m.density.max_value < dv) {
             Ctr again;  // the lookup just counted, repeated with its derivative slots
-            const Df<N> dens = grid_lookup_ad<N>(m.density, p, again);
+            const Df<N> dens = grid_lookup_ad<N>(sc, m, p, again);
             // The reference aliases p_scatter with ray.org (volpathAD.cpp:164), so the
             // line integral below runs from the scatter point forward over [0, t].
             // EST_SCATTER_FROM_ORIGIN integrates the segment actually travelled instead.
             const RayAD<G> ray0 = ray;
             ray.o = p;
-            const DV<N> alb = m.albedo_vol.valid ? grid_lookup3_ad<N>(m.albedo_vol, p) : load_dual3<N>(m.albedo, m.d_albedo);
             const Df<N> sig = load_dual<N>(m.scale, m.d_scale) * dens;
             if (adj != nullptr && m.grad_off >= 0)  // d log(sigma_t(p)) = d density / density
-                grid_scatter(m.density, adj->grad + m.grad_off, p.val(), adj->w / dens.v);
+                grid_scatter(sc, m, adj->grad, p.val(), adj->w / dens.v);
             float ist[N > 0 ? N : 1];
             int_sig_t<N>(sc, m, (sc.est_flags & EST_SCATTER_FROM_ORIGIN) ? ray0 : ray, Df<G>(0.f), Df<G>(t), rng, ist,
                          c, adj);
             Df<N> tmp(1.f);
 #pragma unroll
             for (int j = 0; j < N; ++j) tmp.d[j] = -ist[j];
-            thr = cmul(thr, alb * (sig * tmp / sig.v));
+            k = sig * tmp / sig.v;
             return true;
         }
     }
     float ist[N > 0 ? N : 1];
     int_sig_t<N>(sc, m, ray, Df<G>(0.f), tmax, rng, ist, c, adj);
-    Df<N> tmp(1.f);
 #pragma unroll
-    for (int j = 0; j < N; ++j) tmp.d[j] = -ist[j];
-    thr = thr * tmp;
+    for (int j = 0; j < N; ++j) k.d[j] = -ist[j];
     return false;
+}
+
+// The distance sampling of a vertex: the prefix throughput P takes the factor; `zero` when
+// the factor vanishes (the path ends). True at a scatter point.
+template <int N, int G>
+DT_D bool medium_step(const DevScene &sc, const DevMedium &m, RayAD<G> &ray, const Df<G> &tmax, float r0, float r1,
+                      Rng &rng, DV<N> &P, bool &zero, Ctr &c, const AdjCtx *adj = nullptr) {
+    Df<N> k;
+    if (!sample_distance_ad<N>(sc, m, ray, tmax, r0, r1, rng, k, c, adj)) {
+        zero = fabsf(k.v) <= kEps;
+        P = P * k;
+        return false;
+    }
+    const DV<N> f = (m.albedo_vol.valid ? grid_lookup3_ad<N>(m.albedo_vol, ray.o) : load_dual3<N>(m.albedo, m.d_albedo)) * k;
+    zero = f.is_zero();
+    P = cmul(P, f);
+    return true;
 }
 
 // homogeneous.cpp:52-55 / heterogeneous.cpp:78-91 (residual ratio tracking)
@@ -1138,7 +1177,7 @@ DT_HEAVY float medium_transmittance(const DevScene &sc, const DevMedium &m, floa
             set_error(sc, ERR_TRACK_CAP);
             break;
         }
-        ret *= 1.f - grid_lookup(m.density, o + d * t, c) / m.density.max_value;
+        ret *= 1.f - grid_lookup(sc, m, o + d * t, c) / m.density.max_value;
     }
     return ret;
 }

@@ -31,6 +31,9 @@ struct Scratch {
     // sort of the Li sub-path pairs: keys, values, their double buffers and digit counts
     void *li_sort = nullptr;
     size_t li_sort_bytes = 0;
+    // density cells of a render (DevScene::cells), then the replay's gradient in that layout
+    void *cells = nullptr;
+    size_t cells_bytes = 0;
 
 };
 
@@ -147,6 +150,12 @@ struct dtrt_scene {
 };
 
 namespace dt {
+// Density cells of a render of `paths` camera paths (with_grad: and zeroed gradient cells) in
+// sc, from the scene's grids as they are now, on stream st; nothing when the render is too
+// small for them or the device has no room. Returns the kernels launched.
+int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, bool with_grad, cudaStream_t st);
+// sc.grad_cells summed into the voxels of `grad` (zeroed before); returns the kernels launched
+int gather_cells(const dtrt_scene *s, const DevScene &sc, float *grad, cudaStream_t st);
 template <int N>
 int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on_device, cudaStream_t stream);
 int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_image, float *image, float *d_density,

@@ -209,36 +209,32 @@ DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, int *stack, l
     return ray_intersect_ad<G>(sc, stack, st.ray, false, st.its, c);
 }
 
-// Random numbers of a vertex drawn before its branch, the distance-sampling throughput and
-// the incoming direction: what the volume and interface halves of a vertex share.
-template <int N>
+// Random numbers of a vertex drawn before its branch: what the volume and interface halves
+// of a vertex share (the distance-sampling throughput is folded into the path's P).
 struct alignas(16) VertexIn {
     float r2[4], r3a, r3b, r3c;
-    DV<N> thr;
-    float3 dir_in;
 };
 
 // First part of a vertex of camera path g (volpathAD.cpp:160-164, 306-308): the vertex's
 // random numbers and distance sampling. 0: the path ends here, 1: volume vertex, 2:
 // interface vertex.
 template <int N, int G>
-DT_D int camera_decide(const DevScene &sc, CamState<N, G> &st, VertexIn<N> &vin, Ctr &c) {
+DT_D int camera_decide(const DevScene &sc, CamState<N, G> &st, VertexIn &vin, Ctr &c) {
     Rng &rng = st.rng;
     const float r1a = rng.next1(), r1b = rng.next1();
     vin.r2[0] = rng.next1(); vin.r2[1] = rng.next1(); vin.r2[2] = rng.next1(); vin.r2[3] = rng.next1();
     vin.r3a = rng.next1(); vin.r3b = rng.next1(); vin.r3c = rng.next1();
-    vin.thr = DV<N>(mk(1.f, 1.f, 1.f));
-    vin.dir_in = st.ray.d.val();
-    if (st.med >= 0 && sample_distance_ad<N>(sc, sc.media[st.med], st.ray, st.its.t, r1a, r1b, rng, vin.thr, c))
-        return (st.depth == 0 || vin.thr.is_zero()) ? 0 : 1;
-    return (!st.its.valid() || vin.thr.is_zero()) ? 0 : 2;
+    bool zero = false;
+    if (st.med >= 0 && medium_step<N>(sc, sc.media[st.med], st.ray, st.its.t, r1a, r1b, rng, st.P, zero, c))
+        return (st.depth == 0 || zero) ? 0 : 1;
+    return (!st.its.valid() || zero) ? 0 : 2;
 }
 
 // Volume vertex (volpathAD.cpp:164-305): NEE, volume edge record, phase sampling and the
 // emitter lookup along the new direction. Returns whether the path continues.
 template <int N, int G>
 DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
-                        const VertexIn<N> &vin, const Queue &qe, Ctr &c) {
+                        const VertexIn &vin, const Queue &qe, Ctr &c) {
     Rng &rng = st.rng;
     RayAD<G> &ray = st.ray;
     ItsAD<G> &its = st.its;
@@ -249,19 +245,17 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     const uint64_t key = (uint64_t)g;
     const float *r2 = vin.r2;
     const float r3a = vin.r3a, r3b = vin.r3b;
-    const DV<N> &thr = vin.thr;
-    const float3 dir_in = vin.dir_in;
+    const float3 dir_in = ray.d.val();
     bool alive = false;
     // ------------------------------------------------ volumetric vertex, volpathAD.cpp:164-305
     const DevPhase &ph = sc.phases[sc.media[med].phase_id];
-    const DV<N> Q = cmul(P, thr);
     DV<G> wo;
     float pdf_nee;
     if (mode & MODE_VOLUME_MAIN) {
         DV<N> v = nee_point_ad<N>(sc, stack, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c);
         if (!v.is_zero()) {
             Df<N> pv = phase_eval_ad<N>(ph, -ray.d, wo);
-            if (pv.v > kEps) acc += cmul(Q, v) * (pv * mis_weight(pdf_nee, phase_eval(ph, -dir_in, wo.val())));
+            if (pv.v > kEps) acc += cmul(P, v) * (pv * mis_weight(pdf_nee, phase_eval(ph, -dir_in, wo.val())));
         }
     }
     // edge record before the continuation overwrites the vertex state
@@ -270,7 +264,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
         const long long slot = queue_reserve(sc, qe);
         if (slot >= 0) {
             EdgeRec<N> &r = reinterpret_cast<EdgeRec<N> *>(qe.data)[slot];
-            const float3 x = ray.o.val(), w = cmul(P.val(), thr.val()) * rp.inv_spp, wi = -dir_in;
+            const float3 x = ray.o.val(), w = P.val() * rp.inv_spp, wi = -dir_in;
             r.x0[0] = x.x; r.x0[1] = x.y; r.x0[2] = x.z;
 #pragma unroll
             for (int j = 0; j < G; ++j) {
@@ -285,15 +279,14 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     }
     const Df<N> pvs = phase_sample_ad<N>(ph, -ray.d, r3a, r3b, wo);
     if (pvs.v > kEps) {
-        const DV<N> thr1 = thr * pvs;
+        P = P * pvs;
         ray.d = wo;
         ItsAD<G> its1;
         DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, false, rng, med, depth - 1, its1, pdf_nee, nullptr,
                                            nullptr, c);
         if (!att.is_zero() && (mode & MODE_VOLUME_MAIN))
-            acc += cmul(cmul(P, thr1), att) * mis_weight(phase_eval(ph, -wo.val(), wo.val()), pdf_nee);
+            acc += cmul(P, att) * mis_weight(phase_eval(ph, -wo.val(), wo.val()), pdf_nee);
         its = its1;
-        P = cmul(P, thr1);
         depth -= 1;
         mode &= ~MODE_EMISSION;
         alive = true;
@@ -306,7 +299,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
 // path continues.
 template <int N, int G>
 DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
-                         const VertexIn<N> &vin, const Queue &qe, const Queue &ql, Ctr &c) {
+                         const VertexIn &vin, const Queue &qe, const Queue &ql, Ctr &c) {
     Rng &rng = st.rng;
     RayAD<G> &ray = st.ray;
     ItsAD<G> &its = st.its;
@@ -317,14 +310,12 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
     const uint64_t key = (uint64_t)g;
     const float *r2 = vin.r2;
     const float r3a = vin.r3a, r3b = vin.r3b, r3c = vin.r3c;
-    const DV<N> &thr = vin.thr;
-    const float3 dir_in = vin.dir_in;
+    const float3 dir_in = ray.d.val();
     bool alive = false;
     // ---------------------------------------------------- interface vertex, volpathAD.cpp:306-617
     const DevShape &sh = sc.shapes[its.shape];
     if (is_transition(sh) && target_medium(sc, its.shape, its.ng, -dir_in) != med) return false;
-    const DV<N> Q = cmul(P, thr);
-    if (sh.light_id >= 0 && (mode & MODE_EMISSION)) acc += cmul(Q, le_ad<N>(sc, its, -ray.d));
+    if (sh.light_id >= 0 && (mode & MODE_EMISSION)) acc += cmul(P, le_ad<N>(sc, its, -ray.d));
     if (depth == 0) return false;
     const DevBsdf &b = sc.bsdfs[sh.bsdf_id];
     const bool is_null = b.type == BSDF_NULL;
@@ -338,8 +329,8 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
             float3 n = its0.ng;
             if (dot(n, dir_in) < 0.f) n = -n;
             const int ns = min(max((int)(rp.ddist * its.t.der_max()), 1), 100);
-            const float3 sig = sig_s(sc.media[med], its0.p - n * kShadowEps, c);
-            const float3 w = cmul(cmul(P.val(), thr.val()), sig) * (rp.inv_spp / (float)ns);
+            const float3 sig = sig_s(sc, sc.media[med], its0.p - n * kShadowEps, c);
+            const float3 w = cmul(P.val(), sig) * (rp.inv_spp / (float)ns);
             const float3 *src[8] = {&its0.p, &its0.ng, &n, &dir_in, &its0.fr.s, &its0.fr.t, &its0.fr.n, &its0.wi};
             float *dst[8] = {r.p, r.ng, r.n, r.rd, r.fs, r.ft, r.fn, r.wi};
             for (int k = 0; k < 8; ++k) { dst[k][0] = src[k]->x; dst[k][1] = src[k]->y; dst[k][2] = src[k]->z; }
@@ -356,7 +347,7 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         const long long slot = queue_reserve(sc, qe);
         if (slot >= 0) {
             EdgeRec<N> &r = reinterpret_cast<EdgeRec<N> *>(qe.data)[slot];
-            const float3 x = its0.p, w = cmul(P.val(), thr.val()) * rp.inv_spp;
+            const float3 x = its0.p, w = P.val() * rp.inv_spp;
             r.x0[0] = x.x; r.x0[1] = x.y; r.x0[2] = x.z;
 #pragma unroll
             for (int j = 0; j < G; ++j) {
@@ -381,7 +372,7 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         if (!v.is_zero()) {
             const DV<N> bv = bsdf_eval_ad<N>(b, its.wi, wo);
             const float bp = bsdf_pdf(b, its0.wi, wo.val());
-            acc += cmul(cmul(Q, v), bv) * mis_weight(pdf_nee, bp);
+            acc += cmul(cmul(P, v), bv) * mis_weight(pdf_nee, bp);
         }
     }
     float bpdf, beta;
@@ -392,20 +383,17 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         ray.o = its.p;
         ray.d = wo;
         const int med1 = is_transition(sh) ? target_medium(sc, its.shape, its.ng, wo.val()) : med;
-        DV<N> thr1 = thr;
         ItsAD<G> its1;
         if (is_null) {
             ray_intersect_ad<G>(sc, stack, ray, true, its1, c);
         } else {
             DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, true, rng, med1, depth - 1, its1, pdf_nee,
                                                nullptr, nullptr, c);
-            thr1 = cmul(thr1, bw);
-            if (!att.is_zero() && (mode & MODE_SURFACE_MAIN))
-                acc += cmul(cmul(P, thr1), att) * mis_weight(bpdf, pdf_nee);
+            P = cmul(P, bw);
+            if (!att.is_zero() && (mode & MODE_SURFACE_MAIN)) acc += cmul(P, att) * mis_weight(bpdf, pdf_nee);
             mode &= ~MODE_EMISSION;
         }
         its = its1;
-        P = cmul(P, thr1);
         med = med1;
         depth -= 1;
         alive = true;
@@ -418,7 +406,7 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
 template <int N, int G>
 DT_D bool camera_step(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
                       const Queue &qe, const Queue &ql, Ctr &c) {
-    VertexIn<N> vin;
+    VertexIn vin;
     const int kind = camera_decide<N, G>(sc, st, vin, c);
     if (kind == 1) return camera_volume<N, G>(sc, rp, stack, g, st, vin, qe, c);
     if (kind == 2) return camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
@@ -528,12 +516,12 @@ DT_D bool interface_back(const DevScene &sc, int shape) {
 // After a vertex of level L: a continuing path draws the random numbers and samples the
 // distance of level L+1 right away and is queued as a volume or interface vertex of L+1.
 template <int N, int G>
-DT_D int camera_next(const DevScene &sc, CamState<N, G> &st, bool alive, VertexIn<N> *vins, int id, int *qv,
+DT_D int camera_next(const DevScene &sc, CamState<N, G> &st, bool alive, VertexIn *vins, int id, int *qv,
                      unsigned long long *cnt_v, int *qs, unsigned long long *cnt_s, unsigned long long *cnt_s_back,
                      long long cap, Ctr &c) {
     int kind = 0;
     if (alive && st.mode != 0) {
-        VertexIn<N> vin;
+        VertexIn vin;
         kind = camera_decide<N, G>(sc, st, vin, c);
         if (kind) vins[id] = vin;
     }
@@ -570,7 +558,7 @@ DT_D void store_state(CamState<N, G> *states, int id, const CamState<N, G> &st, 
 // the path goes on to level 1's distance sampling; a volume vertex is queued for level 0.
 template <int N, int G>
 __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
-                                                      VertexIn<N> *vins, int *qv0, unsigned long long *cnt_v0,
+                                                      VertexIn *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, unsigned long long *cnt_s1_back,
                                                       long long cap, Queue qe, Queue ql, unsigned long long *ctr) {
@@ -584,7 +572,7 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene s
     if (gi < rp.path_count) {
         const long long g = rp.path_begin + gi;
         if (camera_start<N, G>(sc, rp, stack, g, st, c) && st.mode != 0) {
-            VertexIn<N> vin;
+            VertexIn vin;
             kind = camera_decide<N, G>(sc, st, vin, c);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
@@ -603,7 +591,7 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene s
 // level; a continuing path then runs level L+1's distance sampling (camera_next).
 template <int N, int G, bool kVolume>
 __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
-                                                       VertexIn<N> *vins, const int *q_in,
+                                                       VertexIn *vins, const int *q_in,
                                                        const unsigned long long *cnt_in,
                                                        const unsigned long long *cnt_in_back, int *qv_next,
                                                        unsigned long long *cnt_v_next, int *qs_next,
@@ -632,7 +620,7 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_vertex(DevScene 
         } else {
             st = states[id];
         }
-        const VertexIn<N> vin = vins[id];
+        const VertexIn vin = vins[id];
         const long long g = rp.path_begin + id;
         const bool alive = kVolume ? camera_volume<N, G>(sc, rp, stack, g, st, vin, qe, c)
                                    : camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);

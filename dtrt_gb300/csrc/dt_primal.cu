@@ -193,6 +193,7 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     DT_PCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
     DT_PCK(cudaEventRecord(e0, st));
+    launches += (uint64_t)prepare_cells(s, sc, total, false, st);
     for (long long b0 = 0; b0 < total; b0 += B) {
         rp.path_begin = b0;
         rp.path_count = std::min(B, total - b0);

@@ -32,7 +32,7 @@ namespace dt {
 // (dt_camera_n*.cu).
 template <int N, int G>
 struct CameraStage {
-    static constexpr size_t state_bytes = sizeof(CamState<N, G>), vertex_bytes = sizeof(VertexIn<N>),
+    static constexpr size_t state_bytes = sizeof(CamState<N, G>), vertex_bytes = sizeof(VertexIn),
                             hit_bytes = sizeof(ItsAD<G>);
     static void wave(const DevScene &sc, const RenderParams &rp, const CamWave &w, int sms, const Queue &qe,
                      const Queue &ql, double *acc1, unsigned long long *ctr, cudaStream_t st);
@@ -47,7 +47,7 @@ template <int N, int G>
 void CameraStage<N, G>::wave(const DevScene &sc, const RenderParams &rp, const CamWave &w, int sms, const Queue &qe,
                              const Queue &ql, double *acc1, unsigned long long *ctr, cudaStream_t st) {
     CamState<N, G> *states = (CamState<N, G> *)w.states;
-    VertexIn<N> *vins = (VertexIn<N> *)w.vins;
+    VertexIn *vins = (VertexIn *)w.vins;
     int *qa = w.q, *qb = qa + w.cap, *qv = qb + w.cap, *qs = qv + w.cap;
     // volume and interface vertices queued per level [0, levels] (interface: pushed from the
     // front of the queue, scnt, and from its back, sbk)
@@ -192,6 +192,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
 
     // ---------------------------------------------------------------- pass 1
     const long long total = (long long)npix * std::max(0, o->spp);
+    launches += (uint64_t)prepare_cells(s, sc, total, false, st);
     if (total > 0) {
         const long long unit = std::max<long long>(128, (long long)rp.spp % 32 == 0 ? std::max(rp.spp, 128) : 128);
         // without records a batch is bounded by the path states alone
@@ -207,7 +208,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         const size_t state_size = fixed_rays ? CameraStage<N, 0>::state_bytes : CameraStage<N, N>::state_bytes,
                      hit_size = fixed_rays ? CameraStage<N, 0>::hit_bytes : CameraStage<N, N>::hit_bytes;
         const size_t state_bytes = ((size_t)Bw * state_size + 255) & ~(size_t)255;
-        if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, state_bytes + (size_t)Bw * sizeof(VertexIn<N>)) &&
+        if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, state_bytes + (size_t)Bw * sizeof(VertexIn)) &&
                            ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * Bw * sizeof(int)) &&
                            ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * (levels + 1) * sizeof(unsigned long long)))) {
             if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
@@ -241,7 +242,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                     // each queued vertex's state and inputs are written once and read once (a
                     // volume vertex's without the hit record); an ended path writes its sums,
                     // which k_cam_accum reads
-                    const uint64_t sv = state_size + sizeof(VertexIn<N>), si = hit_size;
+                    const uint64_t sv = state_size + sizeof(VertexIn), si = hit_size;
                     uint64_t vol = 0, itf = 0;
                     for (int L = 0; L < levels; ++L) {
                         vol += lc[L];

@@ -153,6 +153,8 @@ struct DevScene {
     int num_pedges;
     double pedge_sum;
     DevCamera cam;
+    const float4 *cells;           // density cells with their corners together, [voxel][2] in grad_off order (or NULL)
+    float4 *grad_cells;            // the density gradient of the replay in the same layout (or NULL)
     int tracking_cap;
     int moving_geometry;           // any vertex velocity present
     int has_grid_media;            // a heterogeneous medium exists (transmittance is a random estimate)
