@@ -47,7 +47,7 @@ struct alignas(16) AdjState {
 };
 
 template <int N>
-DT_D bool replay_start(const DevScene &sc, const RenderParams &rp, int *stack, long long g, AdjState<N> &st, Ctr &c) {
+DT_D bool replay_start(const DevScene &sc, const RenderParams &rp, long long g, AdjState<N> &st, Ctr &c) {
     const int pixel = (int)(g / rp.spp);
     const int ix = rp.crop_x + pixel % rp.out_w, iy = rp.crop_y + pixel / rp.out_w;
     st.rng.init(rp.seed, (uint64_t)g);
@@ -65,7 +65,7 @@ DT_D bool replay_start(const DevScene &sc, const RenderParams &rp, int *stack, l
     st.ne = 0;
     st.P = mk(1.f, 1.f, 1.f);
     st.acc = mk(0.f, 0.f, 0.f);
-    return ray_intersect_ad<N>(sc, stack, st.ray, false, st.its, c);
+    return ray_intersect_ad<N>(sc, st.ray, false, st.its, c);
 }
 
 // One vertex of the replayed path (camera_step's branches, values only). Pass B scatters
@@ -93,7 +93,7 @@ DT_D int replay_decide(const DevScene &sc, const RenderParams &rp, bool pass_b, 
 }
 
 template <int N>
-DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, bool pass_b, float3 gpix, AdjCtx &adj,
+DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, bool pass_b, float3 gpix, AdjCtx &adj,
                         Ctr &c, float3 *ev, AdjState<N> &st, const VertexIn &vin) {
     Rng &rng = st.rng;
     RayAD<N> &ray = st.ray;
@@ -115,12 +115,12 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
         if (pass_b && k < kReplayEvents) {
             const float3 e = ev[k];
             adj.w = dot(gpix, e) * rp.inv_spp;
-            nee_point_ad<N>(sc, stack, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c,
+            nee_point_ad<N>(sc, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c,
                             is_zero3(e, 0.f) ? nullptr : hook);
             acc = acc + e;
         } else {
             const Rng saved = rng;
-            DV<N> v = nee_point_ad<N>(sc, stack, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c);
+            DV<N> v = nee_point_ad<N>(sc, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c);
             float3 e = zero;
             if (!v.is_zero()) {
                 const Df<N> pv = phase_eval_ad<N>(ph, -ray.d, wo);
@@ -133,7 +133,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
                 adj.w = dot(gpix, e) * rp.inv_spp;
                 DV<N> wo2;
                 float pdf2;
-                nee_point_ad<N>(sc, stack, ray.o, r2, rng, med, depth - 1, wo2, pdf2, c, hook);
+                nee_point_ad<N>(sc, ray.o, r2, rng, med, depth - 1, wo2, pdf2, c, hook);
                 rng = after;
             }
             if (!pass_b && k < kReplayEvents) ev[k] = e;
@@ -149,12 +149,12 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
         if (pass_b && k < kReplayEvents) {
             const float3 e = ev[k];
             adj.w = dot(gpix, e) * rp.inv_spp;
-            look_for_emitter_ad<N>(sc, stack, ray, false, rng, med, depth - 1, its1, pdf_nee, nullptr, nullptr,
+            look_for_emitter_ad<N>(sc, ray, false, rng, med, depth - 1, its1, pdf_nee, nullptr, nullptr,
                                    c, is_zero3(e, 0.f) ? nullptr : hook);
             acc = acc + e;
         } else {
             const Rng saved = rng;
-            DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, false, rng, med, depth - 1, its1, pdf_nee,
+            DV<N> att = look_for_emitter_ad<N>(sc, ray, false, rng, med, depth - 1, its1, pdf_nee,
                                                nullptr, nullptr, c);
             float3 e = zero;
             if (!att.is_zero() && (mode & MODE_VOLUME_MAIN))
@@ -165,7 +165,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
                 adj.w = dot(gpix, e) * rp.inv_spp;
                 ItsAD<N> its2;
                 float pdf2;
-                look_for_emitter_ad<N>(sc, stack, ray, false, rng, med, depth - 1, its2, pdf2, nullptr, nullptr,
+                look_for_emitter_ad<N>(sc, ray, false, rng, med, depth - 1, its2, pdf2, nullptr, nullptr,
                                        c, hook);
                 rng = after;
             }
@@ -181,7 +181,7 @@ DT_D bool replay_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
 }
 
 template <int N>
-DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack, bool pass_b, float3 gpix,
+DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, bool pass_b, float3 gpix,
                          AdjCtx &adj, Ctr &c, float3 *ev, AdjState<N> &st, const VertexIn &vin) {
     Rng &rng = st.rng;
     RayAD<N> &ray = st.ray;
@@ -210,12 +210,12 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         if (pass_b && k < kReplayEvents) {
             const float3 e = ev[k];
             adj.w = dot(gpix, e) * rp.inv_spp;
-            nee_surface_ad<N>(sc, stack, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c,
+            nee_surface_ad<N>(sc, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c,
                               is_zero3(e, 0.f) ? nullptr : hook, &b);
             acc = acc + e;
         } else {
             const Rng saved = rng;
-            DV<N> v = nee_surface_ad<N>(sc, stack, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c, nullptr, &b);
+            DV<N> v = nee_surface_ad<N>(sc, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c, nullptr, &b);
             float3 e = zero;
             if (!v.is_zero()) {
                 const DV<N> bv = bsdf_eval_ad<N>(b, its.wi, wo);
@@ -228,7 +228,7 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
                 adj.w = dot(gpix, e) * rp.inv_spp;
                 DV<N> wo2;
                 float pdf2;
-                nee_surface_ad<N>(sc, stack, its, fr, r2, rng, med, depth - 1, wo2, pdf2, c, hook, &b);
+                nee_surface_ad<N>(sc, its, fr, r2, rng, med, depth - 1, wo2, pdf2, c, hook, &b);
                 rng = after;
             }
             if (!pass_b && k < kReplayEvents) ev[k] = e;
@@ -245,19 +245,19 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         const int med1 = is_transition(sh) ? target_medium(sc, its.shape, its.ng, wo.val()) : med;
         ItsAD<N> its1;
         if (is_null) {
-            ray_intersect_ad<N>(sc, stack, ray, true, its1, c);
+            ray_intersect_ad<N>(sc, ray, true, its1, c);
         } else {
             P = cmul(P, bw.val());
             const int k = ne++;
             if (pass_b && k < kReplayEvents) {
                 const float3 e = ev[k];
                 adj.w = dot(gpix, e) * rp.inv_spp;
-                look_for_emitter_ad<N>(sc, stack, ray, true, rng, med1, depth - 1, its1, pdf_nee, nullptr, nullptr,
+                look_for_emitter_ad<N>(sc, ray, true, rng, med1, depth - 1, its1, pdf_nee, nullptr, nullptr,
                                        c, is_zero3(e, 0.f) ? nullptr : hook);
                 acc = acc + e;
             } else {
                 const Rng saved = rng;
-                DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, true, rng, med1, depth - 1, its1, pdf_nee,
+                DV<N> att = look_for_emitter_ad<N>(sc, ray, true, rng, med1, depth - 1, its1, pdf_nee,
                                                    nullptr, nullptr, c);
                 float3 e = zero;
                 if (!att.is_zero() && (mode & MODE_SURFACE_MAIN))
@@ -268,7 +268,7 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
                     adj.w = dot(gpix, e) * rp.inv_spp;
                     ItsAD<N> its2;
                     float pdf2;
-                    look_for_emitter_ad<N>(sc, stack, ray, true, rng, med1, depth - 1, its2, pdf2, nullptr,
+                    look_for_emitter_ad<N>(sc, ray, true, rng, med1, depth - 1, its2, pdf2, nullptr,
                                            nullptr, c, hook);
                     rng = after;
                 }
@@ -286,22 +286,22 @@ DT_D bool replay_surface(const DevScene &sc, const RenderParams &rp, int *stack,
 }
 
 template <int N>
-DT_D bool replay_step(const DevScene &sc, const RenderParams &rp, int *stack, bool pass_b, float3 total, float3 gpix,
+DT_D bool replay_step(const DevScene &sc, const RenderParams &rp, bool pass_b, float3 total, float3 gpix,
                       AdjCtx &adj, Ctr &c, float3 *ev, AdjState<N> &st) {
     VertexIn vin;
     const int kind = replay_decide<N>(sc, rp, pass_b, total, gpix, adj, c, st, vin);
-    if (kind == 1) return replay_volume<N>(sc, rp, stack, pass_b, gpix, adj, c, ev, st, vin);
-    if (kind == 2) return replay_surface<N>(sc, rp, stack, pass_b, gpix, adj, c, ev, st, vin);
+    if (kind == 1) return replay_volume<N>(sc, rp, pass_b, gpix, adj, c, ev, st, vin);
+    if (kind == 2) return replay_surface<N>(sc, rp, pass_b, gpix, adj, c, ev, st, vin);
     return false;
 }
 
 template <int N>
-DT_D float3 replay_path(const DevScene &sc, const RenderParams &rp, int *stack, long long g, bool pass_b, float3 total,
+DT_D float3 replay_path(const DevScene &sc, const RenderParams &rp, long long g, bool pass_b, float3 total,
                         float3 gpix, AdjCtx &adj, Ctr &c, float3 *ev) {
     AdjState<N> st;
-    bool alive = replay_start<N>(sc, rp, stack, g, st, c);
+    bool alive = replay_start<N>(sc, rp, g, st, c);
     while (alive && st.mode != 0) {
-        alive = replay_step<N>(sc, rp, stack, pass_b, total, gpix, adj, c, ev, st);
+        alive = replay_step<N>(sc, rp, pass_b, total, gpix, adj, c, ev, st);
         ++st.level;
     }
     return st.acc;
@@ -311,7 +311,7 @@ DT_D float3 replay_path(const DevScene &sc, const RenderParams &rp, int *stack, 
 // when the path and its pixel's dL/dI are non-zero. img_acc (optional) receives the image,
 // FP64 [npix][3]. Contains warp collectives: all 32 lanes of a warp must call it together.
 template <int N>
-DT_D void adjoint_one(const DevScene &sc, const RenderParams &rp, int *stack, long long gi, const float *dimg,
+DT_D void adjoint_one(const DevScene &sc, const RenderParams &rp, long long gi, const float *dimg,
                       float *grad, double *img_acc, Ctr &c, long long stride = 1) {
     // stride > 1 (autotuning samples): path gi*stride of the range
     const bool active = gi * stride < rp.path_count;
@@ -321,11 +321,11 @@ DT_D void adjoint_one(const DevScene &sc, const RenderParams &rp, int *stack, lo
     float3 ev[kReplayEvents];
     float3 total = mk(0.f, 0.f, 0.f);
     if (active) {
-        total = replay_path<N>(sc, rp, stack, g, false, total, total, adj, c, ev);
+        total = replay_path<N>(sc, rp, g, false, total, total, adj, c, ev);
         if (grad != nullptr && dimg != nullptr && !is_zero3(total, 0.f)) {
             const float3 gp = mk(__ldg(dimg + 3 * (size_t)pixel), __ldg(dimg + 3 * (size_t)pixel + 1),
                                  __ldg(dimg + 3 * (size_t)pixel + 2));
-            if (!is_zero3(gp, 0.f)) replay_path<N>(sc, rp, stack, g, true, total, gp, adj, c, ev);
+            if (!is_zero3(gp, 0.f)) replay_path<N>(sc, rp, g, true, total, gp, adj, c, ev);
         }
     }
     if (img_acc != nullptr) {
@@ -346,9 +346,8 @@ DT_D void adjoint_one(const DevScene &sc, const RenderParams &rp, int *stack, lo
 template <int N>
 __global__ void __launch_bounds__(kBlock) k_adjoint(DevScene sc, RenderParams rp, const float *dimg, float *grad,
                                                     double *img_acc, unsigned long long *ctr, long long stride = 1) {
-    __shared__ int s_stack[kStackDepth * kBlock];
     Ctr c;
-    adjoint_one<N>(sc, rp, s_stack + threadIdx.x, (long long)blockIdx.x * kBlock + threadIdx.x, dimg, grad, img_acc, c,
+    adjoint_one<N>(sc, rp, (long long)blockIdx.x * kBlock + threadIdx.x, dimg, grad, img_acc, c,
                    stride);
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
@@ -390,8 +389,6 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderPara
                                                       unsigned long long *cnt_s1, const float *dimg, float *grad,
                                                       const float3 *totals, float3 *evbuf, QueueEnds qx, bool pass_b,
                                                       unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     int kind = 0;
@@ -407,12 +404,12 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderPara
             gp = pixel_dldi(rp, dimg, g);
         }
         run = !pass_b || (!is_zero3(total, 0.f) && !is_zero3(gp, 0.f));
-        if (run && replay_start<N>(sc, rp, stack, g, st, c) && st.mode != 0) {
+        if (run && replay_start<N>(sc, rp, g, st, c) && st.mode != 0) {
             VertexIn vin;
             kind = replay_decide<N>(sc, rp, pass_b, total, gp, adj, c, st, vin);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
-                next = replay_surface<N>(sc, rp, stack, pass_b, gp, adj, c, evbuf + (size_t)gi * kReplayEvents, st, vin);
+                next = replay_surface<N>(sc, rp, pass_b, gp, adj, c, evbuf + (size_t)gi * kReplayEvents, st, vin);
                 ++st.level;
             }
         }
@@ -433,8 +430,6 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderPar
                                                        unsigned long long *cnt_s_next, const float *dimg, float *grad,
                                                        const float3 *totals, float3 *evbuf, QueueEnds qx, bool pass_b,
                                                        unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long nf = (long long)*cnt_in, n = nf + (kVolume ? 0 : (long long)cnt_in[qx.back]);
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
@@ -445,8 +440,8 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderPar
         const float3 total = pass_b ? totals[id] : zero, gp = pass_b ? pixel_dldi(rp, dimg, rp.path_begin + id) : zero;
         AdjCtx adj{grad, 0.f};
         float3 *ev = evbuf + (size_t)id * kReplayEvents;
-        const bool alive = kVolume ? replay_volume<N>(sc, rp, stack, pass_b, gp, adj, c, ev, st, vin)
-                                   : replay_surface<N>(sc, rp, stack, pass_b, gp, adj, c, ev, st, vin);
+        const bool alive = kVolume ? replay_volume<N>(sc, rp, pass_b, gp, adj, c, ev, st, vin)
+                                   : replay_surface<N>(sc, rp, pass_b, gp, adj, c, ev, st, vin);
         ++st.level;
         replay_next<N>(sc, rp, st, alive, pass_b, total, gp, adj, vins, id, qv_next, cnt_v_next, qs_next, cnt_s_next,
                        qx, c);
@@ -535,8 +530,6 @@ __global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N>
                                                        unsigned long long *cnt_v1, int *qs1,
                                                        unsigned long long *cnt_s1, const float3 *totals,
                                                        float3 *evbuf, QueueEnds qx, bool pass_b) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < bw.count;
     long long g = 0;
@@ -554,12 +547,12 @@ __global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N>
             gp = pixel_dldi(it.rp, it.dimg, g);
         }
         run = !pass_b || (it.grad && !is_zero3(total, 0.f) && !is_zero3(gp, 0.f));
-        if (run && replay_start<N>(it.sc, it.rp, stack, g, st, c) && st.mode != 0) {
+        if (run && replay_start<N>(it.sc, it.rp, g, st, c) && st.mode != 0) {
             VertexIn vin;
             kind = replay_decide<N>(it.sc, it.rp, pass_b, total, gp, adj, c, st, vin);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
-                next = replay_surface<N>(it.sc, it.rp, stack, pass_b, gp, adj, c, evbuf + (size_t)gi * kReplayEvents,
+                next = replay_surface<N>(it.sc, it.rp, pass_b, gp, adj, c, evbuf + (size_t)gi * kReplayEvents,
                                          st, vin);
                 ++st.level;
             }
@@ -577,8 +570,6 @@ __global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N
                                                         int *qv_next, unsigned long long *cnt_v_next, int *qs_next,
                                                         unsigned long long *cnt_s_next, const float3 *totals,
                                                         float3 *evbuf, QueueEnds qx, bool pass_b) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long nf = (long long)*cnt_in, n = nf + (kVolume ? 0 : (long long)cnt_in[qx.back]);
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
@@ -591,8 +582,8 @@ __global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N
         const float3 total = pass_b ? totals[id] : zero, gp = pass_b ? pixel_dldi(it.rp, it.dimg, g) : zero;
         AdjCtx adj{it.grad, 0.f};
         float3 *ev = evbuf + (size_t)id * kReplayEvents;
-        const bool alive = kVolume ? replay_volume<N>(it.sc, it.rp, stack, pass_b, gp, adj, c, ev, st, vin)
-                                   : replay_surface<N>(it.sc, it.rp, stack, pass_b, gp, adj, c, ev, st, vin);
+        const bool alive = kVolume ? replay_volume<N>(it.sc, it.rp, pass_b, gp, adj, c, ev, st, vin)
+                                   : replay_surface<N>(it.sc, it.rp, pass_b, gp, adj, c, ev, st, vin);
         ++st.level;
         replay_next<N>(it.sc, it.rp, st, alive, pass_b, total, gp, adj, vins, id, qv_next, cnt_v_next, qs_next,
                        cnt_s_next, qx, c);

@@ -1549,13 +1549,12 @@ int dtrt_render_adjoint(dtrt_scene *scene, const dtrt_render_options *opts, cons
 
 namespace dt {
 __global__ void __launch_bounds__(kBlock) k_trace(DevScene sc, const float *rays, int n, int *hits, float *t) {
-    __shared__ int s_stack[kStackDepth * kBlock];
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
     const float *r = rays + 8 * (size_t)i;
     Ctr c;
     float th;
-    const int prim = closest_hit(sc, s_stack + threadIdx.x, mk(r[0], r[1], r[2]), mk(r[4], r[5], r[6]), r[3], r[7], th, c);
+    const int prim = closest_hit(sc, mk(r[0], r[1], r[2]), mk(r[4], r[5], r[6]), r[3], r[7], th, c);
     hits[2 * i] = prim;
     hits[2 * i + 1] = prim >= 0 ? sc.tris[prim].w : -1;
     t[i] = prim >= 0 ? th : INFINITY;

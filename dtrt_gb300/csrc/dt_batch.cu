@@ -33,12 +33,10 @@ namespace dt {
 __global__ void __launch_bounds__(kBlock) k_batch(const BatchItemDev *items, const long long *cbeg, const int *order,
                                                   int n, long long total_chunks, int chunk, long long sample_stride,
                                                   unsigned long long *next) {
-    __shared__ int s_stack[kStackDepth * kBlock];
     // the current item's scene and parameters, one copy per warp: the path code reads them
     // at every step, and shared memory serves those uniform reads like kernel parameters do
     __shared__ DevScene s_sc[kBlock / 32];
     __shared__ RenderParams s_rp[kBlock / 32];
-    int *stack = s_stack + threadIdx.x;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int cur = -1;
@@ -75,7 +73,7 @@ __global__ void __launch_bounds__(kBlock) k_batch(const BatchItemDev *items, con
         const long long base = ((long long)c - cbeg[lo]) * chunk;
         Ctr ctr;
         for (int k = lane; k < chunk; k += 32)  // sample_stride > 1 (tuning): every stride-th path
-            adjoint_one<0>(s_sc[warp], s_rp[warp], stack, base + k, dimg, grad, img_acc, ctr, sample_stride);
+            adjoint_one<0>(s_sc[warp], s_rp[warp], base + k, dimg, grad, img_acc, ctr, sample_stride);
     }
 }
 

@@ -60,14 +60,18 @@ DT_D float3 f3(float4 a) { return mk(a.x, a.y, a.z); }
 // ------------------------------------------------------------------ BVH closest hit
 // Replaces rtcIntersect1 (src/scene.cpp:172 and its other call sites): closest
 // triangle with t in [tmin, tmax]. Two-child node tests against the current best
-// distance; the per-thread stack lives in shared memory (stride kBlock).
+// distance. The stack is local memory: its few entries in use stay in L1, and the L1 that
+// a stack of 48 entries per thread in shared memory took (24 KB a block) goes to nodes,
+// voxels and path states (C2 forward 107.2 -> 96.5 ms, C3 66.9 -> 63.7, primal mesh 2.27 ->
+// 2.00; 24 entries in shared memory 101.2, 66.8, 2.13).
 constexpr int kStackExit = (int)0x80000000;
 // Hard bound on null-interface crossings of one transmittance / emitter-lookup chain
 // (the reference bounds them by max_interactions, which can be -1 = unbounded).
 constexpr int kMaxInteractions = 4096;
 
-DT_HEAVY int closest_hit(const DevScene &sc, int *stack, float3 o, float3 d, float tmin, float tmax, float &t_hit,
+DT_HEAVY int closest_hit(const DevScene &sc, float3 o, float3 d, float tmin, float tmax, float &t_hit,
                      Ctr &c) {
+    int stack[kStackDepth];
     c.rays++;
     const float3 inv = mk(1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x)),
                           1.0f / (fabsf(d.y) > 1e-30f ? d.y : copysignf(1e-30f, d.y)),
@@ -103,7 +107,7 @@ DT_HEAVY int closest_hit(const DevScene &sc, int *stack, float3 o, float3 d, flo
                     code = kStackExit;
                     break;
                 }
-                stack[sp * kBlock] = farc;
+                stack[sp] = farc;
                 ++sp;
                 code = nearc;
             } else if (hl) {
@@ -111,7 +115,7 @@ DT_HEAVY int closest_hit(const DevScene &sc, int *stack, float3 o, float3 d, flo
             } else if (hr) {
                 code = ch.y;
             } else {
-                code = sp > 0 ? stack[(--sp) * kBlock] : kStackExit;
+                code = sp > 0 ? stack[--sp] : kStackExit;
             }
         }
         if (code == kStackExit) break;
@@ -139,7 +143,7 @@ DT_HEAVY int closest_hit(const DevScene &sc, int *stack, float3 o, float3 d, flo
                 best = __float_as_int(A.w);
             }
         }
-        code = sp > 0 ? stack[(--sp) * kBlock] : kStackExit;
+        code = sp > 0 ? stack[--sp] : kStackExit;
     }
     t_hit = best_t;
     return best;
@@ -1194,9 +1198,9 @@ DT_HEAVY Df<N> medium_transmittance_ad(const DevScene &sc, const DevMedium &m, c
 }
 
 // ------------------------------------------------------------------ scene queries, scene.cpp
-DT_D bool ray_intersect(const DevScene &sc, int *stack, float3 o, float3 d, bool on_surface, Its &its, Ctr &c) {
+DT_D bool ray_intersect(const DevScene &sc, float3 o, float3 d, bool on_surface, Its &its, Ctr &c) {
     float th;
-    const int prim = closest_hit(sc, stack, o, d, on_surface ? kShadowEps : 0.f, INFINITY, th, c);
+    const int prim = closest_hit(sc, o, d, on_surface ? kShadowEps : 0.f, INFINITY, th, c);
     if (prim < 0) {
         its.shape = -1;
         its.t = INFINITY;
@@ -1207,10 +1211,10 @@ DT_D bool ray_intersect(const DevScene &sc, int *stack, float3 o, float3 d, bool
 }
 
 template <int N>
-DT_D bool ray_intersect_ad(const DevScene &sc, int *stack, const RayAD<N> &ray, bool on_surface, ItsAD<N> &its,
+DT_D bool ray_intersect_ad(const DevScene &sc, const RayAD<N> &ray, bool on_surface, ItsAD<N> &its,
                            Ctr &c) {
     float th;
-    const int prim = closest_hit(sc, stack, ray.o.val(), ray.d.val(), on_surface ? kShadowEps : 0.f, INFINITY, th, c);
+    const int prim = closest_hit(sc, ray.o.val(), ray.d.val(), on_surface ? kShadowEps : 0.f, INFINITY, th, c);
     if (prim < 0) {
         its.shape = -1;
         its.t = Df<N>(INFINITY);
@@ -1221,7 +1225,7 @@ DT_D bool ray_intersect_ad(const DevScene &sc, int *stack, const RayAD<N> &ray, 
 }
 
 // scene.cpp:177-237
-DT_HEAVY float eval_transmittance(const DevScene &sc, int *stack, float3 o, float3 d, bool on_surface, int med,
+DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool on_surface, int med,
                               float remaining, Rng &rng, int max_inter, Ctr &c) {
     float tmin = on_surface ? kShadowEps : 0.f;
     float tfar = (1.f - kShadowEps) * remaining;
@@ -1230,7 +1234,7 @@ DT_HEAVY float eval_transmittance(const DevScene &sc, int *stack, float3 o, floa
     while (remaining > 0.f) {
         if (inter >= kMaxInteractions) return 0.f;  // also bounds max_inter == -1
         float tmax = remaining, th;
-        const int prim = closest_hit(sc, stack, o, d, tmin, tfar, th, c);
+        const int prim = closest_hit(sc, o, d, tmin, tfar, th, c);
         Its its;
         if (prim >= 0) {
             const int shape = __ldg(sc.tris + prim).w;
@@ -1252,11 +1256,11 @@ DT_HEAVY float eval_transmittance(const DevScene &sc, int *stack, float3 o, floa
 }
 
 // scene.cpp:617-701
-DT_HEAVY float3 look_for_emitter(const DevScene &sc, int *stack, float3 o, float3 d, bool on_surface, Rng &rng, int med,
+DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on_surface, Rng &rng, int med,
                              int max_inter, Its &its, float &pdf_nee, Ctr &c) {
     float tmin = on_surface ? kShadowEps : 0.f, th;
     const float3 scatter = o;
-    int prim = closest_hit(sc, stack, o, d, tmin, INFINITY, th, c);
+    int prim = closest_hit(sc, o, d, tmin, INFINITY, th, c);
     const float3 zero = mk(0.f, 0.f, 0.f);
     if (prim < 0) {
         its.shape = -1;
@@ -1278,7 +1282,7 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, int *stack, float3 o, float
             }
             if (inter == max_inter || sc.bsdfs[s.bsdf_id].type != BSDF_NULL) break;
             o1 = o1 + d * n1.t;
-            p1 = closest_hit(sc, stack, o1, d, kShadowEps, INFINITY, th, c);
+            p1 = closest_hit(sc, o1, d, kShadowEps, INFINITY, th, c);
             if (p1 < 0) break;
         }
         if (!emitter) return zero;
@@ -1300,7 +1304,7 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, int *stack, float3 o, float
         if (is_transition(s)) med = dot(ni.ng, d) > 0.f ? s.med_ext : s.med_int;
         o = o + d * tmax;
         tmin = kShadowEps;
-        prim = closest_hit(sc, stack, o, d, tmin, INFINITY, th, c);
+        prim = closest_hit(sc, o, d, tmin, INFINITY, th, c);
         if (prim < 0) return zero;
     }
     return zero;
@@ -1323,12 +1327,12 @@ struct Chain {
 
 // scene.cpp:703-793
 template <int N, int G>
-DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray, bool on_surface, Rng &rng, int med,
+DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, RayAD<G> ray, bool on_surface, Rng &rng, int med,
                                int max_inter, ItsAD<G> &its, float &pdf_nee, int *far_shape, float *far_t, Ctr &c,
                                const AdjCtx *adj = nullptr) {
     float tmin = on_surface ? kShadowEps : 0.f, th;
     const float3 scatter = ray.o.val();
-    int prim = closest_hit(sc, stack, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
+    int prim = closest_hit(sc, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
     if (prim < 0) {
         its.shape = -1;
         its.t = Df<G>(INFINITY);
@@ -1358,7 +1362,7 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray,
             }
             if (inter == max_inter || sc.bsdfs[s.bsdf_id].type != BSDF_NULL) break;
             r1.o = r1.o + r1.d * n1.t;
-            p1 = closest_hit(sc, stack, r1.o.val(), r1.d.val(), kShadowEps, INFINITY, th, c);
+            p1 = closest_hit(sc, r1.o.val(), r1.d.val(), kShadowEps, INFINITY, th, c);
             if (p1 < 0) break;
         }
         if (!emitter) return DV<N>();
@@ -1387,14 +1391,14 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, int *stack, RayAD<G> ray,
         ray.o = ray.o + ray.d * tmax;
         tmin = kShadowEps;
         prim = chain.has(inter) ? chain.get(inter)
-                                : closest_hit(sc, stack, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
+                                : closest_hit(sc, ray.o.val(), ray.d.val(), tmin, INFINITY, th, c);
         if (prim < 0) return DV<N>();
     }
     return DV<N>();
 }
 
 // scene.cpp:399-426 (from a point in a medium; wo in world space)
-DT_HEAVY float3 nee_point(const DevScene &sc, int *stack, float3 p, const float rnd[4], Rng &rng, int med, int max_inter,
+DT_HEAVY float3 nee_point(const DevScene &sc, float3 p, const float rnd[4], Rng &rng, int med, int max_inter,
                       float3 &wo, float &pdf, Ctr &c) {
     float3 lp, ln;
     const int l = sample_light(sc, rnd, lp, ln, pdf);
@@ -1404,7 +1408,7 @@ DT_HEAVY float3 nee_point(const DevScene &sc, int *stack, float3 p, const float 
     if (dot(dir, ln) < 0.f && pdf != 0.f) {
         const float dist = length(dir);
         dir = dir / dist;
-        const float tr = eval_transmittance(sc, stack, p, dir, false, med, dist, rng, max_inter, c);
+        const float tr = eval_transmittance(sc, p, dir, false, med, dist, rng, max_inter, c);
         if (tr != 0.f) {
             pdf *= dist * dist / dot(ln, -dir);
             wo = dir;
@@ -1415,7 +1419,7 @@ DT_HEAVY float3 nee_point(const DevScene &sc, int *stack, float3 p, const float 
 }
 
 // scene.cpp:456-491 (from a surface; wo in the local shading frame)
-DT_HEAVY float3 nee_surface(const DevScene &sc, int *stack, const Its &its, const float rnd[4], Rng &rng, int med,
+DT_HEAVY float3 nee_surface(const DevScene &sc, const Its &its, const float rnd[4], Rng &rng, int med,
                         int max_inter, float3 &wo, float &pdf, bool flag, Ctr &c) {
     float3 lp, ln;
     const int l = sample_light(sc, rnd, lp, ln, pdf);
@@ -1432,7 +1436,7 @@ DT_HEAVY float3 nee_surface(const DevScene &sc, int *stack, const Its &its, cons
         wo = its.to_local(dir);
         if (flag && signum(its.wi.z) != signum(wo.z)) --max_inter;
         if (max_inter >= 0) {
-            const float tr = eval_transmittance(sc, stack, its.p, dir, true, med, dist, rng, max_inter, c);
+            const float tr = eval_transmittance(sc, its.p, dir, true, med, dist, rng, max_inter, c);
             if (tr != 0.f) {
                 pdf *= dist * dist / dot(ln, -dir);
                 return le_normal(sc.emitters[l], ln, -dir) * (tr / pdf);
@@ -1444,7 +1448,7 @@ DT_HEAVY float3 nee_surface(const DevScene &sc, int *stack, const Its &its, cons
 
 // scene.cpp:428-454 (AD, from a point; the light sample carries no derivative)
 template <int N, int G>
-DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<G> &p, const float rnd[4], Rng &rng, int med,
+DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, const DV<G> &p, const float rnd[4], Rng &rng, int med,
                         int max_inter, DV<G> &wo, float &pdf, Ctr &c, const AdjCtx *adj = nullptr) {
     float3 lp, ln;
     float pdf0;
@@ -1459,7 +1463,7 @@ DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<G> &p, cons
         int far_shape = -1;
         float far_t = 0.f;
         RayAD<G> r{p, DV<G>(dir)};
-        DV<N> v = look_for_emitter_ad<N>(sc, stack, r, false, rng, med, max_inter, near_its, pdf, &far_shape, &far_t, c,
+        DV<N> v = look_for_emitter_ad<N>(sc, r, false, rng, med, max_inter, near_its, pdf, &far_shape, &far_t, c,
                                          adj);
         if (!v.is_zero() && pdf > kEps && far_shape == sc.emitters[l].shape_id && fabsf(far_t - dist) < kShadowEps) {
             wo = DV<G>(dir);
@@ -1475,7 +1479,7 @@ DT_HEAVY DV<N> nee_point_ad(const DevScene &sc, int *stack, const DV<G> &p, cons
 // traced: the contribution is zero either way (a near-specular dielectric is zero for almost
 // every light sample). Random numbers such a chain would have drawn are not drawn.
 template <int N, int G>
-DT_HEAVY DV<N> nee_surface_ad(const DevScene &sc, int *stack, const ItsAD<G> &its, const FrameAD<G> &fr, const float rnd[4],
+DT_HEAVY DV<N> nee_surface_ad(const DevScene &sc, const ItsAD<G> &its, const FrameAD<G> &fr, const float rnd[4],
                           Rng &rng, int med, int max_inter, DV<G> &wo, float &pdf, Ctr &c, const AdjCtx *adj = nullptr,
                           const DevBsdf *bsdf = nullptr) {
     float3 lp, ln;
@@ -1497,7 +1501,7 @@ DT_HEAVY DV<N> nee_surface_ad(const DevScene &sc, int *stack, const ItsAD<G> &it
         int far_shape = -1;
         float far_t = 0.f;
         RayAD<G> r{its.p, DV<G>(dir)};
-        DV<N> v = look_for_emitter_ad<N>(sc, stack, r, true, rng, med, max_inter, near_its, pdf, &far_shape, &far_t, c,
+        DV<N> v = look_for_emitter_ad<N>(sc, r, true, rng, med, max_inter, near_its, pdf, &far_shape, &far_t, c,
                                          adj);
         if (!v.is_zero() && pdf > kEps && far_shape == sc.emitters[l].shape_id && fabsf(far_t - dist) < kShadowEps) {
             wo = fr.to_local(dir);
@@ -1519,7 +1523,7 @@ struct alignas(16) LiState {
 };
 
 // First hit of the path; false when the loop would not run at all.
-DT_D bool li_start(const DevScene &sc, int *stack, LiState &s, float3 o, float3 d, int max_depth, int med,
+DT_D bool li_start(const DevScene &sc, LiState &s, float3 o, float3 d, int max_depth, int med,
                    bool inc_emission, Ctr &c, bool on_surface = true) {
     s.its = Its();
     s.o = o;
@@ -1530,12 +1534,12 @@ DT_D bool li_start(const DevScene &sc, int *stack, LiState &s, float3 o, float3 
     s.depth = 0;
     s.max_depth = max_depth;
     s.inc_emission = inc_emission ? 1 : 0;
-    ray_intersect(sc, stack, o, d, on_surface, s.its, c);
+    ray_intersect(sc, o, d, on_surface, s.its, c);
     return s.depth <= s.max_depth;
 }
 
 // One vertex (one iteration of the loop at s.depth): false when the path ends.
-DT_D bool li_step(const DevScene &sc, int *stack, LiState &s, Ctr &c) {
+DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     Rng &rng = s.rng;
     Its &its = s.its;
     float3 &o = s.o, &d = s.d, &ret = s.ret, &thr = s.thr;
@@ -1553,7 +1557,7 @@ DT_D bool li_step(const DevScene &sc, int *stack, LiState &s, Ctr &c) {
         const DevPhase &ph = sc.phases[sc.media[med].phase_id];
         float3 wo;
         float pdf_nee;
-        const float3 v = nee_point(sc, stack, o, r2, rng, med, max_inter, wo, pdf_nee, c);
+        const float3 v = nee_point(sc, o, r2, rng, med, max_inter, wo, pdf_nee, c);
         if (!is_zero3(v)) {
             const float pv = phase_eval(ph, -d, wo);
             if (pv > kEps) ret += cmul(thr, v) * (mis_weight(pdf_nee, pv) * pv);
@@ -1562,7 +1566,7 @@ DT_D bool li_step(const DevScene &sc, int *stack, LiState &s, Ctr &c) {
         if (pv < kEps) return false;
         thr = thr * pv;
         d = wo;
-        const float3 att = look_for_emitter(sc, stack, o, d, false, rng, med, max_inter, its, pdf_nee, c);
+        const float3 att = look_for_emitter(sc, o, d, false, rng, med, max_inter, its, pdf_nee, c);
         if (!is_zero3(att)) ret += cmul(thr, att) * mis_weight(phase_eval(ph, -d, wo), pdf_nee);
         s.inc_emission = 0;
     } else {
@@ -1574,7 +1578,7 @@ DT_D bool li_step(const DevScene &sc, int *stack, LiState &s, Ctr &c) {
         float3 wo;
         float pdf_nee;
         if (b.type != BSDF_NULL) {
-            const float3 v = nee_surface(sc, stack, its, r2, rng, med, max_inter, wo, pdf_nee, false, c);
+            const float3 v = nee_surface(sc, its, r2, rng, med, max_inter, wo, pdf_nee, false, c);
             if (!is_zero3(v))
                 ret += cmul(cmul(thr, v), bsdf_eval(b, its.wi, wo)) * mis_weight(pdf_nee, bsdf_pdf(b, its.wi, wo));
         }
@@ -1586,9 +1590,9 @@ DT_D bool li_step(const DevScene &sc, int *stack, LiState &s, Ctr &c) {
         d = wo;
         if (is_transition(sh)) med = dot(wo, its.ng) > 0.f ? sh.med_ext : sh.med_int;
         if (b.type == BSDF_NULL) {
-            ray_intersect(sc, stack, o, d, true, its, c);
+            ray_intersect(sc, o, d, true, its, c);
         } else {
-            const float3 att = look_for_emitter(sc, stack, o, d, true, rng, med, max_inter, its, pdf_nee, c);
+            const float3 att = look_for_emitter(sc, o, d, true, rng, med, max_inter, its, pdf_nee, c);
             thr = cmul(thr, bw);
             if (!is_zero3(att, 1e-12f)) ret += cmul(thr, att) * mis_weight(bpdf, pdf_nee);
             s.inc_emission = 0;
@@ -1598,12 +1602,12 @@ DT_D bool li_step(const DevScene &sc, int *stack, LiState &s, Ctr &c) {
     return s.depth <= max_depth;
 }
 
-DT_D float3 li_path(const DevScene &sc, int *stack, Rng &rng, float3 o, float3 d, int max_depth, int med,
+DT_D float3 li_path(const DevScene &sc, Rng &rng, float3 o, float3 d, int max_depth, int med,
                     bool inc_emission, Ctr &c, bool on_surface = true) {
     LiState s;
     s.rng = rng;
-    bool alive = li_start(sc, stack, s, o, d, max_depth, med, inc_emission, c, on_surface);
-    while (alive) alive = li_step(sc, stack, s, c);
+    bool alive = li_start(sc, s, o, d, max_depth, med, inc_emission, c, on_surface);
+    while (alive) alive = li_step(sc, s, c);
     rng = s.rng;
     return s.ret;
 }

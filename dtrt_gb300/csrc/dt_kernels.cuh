@@ -189,7 +189,7 @@ struct alignas(16) CamState {  // 16-byte aligned: whole-state copies compile to
 
 // Path start: jittered primary ray and first intersection. False: nothing was hit.
 template <int N, int G>
-DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st, Ctr &c) {
+DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, long long g, CamState<N, G> &st, Ctr &c) {
     const int pixel = (int)(g / rp.spp);
     const int ix = rp.crop_x + pixel % rp.out_w, iy = rp.crop_y + pixel / rp.out_w;
     st.rng.init(rp.seed, (uint64_t)g);
@@ -206,7 +206,7 @@ DT_D bool camera_start(const DevScene &sc, const RenderParams &rp, int *stack, l
     st.level = 0;
     st.P = DV<N>(mk(1.f, 1.f, 1.f));
     st.acc = DV<N>();
-    return ray_intersect_ad<G>(sc, stack, st.ray, false, st.its, c);
+    return ray_intersect_ad<G>(sc, st.ray, false, st.its, c);
 }
 
 // Random numbers of a vertex drawn before its branch: what the volume and interface halves
@@ -233,7 +233,7 @@ DT_D int camera_decide(const DevScene &sc, CamState<N, G> &st, VertexIn &vin, Ct
 // Volume vertex (volpathAD.cpp:164-305): NEE, volume edge record, phase sampling and the
 // emitter lookup along the new direction. Returns whether the path continues.
 template <int N, int G>
-DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
+DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, long long g, CamState<N, G> &st,
                         const VertexIn &vin, const Queue &qe, Ctr &c) {
     Rng &rng = st.rng;
     RayAD<G> &ray = st.ray;
@@ -252,7 +252,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
     DV<G> wo;
     float pdf_nee;
     if (mode & MODE_VOLUME_MAIN) {
-        DV<N> v = nee_point_ad<N>(sc, stack, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c);
+        DV<N> v = nee_point_ad<N>(sc, ray.o, r2, rng, med, depth - 1, wo, pdf_nee, c);
         if (!v.is_zero()) {
             Df<N> pv = phase_eval_ad<N>(ph, -ray.d, wo);
             if (pv.v > kEps) acc += cmul(P, v) * (pv * mis_weight(pdf_nee, phase_eval(ph, -dir_in, wo.val())));
@@ -282,7 +282,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
         P = P * pvs;
         ray.d = wo;
         ItsAD<G> its1;
-        DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, false, rng, med, depth - 1, its1, pdf_nee, nullptr,
+        DV<N> att = look_for_emitter_ad<N>(sc, ray, false, rng, med, depth - 1, its1, pdf_nee, nullptr,
                                            nullptr, c);
         if (!att.is_zero() && (mode & MODE_VOLUME_MAIN))
             acc += cmul(P, att) * mis_weight(phase_eval(ph, -wo.val(), wo.val()), pdf_nee);
@@ -298,7 +298,7 @@ DT_D bool camera_volume(const DevScene &sc, const RenderParams &rp, int *stack, 
 // BSDF sampling and the emitter lookup (or null-interface crossing). Returns whether the
 // path continues.
 template <int N, int G>
-DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
+DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, long long g, CamState<N, G> &st,
                          const VertexIn &vin, const Queue &qe, const Queue &ql, Ctr &c) {
     Rng &rng = st.rng;
     RayAD<G> &ray = st.ray;
@@ -368,7 +368,7 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
     DV<G> wo;
     float pdf_nee;
     if (!is_null && (mode & MODE_SURFACE_MAIN)) {
-        DV<N> v = nee_surface_ad<N>(sc, stack, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c, nullptr, &b);
+        DV<N> v = nee_surface_ad<N>(sc, its, fr, r2, rng, med, depth - 1, wo, pdf_nee, c, nullptr, &b);
         if (!v.is_zero()) {
             const DV<N> bv = bsdf_eval_ad<N>(b, its.wi, wo);
             const float bp = bsdf_pdf(b, its0.wi, wo.val());
@@ -385,9 +385,9 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
         const int med1 = is_transition(sh) ? target_medium(sc, its.shape, its.ng, wo.val()) : med;
         ItsAD<G> its1;
         if (is_null) {
-            ray_intersect_ad<G>(sc, stack, ray, true, its1, c);
+            ray_intersect_ad<G>(sc, ray, true, its1, c);
         } else {
-            DV<N> att = look_for_emitter_ad<N>(sc, stack, ray, true, rng, med1, depth - 1, its1, pdf_nee,
+            DV<N> att = look_for_emitter_ad<N>(sc, ray, true, rng, med1, depth - 1, its1, pdf_nee,
                                                nullptr, nullptr, c);
             P = cmul(P, bw);
             if (!att.is_zero() && (mode & MODE_SURFACE_MAIN)) acc += cmul(P, att) * mis_weight(bpdf, pdf_nee);
@@ -404,12 +404,12 @@ DT_D bool camera_surface(const DevScene &sc, const RenderParams &rp, int *stack,
 // One vertex of camera path g. Returns whether the path continues; st.level is advanced
 // by the caller.
 template <int N, int G>
-DT_D bool camera_step(const DevScene &sc, const RenderParams &rp, int *stack, long long g, CamState<N, G> &st,
+DT_D bool camera_step(const DevScene &sc, const RenderParams &rp, long long g, CamState<N, G> &st,
                       const Queue &qe, const Queue &ql, Ctr &c) {
     VertexIn vin;
     const int kind = camera_decide<N, G>(sc, st, vin, c);
-    if (kind == 1) return camera_volume<N, G>(sc, rp, stack, g, st, vin, qe, c);
-    if (kind == 2) return camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
+    if (kind == 1) return camera_volume<N, G>(sc, rp, g, st, vin, qe, c);
+    if (kind == 2) return camera_surface<N, G>(sc, rp, g, st, vin, qe, ql, c);
     return false;
 }
 
@@ -448,8 +448,6 @@ DT_D void accumulate_path(const RenderParams &rp, bool active, int pixel, const 
 template <int N, int G>
 __global__ void __launch_bounds__(kBlock) k_camera(DevScene sc, RenderParams rp, Queue qe, Queue ql, double *acc1,
                                                    unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < rp.path_count;
     const long long g = rp.path_begin + (active ? gi : 0);
@@ -457,9 +455,9 @@ __global__ void __launch_bounds__(kBlock) k_camera(DevScene sc, RenderParams rp,
     DV<N> acc;
     if (active) {
         CamState<N, G> st;
-        bool alive = camera_start<N, G>(sc, rp, stack, g, st, c);
+        bool alive = camera_start<N, G>(sc, rp, g, st, c);
         while (alive && st.mode != 0) {
-            alive = camera_step<N, G>(sc, rp, stack, g, st, qe, ql, c);
+            alive = camera_step<N, G>(sc, rp, g, st, qe, ql, c);
             ++st.level;
         }
         acc = st.acc * rp.inv_spp;
@@ -470,6 +468,11 @@ __global__ void __launch_bounds__(kBlock) k_camera(DevScene sc, RenderParams rp,
 
 // AUTO schedule: the wavefront from this many camera paths per render batch
 constexpr long long kWavefrontMinPaths = 1 << 16;
+// Blocks per SM of the camera kernels without ray derivatives: they wait on L1 and L2, so
+// warps count more than spills, up to the point where the slots no longer fit (C1, nder 3:
+// 14.4 / 14.1 / 13.5 / 13.9 ms at 3 / 4 / 5 / 6 blocks; C3, nder 8: 71.0 / 68.0 / 68.3 / 68.8).
+template <int N>
+constexpr int kCamBlocks = N > 4 ? 4 : 5;
 
 // Wavefront schedule: paths that continue are compacted into a queue of path indices
 // after every vertex, so each launch runs one vertex of live paths only (a warp no longer
@@ -557,13 +560,11 @@ DT_D void store_state(CamState<N, G> *states, int id, const CamState<N, G> &st, 
 // sampling. An interface vertex (every path from a camera outside media) runs here too and
 // the path goes on to level 1's distance sampling; a volume vertex is queued for level 0.
 template <int N, int G>
-__global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
+__global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                       VertexIn *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, unsigned long long *cnt_s1_back,
                                                       long long cap, Queue qe, Queue ql, unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     int kind = 0;
@@ -571,12 +572,12 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene s
     bool next = false;
     if (gi < rp.path_count) {
         const long long g = rp.path_begin + gi;
-        if (camera_start<N, G>(sc, rp, stack, g, st, c) && st.mode != 0) {
+        if (camera_start<N, G>(sc, rp, g, st, c) && st.mode != 0) {
             VertexIn vin;
             kind = camera_decide<N, G>(sc, st, vin, c);
             if (kind == 1) vins[gi] = vin;
             if (kind == 2) {
-                next = camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
+                next = camera_surface<N, G>(sc, rp, g, st, vin, qe, ql, c);
                 ++st.level;
             }
         }
@@ -590,7 +591,7 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_start(DevScene s
 // Vertex level L, one launch per kind: the volume (kVolume) or interface vertices of the
 // level; a continuing path then runs level L+1's distance sampling (camera_next).
 template <int N, int G, bool kVolume>
-__global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
+__global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                        VertexIn *vins, const int *q_in,
                                                        const unsigned long long *cnt_in,
                                                        const unsigned long long *cnt_in_back, int *qv_next,
@@ -598,8 +599,6 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_vertex(DevScene 
                                                        unsigned long long *cnt_s_next,
                                                        unsigned long long *cnt_s_next_back, long long cap, Queue qe,
                                                        Queue ql, unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long nf = (long long)*cnt_in, n = nf + (cnt_in_back ? (long long)*cnt_in_back : 0);
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
@@ -622,8 +621,8 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? 4 : 1) k_cam_vertex(DevScene 
         }
         const VertexIn vin = vins[id];
         const long long g = rp.path_begin + id;
-        const bool alive = kVolume ? camera_volume<N, G>(sc, rp, stack, g, st, vin, qe, c)
-                                   : camera_surface<N, G>(sc, rp, stack, g, st, vin, qe, ql, c);
+        const bool alive = kVolume ? camera_volume<N, G>(sc, rp, g, st, vin, qe, c)
+                                   : camera_surface<N, G>(sc, rp, g, st, vin, qe, ql, c);
         ++st.level;
         const int nk = camera_next<N, G>(sc, st, alive, vins, id, qv_next, cnt_v_next, qs_next, cnt_s_next,
                                       cnt_s_next_back, cap, c);
@@ -785,8 +784,6 @@ DT_D float3 edge_subpath_dir(const EdgePoint &ep, int sgn) {
 template <int N>
 __global__ void __launch_bounds__(kBlock, 8) k_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                  long long rec_count, Queue qli, unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     uint32_t nsamples = 0;
@@ -831,7 +828,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_edge(DevScene sc, RenderParams rp
         }
         if (ok) {
             const float tr =
-                eval_transmittance(sc, stack, tof(x0), w1f, r.kind == 0, med1, (float)ep.dist, rng, r.depth, c);
+                eval_transmittance(sc, tof(x0), w1f, r.kind == 0, med1, (float)ep.dist, rng, r.depth, c);
             ok = tr > kEps;
         }
         if (ok) {
@@ -901,8 +898,6 @@ template <int N>
 __global__ void __launch_bounds__(kBlock, 6) k_li(DevScene sc, RenderParams rp, Queue qli, long long begin, long long count,
                                                double *acc1, double *acc2, const int *perm,
                                                unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     // perm: the pairs in sorted order (a pair's two slots stay in adjacent lanes), or queue order
     const long long slot = perm && gi < count ? 2LL * __ldg(perm + (gi >> 1)) + (gi & 1) : begin + gi;
@@ -913,7 +908,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_li(DevScene sc, RenderParams rp, 
         Rng rng;
         rng.init(rp.seed, t.key);
         n = 1;
-        const float3 L = li_path(sc, stack, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
+        const float3 L = li_path(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
         if (!is_zero3(L, 0.f)) {
             const float3 wl = cmul(f3(t.w), L);
             const bool prim = (t.flags & 2) != 0;
@@ -935,8 +930,6 @@ __global__ void __launch_bounds__(kBlock, 6) k_li(DevScene sc, RenderParams rp, 
 template <int N>
 __global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Queue ql, long long count, double *acc1,
                                                  unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     if (gi < count) {
@@ -959,7 +952,7 @@ __global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Q
             float r4[4];
             r4[0] = rng.next1(); r4[1] = rng.next1(); r4[2] = rng.next1(); r4[3] = rng.next1();
             if (b.type == BSDF_NULL) {
-                att = nee_surface(sc, stack, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, true, c);
+                att = nee_surface(sc, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, true, c);
                 if (!is_zero3(att)) {
                     wo = its0.to_world(wo);
                     pv = phase_eval(ph, -rd, wo);
@@ -974,14 +967,14 @@ __global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Q
                     }
                     if (md1 > 0) {
                         const int med1 = is_transition(sh) ? target_medium(sc, r.shape, its0.ng, wo) : med;
-                        att = look_for_emitter(sc, stack, its0.p, wo, true, rng, med1, md1, its1, pdf_nee, c);
+                        att = look_for_emitter(sc, its0.p, wo, true, rng, med1, md1, its1, pdf_nee, c);
                         if (!is_zero3(att)) lins += att * (pv * mis_weight(phase_eval(ph, -rd, wo), pdf_nee));
-                        lins += li_path(sc, stack, rng, its0.p, wo, md1, med1, false, c) * pv;
+                        lins += li_path(sc, rng, its0.p, wo, md1, med1, false, c) * pv;
                     }
                 }
                 continue;
             }
-            att = nee_surface(sc, stack, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, false, c);
+            att = nee_surface(sc, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, false, c);
             if (!is_zero3(att)) {
                 wo = its0.to_world(wo);
                 if (dot(wo, n) < -kEps) {
@@ -993,9 +986,9 @@ __global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Q
             if ((pv = phase_sample(ph, -rd, u, v, wo)) > kEps) {
                 const float wdn = dot(wo, n);
                 if (wdn < -kEps) {
-                    att = look_for_emitter(sc, stack, its0.p, wo, true, rng, med, max_depth - 1, its1, pdf_nee, c);
+                    att = look_for_emitter(sc, its0.p, wo, true, rng, med, max_depth - 1, its1, pdf_nee, c);
                     if (!is_zero3(att)) lins += att * (pv * mis_weight(phase_eval(ph, -rd, wo), pdf_nee));
-                    lins += li_path(sc, stack, rng, its0.p, wo, max_depth - 1, med, false, c) * pv;
+                    lins += li_path(sc, rng, its0.p, wo, max_depth - 1, med, false, c) * pv;
                 } else if (wdn > kEps) {
                     if (sh.light_id >= 0) lins += le(sc, its0, -wo) * pv;
                     if (max_depth > 1) {
@@ -1003,7 +996,7 @@ __global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Q
                         its2.wi = its2.to_local(-wo);
                         float r4b[4];
                         r4b[0] = rng.next1(); r4b[1] = rng.next1(); r4b[2] = rng.next1(); r4b[3] = rng.next1();
-                        att = nee_surface(sc, stack, its2, r4b, rng, med, max_depth - 2, wo, pdf_nee, false, c);
+                        att = nee_surface(sc, its2, r4b, rng, med, max_depth - 2, wo, pdf_nee, false, c);
                         if (!is_zero3(att))
                             lins += cmul(bsdf_eval(b, its2.wi, wo), att) *
                                     (pv * mis_weight(pdf_nee, bsdf_pdf(b, its2.wi, wo)));
@@ -1015,9 +1008,9 @@ __global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Q
                             wo = its2.to_world(wo);
                             const int med1 = is_transition(sh) ? target_medium(sc, r.shape, its2.ng, wo) : med;
                             Its its3;
-                            att = look_for_emitter(sc, stack, its2.p, wo, true, rng, med1, max_depth - 2, its3, pdf_nee, c);
+                            att = look_for_emitter(sc, its2.p, wo, true, rng, med1, max_depth - 2, its3, pdf_nee, c);
                             if (!is_zero3(att, 1e-12f)) lins += cmul(t1, att) * mis_weight(bp, pdf_nee);
-                            lins += cmul(t1, li_path(sc, stack, rng, its2.p, wo, max_depth - 2, med1, false, c));
+                            lins += cmul(t1, li_path(sc, rng, its2.p, wo, max_depth - 2, med1, false, c));
                         }
                     }
                 }
@@ -1084,8 +1077,6 @@ __global__ void k_primary_keys(RenderParams rp, unsigned *keys, int *vals) {
 template <int N>
 __global__ void __launch_bounds__(kBlock) k_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                     unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     uint32_t n = 0;
@@ -1118,7 +1109,7 @@ __global__ void __launch_bounds__(kBlock) k_primary(DevScene sc, RenderParams rp
         if (moving && lx >= 0 && ly >= 0 && lx < rp.out_w && ly < rp.out_h) {
             float3 o, d;
             camera_ray(cam, ipx + fx, ipy + fy, o, d);
-            const float tr = eval_transmittance(sc, stack, o, d, false, cam.med_id, maxd, rng, rp.max_bounces - 1, c);
+            const float tr = eval_transmittance(sc, o, d, false, cam.med_id, maxd, rng, rp.max_bounces - 1, c);
             if (tr > kEps) {
                 const long long slot = queue_reserve_n(sc, qli, 2);  // the pair in adjacent slots
                 for (int sgn = 0; sgn < 2 && slot >= 0; ++sgn) {

@@ -17,8 +17,6 @@ namespace dt {
 
 __global__ void __launch_bounds__(kBlock, 6) k_primal(DevScene sc, RenderParams rp, double *img_acc,
                                                    unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < rp.path_count;
     const long long g = rp.path_begin + (active ? gi : 0);
@@ -32,7 +30,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_primal(DevScene sc, RenderParams 
         const double jx = rng.next1d(), jy = rng.next1d();  // samplePrimaryRay(ix, iy, next2D())
         float3 o, d;
         camera_ray(sc.cam, ix + jx, iy + jy, o, d);
-        L = li_path(sc, stack, rng, o, d, rp.max_bounces, sc.cam.med_id, true, c, false) * rp.inv_spp;
+        L = li_path(sc, rng, o, d, rp.max_bounces, sc.cam.med_id, true, c, false) * rp.inv_spp;
     }
     const unsigned full = 0xffffffffu;
     const int p0 = __shfl_sync(full, pixel, 0);
@@ -53,8 +51,6 @@ __global__ void __launch_bounds__(kBlock, 6) k_primal(DevScene sc, RenderParams 
 __global__ void __launch_bounds__(kBlock) k_primal_start(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
                                                          int *q_out, unsigned long long *cnt_out,
                                                          unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     bool live = false;
@@ -67,7 +63,7 @@ __global__ void __launch_bounds__(kBlock) k_primal_start(DevScene sc, RenderPara
         const double jx = st.rng.next1d(), jy = st.rng.next1d();
         float3 o, d;
         camera_ray(sc.cam, ix + jx, iy + jy, o, d);
-        live = li_start(sc, stack, st, o, d, rp.max_bounces, sc.cam.med_id, true, c, false);
+        live = li_start(sc, st, o, d, rp.max_bounces, sc.cam.med_id, true, c, false);
         if (live) states[gi] = st;
         rets[gi] = mk(0.f, 0.f, 0.f);
     }
@@ -78,14 +74,12 @@ __global__ void __launch_bounds__(kBlock) k_primal_start(DevScene sc, RenderPara
 __global__ void __launch_bounds__(kBlock, 6) k_primal_level(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
                                                          const int *q_in, const unsigned long long *cnt_in, int *q_out,
                                                          unsigned long long *cnt_out, unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long n = (long long)*cnt_in;
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
         const int id = q_in[i];
         LiState st = states[id];
-        const bool alive = li_step(sc, stack, st, c);
+        const bool alive = li_step(sc, st, c);
         if (alive) states[id] = st;
         else rets[id] = st.ret;
         push_path(q_out, cnt_out, id, alive);

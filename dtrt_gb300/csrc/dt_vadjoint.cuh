@@ -123,7 +123,7 @@ enum { VR_VALUE = 0, VR_FRAME = 1, VR_CHAIN = 2 };
 //   VR_CHAIN: walks the x0 gradient slots back to front (needs xadj)
 constexpr int kVMaxLevels = 32;
 
-DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, int *stack, long long g, int pixel, int stage,
+DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g, int pixel, int stage,
                          float3 total, float3 gpix, float *grad, Queue qe, const float *xadj, long long chain_base,
                          Ctr &c) {
     const float3 zero = mk(0.f, 0.f, 0.f);
@@ -144,7 +144,7 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, int *stack,
     int cprim[kVMaxLevels];
     float3 cd[kVMaxLevels], cp[kVMaxLevels];
     int nlev = 0;
-    bool alive = ray_intersect_ad<1>(sc, stack, ray, false, its, c);
+    bool alive = ray_intersect_ad<1>(sc, ray, false, its, c);
     for (int level = 0; alive && mode != 0; ++level) {
         alive = false;
         rng.next1(); rng.next1();  // distance-sampling draws (no medium)
@@ -199,7 +199,7 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, int *stack,
         DV<1> wo;
         float pdf_nee;
         if (!is_null && (mode & MODE_SURFACE_MAIN)) {
-            DV<1> v = nee_surface_ad<1>(sc, stack, its, fr, r2, rng, -1, depth - 1, wo, pdf_nee, c);
+            DV<1> v = nee_surface_ad<1>(sc, its, fr, r2, rng, -1, depth - 1, wo, pdf_nee, c);
             if (!v.is_zero()) {
                 const DV<1> bv = bsdf_eval_ad<1>(b, its.wi, wo);
                 const float bp = bsdf_pdf(b, its0.wi, wo.val());
@@ -230,9 +230,9 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, int *stack,
             float3 thr1 = mk(1.f, 1.f, 1.f);
             ItsAD<1> its1;
             if (is_null) {
-                ray_intersect_ad<1>(sc, stack, ray, true, its1, c);
+                ray_intersect_ad<1>(sc, ray, true, its1, c);
             } else {
-                DV<1> att = look_for_emitter_ad<1>(sc, stack, ray, true, rng, -1, depth - 1, its1, pdf_nee, nullptr,
+                DV<1> att = look_for_emitter_ad<1>(sc, ray, true, rng, -1, depth - 1, its1, pdf_nee, nullptr,
                                                    nullptr, c);
                 thr1 = bw.val();
                 if (!att.is_zero() && (mode & MODE_SURFACE_MAIN))
@@ -262,8 +262,6 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, int *stack,
 __global__ void __launch_bounds__(kBlock) k_vadj_camera(DevScene sc, RenderParams rp, const float *dimg, float *grad,
                                                         Queue qe, double *img_acc, int levels,
                                                         unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < rp.path_count;
     const long long g = rp.path_begin + (active ? gi : 0);
@@ -271,11 +269,11 @@ __global__ void __launch_bounds__(kBlock) k_vadj_camera(DevScene sc, RenderParam
     Ctr c;
     float3 total = mk(0.f, 0.f, 0.f);
     if (active) {
-        total = vreplay_path(sc, rp, stack, g, pixel, VR_VALUE, total, total, grad, qe, nullptr, gi * levels, c);
+        total = vreplay_path(sc, rp, g, pixel, VR_VALUE, total, total, grad, qe, nullptr, gi * levels, c);
         const float3 gp = mk(__ldg(dimg + 3 * (size_t)pixel), __ldg(dimg + 3 * (size_t)pixel + 1),
                              __ldg(dimg + 3 * (size_t)pixel + 2));
         if (!is_zero3(total, 0.f) && !is_zero3(gp, 0.f))
-            vreplay_path(sc, rp, stack, g, pixel, VR_FRAME, total, gp, grad, qe, nullptr, gi * levels, c);
+            vreplay_path(sc, rp, g, pixel, VR_FRAME, total, gp, grad, qe, nullptr, gi * levels, c);
     }
     if (img_acc != nullptr) {
         const unsigned full = 0xffffffffu;
@@ -295,14 +293,13 @@ __global__ void __launch_bounds__(kBlock) k_vadj_camera(DevScene sc, RenderParam
 // one thread per camera path: the x0 gradient slots back to front
 __global__ void __launch_bounds__(kBlock) k_vadj_chain(DevScene sc, RenderParams rp, float *grad, const float *xadj,
                                                        int levels, unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     if (gi >= rp.path_count) return;
     const long long g = rp.path_begin + gi;
     Ctr c;
     Queue none{nullptr, nullptr, 0};
     const float3 z = mk(0.f, 0.f, 0.f);
-    vreplay_path(sc, rp, s_stack + threadIdx.x, g, (int)(g / rp.spp), VR_CHAIN, z, z, grad, none, xadj, gi * levels, c);
+    vreplay_path(sc, rp, g, (int)(g / rp.spp), VR_CHAIN, z, z, grad, none, xadj, gi * levels, c);
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
@@ -310,8 +307,6 @@ __global__ void __launch_bounds__(kBlock) k_vadj_chain(DevScene sc, RenderParams
 // the gradient coefficients instead of per-slot scalars
 __global__ void __launch_bounds__(kBlock) k_vadj_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                       long long rec_count, Queue qli, unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     uint32_t nsamples = 0;
@@ -349,7 +344,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_edge(DevScene sc, RenderParams 
             ok = !is_zero3(val);
         }
         if (ok) {
-            const float tr = eval_transmittance(sc, stack, tof(x0), w1f, true, med1, (float)dist, rng, r.depth, c);
+            const float tr = eval_transmittance(sc, tof(x0), w1f, true, med1, (float)dist, rng, r.depth, c);
             ok = tr > kEps;
         }
         if (ok) {
@@ -381,8 +376,6 @@ __global__ void __launch_bounds__(kBlock) k_vadj_edge(DevScene sc, RenderParams 
 // one thread per primary-edge sample: k_primary's geometry with the projection Jacobian
 __global__ void __launch_bounds__(kBlock) k_vadj_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                          unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     uint32_t n = 0;
@@ -411,7 +404,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_primary(DevScene sc, RenderPara
             }
             float3 o, d;
             camera_ray(cam, ipx + fx, ipy + fy, o, d);
-            const float tr = eval_transmittance(sc, stack, o, d, false, cam.med_id, maxd, rng, rp.max_bounces - 1, c);
+            const float tr = eval_transmittance(sc, o, d, false, cam.med_id, maxd, rng, rp.max_bounces - 1, c);
             if (tr > kEps) {
                 const long long slot = queue_reserve_n(sc, qli, 2);  // the pair in adjacent slots
                 for (int sgn = 0; sgn < 2 && slot >= 0; ++sgn) {
@@ -441,8 +434,6 @@ __global__ void __launch_bounds__(kBlock) k_vadj_primary(DevScene sc, RenderPara
 __global__ void __launch_bounds__(kBlock, 6) k_vadj_li(DevScene sc, RenderParams rp, Queue qli, long long count,
                                                     const float *dimg, float *grad, float *xadj, const int *perm,
                                                     unsigned long long *ctr) {
-    __shared__ int s_stack[kStackDepth * kBlock];
-    int *stack = s_stack + threadIdx.x;
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
     uint32_t n = 0;
@@ -452,7 +443,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_vadj_li(DevScene sc, RenderParams
         Rng rng;
         rng.init(rp.seed, t.key);
         n = 1;
-        const float3 L = li_path(sc, stack, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
+        const float3 L = li_path(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
         const float3 gp = mk(__ldg(dimg + 3 * (size_t)t.pixel), __ldg(dimg + 3 * (size_t)t.pixel + 1),
                              __ldg(dimg + 3 * (size_t)t.pixel + 2));
         const float K = dot(gp, cmul(f3(t.w), L));
