@@ -1052,6 +1052,7 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
         return DTRT_ERR_CUDA;
     if (!any_normals) ds.normal_der = nullptr;
     ds.num_bsdfs = d->num_bsdfs;
+    for (const DevBsdf &b : bsdfs) ds.has_null |= b.type == BSDF_NULL ? 1 : 0;
     ds.num_phases = d->num_phases;
     ds.num_emitters = d->num_emitters;
     ds.num_media = d->num_media;

@@ -69,8 +69,8 @@ constexpr int kStackExit = (int)0x80000000;
 // (the reference bounds them by max_interactions, which can be -1 = unbounded).
 constexpr int kMaxInteractions = 4096;
 
-DT_HEAVY int closest_hit(const DevScene &sc, float3 o, float3 d, float tmin, float tmax, float &t_hit,
-                     Ctr &c) {
+DT_HEAVY int closest_hit(const DevScene &sc, float3 o, float3 d, float tmin, float tmax, float &t_hit, Ctr &c,
+                         bool any = false) {
     int stack[kStackDepth];
     c.rays++;
     const float3 inv = mk(1.0f / (fabsf(d.x) > 1e-30f ? d.x : copysignf(1e-30f, d.x)),
@@ -143,6 +143,7 @@ DT_HEAVY int closest_hit(const DevScene &sc, float3 o, float3 d, float tmin, flo
                 best = __float_as_int(A.w);
             }
         }
+        if (any && best >= 0) break;
         code = sp > 0 ? stack[--sp] : kStackExit;
     }
     t_hit = best_t;
@@ -1234,7 +1235,8 @@ DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool o
     while (remaining > 0.f) {
         if (inter >= kMaxInteractions) return 0.f;  // also bounds max_inter == -1
         float tmax = remaining, th;
-        const int prim = closest_hit(sc, o, d, tmin, tfar, th, c);
+        // any hit blocks where no surface lets light through
+        const int prim = closest_hit(sc, o, d, tmin, tfar, th, c, !sc.has_null);
         Its its;
         if (prim >= 0) {
             const int shape = __ldg(sc.tris + prim).w;

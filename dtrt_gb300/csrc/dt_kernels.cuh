@@ -782,7 +782,7 @@ DT_D float3 edge_subpath_dir(const EdgePoint &ep, int sgn) {
 
 // eight resident blocks per SM: the kernel waits on the FP64 pipe and on traversal latency
 template <int N>
-__global__ void __launch_bounds__(kBlock, 8) k_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
+__global__ void __launch_bounds__(kBlock, 12) k_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                  long long rec_count, Queue qli, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
@@ -895,7 +895,7 @@ __global__ void k_li_keys(DevScene sc, const Task *tasks, long long npairs, unsi
 // Six resident blocks per SM (80 registers, a few spilled): traversal is latency bound and
 // the extra warps hide more of it than the spills cost (C2 Li stage 121 -> 102 ms).
 template <int N>
-__global__ void __launch_bounds__(kBlock, 6) k_li(DevScene sc, RenderParams rp, Queue qli, long long begin, long long count,
+__global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, Queue qli, long long begin, long long count,
                                                double *acc1, double *acc2, const int *perm,
                                                unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_li(DevScene sc, RenderParams rp, 
 
 // ====================================================================== Lins records
 template <int N>
-__global__ void __launch_bounds__(kBlock) k_lins(DevScene sc, RenderParams rp, Queue ql, long long count, double *acc1,
+__global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp, Queue ql, long long count, double *acc1,
                                                  unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
@@ -1075,7 +1075,7 @@ __global__ void k_primary_keys(RenderParams rp, unsigned *keys, int *vals) {
 }
 
 template <int N>
-__global__ void __launch_bounds__(kBlock) k_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
+__global__ void __launch_bounds__(kBlock, 10) k_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                     unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;

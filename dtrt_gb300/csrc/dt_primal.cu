@@ -15,7 +15,7 @@
 
 namespace dt {
 
-__global__ void __launch_bounds__(kBlock, 6) k_primal(DevScene sc, RenderParams rp, double *img_acc,
+__global__ void __launch_bounds__(kBlock, 10) k_primal(DevScene sc, RenderParams rp, double *img_acc,
                                                    unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < rp.path_count;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kBlock) k_primal_start(DevScene sc, RenderPara
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
-__global__ void __launch_bounds__(kBlock, 6) k_primal_level(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
+__global__ void __launch_bounds__(kBlock, 8) k_primal_level(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
                                                          const int *q_in, const unsigned long long *cnt_in, int *q_out,
                                                          unsigned long long *cnt_out, unsigned long long *ctr) {
     const long long n = (long long)*cnt_in;

@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_chain(DevScene sc, RenderParams
 
 // one thread per (edge record, edge sample): k_edge's geometry, then two VLiTasks carrying
 // the gradient coefficients instead of per-slot scalars
-__global__ void __launch_bounds__(kBlock) k_vadj_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
+__global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                       long long rec_count, Queue qli, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_edge(DevScene sc, RenderParams 
 }
 
 // one thread per primary-edge sample: k_primary's geometry with the projection Jacobian
-__global__ void __launch_bounds__(kBlock) k_vadj_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
+__global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                          unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     Ctr c;
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_primary(DevScene sc, RenderPara
 
 // one thread per VLiTask: Li, then K = dot(dL/dI, w (x) Li) times the coefficients; six
 // resident blocks per SM and the pairs in sorted order (perm, or queue order), as k_li
-__global__ void __launch_bounds__(kBlock, 6) k_vadj_li(DevScene sc, RenderParams rp, Queue qli, long long count,
+__global__ void __launch_bounds__(kBlock, 10) k_vadj_li(DevScene sc, RenderParams rp, Queue qli, long long count,
                                                     const float *dimg, float *grad, float *xadj, const int *perm,
                                                     unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
