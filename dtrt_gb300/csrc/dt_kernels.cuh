@@ -892,35 +892,40 @@ __global__ void k_li_keys(DevScene sc, const Task *tasks, long long npairs, unsi
     vals[m] = (int)m;
 }
 
-// Six resident blocks per SM (80 registers, a few spilled): traversal is latency bound and
-// the extra warps hide more of it than the spills cost (C2 Li stage 121 -> 102 ms).
-template <int N>
+// Eight resident blocks per SM: the kernel issues on half the cycles with 11 of 32 lanes
+// active, and more warps hide more of the traversal's latency than their spills cost. The two
+// sub-paths of a sample share pixel and slot weights: their lanes add up the radiance first
+// and each adds every other slot, half the FP64 atomics.
+template <int N, bool kSurf>
 __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, Queue qli, long long begin, long long count,
                                                double *acc1, double *acc2, const int *perm,
                                                unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     // perm: the pairs in sorted order (a pair's two slots stay in adjacent lanes), or queue order
     const long long slot = perm && gi < count ? 2LL * __ldg(perm + (gi >> 1)) + (gi & 1) : begin + gi;
+    const LiTask<N> &t = reinterpret_cast<const LiTask<N> *>(qli.data)[slot];
     Ctr c;
     uint32_t n = 0;
+    float3 wl = mk(0.f, 0.f, 0.f);
     if (gi < count) {
-        const LiTask<N> &t = reinterpret_cast<const LiTask<N> *>(qli.data)[slot];
         Rng rng;
         rng.init(rp.seed, t.key);
         n = 1;
-        const float3 L = li_path(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
-        if (!is_zero3(L, 0.f)) {
-            const float3 wl = cmul(f3(t.w), L);
-            const bool prim = (t.flags & 2) != 0;
-            double *acc = prim ? acc2 : acc1 + (size_t)rp.npix * 3;  // slot j of the derivative images
+        wl = cmul(f3(t.w), li_path<kSurf>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c));
+    }
+    wl = mk(wl.x + __shfl_xor_sync(0xffffffffu, wl.x, 1), wl.y + __shfl_xor_sync(0xffffffffu, wl.y, 1),
+            wl.z + __shfl_xor_sync(0xffffffffu, wl.z, 1));
+    if (gi < count && !is_zero3(wl, 0.f)) {
+        const bool prim = (t.flags & 2) != 0;
+        double *acc = prim ? acc2 : acc1 + (size_t)rp.npix * 3;  // slot j of the derivative images
+        const bool alone = (gi ^ 1) >= count;
 #pragma unroll
-            for (int j = 0; j < N; ++j) {
-                if (t.s[j] == 0.f) continue;
-                double *a = acc + ((size_t)j * rp.npix + t.pixel) * 3;
-                atomicAdd(a, (double)(wl.x * t.s[j]));
-                atomicAdd(a + 1, (double)(wl.y * t.s[j]));
-                atomicAdd(a + 2, (double)(wl.z * t.s[j]));
-            }
+        for (int j = 0; j < N; ++j) {
+            if (t.s[j] == 0.f || (!alone && ((j ^ (int)gi) & 1))) continue;
+            double *a = acc + ((size_t)j * rp.npix + t.pixel) * 3;
+            atomicAdd(a, (double)(wl.x * t.s[j]));
+            atomicAdd(a + 1, (double)(wl.y * t.s[j]));
+            atomicAdd(a + 2, (double)(wl.z * t.s[j]));
         }
     }
     if (ctr) flush_counters(ctr, K_LI, c, CT_LI, n);

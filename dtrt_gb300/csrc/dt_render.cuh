@@ -183,7 +183,8 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                      const int *perm = li_sorted ? sort_li_pairs(sc, (const LiTask<N> *)qli.data, (long long)n, sb,
                                                                  li_cap, st, launches)
                                                  : nullptr;
-                     k_li<N><<<blocks(n), kBlock, 0, st>>>(sc, rp, qli, 0, n, sb.acc1, sb.acc2, perm, ctr);
+                     const auto k = surfaces_only(sc) ? k_li<N, true> : k_li<N, false>;
+                     k<<<blocks(n), kBlock, 0, st>>>(sc, rp, qli, 0, n, sb.acc1, sb.acc2, perm, ctr);
                  })))
                 return rc;
         DT_CK(cudaMemsetAsync(sb.counts + 2, 0, sizeof(unsigned long long), st));
@@ -454,7 +455,8 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
         const unsigned long long n = std::min<unsigned long long>(hcnt[2], kNoallocLiCap);
         tot_li += n;
         if (n) {
-            k_li<N><<<blocks(n), kBlock, 0, st>>>(sc, rp, qli, 0, n, acc1, acc2, nullptr, nullptr);
+            const auto k = surfaces_only(sc) ? k_li<N, true> : k_li<N, false>;
+            k<<<blocks(n), kBlock, 0, st>>>(sc, rp, qli, 0, n, acc1, acc2, nullptr, nullptr);
             if ((rc = launched())) return rc;
         }
         DT_CK(cudaMemsetAsync(counts + 2, 0, sizeof(unsigned long long), st));

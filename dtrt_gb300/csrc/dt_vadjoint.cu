@@ -146,8 +146,8 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
             const int *perm =
                 li_sorted ? sort_li_pairs(sc, (const VLiTask *)qli.data, (long long)n, sb, li_cap, st, launches)
                           : nullptr;
-            k_vadj_li<<<blocks((long long)n), kBlock, 0, st>>>(sc, rp, qli, (long long)n, dimg, grad, xadj, perm,
-                                                               ctr);
+            const auto k = surfaces_only(sc) ? k_vadj_li<true> : k_vadj_li<false>;
+            k<<<blocks((long long)n), kBlock, 0, st>>>(sc, rp, qli, (long long)n, dimg, grad, xadj, perm, ctr);
             ++launches;
             DT_VCK(cudaGetLastError());
         }

@@ -429,28 +429,40 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, Render
     if (ctr) flush_counters(ctr, K_PRIMARY, c, CT_PRIMARY, n);
 }
 
-// one thread per VLiTask: Li, then K = dot(dL/dI, w (x) Li) times the coefficients; six
-// resident blocks per SM and the pairs in sorted order (perm, or queue order), as k_li
+// one thread per VLiTask: Li, then K = dot(dL/dI, w (x) Li) times the coefficients; the pairs
+// in sorted order (perm, or queue order) as k_li. The two sub-paths of a sample share the
+// coefficients: their lanes add up K first and each scatters half of the nine values.
+template <bool kSurf>
 __global__ void __launch_bounds__(kBlock, 10) k_vadj_li(DevScene sc, RenderParams rp, Queue qli, long long count,
                                                     const float *dimg, float *grad, float *xadj, const int *perm,
                                                     unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
+    const long long slot = perm && gi < count ? 2LL * __ldg(perm + (gi >> 1)) + (gi & 1) : gi;
+    const VLiTask &t = reinterpret_cast<const VLiTask *>(qli.data)[slot];
     Ctr c;
     uint32_t n = 0;
+    float K = 0.f;
     if (gi < count) {
-        const long long slot = perm ? 2LL * __ldg(perm + (gi >> 1)) + (gi & 1) : gi;
-        const VLiTask &t = reinterpret_cast<const VLiTask *>(qli.data)[slot];
         Rng rng;
         rng.init(rp.seed, t.key);
         n = 1;
-        const float3 L = li_path(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
+        const float3 L = li_path<kSurf>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
         const float3 gp = mk(__ldg(dimg + 3 * (size_t)t.pixel), __ldg(dimg + 3 * (size_t)t.pixel + 1),
                              __ldg(dimg + 3 * (size_t)t.pixel + 2));
-        const float K = dot(gp, cmul(f3(t.w), L));
-        if (K != 0.f && isfinite(K)) {
+        K = dot(gp, cmul(f3(t.w), L));
+        if (!isfinite(K)) K = 0.f;
+    }
+    K += __shfl_xor_sync(0xffffffffu, K, 1);
+    if (gi < count && K != 0.f && isfinite(K)) {
+        const bool alone = (gi ^ 1) >= count;
+        const float3 x = f3(t.cx) * K;
+        if (alone || !(gi & 1)) {
             scatter3(grad, t.v0, f3(t.c0) * K);
+            if (t.chain >= 0) scatter3(xadj, t.chain, mk(x.x, alone ? x.y : 0.f, alone ? x.z : 0.f));
+        }
+        if (alone || (gi & 1)) {
             scatter3(grad, t.v1, f3(t.c1) * K);
-            if (t.chain >= 0) scatter3(xadj, t.chain, f3(t.cx) * K);
+            if (t.chain >= 0 && !alone) scatter3(xadj, t.chain, mk(0.f, x.y, x.z));
         }
     }
     if (ctr) flush_counters(ctr, K_LI, c, CT_LI, n);
