@@ -297,11 +297,8 @@ int enqueue_chunk(dtrt_batch *b, const AdjWave &w, BatchWave bw, cudaStream_t st
             for (int L = 0; L < levels; ++L) {
                 int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
                 int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
-                k_badj_vertex<0, true><<<gw, kBlock, 0, st>>>(bw, states, vins, qvl, vc + L, qvn, vc + L + 1, qsn,
-                                                             scn + L + 1, w.tots, w.ev, qx, pb);
-                if (L > 0)
-                    k_badj_vertex<0, false><<<gw, kBlock, 0, st>>>(bw, states, vins, qsl, scn + L, qvn, vc + L + 1,
-                                                                  qsn, scn + L + 1, w.tots, w.ev, qx, pb);
+                k_badj_vertex<0><<<gw, kBlock, 0, st>>>(bw, states, vins, qvl, vc + L, qsl, scn + L, qvn, vc + L + 1, qsn,
+                                                        scn + L + 1, w.tots, w.ev, qx, pb);
             }
             if (pass == 0) k_badj_totals<0><<<blocks(bw.count), kBlock, 0, st>>>(bw, states, w.tots);
         }

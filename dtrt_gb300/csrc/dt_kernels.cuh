@@ -9,8 +9,8 @@
 //              dual prefix throughput; emits EdgeRec (surface / volume edge term) and
 //              LinsRec (Lins interface term) records instead of recursing. Megakernel
 //              k_camera (one thread per path) or wavefront k_cam_start / k_cam_vertex /
-//              k_cam_accum (one launch per vertex kind and level over the compacted paths
-//              of that kind, each ending with the next level's distance sampling)
+//              k_cam_accum (one launch per level over its compacted volume and interface
+//              vertices, each ending with the next level's distance sampling)
 //   k_edge     one thread per (edge record, edge sample): FP64 silhouette test and
 //              edge-point solve, the visibility gate, then two LiTask sub-paths
 //   k_lins     one thread per Lins record: the Lins estimate with its Li sub-paths
@@ -588,23 +588,48 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_star
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
-// Vertex level L, one launch per kind: the volume (kVolume) or interface vertices of the
-// level; a continuing path then runs level L+1's distance sampling (camera_next).
-template <int N, int G, bool kVolume>
+// Entries of a level's launch: the volume vertices, padded to whole warps, then the interface
+// vertices from both ends of their queue. One launch takes both kinds: a late level's few
+// paths take as long as its slowest vertex (100 to 200 us at C3), and two launches took twice
+// that (C3 forward MS_C3A -> MS_C3B ms, density adjoint MS_DA -> MS_DB).
+struct LevelQueue {
+    long long nv, nvp, nf, n;
+    DT_D LevelQueue(int kind, const unsigned long long *cnt_v, const unsigned long long *cnt_s, const unsigned long long *cnt_back) {
+        nv = kind == 2 ? 0 : (long long)*cnt_v;
+        nvp = (nv + 31) & ~31ll;
+        nf = kind == 1 ? 0 : (long long)*cnt_s;
+        n = nvp + nf + (kind == 1 ? 0 : (long long)*cnt_back);
+    }
+    DT_D bool volume(long long i) const { return i < nvp; }  // warp-uniform
+    DT_D bool none(long long i) const { return i >= nv && i < nvp; }
+    DT_D int path(const int *qv, const int *qs, long long cap, long long i) const {
+        if (i < nvp) return qv[i];
+        i -= nvp;
+        return i < nf ? qs[i] : qs[cap - 1 - (i - nf)];
+    }
+};
+
+// Vertex level L: its volume and interface vertices; a continuing path then runs level L+1's
+// distance sampling (camera_next).
+template <int N, int G, int kKind>
 __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
-                                                       VertexIn *vins, const int *q_in,
-                                                       const unsigned long long *cnt_in,
-                                                       const unsigned long long *cnt_in_back, int *qv_next,
+                                                       VertexIn *vins, const int *qv, const unsigned long long *cnt_v,
+                                                       const int *qs, const unsigned long long *cnt_s,
+                                                       const unsigned long long *cnt_s_back, int *qv_next,
                                                        unsigned long long *cnt_v_next, int *qs_next,
                                                        unsigned long long *cnt_s_next,
                                                        unsigned long long *cnt_s_next_back, long long cap, Queue qe,
                                                        Queue ql, unsigned long long *ctr) {
-    const long long nf = (long long)*cnt_in, n = nf + (cnt_in_back ? (long long)*cnt_in_back : 0);
+    const LevelQueue lq(kKind, cnt_v, cnt_s, cnt_s_back);
     Ctr c;
-    for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
-        const int id = i < nf ? q_in[i] : q_in[cap - 1 - (i - nf)];
+    for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < lq.n; i += (long long)gridDim.x * kBlock) {
+        if (lq.none(i)) continue;
+        const int id = lq.path(qv, qs, cap, i);
         CamState<N, G> st;
-        if (kVolume) {
+        const VertexIn vin = vins[id];
+        const long long g = rp.path_begin + id;
+        bool alive;
+        if (kKind == 1 || (kKind == 0 && lq.volume(i))) {
             // a volume vertex writes the hit record (of its continuation) without reading it:
             // the record stays in HBM (380 B of 848 at nder 8)
             const CamState<N, G> &s0 = states[id];
@@ -616,13 +641,11 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vert
             st.depth = s0.depth;
             st.mode = s0.mode;
             st.level = s0.level;
+            alive = camera_volume<N, G>(sc, rp, g, st, vin, qe, c);
         } else {
             st = states[id];
+            alive = camera_surface<N, G>(sc, rp, g, st, vin, qe, ql, c);
         }
-        const VertexIn vin = vins[id];
-        const long long g = rp.path_begin + id;
-        const bool alive = kVolume ? camera_volume<N, G>(sc, rp, g, st, vin, qe, c)
-                                   : camera_surface<N, G>(sc, rp, g, st, vin, qe, ql, c);
         ++st.level;
         const int nk = camera_next<N, G>(sc, st, alive, vins, id, qv_next, cnt_v_next, qs_next, cnt_s_next,
                                       cnt_s_next_back, cap, c);
