@@ -88,15 +88,11 @@ cudaError_t launch_adjoint_wave(const DevScene &sc, const RenderParams &range, c
             for (int L = 0; L < levels; ++L) {
                 int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
                 int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
-                k_adj_vertex<0, true><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vc + L, qvn, vc + L + 1, qsn,
-                                                            sc_ + L + 1, dimg, grad, w.tots, w.ev, qx, b, ctr);
-                if (L > 0)  // level 0's interface vertices ran in k_adj_start
-                    k_adj_vertex<0, false><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qsl, sc_ + L, qvn, vc + L + 1,
-                                                                 qsn, sc_ + L + 1, dimg, grad, w.tots, w.ev, qx, b,
-                                                                 ctr);
+                k_adj_vertex<0><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vc + L, qsl, sc_ + L, qvn, vc + L + 1,
+                                                       qsn, sc_ + L + 1, dimg, grad, w.tots, w.ev, qx, b, ctr);
             }
             if (pass == 0) k_adj_totals<0><<<blocks(rp.path_count), kBlock, 0, st>>>(rp, states, w.tots, img_acc);
-            if (launches) *launches += 2 * levels + (pass == 0 ? 1 : 0);  // start, 2 per level (1 at level 0), totals in pass A
+            if (launches) *launches += 1 + levels + (pass == 0 ? 1 : 0);  // start, the levels, totals in pass A
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }

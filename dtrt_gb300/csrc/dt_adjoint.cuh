@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_start(DevScene sc, RenderPara
 
 // Vertex level of one pass: its volume and interface vertices, each continuing path then
 // running level L+1's distance sampling (replay_next).
-template <int N, int kKind>
+template <int N>
 __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderParams rp, AdjState<N> *states,
                                                        VertexIn *vins, const int *qv, const unsigned long long *cnt_v,
                                                        const int *qs, const unsigned long long *cnt_s, int *qv_next,
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderPar
                                                        unsigned long long *cnt_s_next, const float *dimg, float *grad,
                                                        const float3 *totals, float3 *evbuf, QueueEnds qx, bool pass_b,
                                                        unsigned long long *ctr) {
-    const LevelQueue lq(kKind, cnt_v, cnt_s, cnt_s + qx.back);
+    const LevelQueue lq(cnt_v, cnt_s, cnt_s + qx.back);
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < lq.n; i += (long long)gridDim.x * kBlock) {
         if (lq.none(i)) continue;
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_adj_vertex(DevScene sc, RenderPar
         const float3 total = pass_b ? totals[id] : zero, gp = pass_b ? pixel_dldi(rp, dimg, rp.path_begin + id) : zero;
         AdjCtx adj{grad, 0.f};
         float3 *ev = evbuf + (size_t)id * kReplayEvents;
-        const bool alive = kKind == 1 || (kKind == 0 && lq.volume(i)) ? replay_volume<N>(sc, rp, pass_b, gp, adj, c, ev, st, vin)
+        const bool alive = lq.volume(i) ? replay_volume<N>(sc, rp, pass_b, gp, adj, c, ev, st, vin)
                                         : replay_surface<N>(sc, rp, pass_b, gp, adj, c, ev, st, vin);
         ++st.level;
         replay_next<N>(sc, rp, st, alive, pass_b, total, gp, adj, vins, id, qv_next, cnt_v_next, qs_next, cnt_s_next,
@@ -565,14 +565,14 @@ __global__ void __launch_bounds__(kBlock) k_badj_start(BatchWave bw, AdjState<N>
     if (run) states[gi] = st;
 }
 
-template <int N, int kKind = 0>
+template <int N>
 __global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N> *states, VertexIn *vins,
                                                         const int *qv, const unsigned long long *cnt_v, const int *qs,
                                                         const unsigned long long *cnt_s, int *qv_next,
                                                         unsigned long long *cnt_v_next, int *qs_next,
                                                         unsigned long long *cnt_s_next, const float3 *totals,
                                                         float3 *evbuf, QueueEnds qx, bool pass_b) {
-    const LevelQueue lq(kKind, cnt_v, cnt_s, cnt_s + qx.back);
+    const LevelQueue lq(cnt_v, cnt_s, cnt_s + qx.back);
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < lq.n; i += (long long)gridDim.x * kBlock) {
         if (lq.none(i)) continue;
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kBlock) k_badj_vertex(BatchWave bw, AdjState<N
         const float3 total = pass_b ? totals[id] : zero, gp = pass_b ? pixel_dldi(it.rp, it.dimg, g) : zero;
         AdjCtx adj{it.grad, 0.f};
         float3 *ev = evbuf + (size_t)id * kReplayEvents;
-        const bool alive = kKind == 1 || (kKind == 0 && lq.volume(i)) ? replay_volume<N>(it.sc, it.rp, pass_b, gp, adj, c, ev, st, vin)
+        const bool alive = lq.volume(i) ? replay_volume<N>(it.sc, it.rp, pass_b, gp, adj, c, ev, st, vin)
                                         : replay_surface<N>(it.sc, it.rp, pass_b, gp, adj, c, ev, st, vin);
         ++st.level;
         replay_next<N>(it.sc, it.rp, st, alive, pass_b, total, gp, adj, vins, id, qv_next, cnt_v_next, qs_next,

@@ -590,15 +590,15 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_star
 
 // Entries of a level's launch: the volume vertices, padded to whole warps, then the interface
 // vertices from both ends of their queue. One launch takes both kinds: a late level's few
-// paths take as long as its slowest vertex (100 to 200 us at C3), and two launches took twice
-// that (C3 forward MS_C3A -> MS_C3B ms, density adjoint MS_DA -> MS_DB).
+// paths take as long as its slowest vertex (130 to 200 us in a 128^3 cloud), and two launches
+// took twice that (density step 6.7 -> 4.7 ms, batch 5.4 -> 3.5, density adjoint 40.3 -> 39.7).
 struct LevelQueue {
     long long nv, nvp, nf, n;
-    DT_D LevelQueue(int kind, const unsigned long long *cnt_v, const unsigned long long *cnt_s, const unsigned long long *cnt_back) {
-        nv = kind == 2 ? 0 : (long long)*cnt_v;
+    DT_D LevelQueue(const unsigned long long *cnt_v, const unsigned long long *cnt_s, const unsigned long long *cnt_back) {
+        nv = (long long)*cnt_v;
         nvp = (nv + 31) & ~31ll;
-        nf = kind == 1 ? 0 : (long long)*cnt_s;
-        n = nvp + nf + (kind == 1 ? 0 : (long long)*cnt_back);
+        nf = (long long)*cnt_s;
+        n = nvp + nf + (long long)*cnt_back;
     }
     DT_D bool volume(long long i) const { return i < nvp; }  // warp-uniform
     DT_D bool none(long long i) const { return i >= nv && i < nvp; }
@@ -611,7 +611,7 @@ struct LevelQueue {
 
 // Vertex level L: its volume and interface vertices; a continuing path then runs level L+1's
 // distance sampling (camera_next).
-template <int N, int G, int kKind>
+template <int N, int G>
 __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                        VertexIn *vins, const int *qv, const unsigned long long *cnt_v,
                                                        const int *qs, const unsigned long long *cnt_s,
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vert
                                                        unsigned long long *cnt_s_next,
                                                        unsigned long long *cnt_s_next_back, long long cap, Queue qe,
                                                        Queue ql, unsigned long long *ctr) {
-    const LevelQueue lq(kKind, cnt_v, cnt_s, cnt_s_back);
+    const LevelQueue lq(cnt_v, cnt_s, cnt_s_back);
     Ctr c;
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < lq.n; i += (long long)gridDim.x * kBlock) {
         if (lq.none(i)) continue;
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vert
         const VertexIn vin = vins[id];
         const long long g = rp.path_begin + id;
         bool alive;
-        if (kKind == 1 || (kKind == 0 && lq.volume(i))) {
+        if (lq.volume(i)) {
             // a volume vertex writes the hit record (of its continuation) without reading it:
             // the record stays in HBM (380 B of 848 at nder 8)
             const CamState<N, G> &s0 = states[id];

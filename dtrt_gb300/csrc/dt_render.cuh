@@ -42,7 +42,7 @@ struct CameraStage {
 
 inline unsigned path_blocks(long long n) { return (unsigned)((n + kBlock - 1) / kBlock); }
 
-// Wavefront schedule: start, two launches per vertex level (one at level 0), pixel sums
+// Wavefront schedule: start (with level 0's interface vertices), a launch per vertex level, pixel sums
 template <int N, int G>
 void CameraStage<N, G>::wave(const DevScene &sc, const RenderParams &rp, const CamWave &w, int sms, const Queue &qe,
                              const Queue &ql, double *acc1, unsigned long long *ctr, cudaStream_t st) {
@@ -61,12 +61,8 @@ void CameraStage<N, G>::wave(const DevScene &sc, const RenderParams &rp, const C
     for (int L = 0; L < w.levels; ++L) {
         int *qvl = (L & 1) ? qv : qa, *qsl = (L & 1) ? qs : qb;
         int *qvn = (L & 1) ? qa : qv, *qsn = (L & 1) ? qb : qs;
-        k_cam_vertex<N, G, true><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vcnt + L, nullptr, qvn, vcnt + L + 1,
-                                                        qsn, scnt + L + 1, sbk + L + 1, w.cap, qe, ql, ctr);
-        if (L > 0)  // level 0's interface vertices ran in k_cam_start
-            k_cam_vertex<N, G, false><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qsl, scnt + L, sbk + L, qvn,
-                                                             vcnt + L + 1, qsn, scnt + L + 1, sbk + L + 1, w.cap, qe,
-                                                             ql, ctr);
+        k_cam_vertex<N, G><<<gw, kBlock, 0, st>>>(sc, rp, states, vins, qvl, vcnt + L, qsl, scnt + L, sbk + L, qvn,
+                                                  vcnt + L + 1, qsn, scnt + L + 1, sbk + L + 1, w.cap, qe, ql, ctr);
     }
     k_cam_accum<N, G><<<path_blocks(rp.path_count), kBlock, 0, st>>>(rp, states, acc1);
 }
@@ -232,7 +228,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                          else CameraStage<N, N>::wave(sc, rp, w, sms, qe, ql, sb.acc1, ctr, st);
                      })))
                     return rc;
-                launches += 2 * levels + 1;  // start, 2 per level (1 at level 0), accumulation
+                launches += levels + 1;  // start, the levels, accumulation
                 if (ctr) {
                     // every launched vertex reads and writes its path's state and vertex inputs;
                     // the start writes them once per path, the accumulation reads the sums
