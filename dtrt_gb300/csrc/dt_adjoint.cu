@@ -181,11 +181,15 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     const long long B = 1ll << 24;  // paths per megakernel launch
     bool wavefront = s->camera_schedule == DTRT_CAMERA_WAVEFRONT ||
                      (s->camera_schedule == DTRT_CAMERA_AUTO && total >= kWavefrontMinPaths);
-    AdjWave w{};
+    AdjWave w[kLanes];
+    int lanes = 1;
     if (wavefront) {
-        const long long cap = std::min<long long>(1ll << 24, std::max<long long>(total, 1));
-        if (ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, AdjWave::bytes(cap, o->max_bounces + 1))) {
-            w.carve(sb.cam_state, cap, o->max_bounces + 1);
+        const long long cap = std::min<long long>(1ll << 21, std::max<long long>(total, 1));
+        lanes = (int)std::min<long long>(kLanes, std::max<long long>(1, (total + cap - 1) / cap));
+        if (lanes > 1 && !ensure_lanes(sb)) lanes = 1;
+        const size_t bytes = (AdjWave::bytes(cap, o->max_bounces + 1) + 255) & ~(size_t)255;
+        if (ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * bytes)) {
+            for (int k = 0; k < lanes; ++k) w[k].carve((char *)sb.cam_state + k * bytes, cap, o->max_bounces + 1);
         } else {
             if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
             cudaGetLastError();  // AUTO: no room for the path states, run the megakernel
@@ -195,9 +199,12 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     if (wavefront) {
         int sms = 0;
         DT_ACK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
-        rp.path_begin = 0;
-        rp.path_count = total;
-        DT_ACK(launch_adjoint_wave(sc, rp, dimg, grad, img_acc, ctr, w, sms, st, &launches));
+        DT_ACK(in_lanes(sb, st, lanes, (total + w[0].cap - 1) / w[0].cap, [&](long long k, int lane, cudaStream_t q) {
+            RenderParams r = rp;
+            r.path_begin = k * w[0].cap;
+            r.path_count = std::min(w[0].cap, total - r.path_begin);
+            return launch_adjoint_wave(sc, r, dimg, grad, img_acc, ctr, w[lane], sms, q, &launches);
+        }));
     } else {
         for (long long b0 = 0; b0 < total; b0 += B) {
             rp.path_begin = b0;
@@ -232,7 +239,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     std::memset(&ls, 0, sizeof(ls));
     ls.camera_paths = (uint64_t)total;
     ls.kernel_launches = launches;
-    ls.batches = (uint64_t)((total + (wavefront ? w.cap : B) - 1) / std::max<long long>(1, wavefront ? w.cap : B));
+    ls.batches = (uint64_t)((total + (wavefront ? w[0].cap : B) - 1) / std::max<long long>(1, wavefront ? w[0].cap : B));
     ls.counters_enabled = ctr != nullptr;
     ls.camera_schedule = wavefront ? DTRT_CAMERA_WAVEFRONT : DTRT_CAMERA_MEGAKERNEL;
     ls.k_rays[0] = ls.rays = hc[0];

@@ -11,6 +11,14 @@ namespace dt {
 
 void set_last_error(const std::string &msg);
 
+// Wavefront batches in flight at once, each on a stream and a workspace of its own: a batch's
+// last levels hold few paths and take as long as their slowest vertex, and the other batches
+// run in the meantime; small batches read neighbouring voxels. C3 forward (33.6 M paths): one
+// lane of 2^23 paths 68.8 ms, 4 lanes of 2^21 63.7, 8 of 2^20 63.1, 8 of 2^19 66.4; its
+// density adjoint: one lane of 2^24 39.7, 8 of 2^20 36.9, 8 of 2^21 35.5; C1 primal: one of
+// 2^22 15.9, 8 of 2^20 14.8, 8 of 2^19 14.1. Eight streams are what the device queues.
+constexpr int kLanes = 8;
+
 // Device buffers reused across renders of one scene, grown on demand.
 struct Scratch {
     double *acc1 = nullptr, *acc2 = nullptr;
@@ -34,10 +42,35 @@ struct Scratch {
     // density cells of a render (DevScene::cells), then the replay's gradient in that layout
     void *cells = nullptr;
     size_t cells_bytes = 0;
-
+    // side streams of the lanes 1..., the fork and join events (made by the first render of several batches)
+    cudaStream_t side[kLanes - 1] = {};
+    cudaEvent_t fork_ev = nullptr, side_ev[kLanes - 1] = {};
 };
 
 bool ensure_buffer(void **ptr, size_t *have, size_t need);
+// The lanes' streams and events: false (and the error cleared) when they cannot be made.
+bool ensure_lanes(Scratch &sb);
+
+// f(batch, lane, stream) for each of n batches, dealt in turn to st and lanes - 1 side streams
+// that fork from st and join it again.
+template <class F>
+cudaError_t in_lanes(Scratch &sb, cudaStream_t st, int lanes, long long n, F f) {
+    cudaError_t e = cudaSuccess;
+    auto ck = [&](cudaError_t r) { e = e == cudaSuccess ? r : e; };
+    if (lanes > 1) {
+        ck(cudaEventRecord(sb.fork_ev, st));
+        for (int k = 1; k < lanes; ++k) ck(cudaStreamWaitEvent(sb.side[k - 1], sb.fork_ev, 0));
+    }
+    for (long long k = 0; k < n && e == cudaSuccess; ++k) {
+        const int lane = (int)(k % lanes);
+        ck(f(k, lane, lane ? sb.side[lane - 1] : st));
+    }
+    for (int k = 1; k < lanes; ++k) {
+        ck(cudaEventRecord(sb.side_ev[k - 1], sb.side[k - 1]));
+        ck(cudaStreamWaitEvent(st, sb.side_ev[k - 1], 0));
+    }
+    return e;
+}
 
 // Buffers of the Li pair sort for queues of li_cap tasks (li_cap / 2 pairs): false (and
 // the allocation error cleared) when the device has no room, the Li kernels then read the
@@ -99,8 +132,8 @@ inline bool static_rays(const DevScene &sc) {
 inline bool surfaces_only(const DevScene &sc) { return sc.num_media == 0 && !sc.has_null && sc.cam.med_id < 0; }
 
 // Camera paths per batch of a scene of static_rays(): its batches hold no records, only path
-// states (2 GB at nder 8)
-constexpr long long kStaticBatchPaths = 1ll << 23;
+// states (256 MB at nder 8), and kLanes of them run at once
+constexpr long long kStaticBatchPaths = 1ll << 20;
 
 // Buffers of the camera wavefront for `cap` paths: path states, vertex inputs, four
 // path-index queues, level counts

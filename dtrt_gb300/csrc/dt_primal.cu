@@ -162,22 +162,17 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     bool wavefront = s->camera_schedule == DTRT_CAMERA_WAVEFRONT ||
                      (s->camera_schedule == DTRT_CAMERA_AUTO && total >= kWavefrontMinPaths && sc.has_grid_media);
     const int levels = o->max_bounces + 2;  // li_step runs at most max_bounces + 1 vertices
-    LiState *states = nullptr;
-    float3 *rets = nullptr;
-    int *qa = nullptr, *qb = nullptr;
-    unsigned long long *lcnt = nullptr;
+    size_t sbytes = 0, wbytes = 0;
+    int lanes = 1;
     if (wavefront) {
-        B = std::min<long long>(1ll << 22, std::max<long long>(total, 1));
-        const size_t sbytes = ((size_t)B * sizeof(LiState) + 255) & ~(size_t)255;
-        if (ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, sbytes + (size_t)B * sizeof(float3)) &&
-            ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)2 * B * sizeof(int)) &&
-            ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)(levels + 1) * sizeof(unsigned long long))) {
-            states = (LiState *)sb.cam_state;
-            rets = (float3 *)((char *)sb.cam_state + sbytes);
-            qa = (int *)sb.cam_q;
-            qb = qa + B;
-            lcnt = (unsigned long long *)sb.cam_cnt;
-        } else {
+        B = std::min<long long>(1ll << 19, std::max<long long>(total, 1));
+        lanes = (int)std::min<long long>(kLanes, std::max<long long>(1, (total + B - 1) / B));
+        if (lanes > 1 && !ensure_lanes(sb)) lanes = 1;
+        sbytes = ((size_t)B * sizeof(LiState) + 255) & ~(size_t)255;
+        wbytes = (sbytes + (size_t)B * sizeof(float3) + 255) & ~(size_t)255;
+        if (!(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * wbytes) &&
+              ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)2 * lanes * B * sizeof(int)) &&
+              ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)lanes * (levels + 1) * sizeof(unsigned long long)))) {
             if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
             cudaGetLastError();  // AUTO: no room for the path states, run the megakernel
             wavefront = false;
@@ -189,24 +184,34 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
     DT_PCK(cudaEventRecord(e0, st));
     launches += (uint64_t)prepare_cells(s, sc, total, false, st);
-    for (long long b0 = 0; b0 < total; b0 += B) {
+    if (wavefront) {
+        const long long nb = (total + B - 1) / B;
+        DT_PCK(in_lanes(sb, st, lanes, nb, [&](long long k, int lane, cudaStream_t q) {
+            RenderParams r = rp;
+            r.path_begin = k * B;
+            r.path_count = std::min(B, total - k * B);
+            LiState *states = (LiState *)((char *)sb.cam_state + lane * wbytes);
+            float3 *rets = (float3 *)((char *)states + sbytes);
+            int *qa = (int *)sb.cam_q + (size_t)2 * lane * B, *qb = qa + B;
+            unsigned long long *lcnt = (unsigned long long *)sb.cam_cnt + (size_t)lane * (levels + 1);
+            const unsigned gw = std::min<unsigned>(blocks(r.path_count), (unsigned)std::max(1, sms) * 16u);
+            const cudaError_t e = cudaMemsetAsync(lcnt, 0, (size_t)(levels + 1) * sizeof(unsigned long long), q);
+            if (e != cudaSuccess) return e;
+            k_primal_start<<<blocks(r.path_count), kBlock, 0, q>>>(sc, r, states, rets, qa, lcnt, ctr);
+            for (int L = 0; L < levels; ++L)
+                k_primal_level<<<gw, kBlock, 0, q>>>(sc, r, states, rets, (L & 1) ? qb : qa, lcnt + L, (L & 1) ? qa : qb,
+                                                     lcnt + L + 1, ctr);
+            k_primal_accum<<<blocks(r.path_count), kBlock, 0, q>>>(r, rets, sb.adj_img);
+            return cudaGetLastError();
+        }));
+        launches += (uint64_t)nb * (levels + 2);
+    }
+    for (long long b0 = wavefront ? total : 0; b0 < total; b0 += B) {
         rp.path_begin = b0;
         rp.path_count = std::min(B, total - b0);
-        if (!wavefront) {
-            const auto k = surfaces_only(sc) ? k_primal<true> : k_primal<false>;
-            k<<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, sb.adj_img, ctr);
-            ++launches;
-            DT_PCK(cudaGetLastError());
-            continue;
-        }
-        const unsigned gw = std::min<unsigned>(blocks(rp.path_count), (unsigned)std::max(1, sms) * 16u);
-        DT_PCK(cudaMemsetAsync(lcnt, 0, (size_t)(levels + 1) * sizeof(unsigned long long), st));
-        k_primal_start<<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, states, rets, qa, lcnt, ctr);
-        for (int L = 0; L < levels; ++L)
-            k_primal_level<<<gw, kBlock, 0, st>>>(sc, rp, states, rets, (L & 1) ? qb : qa, lcnt + L, (L & 1) ? qa : qb,
-                                                  lcnt + L + 1, ctr);
-        k_primal_accum<<<blocks(rp.path_count), kBlock, 0, st>>>(rp, rets, sb.adj_img);
-        launches += levels + 2;
+        const auto k = surfaces_only(sc) ? k_primal<true> : k_primal<false>;
+        k<<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, sb.adj_img, ctr);
+        ++launches;
         DT_PCK(cudaGetLastError());
     }
     DT_PCK(cudaEventRecord(e1, st));

@@ -204,10 +204,15 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                          (s->camera_schedule == DTRT_CAMERA_AUTO && Bw >= kWavefrontMinPaths);
         const size_t state_size = fixed_rays ? CameraStage<N, 0>::state_bytes : CameraStage<N, N>::state_bytes,
                      hit_size = fixed_rays ? CameraStage<N, 0>::hit_bytes : CameraStage<N, N>::hit_bytes;
-        const size_t state_bytes = ((size_t)Bw * state_size + 255) & ~(size_t)255;
-        if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, state_bytes + (size_t)Bw * sizeof(VertexIn)) &&
-                           ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * Bw * sizeof(int)) &&
-                           ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * (levels + 1) * sizeof(unsigned long long)))) {
+        const size_t state_bytes = ((size_t)Bw * state_size + 255) & ~(size_t)255,
+                     work_bytes = (state_bytes + (size_t)Bw * sizeof(VertexIn) + 255) & ~(size_t)255;
+        const long long nb = (total + B - 1) / B;
+        // several batches in flight; the counters read each batch's level counts, so one then
+        int lanes = wavefront && fixed_rays && !ctr ? (int)std::min<long long>(kLanes, nb) : 1;
+        if (lanes > 1 && !ensure_lanes(sb)) lanes = 1;
+        if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * work_bytes) &&
+                           ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * lanes * Bw * sizeof(int)) &&
+                           ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * lanes * (levels + 1) * sizeof(unsigned long long)))) {
             if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
             cudaGetLastError();  // AUTO: no room for the path states, run the megakernel
             wavefront = false;
@@ -215,9 +220,29 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         int sms = 0;
         DT_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
         used_wavefront = wavefront;
-        const CamWave w{sb.cam_state, (char *)sb.cam_state + state_bytes, (int *)sb.cam_q,
-                        (unsigned long long *)sb.cam_cnt, Bw, levels};
-        for (long long b0 = 0; b0 < total; b0 += B) {
+        auto workspace = [&](int lane) {
+            char *base = (char *)sb.cam_state + lane * work_bytes;
+            return CamWave{base, base + state_bytes, (int *)sb.cam_q + (size_t)4 * lane * Bw,
+                           (unsigned long long *)sb.cam_cnt + (size_t)3 * lane * (levels + 1), Bw, levels};
+        };
+        const CamWave w = workspace(0);
+        if (wavefront && fixed_rays && !ctr) {
+            cudaError_t e = cudaSuccess;
+            if ((rc = timed(ms_camera, [&] {
+                     e = in_lanes(sb, st, lanes, nb, [&](long long k, int lane, cudaStream_t q) {
+                         RenderParams r = rp;
+                         r.path_begin = k * B;
+                         r.path_count = std::min(B, total - k * B);
+                         CameraStage<N, 0>::wave(sc, r, workspace(lane), sms, qe, ql, sb.acc1, nullptr, q);
+                         return cudaGetLastError();
+                     });
+                 })))
+                return rc;
+            DT_CK(e);
+            batches = (uint64_t)nb;
+            launches += (uint64_t)nb * (levels + 2) - 1;
+        }
+        for (long long b0 = wavefront && fixed_rays && !ctr ? total : 0; b0 < total; b0 += B) {
             ++batches;
             rp.path_begin = b0;
             rp.path_count = std::min(B, total - b0);
