@@ -478,8 +478,9 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
         cam.inv_w = 1.0 / c.width;
         cam.inv_h = 1.0 / c.height;
         cam.ndc_ky = -2.0 / aspect;
-        cam.plane_kx = 2.0 / fov;
-        cam.plane_ky = -2.0 / (aspect * fov);
+        cam.px_ndc[0] = 2.0 * cam.inv_w;
+        cam.px_ndc[1] = cam.inv_h * cam.ndc_ky;
+        cam.ndc_y0 = -0.5 * cam.ndc_ky;
     }
     const bool cropped = c.crop_width > 0 && c.crop_height > 0;
     cam.crop_x = cropped ? c.crop_offset_x : 0;
@@ -888,14 +889,14 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
     // ------------------------------------------------------------ primary edges, edge_manager.cpp:6-110
     std::vector<DevPrimaryEdge> pedges;
     std::vector<double> plen;
-    std::vector<float> pjac;
+    std::vector<double> pjac;
     std::vector<int> pverts;
     const double aspect = (double)c.width / c.height, fov = c2ndc[0];
     // every edge is projected on its own (host threads, one output slot per candidate
     // edge), then the kept ones are gathered in edge order: the same arrays as a serial loop
     struct PEdgeOut {
         DevPrimaryEdge pe;
-        float jac[24];
+        double jac[12];
         bool ok;
     };
     std::vector<int2> cand;  // (shape, edge of the shape)
@@ -977,20 +978,31 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
             DevPrimaryEdge pe;
             std::memset(&pe, 0, sizeof(pe));
             pe.v0s[0] = c0[0].v * c.width; pe.v0s[1] = c0[1].v * c.height;
-            pe.v1s[0] = c1[0].v * c.width; pe.v1s[1] = c1[1].v * c.height;
+            pe.dvs[0] = c1[0].v * c.width - pe.v0s[0]; pe.dvs[1] = c1[1].v * c.height - pe.v0s[1];
             for (int j = 0; j < N; ++j) {
                 pe.d0[j][0] = (float)(c0[0].d[j] * c.width); pe.d0[j][1] = (float)(c0[1].d[j] * c.height);
                 pe.d1[j][0] = (float)(c1[0].d[j] * c.width); pe.d1[j][1] = (float)(c1[1].d[j] * c.height);
             }
-            const double *srcs[4] = {&v0p.x, &v1p.x, &v0l.x, &v1l.x};
-            double *dsts[4] = {pe.v0p, pe.v1p, pe.v0c, pe.v1c};
-            for (int q = 0; q < 4; ++q)
-                for (int a = 0; a < 3; ++a) dsts[q][a] = srcs[q][a];
+            for (int a = 0; a < 3; ++a) {
+                pe.v0c[a] = (&v0l.x)[a];
+                pe.dvc[a] = (&v1l.x)[a] - (&v0l.x)[a];
+            }
             {
-                const double nx = pe.v1s[1] - pe.v0s[1], ny = pe.v0s[0] - pe.v1s[0], nl = std::sqrt(nx * nx + ny * ny);
+                const double nx = pe.dvs[1], ny = -pe.dvs[0], nl = std::sqrt(nx * nx + ny * ny);
                 pe.n[0] = nx / nl;
                 pe.n[1] = ny / nl;
-                pe.inv_lenp = 1.0 / dnorm(sub(v1p, v0p));
+                pe.dn[0] = pe.n[0] * 1e-4 * (2.0 / c.width);
+                pe.dn[1] = pe.n[1] * 1e-4 * (-2.0 / (aspect * c.height));
+                // image-plane parameter of each screen endpoint, along v1p - v0p
+                const D3 dp = sub(v1p, v0p);
+                double tp[2];
+                for (int q = 0; q < 2; ++q) {
+                    const HD *cs = q ? c1 : c0;
+                    const D3 pp = {(cs[0].v - 0.5) * (2.0 / fov), (cs[1].v - 0.5) * (-2.0 / (aspect * fov)), 1.0};
+                    tp[q] = ddot(sub(pp, v0p), dp) / ddot(dp, dp);
+                }
+                pe.t0[0] = tp[0];
+                pe.t0[1] = tp[1] - tp[0];
                 pe.cb = dnorm(v0p) / dnorm(v0l);
                 pe.cc = dnorm(v1p) / dnorm(v1l);
             }
@@ -1016,10 +1028,10 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
                 HD k0[2], k1[2];
                 const bool vis = clip_line(q0, q1, k0, k1, xmin, xmax, ymin, ymax);
                 for (int q = 0; q < 6; ++q) {
-                    po.jac[q] = vis ? (float)(k0[0].d[q] * c.width) : 0.f;
-                    po.jac[6 + q] = vis ? (float)(k0[1].d[q] * c.height) : 0.f;
-                    po.jac[12 + q] = vis ? (float)(k1[0].d[q] * c.width) : 0.f;
-                    po.jac[18 + q] = vis ? (float)(k1[1].d[q] * c.height) : 0.f;
+                    const double j0 = vis ? pe.n[0] * k0[0].d[q] * c.width + pe.n[1] * k0[1].d[q] * c.height : 0.0;
+                    const double j1 = vis ? pe.n[0] * k1[0].d[q] * c.width + pe.n[1] * k1[1].d[q] * c.height : 0.0;
+                    po.jac[q] = j0;
+                    po.jac[6 + q] = j1 - j0;
                 }
                 po.ok = true;
             }
@@ -1030,8 +1042,8 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
         if (!po.ok) continue;
         const DevEdge &e = edges[shapes[cand[ci].x].edge_off + cand[ci].y];
         pedges.push_back(po.pe);
-        plen.push_back(std::hypot(po.pe.v0s[0] - po.pe.v1s[0], po.pe.v0s[1] - po.pe.v1s[1]));
-        pjac.insert(pjac.end(), po.jac, po.jac + 24);
+        plen.push_back(std::hypot(po.pe.dvs[0], po.pe.dvs[1]));
+        pjac.insert(pjac.end(), po.jac, po.jac + 12);
         pverts.push_back(e.v0);
         pverts.push_back(e.v1);
     }

@@ -65,8 +65,85 @@ DT_HD double3_ operator-(double3_ a, double3_ b) { return mkd(a.x - b.x, a.y - b
 DT_HD double3_ operator*(double3_ a, double s) { return mkd(a.x * s, a.y * s, a.z * s); }
 DT_HD double dotd(double3_ a, double3_ b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 DT_HD double3_ crossd(double3_ a, double3_ b) { return mkd(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x); }
-DT_HD double lengthd(double3_ a) { return sqrt(dotd(a, a)); }
-DT_HD double3_ normalized(double3_ a) { return a * (1.0 / lengthd(a)); }
+
+// ------------------------------------------------------------------ FP64 math
+// The FP64 pipe issues two lanes a cycle per SM (1/64 of FP32), and the edge kernels are bound
+// by it: a library division or square root takes about ten of its instructions, acos or sincos
+// about forty. These take 3 (reciprocal), 6 (square root with its reciprocal) and 19 (sine and
+// cosine on [0, pi]), to the last two bits. Seeds are FP32, moved by shifts of the bits.
+#ifdef __CUDA_ARCH__
+DT_HD uint64_t bits_of(double x) { return (uint64_t)__double_as_longlong(x); }
+DT_HD double of_bits(uint64_t b) { return __longlong_as_double((long long)b); }
+DT_HD float seed_rcp(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+DT_HD float seed_rsqrt(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+DT_HD uint32_t bits_of(float x) { return __float_as_uint(x); }
+DT_HD float of_bits(uint32_t b) { return __uint_as_float(b); }
+#else
+DT_HD uint64_t bits_of(double x) { uint64_t b; __builtin_memcpy(&b, &x, 8); return b; }
+DT_HD double of_bits(uint64_t b) { double x; __builtin_memcpy(&x, &b, 8); return x; }
+DT_HD float seed_rcp(float x) { return 1.0f / x; }
+DT_HD float seed_rsqrt(float x) { return 1.0f / sqrtf(x); }
+DT_HD uint32_t bits_of(float x) { uint32_t b; __builtin_memcpy(&b, &x, 4); return b; }
+DT_HD float of_bits(uint32_t b) { float x; __builtin_memcpy(&x, &b, 4); return x; }
+#endif
+// |x| cut to FP32, and back; x within 2^+-125
+constexpr uint64_t kExpShift = 896ull << 52;  // difference of the exponent biases
+DT_HD bool fp32_range(double x) { return ((uint32_t)(bits_of(x) >> 52) & 0x7ffu) - 898u <= 250u; }
+DT_HD float cut(double x) { return of_bits((uint32_t)(((bits_of(x) & 0x7fffffffffffffffull) - kExpShift) >> 29)); }
+DT_HD double widen(float x) { return of_bits((uint64_t)(((uint64_t)bits_of(x) << 29) + kExpShift)); }  // x > 0, normal
+
+// 1 / x: one third-order Newton step, r (1 + e + e^2) with e = 1 - x r of 2^-22
+DT_HD double rcp_d(double x) {
+    if (!fp32_range(x)) return 1.0 / x;
+    const double r = of_bits((uint64_t)(bits_of(widen(seed_rcp(cut(x)))) | (bits_of(x) & 0x8000000000000000ull)));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+// 1 / sqrt(x) and root = sqrt(x): one third-order step, y (1 + e / 2 + 3 e^2 / 8), e = 1 - x y^2
+DT_HD double rsqrt_d(double x, double &root) {
+    if (!(x > 0.0) || !fp32_range(x)) {
+        root = sqrt(x);
+        return 1.0 / root;
+    }
+    const double y = widen(seed_rsqrt(cut(x))), t = x * y;
+    const double e = fma(-t, y, 1.0), p = fma(0.375, e, 0.5) * e;
+    root = fma(t, p, t);
+    return fma(y, p, y);
+}
+// sine and cosine of x in [0, pi]: Taylor polynomials around the nearest multiple of pi / 2
+// (terms to r^15 and r^16; the next ones are below 5e-17 on |r| <= pi / 4)
+DT_HD void sincos_d(double x, double &s, double &c) {
+    const float xf = (float)x;
+    const int k = xf < 0.78539816f ? 0 : (xf < 2.35619449f ? 1 : 2);
+    const double hi = k == 0 ? 0.0 : (k == 1 ? 1.5707963267948966 : 3.141592653589793);
+    const double lo = k == 0 ? 0.0 : (k == 1 ? 6.123233995736766e-17 : 1.2246467991473532e-16);
+    const double r = (x - hi) - lo, q = r * r;
+    double a = fma(q, -1.0 / 1307674368000.0, 1.0 / 6227020800.0);
+    a = fma(q, a, -1.0 / 39916800.0);
+    a = fma(q, a, 1.0 / 362880.0);
+    a = fma(q, a, -1.0 / 5040.0);
+    a = fma(q, a, 1.0 / 120.0);
+    a = fma(q, a, -1.0 / 6.0);
+    const double sr = fma(r * q, a, r);
+    double b = fma(q, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
+    b = fma(q, b, 1.0 / 479001600.0);
+    b = fma(q, b, -1.0 / 3628800.0);
+    b = fma(q, b, 1.0 / 40320.0);
+    b = fma(q, b, -1.0 / 720.0);
+    b = fma(q, b, 1.0 / 24.0);
+    b = fma(q, b, -0.5);
+    const double cr = fma(q, b, 1.0);
+    s = k == 0 ? sr : (k == 1 ? cr : -sr);
+    c = k == 0 ? cr : (k == 1 ? -sr : -cr);
+}
+// The angle in [0, pi] whose sine and cosine are s and c: FP32 atan2, then the angle left over
+// from its FP64 sine and cosine (below 1e-6, where the angle is its sine)
+DT_HD double angle_d(double s, double c) {
+    const double a = (double)atan2f((float)s, (float)c);
+    double sa, ca;
+    sincos_d(a, sa, ca);
+    return a + fma(s, ca, -(c * sa));
+}
 
 // ------------------------------------------------------------------ FP32 dual number
 // value + N derivative slots; simpleAD.h:20-245 chain rules

@@ -136,9 +136,9 @@ DT_D long long queue_reserve_n(const DevScene &sc, const Queue &q, unsigned k) {
     return (long long)slot;
 }
 
-// camera.cpp:52-60 / 75-83 / 40-50
-DT_D void camera_ray(const DevCamera &cam, double x, double y, float3 &o, float3 &d) {
-    const float3 ndc = mk((float)((x * cam.inv_w - 0.5) * 2.0), (float)((y * cam.inv_h - 0.5) * cam.ndc_ky), 1.f);
+// camera.cpp:52-60 / 75-83 / 40-50, from the NDC point
+DT_D void camera_ray_ndc(const DevCamera &cam, float nx, float ny, float3 &o, float3 &d) {
+    const float3 ndc = mk(nx, ny, 1.f);
     const float *m = cam.ndc2cam;
     float3 dc = normalize(mk(m[0] * ndc.x + m[1] * ndc.y + m[2] * ndc.z, m[3] * ndc.x + m[4] * ndc.y + m[5] * ndc.z,
                              m[6] * ndc.x + m[7] * ndc.y + m[8] * ndc.z));
@@ -146,6 +146,9 @@ DT_D void camera_ray(const DevCamera &cam, double x, double y, float3 &o, float3
     o = mk(c[3], c[7], c[11]);
     d = mk(c[0] * dc.x + c[1] * dc.y + c[2] * dc.z, c[4] * dc.x + c[5] * dc.y + c[6] * dc.z,
            c[8] * dc.x + c[9] * dc.y + c[10] * dc.z);
+}
+DT_D void camera_ray(const DevCamera &cam, double x, double y, float3 &o, float3 &d) {
+    camera_ray_ndc(cam, (float)((x * cam.inv_w - 0.5) * 2.0), (float)((y * cam.inv_h - 0.5) * cam.ndc_ky), o, d);
 }
 template <int N>
 DT_D RayAD<N> camera_ray_ad(const DevCamera &cam, double x, double y) {
@@ -680,7 +683,7 @@ DT_D int sample_reuse(const double *cdf, int n, double &u, double &pdf) {
     while (idx < n - 1 && __double_as_longlong(__ldg(cdf + idx + 1)) == __double_as_longlong(__ldg(cdf + idx))) ++idx;
     const double c0 = __ldg(cdf + idx);
     pdf = __ldg(cdf + idx + 1) - c0;
-    u = (u - c0) / pdf;
+    u = (u - c0) * rcp_d(pdf);
     return idx;
 }
 
@@ -712,9 +715,10 @@ DT_D int is_silhouette(const DevScene &sc, const DevEdge &e, const double3_ &p) 
 // volpathAD.cpp:231-280 / 540-589 (ALTERNATIVE_EDGE_SAMPLING): the edge point seen from x0
 // at parameter t, by angular interpolation between the edge's endpoints, in FP64 (near-
 // degenerate triangles cancel). w0 : wb = sin(theta (1 - t)) / l0 : sin(theta t) / l1,
-// normalised to a sum of 1; the angular pdf is the edge pdf / theta (theta returned). theta = acos(cos theta) as in the
-// reference; sin(theta t) and cos(theta t) come from one sincos and sin(theta (1 - t)) =
-// sin(theta) cos(theta t) - cos(theta) sin(theta t), with sin(theta) = |e0 x e1| / (l0 l1).
+// normalised to a sum of 1; the angular pdf is the edge pdf / theta (theta returned). theta comes
+// from its sine |e0 x e1| / (l0 l1) and cosine (the reference's acos loses the small angles);
+// sin(theta t) and cos(theta t) come from one sincos and sin(theta (1 - t)) = sin(theta)
+// cos(theta t) - cos(theta) sin(theta t).
 struct EdgePoint {
     double3_ w1, nrm;   // unit direction to the edge point, unit normal of (x0, v0, v1)
     double dist, inv_dist, w0, wb, theta;
@@ -723,23 +727,22 @@ DT_D bool edge_point_solve(const DevScene &sc, const DevEdge &e, const double3_ 
     const double3_ v0 = tod(f3(__ldg(sc.verts + e.v0))), v1 = tod(f3(__ldg(sc.verts + e.v1)));
     const double3_ e0 = v0 - x0, e1 = v1 - x0;
     const double3_ cr = crossd(e0, e1);
-    const double lc = lengthd(cr);
-    ep.nrm = cr * (1.0 / lc);
-    const double l0 = lengthd(e0), l1 = lengthd(e1), inv_l01 = 1.0 / (l0 * l1);
-    const double c = fmin(1.0, fmax(-1.0, dotd(e0, e1) * inv_l01));
-    const double theta = acos(c);
-    if (theta < kEpsD || theta > kPiD - kEpsD) return false;
+    double lc, l0, l1;
+    ep.nrm = cr * rsqrt_d(dotd(cr, cr), lc);
+    const double inv_l01 = rsqrt_d(dotd(e0, e0), l0) * rsqrt_d(dotd(e1, e1), l1);
+    const double c = dotd(e0, e1) * inv_l01, s = lc * inv_l01;
+    const double theta = angle_d(s, c);
+    if (!(theta >= kEpsD && theta <= kPiD - kEpsD)) return false;
     double st, ct;
-    sincos(theta * t, &st, &ct);
+    sincos_d(theta * t, st, ct);
     // the common factor 1 / sin(theta) of both weights cancels in the normalisation
-    double w0 = (lc * inv_l01 * ct - c * st) * l1, wb = st * l0;
-    const double inv = 1.0 / (w0 + wb);
+    double w0 = (s * ct - c * st) * l1, wb = st * l0;
+    const double inv = rcp_d(w0 + wb);
     w0 *= inv;
     wb *= inv;
     if (w0 < -kEpsD || wb < -kEpsD || fabs(w0 + wb - 1.0) > kEpsD) return false;
     const double3_ w = e0 * w0 + e1 * wb;
-    ep.dist = lengthd(w);
-    ep.inv_dist = 1.0 / ep.dist;
+    ep.inv_dist = rsqrt_d(dotd(w, w), ep.dist);
     ep.w1 = w * ep.inv_dist;
     ep.w0 = w0;
     ep.wb = wb;
@@ -803,8 +806,9 @@ DT_D float3 edge_subpath_dir(const EdgePoint &ep, int sgn) {
     return normalize(tof(ep.w1) + tof(ep.nrm) * a);
 }
 
-// eight resident blocks per SM: the kernel waits on the FP64 pipe and on traversal latency
-template <int N>
+// twelve resident blocks per SM: the kernel waits on the FP64 pipe and on traversal latency.
+// With library acos, sincos, square roots and divisions the FP64 pipe was 74 % busy.
+template <int N, bool kSurf>
 __global__ void __launch_bounds__(kBlock, 12) k_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                  long long rec_count, Queue qli, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -833,7 +837,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_edge(DevScene sc, RenderParams r
         float s[N];
         if (ok) ok = edge_point_solve(sc, e, x0, u, ep);
         // slot weight factor 1 / (angular pdf * sppse), angular pdf = pdf / theta
-        if (ok) ok = edge_point_slots<N>(sc, e, ep, r.x0d, ep.theta * rp.inv_sppse / pdf, s);
+        if (ok) ok = edge_point_slots<N>(sc, e, ep, r.x0d, ep.theta * rp.inv_sppse * rcp_d(pdf), s);
         float3 val = mk(0.f, 0.f, 0.f);
         int med1 = r.med;
         const float3 w1f = ok ? tof(ep.w1) : mk(0.f, 0.f, 1.f);
@@ -851,7 +855,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_edge(DevScene sc, RenderParams r
         }
         if (ok) {
             const float tr =
-                eval_transmittance(sc, tof(x0), w1f, r.kind == 0, med1, (float)ep.dist, rng, r.depth, c);
+                eval_transmittance<kSurf>(sc, tof(x0), w1f, r.kind == 0, med1, (float)ep.dist, rng, r.depth, c);
             ok = tr > kEps;
         }
         if (ok) {
@@ -1061,31 +1065,39 @@ __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp
 
 // ====================================================================== primary edges
 // A primary-edge sample's point (edge_manager.cpp:112-134, camera.cpp): the screen point at
-// parameter u along the edge, its pixel, the edge's unit screen normal, and the distance to
-// the edge point in camera space (the edge-point solve of compute_intersection_in_tri,
-// utils.cpp:256-266, with the edge's constants precomputed on the host), in FP64.
+// parameter u along the edge and its pixel, in FP64.
 struct PrimaryPoint {
-    double px, py, nx, ny;
+    double px, py;
     int ipx, ipy;
-    float maxd;
 };
-DT_D void primary_edge_point(const DevCamera &cam, const DevPrimaryEdge &e, double u, PrimaryPoint &pp) {
-    pp.px = e.v0s[0] + (e.v1s[0] - e.v0s[0]) * u;
-    pp.py = e.v0s[1] + (e.v1s[1] - e.v0s[1]) * u;
-    pp.ipx = (int)floor(pp.px);
-    pp.ipy = (int)floor(pp.py);
-    pp.nx = e.n[0];
-    pp.ny = e.n[1];
-    const double a0 = (pp.px * cam.inv_w - 0.5) * cam.plane_kx - e.v0p[0];
-    const double a1 = (pp.py * cam.inv_h - 0.5) * cam.plane_ky - e.v0p[1];
-    const double a2 = 1.0 - e.v0p[2];
-    const double t0 = sqrt(a0 * a0 + a1 * a1 + a2 * a2) * e.inv_lenp;
-    const double bx = (1.0 - t0) * e.cb, by = t0 * e.cc;
-    const double t1 = by / (bx + by);
-    double pc[3];
-    for (int q = 0; q < 3; ++q) pc[q] = e.v0c[q] + t1 * (e.v1c[q] - e.v0c[q]);
-    pp.maxd = (float)sqrt(pc[0] * pc[0] + pc[1] * pc[1] + pc[2] * pc[2]);
+DT_D void primary_edge_point(const DevPrimaryEdge &e, double u, PrimaryPoint &pp) {
+    pp.px = fma(e.dvs[0], u, e.v0s[0]);
+    pp.py = fma(e.dvs[1], u, e.v0s[1]);
+    pp.ipx = __double2int_rd(pp.px);
+    pp.ipy = __double2int_rd(pp.py);
 }
+// The distance to the edge point in camera space (the edge-point solve of
+// compute_intersection_in_tri, utils.cpp:256-266, with the edge's constants from the host).
+DT_D float primary_edge_dist(const DevPrimaryEdge &e, double u) {
+    const double t0 = fma(e.t0[1], u, e.t0[0]);
+    const double by = t0 * e.cc, t1 = by * rcp_d(fma(-e.cb, t0, e.cb) + by);
+    const double x = fma(t1, e.dvc[0], e.v0c[0]), y = fma(t1, e.dvc[1], e.v0c[1]), z = fma(t1, e.dvc[2], e.v0c[2]);
+    double dist;
+    rsqrt_d(x * x + y * y + z * z, dist);
+    return (float)dist;
+}
+// The camera rays through the screen point (0) and 1e-4 pixels to either side of it along the
+// edge's screen normal (-1, 1)
+struct PrimaryNdc {
+    double x, y;
+    DT_D PrimaryNdc(const DevCamera &cam, const PrimaryPoint &pp)
+        : x(fma(pp.px, cam.px_ndc[0], -1.0)), y(fma(pp.py, cam.px_ndc[1], cam.ndc_y0)) {}
+    DT_D void ray(const DevCamera &cam, const DevPrimaryEdge &e, int side, float3 &o, float3 &d) const {
+        const double sx = side == 0 ? x : (side < 0 ? x - e.dn[0] : x + e.dn[0]);
+        const double sy = side == 0 ? y : (side < 0 ? y - e.dn[1] : y + e.dn[1]);
+        camera_ray_ndc(cam, (float)sx, (float)sy, o, d);
+    }
+};
 
 // Sort key of primary-edge sample k: the top 20 bits of its first random number, which
 // picks the edge and the point on it (sample_reuse): samples in key order lie along the
@@ -1102,7 +1114,9 @@ __global__ void k_primary_keys(RenderParams rp, unsigned *keys, int *vals) {
     vals[gi] = (int)gi;
 }
 
-template <int N>
+// Bound by the FP64 pipe (77 % busy with library square roots and divisions and the image-plane
+// point of each sample); what only visible samples need is computed after the visibility test.
+template <int N, bool kSurf>
 __global__ void __launch_bounds__(kBlock, 10) k_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                     unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -1118,9 +1132,9 @@ __global__ void __launch_bounds__(kBlock, 10) k_primary(DevScene sc, RenderParam
         const DevPrimaryEdge &e = sc.pedges[idx];
         const DevCamera &cam = sc.cam;
         PrimaryPoint pp;
-        primary_edge_point(cam, e, u, pp);
+        primary_edge_point(e, u, pp);
         // screen velocity of the edge point along its normal, per slot (FP32)
-        const float uf = (float)u, nxf = (float)pp.nx, nyf = (float)pp.ny;
+        const float uf = (float)u, nxf = (float)e.n[0], nyf = (float)e.n[1];
         float sv[N];
         bool moving = false;
 #pragma unroll
@@ -1130,20 +1144,18 @@ __global__ void __launch_bounds__(kBlock, 10) k_primary(DevScene sc, RenderParam
             moving = moving || fabsf(pdx) > kEps || fabsf(pdy) > kEps;
             sv[j] = nxf * pdx + nyf * pdy;
         }
-        const int ipx = pp.ipx, ipy = pp.ipy;
-        const double fx = pp.px - ipx, fy = pp.py - ipy, nx = pp.nx, ny = pp.ny;
-        const float maxd = pp.maxd;
-        const int lx = ipx - rp.crop_x, ly = ipy - rp.crop_y;
+        const int lx = pp.ipx - rp.crop_x, ly = pp.ipy - rp.crop_y;
         if (moving && lx >= 0 && ly >= 0 && lx < rp.out_w && ly < rp.out_h) {
             float3 o, d;
-            camera_ray(cam, ipx + fx, ipy + fy, o, d);
-            const float tr = eval_transmittance(sc, o, d, false, cam.med_id, maxd, rng, rp.max_bounces - 1, c);
+            const PrimaryNdc ndc(cam, pp);
+            ndc.ray(cam, e, 0, o, d);
+            const float tr = eval_transmittance<kSurf>(sc, o, d, false, cam.med_id, primary_edge_dist(e, u), rng,
+                                                       rp.max_bounces - 1, c);
             if (tr > kEps) {
                 const long long slot = queue_reserve_n(sc, qli, 2);  // the pair in adjacent slots
                 for (int sgn = 0; sgn < 2 && slot >= 0; ++sgn) {
-                    const double delta = sgn == 0 ? -1e-4 : 1e-4;
                     float3 o2, d2;
-                    camera_ray(cam, ipx + fx + nx * delta, ipy + fy + ny * delta, o2, d2);
+                    ndc.ray(cam, e, sgn == 0 ? -1 : 1, o2, d2);
                     LiTask<N> &t = reinterpret_cast<LiTask<N> *>(qli.data)[slot + sgn];
                     t.o[0] = o2.x; t.o[1] = o2.y; t.o[2] = o2.z;
                     t.d[0] = d2.x; t.d[1] = d2.y; t.d[2] = d2.z;

@@ -287,7 +287,8 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
                 const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
                 if ((rc = timed(ms_edge, [&] {
-                         k_edge<N><<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
+                         const auto k = surfaces_only(sc) ? k_edge<N, true> : k_edge<N, false>;
+                         k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
                      })))
                     return rc;
                 if ((rc = drain_li())) return rc;
@@ -310,7 +311,8 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             rp.prim_count = std::min(chunk, ns - k0);
             if ((rc = timed(ms_primary, [&] {
                      const int *perm = li_sorted ? sort_primary_samples(rp, sb, li_cap, st, launches) : nullptr;
-                     k_primary<N><<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
+                     const auto k = surfaces_only(sc) ? k_primary<N, true> : k_primary<N, false>;
+                     k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
                  })))
                 return rc;
             if ((rc = drain_li())) return rc;
@@ -506,7 +508,8 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
             tot_lins += nl;
             for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
                 const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
-                k_edge<N><<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, nullptr);
+                const auto k = surfaces_only(sc) ? k_edge<N, true> : k_edge<N, false>;
+                k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, nullptr);
                 if ((rc = launched())) return rc;
                 if ((rc = drain_li())) return rc;
             }
@@ -526,7 +529,8 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
         for (long long k0 = 0; k0 < ns; k0 += chunk) {
             rp.prim_begin = k0;
             rp.prim_count = std::min(chunk, ns - k0);
-            k_primary<N><<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, nullptr, nullptr);
+            const auto k = surfaces_only(sc) ? k_primary<N, true> : k_primary<N, false>;
+            k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, nullptr, nullptr);
             if ((rc = launched())) return rc;
             if ((rc = drain_li())) return rc;
         }

@@ -96,7 +96,7 @@ struct DevCamera {
     // pipe runs at 1/64 of FP32: one division is about ten of its instructions)
     double inv_w, inv_h;     // 1 / width, 1 / height
     double ndc_ky;           // -2 / aspect
-    double plane_kx, plane_ky;  // 2 / fov, -2 / (aspect fov): pixel to image plane
+    double px_ndc[2], ndc_y0;  // pixel to NDC in one operation: x px_ndc[0] - 1, y px_ndc[1] + ndc_y0
 };
 
 struct DevEdge {
@@ -106,12 +106,14 @@ struct DevEdge {
 };
 
 struct DevPrimaryEdge {
-    double v0s[2], v1s[2];               // screen position in pixels
+    double v0s[2], dvs[2];               // first screen endpoint in pixels, difference to the second
     float d0[kMaxNder][2], d1[kMaxNder][2];
-    double v0p[3], v1p[3], v0c[3], v1c[3]; // image plane and camera-space endpoints
+    double v0c[3], dvc[3];               // first camera-space endpoint, difference to the second
     // per-edge constants of the edge-point solve (utils.cpp:256-266): unit screen-space
-    // normal, 1 / |v1p - v0p|, |v0p| / |v0c| and |v1p| / |v1c|
-    double n[2], inv_lenp, cb, cc;
+    // normal, its 1e-4 pixels in NDC, |v0p| / |v0c| and |v1p| / |v1c| of the image-plane
+    // endpoints vp, and the image-plane parameter t0 of the screen point at u (linear: the
+    // screen point moves along the projected edge) as t0[0] + t0[1] u
+    double n[2], dn[2], cb, cc, t0[2];
 };
 
 struct __align__(16) BvhNode {
@@ -147,7 +149,8 @@ struct DevScene {
     int has_edges;
     // primary edges, edge_manager.cpp
     const DevPrimaryEdge *pedges;
-    const float *pedge_jac;        // [num_pedges][end][x,y][6]: screen-point Jacobian (pixels) w.r.t. (v0, v1)
+    const double *pedge_jac;       // [num_pedges][2][6]: screen velocity of the edge point along the edge normal
+                                   // (pixels) w.r.t. (v0, v1), at u = 0 and its change to u = 1
     const int *pedge_verts;        // [num_pedges][2] global vertex ids of the edge
     const double *pedge_cdf;       // num_pedges+1 entries
     int num_pedges;

@@ -170,7 +170,8 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
         tot_edge += ne;
         for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
             const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
-            k_vadj_edge<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
+            const auto k = surfaces_only(sc) ? k_vadj_edge<true> : k_vadj_edge<false>;
+            k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
             ++launches;
             DT_VCK(cudaGetLastError());
             if ((rc = drain_li())) return rc;
@@ -192,7 +193,8 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
             rp.prim_begin = k0;
             rp.prim_count = std::min(chunk, ns - k0);
             const int *perm = li_sorted ? sort_primary_samples(rp, sb, li_cap, st, launches) : nullptr;
-            k_vadj_primary<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
+            const auto k = surfaces_only(sc) ? k_vadj_primary<true> : k_vadj_primary<false>;
+            k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
             ++launches;
             DT_VCK(cudaGetLastError());
             if ((rc = drain_li())) return rc;

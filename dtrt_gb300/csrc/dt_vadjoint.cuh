@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_chain(DevScene sc, RenderParams
 
 // one thread per (edge record, edge sample): k_edge's geometry, then two VLiTasks carrying
 // the gradient coefficients instead of per-slot scalars
+template <bool kSurf>
 __global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                       long long rec_count, Queue qli, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -344,13 +345,13 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderPar
             ok = !is_zero3(val);
         }
         if (ok) {
-            const float tr = eval_transmittance(sc, tof(x0), w1f, true, med1, (float)dist, rng, r.depth, c);
+            const float tr = eval_transmittance<kSurf>(sc, tof(x0), w1f, true, med1, (float)dist, rng, r.depth, c);
             ok = tr > kEps;
         }
         if (ok) {
             // s(V) = m . (w0 dv0 + wb dv1 - dx0), m = (n_e - (n_e.w1) w1) / (dist pdf sppse)
             // 1 / (dist * angular pdf * sppse), angular pdf = pdf / theta
-            const double nw = dotd(nrm, w1), k2 = ep.theta * rp.inv_sppse / (dist * pdf);
+            const double nw = dotd(nrm, w1), k2 = ep.theta * rp.inv_sppse * ep.inv_dist * rcp_d(pdf);
             const double3_ m = (nrm - w1 * nw) * k2;
             const float3 c0 = tof(m * w0), c1 = tof(m * wb), cx = tof(m * (-(w0 + wb)));
             const long long slot = queue_reserve_n(sc, qli, 2);  // the pair in adjacent slots
@@ -374,6 +375,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderPar
 }
 
 // one thread per primary-edge sample: k_primary's geometry with the projection Jacobian
+template <bool kSurf>
 __global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                          unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -389,28 +391,23 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, Render
         const DevPrimaryEdge &e = sc.pedges[idx];
         const DevCamera &cam = sc.cam;
         PrimaryPoint pp;
-        primary_edge_point(cam, e, u, pp);
-        const int ipx = pp.ipx, ipy = pp.ipy;
-        const double fx = pp.px - ipx, fy = pp.py - ipy, nx = pp.nx, ny = pp.ny;
-        const float maxd = pp.maxd;
-        const int lx = ipx - rp.crop_x, ly = ipy - rp.crop_y;
+        primary_edge_point(e, u, pp);
+        const int lx = pp.ipx - rp.crop_x, ly = pp.ipy - rp.crop_y;
         if (lx >= 0 && ly >= 0 && lx < rp.out_w && ly < rp.out_h) {
-            // screen velocity of the edge point: ((1-u) J0 + u J1) [dv0; dv1], J in pixels
-            const float *J = sc.pedge_jac + (size_t)idx * 24;  // [end][coord][6]
-            float cv[6];
-            for (int q = 0; q < 6; ++q) {
-                const double jx = J[q] * (1.0 - u) + J[12 + q] * u, jy = J[6 + q] * (1.0 - u) + J[18 + q] * u;
-                cv[q] = (float)(nx * jx + ny * jy);
-            }
             float3 o, d;
-            camera_ray(cam, ipx + fx, ipy + fy, o, d);
-            const float tr = eval_transmittance(sc, o, d, false, cam.med_id, maxd, rng, rp.max_bounces - 1, c);
+            const PrimaryNdc ndc(cam, pp);
+            ndc.ray(cam, e, 0, o, d);
+            const float tr = eval_transmittance<kSurf>(sc, o, d, false, cam.med_id, primary_edge_dist(e, u), rng,
+                                                       rp.max_bounces - 1, c);
             if (tr > kEps) {
+                // screen velocity of the edge point along the normal, per coordinate of v0 and v1
+                const double *J = sc.pedge_jac + (size_t)idx * 12;
+                float cv[6];
+                for (int q = 0; q < 6; ++q) cv[q] = (float)fma(J[6 + q], u, J[q]);
                 const long long slot = queue_reserve_n(sc, qli, 2);  // the pair in adjacent slots
                 for (int sgn = 0; sgn < 2 && slot >= 0; ++sgn) {
-                    const double delta = sgn == 0 ? -1e-4 : 1e-4;
                     float3 o2, d2;
-                    camera_ray(cam, ipx + fx + nx * delta, ipy + fy + ny * delta, o2, d2);
+                    ndc.ray(cam, e, sgn == 0 ? -1 : 1, o2, d2);
                     VLiTask &t = reinterpret_cast<VLiTask *>(qli.data)[slot + sgn];
                     t.o[0] = o2.x; t.o[1] = o2.y; t.o[2] = o2.z;
                     t.d[0] = d2.x; t.d[1] = d2.y; t.d[2] = d2.z;
