@@ -476,6 +476,10 @@ constexpr long long kWavefrontMinPaths = 1 << 16;
 // 14.4 / 14.1 / 13.5 / 13.9 ms at 3 / 4 / 5 / 6 blocks; C3, nder 8: 71.0 / 68.0 / 68.3 / 68.8).
 template <int N>
 constexpr int kCamBlocks = N > 4 ? 4 : 5;
+// With ray derivatives (camera stage of C0, nder 1: 3.03 / 2.39 / 2.19 / 2.09 ms at 2 / 3 / 4 /
+// 5 blocks; C2, nder 8: 10.90 / 10.46 / 10.71 / 10.78).
+template <int N>
+constexpr int kCamBlocksAd = N > 4 ? 3 : 4;
 
 // Wavefront schedule: paths that continue are compacted into a queue of path indices
 // after every vertex, so each launch runs one vertex of live paths only (a warp no longer
@@ -563,7 +567,7 @@ DT_D void store_state(CamState<N, G> *states, int id, const CamState<N, G> &st, 
 // sampling. An interface vertex (every path from a camera outside media) runs here too and
 // the path goes on to level 1's distance sampling; a volume vertex is queued for level 0.
 template <int N, int G>
-__global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
+__global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : kCamBlocksAd<N>) k_cam_start(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                       VertexIn *vins, int *qv0, unsigned long long *cnt_v0,
                                                       int *qv1, unsigned long long *cnt_v1, int *qs1,
                                                       unsigned long long *cnt_s1, unsigned long long *cnt_s1_back,
@@ -615,7 +619,7 @@ struct LevelQueue {
 // Vertex level L: its volume and interface vertices; a continuing path then runs level L+1's
 // distance sampling (camera_next).
 template <int N, int G>
-__global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : 1) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
+__global__ void __launch_bounds__(kBlock, G == 0 ? kCamBlocks<N> : kCamBlocksAd<N>) k_cam_vertex(DevScene sc, RenderParams rp, CamState<N, G> *states,
                                                        VertexIn *vins, const int *qv, const unsigned long long *cnt_v,
                                                        const int *qs, const unsigned long long *cnt_s,
                                                        const unsigned long long *cnt_s_back, int *qv_next,

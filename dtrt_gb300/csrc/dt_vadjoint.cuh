@@ -116,6 +116,8 @@ DT_D float3 channel_grad(const DV<3> &v, float3 w) {
 // Stage of a camera-path replay
 enum { VR_VALUE = 0, VR_FRAME = 1, VR_CHAIN = 2 };
 
+// Rays and hits have width 0: the gradient takes path values only, the derivatives are local
+// (with k_vadj_camera and k_vadj_chain at four blocks per SM: C2 vertex adjoint 22.2 -> 21.4 ms).
 // One camera path of k_camera's loop on a surface scene (no media: NEE, emitter lookups
 // and edge visibility consume no random numbers beyond the 9 draws per level), value-only.
 //   VR_VALUE: returns the sum of event contributions; pushes a VEdgeRec per non-null vertex
@@ -135,8 +137,8 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
         jx = rng.next1d();
         jy = rng.next1d();
     }
-    RayAD<1> ray = camera_ray_ad<1>(sc.cam, ix + jx, iy + jy);
-    ItsAD<1> its;
+    RayAD<0> ray = camera_ray_ad<0>(sc.cam, ix + jx, iy + jy);
+    ItsAD<0> its;
     int depth = rp.max_bounces;
     int mode = rp.mode;
     float3 P = mk(1.f, 1.f, 1.f), acc = zero;
@@ -144,7 +146,7 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
     int cprim[kVMaxLevels];
     float3 cd[kVMaxLevels], cp[kVMaxLevels];
     int nlev = 0;
-    bool alive = ray_intersect_ad<1>(sc, ray, false, its, c);
+    bool alive = ray_intersect_ad<0>(sc, ray, false, its, c);
     for (int level = 0; alive && mode != 0; ++level) {
         alive = false;
         rng.next1(); rng.next1();  // distance-sampling draws (no medium)
@@ -161,11 +163,11 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
         }
         const DevShape &sh = sc.shapes[its.shape];
         const float3 Q = P;
-        if (sh.light_id >= 0 && (mode & MODE_EMISSION)) acc = acc + cmul(Q, le_ad<1>(sc, its, -ray.d).val());
+        if (sh.light_id >= 0 && (mode & MODE_EMISSION)) acc = acc + cmul(Q, le_ad<0>(sc, its, -ray.d).val());
         if (depth == 0) break;
         const DevBsdf &b = sc.bsdfs[sh.bsdf_id];
         const bool is_null = b.type == BSDF_NULL;
-        const FrameAD<1> fr = its.frame();
+        const FrameAD<0> fr = its.frame();
         const Its its0 = its.plain();
         // edge record (interface edge term), volpathAD.cpp:513-616
         if (stage == VR_VALUE && !is_null && rp.sppse > 0 && (mode & MODE_SURFACE_BOUNDARY) && sc.has_edges &&
@@ -196,12 +198,12 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
             fr3 = FrameAD<3>(ns3);
             wi3 = fr3.to_local(-dir_in);
         }
-        DV<1> wo;
+        DV<0> wo;
         float pdf_nee;
         if (!is_null && (mode & MODE_SURFACE_MAIN)) {
-            DV<1> v = nee_surface_ad<1>(sc, its, fr, r2, rng, -1, depth - 1, wo, pdf_nee, c);
+            DV<0> v = nee_surface_ad<0>(sc, its, fr, r2, rng, -1, depth - 1, wo, pdf_nee, c);
             if (!v.is_zero()) {
-                const DV<1> bv = bsdf_eval_ad<1>(b, its.wi, wo);
+                const DV<0> bv = bsdf_eval_ad<0>(b, its.wi, wo);
                 const float bp = bsdf_pdf(b, its0.wi, wo.val());
                 const float3 e = cmul(cmul(Q, v.val()), bv.val()) * mis_weight(pdf_nee, bp);
                 if (stage == VR_FRAME && !is_zero3(e, 0.f)) {
@@ -213,7 +215,7 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
             }
         }
         float bpdf, beta;
-        const DV<1> bw = bsdf_sample_ad<1>(b, its, fr, its0, r3a, r3b, r3c, wo, bpdf, beta);
+        const DV<0> bw = bsdf_sample_ad<0>(b, its, fr, its0, r3a, r3b, r3c, wo, bpdf, beta);
         if (!bw.is_zero()) {
             if (stage == VR_FRAME && !is_null) {  // the sampling weight multiplies every later event
                 ItsAD<3> its3;
@@ -228,11 +230,11 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
             ray.o = its.p;
             ray.d = wo;
             float3 thr1 = mk(1.f, 1.f, 1.f);
-            ItsAD<1> its1;
+            ItsAD<0> its1;
             if (is_null) {
-                ray_intersect_ad<1>(sc, ray, true, its1, c);
+                ray_intersect_ad<0>(sc, ray, true, its1, c);
             } else {
-                DV<1> att = look_for_emitter_ad<1>(sc, ray, true, rng, -1, depth - 1, its1, pdf_nee, nullptr,
+                DV<0> att = look_for_emitter_ad<0>(sc, ray, true, rng, -1, depth - 1, its1, pdf_nee, nullptr,
                                                    nullptr, c);
                 thr1 = bw.val();
                 if (!att.is_zero() && (mode & MODE_SURFACE_MAIN))
@@ -259,7 +261,7 @@ DT_D float3 vreplay_path(const DevScene &sc, const RenderParams &rp, long long g
 }
 
 // one thread per camera path: value pass (edge records), then the frame-factor pass
-__global__ void __launch_bounds__(kBlock) k_vadj_camera(DevScene sc, RenderParams rp, const float *dimg, float *grad,
+__global__ void __launch_bounds__(kBlock, 4) k_vadj_camera(DevScene sc, RenderParams rp, const float *dimg, float *grad,
                                                         Queue qe, double *img_acc, int levels,
                                                         unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(kBlock) k_vadj_camera(DevScene sc, RenderParam
 }
 
 // one thread per camera path: the x0 gradient slots back to front
-__global__ void __launch_bounds__(kBlock) k_vadj_chain(DevScene sc, RenderParams rp, float *grad, const float *xadj,
+__global__ void __launch_bounds__(kBlock, 4) k_vadj_chain(DevScene sc, RenderParams rp, float *grad, const float *xadj,
                                                        int levels, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     if (gi >= rp.path_count) return;
