@@ -96,9 +96,9 @@ int gather_cells(const dtrt_scene *s, const DevScene &sc, float *grad, cudaStrea
     return launches;
 }
 
-bool ensure_lanes(Scratch &sb) {
+bool ensure_lanes(Scratch &sb, int lanes) {
     bool ok = sb.fork_ev || cudaEventCreateWithFlags(&sb.fork_ev, cudaEventDisableTiming) == cudaSuccess;
-    for (int k = 0; k < kLanes - 1 && ok; ++k) {
+    for (int k = 0; k < lanes - 1 && ok; ++k) {
         ok = sb.side[k] || cudaStreamCreateWithFlags(&sb.side[k], cudaStreamNonBlocking) == cudaSuccess;
         ok = ok && (sb.side_ev[k] || cudaEventCreateWithFlags(&sb.side_ev[k], cudaEventDisableTiming) == cudaSuccess);
     }

@@ -48,8 +48,8 @@ struct Scratch {
 };
 
 bool ensure_buffer(void **ptr, size_t *have, size_t need);
-// The lanes' streams and events: false (and the error cleared) when they cannot be made.
-bool ensure_lanes(Scratch &sb);
+// Streams and events of `lanes` lanes: false (and the error cleared) when they cannot be made.
+bool ensure_lanes(Scratch &sb, int lanes);
 
 // f(batch, lane, stream) for each of n batches, dealt in turn to st and lanes - 1 side streams
 // that fork from st and join it again.
@@ -82,14 +82,19 @@ inline bool ensure_li_sort(Scratch &sb, uint64_t li_cap) {
     return false;
 }
 
+// Fewer pairs or samples than this run in queue order: the sort's 13 launches take about 60 us,
+// more than it saves them (preview of 3,300 pairs: Li 0.25 -> 0.19 ms; render_scene, some
+// 2^17 samples a stage: 8.7 -> 8.4 ms with 2^18 here against 2^12).
+constexpr long long kSortMin = 1 << 17;
+
 // The n queued Li tasks' pairs (slots 2m, 2m + 1) in key order (k_li_keys) on stream st;
-// nullptr when n is odd or holds one pair (the queue is then read in order). Adds the
+// nullptr when n is odd or small (the queue is then read in order). Adds the
 // kernels it launches to `launches`.
 template <class Task>
 const int *sort_li_pairs(const DevScene &sc, const Task *tasks, long long n, Scratch &sb, uint64_t li_cap,
                          cudaStream_t st, uint64_t &launches) {
     const long long np = n / 2, cap = (long long)(li_cap / 2);
-    if ((n & 1) || np < 2 || np > cap) return nullptr;
+    if ((n & 1) || np < kSortMin || np > cap) return nullptr;
     unsigned *keys = (unsigned *)sb.li_sort, *keys2 = keys + cap;
     int *vals = (int *)(keys2 + cap), *vals2 = vals + cap;
     unsigned *hist = (unsigned *)(vals2 + cap);
@@ -99,12 +104,12 @@ const int *sort_li_pairs(const DevScene &sc, const Task *tasks, long long n, Scr
 }
 
 // The primary-edge samples [rp.prim_begin, + rp.prim_count) in key order (k_primary_keys),
-// in the Li sort's buffers (a chunk holds at most li_cap / 2 samples); nullptr for one.
+// in the Li sort's buffers (a chunk holds at most li_cap / 2 samples); nullptr for few.
 // Adds the kernels it launches to `launches`.
 inline const int *sort_primary_samples(const RenderParams &rp, Scratch &sb, uint64_t li_cap, cudaStream_t st,
                                        uint64_t &launches) {
     const long long cap = (long long)(li_cap / 2);
-    if (rp.prim_count < 2 || rp.prim_count > cap) return nullptr;
+    if (rp.prim_count < kSortMin || rp.prim_count > cap) return nullptr;
     unsigned *keys = (unsigned *)sb.li_sort, *keys2 = keys + cap;
     int *vals = (int *)(keys2 + cap), *vals2 = vals + cap;
     unsigned *hist = (unsigned *)(vals2 + cap);

@@ -187,6 +187,23 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         return DTRT_OK;
     };
 
+    // primary-edge samples, a chunk at most at once
+    uint64_t prim_samples = 0;
+    const long long prim_chunk = std::max<long long>(1, (long long)(li_cap / 2));
+    if (o->sppe > 0 && sc.num_pedges > 0) {
+        prim_samples = (uint64_t)std::ceil(sc.pedge_sum * o->sppe / 128.0) * 128;
+        rp.prim_weight = sc.pedge_sum / (double)prim_samples;
+    }
+    auto run_primary = [&](long long begin, long long count) -> int {
+        rp.prim_begin = begin;
+        rp.prim_count = count;
+        return timed(ms_primary, [&] {
+            const int *perm = li_sorted ? sort_primary_samples(rp, sb, li_cap, st, launches) : nullptr;
+            const auto k = surfaces_only(sc) ? k_primary<N, true> : k_primary<N, false>;
+            k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
+        });
+    };
+    bool prim_done = false;
     // ---------------------------------------------------------------- pass 1
     const long long total = (long long)npix * std::max(0, o->spp);
     launches += (uint64_t)prepare_cells(s, sc, total, false, st);
@@ -209,7 +226,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         const long long nb = (total + B - 1) / B;
         // several batches in flight; the counters read each batch's level counts, so one then
         int lanes = wavefront && fixed_rays && !ctr ? (int)std::min<long long>(kLanes, nb) : 1;
-        if (lanes > 1 && !ensure_lanes(sb)) lanes = 1;
+        if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
         if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * work_bytes) &&
                            ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * lanes * Bw * sizeof(int)) &&
                            ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * lanes * (levels + 1) * sizeof(unsigned long long)))) {
@@ -284,6 +301,15 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             const unsigned long long nl = std::min<unsigned long long>(hcnt[1], rec_cap);
             tot_edge += ne;
             tot_lins += nl;
+            // Lins records run on a side stream beside the edge samples and their Li sub-paths
+            const bool lins_aside = nl && ensure_lanes(sb, 2);
+            if (lins_aside) {
+                DT_CK(cudaEventRecord(sb.fork_ev, st));
+                DT_CK(cudaStreamWaitEvent(sb.side[0], sb.fork_ev, 0));
+                k_lins<N><<<blocks(nl), kBlock, 0, sb.side[0]>>>(sc, rp, ql, nl, sb.acc1, ctr);
+                ++launches;
+                DT_CK(cudaEventRecord(sb.side_ev[0], sb.side[0]));
+            }
             for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
                 const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
                 if ((rc = timed(ms_edge, [&] {
@@ -291,32 +317,27 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                          k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
                      })))
                     return rc;
+                // the primary-edge samples share the last Li launch where the queue holds both
+                if (prim_samples && b0 + B >= total && r0 + per_chunk >= ne &&
+                    2 * (prim_samples + (uint64_t)cnt * rp.sppse) <= li_cap) {
+                    if ((rc = run_primary(0, (long long)prim_samples))) return rc;
+                    prim_done = true;
+                }
                 if ((rc = drain_li())) return rc;
             }
             if (nl)
-                if ((rc = timed(ms_li, [&] { k_lins<N><<<blocks(nl), kBlock, 0, st>>>(sc, rp, ql, nl, sb.acc1, ctr); })))
+                if ((rc = timed(ms_li, [&] {
+                         if (lins_aside) cudaStreamWaitEvent(st, sb.side_ev[0], 0);
+                         else k_lins<N><<<blocks(nl), kBlock, 0, st>>>(sc, rp, ql, nl, sb.acc1, ctr);
+                     })))
                     return rc;
         }
     }
     // ---------------------------------------------------------------- pass 2: primary edges
-    uint64_t prim_samples = 0;
-    if (o->sppe > 0 && sc.num_pedges > 0) {
-        const long long nblock = (long long)std::ceil(sc.pedge_sum * o->sppe / 128.0);
-        const long long ns = nblock * 128;
-        prim_samples = (uint64_t)ns;
-        rp.prim_weight = sc.pedge_sum / (double)ns;
-        const long long chunk = std::max<long long>(1, (long long)(li_cap / 2));
-        for (long long k0 = 0; k0 < ns && !fixed_rays; k0 += chunk) {  // no edge moves on the screen under fixed rays
-            rp.prim_begin = k0;
-            rp.prim_count = std::min(chunk, ns - k0);
-            if ((rc = timed(ms_primary, [&] {
-                     const int *perm = li_sorted ? sort_primary_samples(rp, sb, li_cap, st, launches) : nullptr;
-                     const auto k = surfaces_only(sc) ? k_primary<N, true> : k_primary<N, false>;
-                     k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
-                 })))
-                return rc;
-            if ((rc = drain_li())) return rc;
-        }
+    // (no edge moves on the screen under fixed rays)
+    for (long long k0 = 0; k0 < (long long)prim_samples && !fixed_rays && !prim_done; k0 += prim_chunk) {
+        if ((rc = run_primary(k0, std::min(prim_chunk, (long long)prim_samples - k0)))) return rc;
+        if ((rc = drain_li())) return rc;
     }
     // ---------------------------------------------------------------- finalize
     float *dst = out_on_device ? out : sb.out;
