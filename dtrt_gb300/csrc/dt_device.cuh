@@ -944,6 +944,14 @@ DT_D bool aabb_hit(const DevGrid &g, float3 o, float3 d, float &tn, float &tf) {
     return true;
 }
 
+// Scenes without media and null BSDFs (kNoMedia) or without density grids (kNoGrids) take the Li,
+// Lins and edge kernels' queries without the code they do not need: without media a shadow
+// ray is one any-hit traversal and an emitter lookup one closest hit; without grids a segment's
+// transmittance is one exponential. Their warps waited for instructions in 3 of 14 cycles per
+// issue (kNoMedia, with the pair sums of k_li: C2 forward 89.4 -> 81.1 ms, vertex adjoint 26.7 ->
+// 24.7, primal mesh 1.72 -> 1.55; kNoGrids: C0 forward 18.1 -> 17.4, render_scene 8.3 -> 8.2).
+enum { kAnyMedia = 0, kNoMedia = 1, kNoGrids = 2 };
+
 // ------------------------------------------------------------------ media
 DT_D float3 sig_s(const DevScene &sc, const DevMedium &m, float3 x, Ctr &c) {  // homogeneous.h:57, heterogeneous.h:88-90
     if (m.type == MEDIUM_HOMOGENEOUS) return f3(m.sigma_s);
@@ -951,9 +959,10 @@ DT_D float3 sig_s(const DevScene &sc, const DevMedium &m, float3 x, Ctr &c) {  /
 }
 
 // homogeneous.cpp:6-24 / heterogeneous.cpp:9-37; moves `o` to the scatter point
+template <int kMedia = kAnyMedia>
 DT_HEAVY bool sample_distance(const DevScene &sc, const DevMedium &m, float3 &o, float3 d, float tmax, float r0, float r1,
                           Rng &rng, float3 &thr, Ctr &c) {
-    if (m.type == MEDIUM_HOMOGENEOUS) {
+    if (kMedia == kNoGrids || m.type == MEDIUM_HOMOGENEOUS) {
         if (m.sampling_weight > kEps) {
             const float t = -logf(r0) / m.sigma_t;
             if (t < tmax) {
@@ -1170,9 +1179,10 @@ DT_D bool medium_step(const DevScene &sc, const DevMedium &m, RayAD<G> &ray, con
 }
 
 // homogeneous.cpp:52-55 / heterogeneous.cpp:78-91 (residual ratio tracking)
+template <int kMedia = kAnyMedia>
 DT_HEAVY float medium_transmittance(const DevScene &sc, const DevMedium &m, float3 o, float3 d, float tmin, float tmax,
                                 Rng &rng, Ctr &c) {
-    if (m.type == MEDIUM_HOMOGENEOUS) return expf((tmin - tmax) * m.sigma_t);
+    if (kMedia == kNoGrids || m.type == MEDIUM_HOMOGENEOUS) return expf((tmin - tmax) * m.sigma_t);
     float ret = 1.f, t = tmin;
     int steps = 0;
     while (ret > kEps) {
@@ -1225,20 +1235,14 @@ DT_D bool ray_intersect_ad(const DevScene &sc, const RayAD<N> &ray, bool on_surf
     return true;
 }
 
-// Scenes of opaque surfaces alone (no medium, no null BSDF: host, surfaces_only()) take these
-// queries with kSurf: a shadow ray is one any-hit traversal, an emitter lookup one closest
-// hit, and the tracking loops and chains leave the kernel, whose warps waited for
-// instructions in 3 of 14 cycles per issue (with the pair sums of k_li: C2 forward 89.4 ->
-// 81.1 ms, vertex adjoint 26.7 -> 24.7, primal mesh 1.72 -> 1.55).
-
 // scene.cpp:177-237
-template <bool kSurf = false>
+template <int kMedia = kAnyMedia>
 DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool on_surface, int med,
                               float remaining, Rng &rng, int max_inter, Ctr &c) {
     float tmin = on_surface ? kShadowEps : 0.f;
     float tfar = (1.f - kShadowEps) * remaining;
     float tr = 1.f;
-    if constexpr (kSurf) {
+    if constexpr (kMedia == kNoMedia) {
         float th;
         return remaining > 0.f && closest_hit(sc, o, d, tmin, tfar, th, c, true) >= 0 ? 0.f : 1.f;
     }
@@ -1255,7 +1259,7 @@ DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool o
             shape_intersect(sc, prim, o, d, its);
             if (its.t < tmax) tmax = its.t;
         }
-        if (med >= 0) tr *= medium_transmittance(sc, sc.media[med], o, d, tmin, tmax, rng, c);
+        if (med >= 0) tr *= medium_transmittance<kMedia>(sc, sc.media[med], o, d, tmin, tmax, rng, c);
         if (prim < 0) break;
         const DevShape &s = sc.shapes[its.shape];
         if (is_transition(s)) med = dot(its.ng, d) > 0.f ? s.med_ext : s.med_int;
@@ -1269,7 +1273,7 @@ DT_HEAVY float eval_transmittance(const DevScene &sc, float3 o, float3 d, bool o
 }
 
 // scene.cpp:617-701
-template <bool kSurf = false>
+template <int kMedia = kAnyMedia>
 DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on_surface, Rng &rng, int med,
                              int max_inter, Its &its, float &pdf_nee, Ctr &c) {
     float tmin = on_surface ? kShadowEps : 0.f, th;
@@ -1282,7 +1286,7 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on
         return zero;
     }
     shape_intersect(sc, prim, o, d, its);
-    if constexpr (kSurf) {
+    if constexpr (kMedia == kNoMedia) {
         const DevShape &s = sc.shapes[its.shape];
         if (s.light_id < 0) return zero;
         const float3 dp = its.p - scatter;
@@ -1290,7 +1294,7 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on
         pdf_nee = sc.light_pmf[s.light_id] / (sc.light_area[s.light_id] * G);
         return le(sc, its, -d);
     }
-    if (sc.has_grid_media) {  // geometry first: chains that miss every emitter skip transmittance
+    if (kMedia == kAnyMedia && sc.has_grid_media) {  // geometry first: chains that miss every emitter skip transmittance
         float3 o1 = o;
         Its n1 = its;
         int p1 = prim;
@@ -1314,7 +1318,7 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on
     for (int inter = 0; inter < kMaxInteractions; ++inter) {
         if (inter > 0) shape_intersect(sc, prim, o, d, ni);
         const float tmax = ni.t;
-        if (med >= 0) tr *= medium_transmittance(sc, sc.media[med], o, d, tmin, tmax, rng, c);
+        if (med >= 0) tr *= medium_transmittance<kMedia>(sc, sc.media[med], o, d, tmin, tmax, rng, c);
         const DevShape &s = sc.shapes[ni.shape];
         if (s.light_id >= 0) {
             const float3 dp = ni.p - scatter;
@@ -1420,6 +1424,7 @@ DT_HEAVY DV<N> look_for_emitter_ad(const DevScene &sc, RayAD<G> ray, bool on_sur
 }
 
 // scene.cpp:399-426 (from a point in a medium; wo in world space)
+template <int kMedia = kAnyMedia>
 DT_HEAVY float3 nee_point(const DevScene &sc, float3 p, const float rnd[4], Rng &rng, int med, int max_inter,
                       float3 &wo, float &pdf, Ctr &c) {
     float3 lp, ln;
@@ -1430,7 +1435,7 @@ DT_HEAVY float3 nee_point(const DevScene &sc, float3 p, const float rnd[4], Rng 
     if (dot(dir, ln) < 0.f && pdf != 0.f) {
         const float dist = length(dir);
         dir = dir / dist;
-        const float tr = eval_transmittance(sc, p, dir, false, med, dist, rng, max_inter, c);
+        const float tr = eval_transmittance<kMedia>(sc, p, dir, false, med, dist, rng, max_inter, c);
         if (tr != 0.f) {
             pdf *= dist * dist / dot(ln, -dir);
             wo = dir;
@@ -1441,7 +1446,7 @@ DT_HEAVY float3 nee_point(const DevScene &sc, float3 p, const float rnd[4], Rng 
 }
 
 // scene.cpp:456-491 (from a surface; wo in the local shading frame)
-template <bool kSurf = false>
+template <int kMedia = kAnyMedia>
 DT_HEAVY float3 nee_surface(const DevScene &sc, const Its &its, const float rnd[4], Rng &rng, int med,
                         int max_inter, float3 &wo, float &pdf, bool flag, Ctr &c) {
     float3 lp, ln;
@@ -1459,7 +1464,7 @@ DT_HEAVY float3 nee_surface(const DevScene &sc, const Its &its, const float rnd[
         wo = its.to_local(dir);
         if (flag && signum(its.wi.z) != signum(wo.z)) --max_inter;
         if (max_inter >= 0) {
-            const float tr = eval_transmittance<kSurf>(sc, its.p, dir, true, med, dist, rng, max_inter, c);
+            const float tr = eval_transmittance<kMedia>(sc, its.p, dir, true, med, dist, rng, max_inter, c);
             if (tr != 0.f) {
                 pdf *= dist * dist / dot(ln, -dir);
                 return le_normal(sc.emitters[l], ln, -dir) * (tr / pdf);
@@ -1561,9 +1566,9 @@ DT_D bool li_start(const DevScene &sc, LiState &s, float3 o, float3 d, int max_d
     return s.depth <= s.max_depth;
 }
 
-// One vertex (one iteration of the loop at s.depth): false when the path ends. With kSurf an
+// One vertex (one iteration of the loop at s.depth): false when the path ends. With kNoMedia an
 // escaped path ends before it draws the vertex's random numbers, which nothing reads.
-template <bool kSurf = false>
+template <int kMedia = kAnyMedia>
 DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     Rng &rng = s.rng;
     Its &its = s.its;
@@ -1571,19 +1576,19 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     int &med = s.med;
     const int depth = s.depth, max_depth = s.max_depth;
     const int max_inter = max_depth - depth - 1;
-    if (kSurf && !its.valid()) return false;
+    if (kMedia == kNoMedia && !its.valid()) return false;
     const float r1a = rng.next1(), r1b = rng.next1();
     float r2[4];
     r2[0] = rng.next1(); r2[1] = rng.next1(); r2[2] = rng.next1(); r2[3] = rng.next1();
     const float r3a = rng.next1(), r3b = rng.next1(), r3c = rng.next1();
-    const bool inside = !kSurf && med >= 0 && sample_distance(sc, sc.media[med], o, d, its.t, r1a, r1b, rng, thr, c);
+    const bool inside = kMedia != kNoMedia && med >= 0 && sample_distance<kMedia>(sc, sc.media[med], o, d, its.t, r1a, r1b, rng, thr, c);
     if (inside) {
         if (depth >= max_depth) return false;
         if (is_zero3(thr)) return false;
         const DevPhase &ph = sc.phases[sc.media[med].phase_id];
         float3 wo;
         float pdf_nee;
-        const float3 v = nee_point(sc, o, r2, rng, med, max_inter, wo, pdf_nee, c);
+        const float3 v = nee_point<kMedia>(sc, o, r2, rng, med, max_inter, wo, pdf_nee, c);
         if (!is_zero3(v)) {
             const float pv = phase_eval(ph, -d, wo);
             if (pv > kEps) ret += cmul(thr, v) * (mis_weight(pdf_nee, pv) * pv);
@@ -1592,7 +1597,7 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
         if (pv < kEps) return false;
         thr = thr * pv;
         d = wo;
-        const float3 att = look_for_emitter(sc, o, d, false, rng, med, max_inter, its, pdf_nee, c);
+        const float3 att = look_for_emitter<kMedia>(sc, o, d, false, rng, med, max_inter, its, pdf_nee, c);
         if (!is_zero3(att)) ret += cmul(thr, att) * mis_weight(phase_eval(ph, -d, wo), pdf_nee);
         s.inc_emission = 0;
     } else {
@@ -1604,7 +1609,7 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
         float3 wo;
         float pdf_nee;
         if (b.type != BSDF_NULL) {
-            const float3 v = nee_surface<kSurf>(sc, its, r2, rng, med, max_inter, wo, pdf_nee, false, c);
+            const float3 v = nee_surface<kMedia>(sc, its, r2, rng, med, max_inter, wo, pdf_nee, false, c);
             if (!is_zero3(v))
                 ret += cmul(cmul(thr, v), bsdf_eval(b, its.wi, wo)) * mis_weight(pdf_nee, bsdf_pdf(b, its.wi, wo));
         }
@@ -1618,7 +1623,7 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
         if (b.type == BSDF_NULL) {
             ray_intersect(sc, o, d, true, its, c);
         } else {
-            const float3 att = look_for_emitter<kSurf>(sc, o, d, true, rng, med, max_inter, its, pdf_nee, c);
+            const float3 att = look_for_emitter<kMedia>(sc, o, d, true, rng, med, max_inter, its, pdf_nee, c);
             thr = cmul(thr, bw);
             if (!is_zero3(att, 1e-12f)) ret += cmul(thr, att) * mis_weight(bpdf, pdf_nee);
             s.inc_emission = 0;
@@ -1628,13 +1633,13 @@ DT_D bool li_step(const DevScene &sc, LiState &s, Ctr &c) {
     return s.depth <= max_depth;
 }
 
-template <bool kSurf = false>
+template <int kMedia = kAnyMedia>
 DT_D float3 li_path(const DevScene &sc, Rng &rng, float3 o, float3 d, int max_depth, int med,
                     bool inc_emission, Ctr &c, bool on_surface = true) {
     LiState s;
     s.rng = rng;
     bool alive = li_start(sc, s, o, d, max_depth, med, inc_emission, c, on_surface);
-    while (alive) alive = li_step<kSurf>(sc, s, c);
+    while (alive) alive = li_step<kMedia>(sc, s, c);
     rng = s.rng;
     return s.ret;
 }

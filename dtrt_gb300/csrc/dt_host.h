@@ -133,8 +133,11 @@ inline bool static_rays(const DevScene &sc) {
     return true;
 }
 
-// Opaque surfaces alone: the Li kernels' kSurf queries apply
-inline bool surfaces_only(const DevScene &sc) { return sc.num_media == 0 && !sc.has_null && sc.cam.med_id < 0; }
+// The queries that apply to the scene's Li, Lins and edge kernels
+inline int media_kind(const DevScene &sc) {
+    if (sc.num_media == 0 && !sc.has_null && sc.cam.med_id < 0) return kNoMedia;
+    return sc.has_grid_media ? kAnyMedia : kNoGrids;
+}
 
 // Camera paths per batch of a scene of static_rays(): its batches hold no records, only path
 // states (256 MB at nder 8), and kLanes of them run at once

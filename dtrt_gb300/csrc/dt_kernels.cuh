@@ -812,7 +812,7 @@ DT_D float3 edge_subpath_dir(const EdgePoint &ep, int sgn) {
 
 // twelve resident blocks per SM: the kernel waits on the FP64 pipe and on traversal latency.
 // With library acos, sincos, square roots and divisions the FP64 pipe was 74 % busy.
-template <int N, bool kSurf>
+template <int N, int kMedia>
 __global__ void __launch_bounds__(kBlock, 12) k_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                  long long rec_count, Queue qli, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_edge(DevScene sc, RenderParams r
         }
         if (ok) {
             const float tr =
-                eval_transmittance<kSurf>(sc, tof(x0), w1f, r.kind == 0, med1, (float)ep.dist, rng, r.depth, c);
+                eval_transmittance<kMedia>(sc, tof(x0), w1f, r.kind == 0, med1, (float)ep.dist, rng, r.depth, c);
             ok = tr > kEps;
         }
         if (ok) {
@@ -927,7 +927,7 @@ __global__ void k_li_keys(DevScene sc, const Task *tasks, long long npairs, unsi
 // active, and more warps hide more of the traversal's latency than their spills cost. The two
 // sub-paths of a sample share pixel and slot weights: their lanes add up the radiance first
 // and each adds every other slot, half the FP64 atomics.
-template <int N, bool kSurf>
+template <int N, int kMedia>
 __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, Queue qli, long long begin, long long count,
                                                double *acc1, double *acc2, const int *perm,
                                                unsigned long long *ctr) {
@@ -942,7 +942,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, 
         Rng rng;
         rng.init(rp.seed, t.key);
         n = 1;
-        wl = cmul(f3(t.w), li_path<kSurf>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c));
+        wl = cmul(f3(t.w), li_path<kMedia>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c));
     }
     wl = mk(wl.x + __shfl_xor_sync(0xffffffffu, wl.x, 1), wl.y + __shfl_xor_sync(0xffffffffu, wl.y, 1),
             wl.z + __shfl_xor_sync(0xffffffffu, wl.z, 1));
@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, 
 }
 
 // ====================================================================== Lins records
-template <int N>
+template <int N, int kMedia>
 __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp, Queue ql, long long count, double *acc1,
                                                  unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp
             float r4[4];
             r4[0] = rng.next1(); r4[1] = rng.next1(); r4[2] = rng.next1(); r4[3] = rng.next1();
             if (b.type == BSDF_NULL) {
-                att = nee_surface(sc, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, true, c);
+                att = nee_surface<kMedia>(sc, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, true, c);
                 if (!is_zero3(att)) {
                     wo = its0.to_world(wo);
                     pv = phase_eval(ph, -rd, wo);
@@ -1003,14 +1003,14 @@ __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp
                     }
                     if (md1 > 0) {
                         const int med1 = is_transition(sh) ? target_medium(sc, r.shape, its0.ng, wo) : med;
-                        att = look_for_emitter(sc, its0.p, wo, true, rng, med1, md1, its1, pdf_nee, c);
+                        att = look_for_emitter<kMedia>(sc, its0.p, wo, true, rng, med1, md1, its1, pdf_nee, c);
                         if (!is_zero3(att)) lins += att * (pv * mis_weight(phase_eval(ph, -rd, wo), pdf_nee));
-                        lins += li_path(sc, rng, its0.p, wo, md1, med1, false, c) * pv;
+                        lins += li_path<kMedia>(sc, rng, its0.p, wo, md1, med1, false, c) * pv;
                     }
                 }
                 continue;
             }
-            att = nee_surface(sc, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, false, c);
+            att = nee_surface<kMedia>(sc, its0, r4, rng, med, max_depth - 1, wo, pdf_nee, false, c);
             if (!is_zero3(att)) {
                 wo = its0.to_world(wo);
                 if (dot(wo, n) < -kEps) {
@@ -1022,9 +1022,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp
             if ((pv = phase_sample(ph, -rd, u, v, wo)) > kEps) {
                 const float wdn = dot(wo, n);
                 if (wdn < -kEps) {
-                    att = look_for_emitter(sc, its0.p, wo, true, rng, med, max_depth - 1, its1, pdf_nee, c);
+                    att = look_for_emitter<kMedia>(sc, its0.p, wo, true, rng, med, max_depth - 1, its1, pdf_nee, c);
                     if (!is_zero3(att)) lins += att * (pv * mis_weight(phase_eval(ph, -rd, wo), pdf_nee));
-                    lins += li_path(sc, rng, its0.p, wo, max_depth - 1, med, false, c) * pv;
+                    lins += li_path<kMedia>(sc, rng, its0.p, wo, max_depth - 1, med, false, c) * pv;
                 } else if (wdn > kEps) {
                     if (sh.light_id >= 0) lins += le(sc, its0, -wo) * pv;
                     if (max_depth > 1) {
@@ -1032,7 +1032,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp
                         its2.wi = its2.to_local(-wo);
                         float r4b[4];
                         r4b[0] = rng.next1(); r4b[1] = rng.next1(); r4b[2] = rng.next1(); r4b[3] = rng.next1();
-                        att = nee_surface(sc, its2, r4b, rng, med, max_depth - 2, wo, pdf_nee, false, c);
+                        att = nee_surface<kMedia>(sc, its2, r4b, rng, med, max_depth - 2, wo, pdf_nee, false, c);
                         if (!is_zero3(att))
                             lins += cmul(bsdf_eval(b, its2.wi, wo), att) *
                                     (pv * mis_weight(pdf_nee, bsdf_pdf(b, its2.wi, wo)));
@@ -1044,9 +1044,9 @@ __global__ void __launch_bounds__(kBlock, 5) k_lins(DevScene sc, RenderParams rp
                             wo = its2.to_world(wo);
                             const int med1 = is_transition(sh) ? target_medium(sc, r.shape, its2.ng, wo) : med;
                             Its its3;
-                            att = look_for_emitter(sc, its2.p, wo, true, rng, med1, max_depth - 2, its3, pdf_nee, c);
+                            att = look_for_emitter<kMedia>(sc, its2.p, wo, true, rng, med1, max_depth - 2, its3, pdf_nee, c);
                             if (!is_zero3(att, 1e-12f)) lins += cmul(t1, att) * mis_weight(bp, pdf_nee);
-                            lins += cmul(t1, li_path(sc, rng, its2.p, wo, max_depth - 2, med1, false, c));
+                            lins += cmul(t1, li_path<kMedia>(sc, rng, its2.p, wo, max_depth - 2, med1, false, c));
                         }
                     }
                 }
@@ -1120,7 +1120,7 @@ __global__ void k_primary_keys(RenderParams rp, unsigned *keys, int *vals) {
 
 // Bound by the FP64 pipe (77 % busy with library square roots and divisions and the image-plane
 // point of each sample); what only visible samples need is computed after the visibility test.
-template <int N, bool kSurf>
+template <int N, int kMedia>
 __global__ void __launch_bounds__(kBlock, 10) k_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                     unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -1153,7 +1153,7 @@ __global__ void __launch_bounds__(kBlock, 10) k_primary(DevScene sc, RenderParam
             float3 o, d;
             const PrimaryNdc ndc(cam, pp);
             ndc.ray(cam, e, 0, o, d);
-            const float tr = eval_transmittance<kSurf>(sc, o, d, false, cam.med_id, primary_edge_dist(e, u), rng,
+            const float tr = eval_transmittance<kMedia>(sc, o, d, false, cam.med_id, primary_edge_dist(e, u), rng,
                                                        rp.max_bounces - 1, c);
             if (tr > kEps) {
                 const long long slot = queue_reserve_n(sc, qli, 2);  // the pair in adjacent slots

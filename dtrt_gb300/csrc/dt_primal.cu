@@ -15,7 +15,7 @@
 
 namespace dt {
 
-template <bool kSurf>
+template <int kMedia>
 __global__ void __launch_bounds__(kBlock, 10) k_primal(DevScene sc, RenderParams rp, double *img_acc,
                                                    unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(kBlock, 10) k_primal(DevScene sc, RenderParams
         const double jx = rng.next1d(), jy = rng.next1d();  // samplePrimaryRay(ix, iy, next2D())
         float3 o, d;
         camera_ray(sc.cam, ix + jx, iy + jy, o, d);
-        L = li_path<kSurf>(sc, rng, o, d, rp.max_bounces, sc.cam.med_id, true, c, false) * rp.inv_spp;
+        L = li_path<kMedia>(sc, rng, o, d, rp.max_bounces, sc.cam.med_id, true, c, false) * rp.inv_spp;
     }
     const unsigned full = 0xffffffffu;
     const int p0 = __shfl_sync(full, pixel, 0);
@@ -209,7 +209,7 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     for (long long b0 = wavefront ? total : 0; b0 < total; b0 += B) {
         rp.path_begin = b0;
         rp.path_count = std::min(B, total - b0);
-        const auto k = surfaces_only(sc) ? k_primal<true> : k_primal<false>;
+        const auto k = media_kind(sc) == kNoMedia ? k_primal<kNoMedia> : k_primal<kAnyMedia>;
         k<<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, sb.adj_img, ctr);
         ++launches;
         DT_PCK(cudaGetLastError());

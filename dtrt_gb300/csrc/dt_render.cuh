@@ -85,6 +85,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     using clk = std::chrono::steady_clock;
     const auto t_start = clk::now();
     DevScene sc = s->dev;
+    const int media = media_kind(sc);
     Scratch &sb = s->scratch;
     const DevCamera &cam = sc.cam;
     const bool cropped = cam.crop_w > 0 && cam.crop_h > 0;
@@ -179,7 +180,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                      const int *perm = li_sorted ? sort_li_pairs(sc, (const LiTask<N> *)qli.data, (long long)n, sb,
                                                                  li_cap, st, launches)
                                                  : nullptr;
-                     const auto k = surfaces_only(sc) ? k_li<N, true> : k_li<N, false>;
+                     const auto k = media == kNoMedia ? k_li<N, kNoMedia> : (media == kNoGrids ? k_li<N, kNoGrids> : k_li<N, kAnyMedia>);
                      k<<<blocks(n), kBlock, 0, st>>>(sc, rp, qli, 0, n, sb.acc1, sb.acc2, perm, ctr);
                  })))
                 return rc;
@@ -199,9 +200,13 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         rp.prim_count = count;
         return timed(ms_primary, [&] {
             const int *perm = li_sorted ? sort_primary_samples(rp, sb, li_cap, st, launches) : nullptr;
-            const auto k = surfaces_only(sc) ? k_primary<N, true> : k_primary<N, false>;
+            const auto k = media == kNoMedia ? k_primary<N, kNoMedia> : (media == kNoGrids ? k_primary<N, kNoGrids> : k_primary<N, kAnyMedia>);
             k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
         });
+    };
+    auto run_lins = [&](cudaStream_t q, unsigned long long nl) {
+        const auto k = media == kNoGrids ? k_lins<N, kNoGrids> : k_lins<N, kAnyMedia>;
+        k<<<blocks(nl), kBlock, 0, q>>>(sc, rp, ql, nl, sb.acc1, ctr);
     };
     bool prim_done = false;
     // ---------------------------------------------------------------- pass 1
@@ -306,14 +311,14 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             if (lins_aside) {
                 DT_CK(cudaEventRecord(sb.fork_ev, st));
                 DT_CK(cudaStreamWaitEvent(sb.side[0], sb.fork_ev, 0));
-                k_lins<N><<<blocks(nl), kBlock, 0, sb.side[0]>>>(sc, rp, ql, nl, sb.acc1, ctr);
+                run_lins(sb.side[0], nl);
                 ++launches;
                 DT_CK(cudaEventRecord(sb.side_ev[0], sb.side[0]));
             }
             for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
                 const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
                 if ((rc = timed(ms_edge, [&] {
-                         const auto k = surfaces_only(sc) ? k_edge<N, true> : k_edge<N, false>;
+                         const auto k = media == kNoMedia ? k_edge<N, kNoMedia> : (media == kNoGrids ? k_edge<N, kNoGrids> : k_edge<N, kAnyMedia>);
                          k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
                      })))
                     return rc;
@@ -328,7 +333,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             if (nl)
                 if ((rc = timed(ms_li, [&] {
                          if (lins_aside) cudaStreamWaitEvent(st, sb.side_ev[0], 0);
-                         else k_lins<N><<<blocks(nl), kBlock, 0, st>>>(sc, rp, ql, nl, sb.acc1, ctr);
+                         else run_lins(st, nl);
                      })))
                     return rc;
         }
@@ -427,6 +432,7 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
     using clk = std::chrono::steady_clock;
     const auto t_start = clk::now();
     DevScene sc = s->dev;
+    const int media = media_kind(sc);
     const DevCamera &cam = sc.cam;
     const bool cropped = cam.crop_w > 0 && cam.crop_h > 0;
     RenderParams rp{};
@@ -499,7 +505,7 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
         const unsigned long long n = std::min<unsigned long long>(hcnt[2], kNoallocLiCap);
         tot_li += n;
         if (n) {
-            const auto k = surfaces_only(sc) ? k_li<N, true> : k_li<N, false>;
+            const auto k = media == kNoMedia ? k_li<N, kNoMedia> : (media == kNoGrids ? k_li<N, kNoGrids> : k_li<N, kAnyMedia>);
             k<<<blocks(n), kBlock, 0, st>>>(sc, rp, qli, 0, n, acc1, acc2, nullptr, nullptr);
             if ((rc = launched())) return rc;
         }
@@ -529,13 +535,14 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
             tot_lins += nl;
             for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
                 const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
-                const auto k = surfaces_only(sc) ? k_edge<N, true> : k_edge<N, false>;
+                const auto k = media == kNoMedia ? k_edge<N, kNoMedia> : (media == kNoGrids ? k_edge<N, kNoGrids> : k_edge<N, kAnyMedia>);
                 k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, nullptr);
                 if ((rc = launched())) return rc;
                 if ((rc = drain_li())) return rc;
             }
             if (nl) {
-                k_lins<N><<<blocks(nl), kBlock, 0, st>>>(sc, rp, ql, nl, acc1, nullptr);
+                const auto k = media == kNoGrids ? k_lins<N, kNoGrids> : k_lins<N, kAnyMedia>;
+                k<<<blocks(nl), kBlock, 0, st>>>(sc, rp, ql, nl, acc1, nullptr);
                 if ((rc = launched())) return rc;
             }
         }
@@ -550,7 +557,7 @@ int render_n_noalloc(dtrt_scene *s, const dtrt_render_options *o, float *out, in
         for (long long k0 = 0; k0 < ns; k0 += chunk) {
             rp.prim_begin = k0;
             rp.prim_count = std::min(chunk, ns - k0);
-            const auto k = surfaces_only(sc) ? k_primary<N, true> : k_primary<N, false>;
+            const auto k = media == kNoMedia ? k_primary<N, kNoMedia> : (media == kNoGrids ? k_primary<N, kNoGrids> : k_primary<N, kAnyMedia>);
             k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, nullptr, nullptr);
             if ((rc = launched())) return rc;
             if ((rc = drain_li())) return rc;

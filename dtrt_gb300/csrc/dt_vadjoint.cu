@@ -146,7 +146,7 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
             const int *perm =
                 li_sorted ? sort_li_pairs(sc, (const VLiTask *)qli.data, (long long)n, sb, li_cap, st, launches)
                           : nullptr;
-            const auto k = surfaces_only(sc) ? k_vadj_li<true> : k_vadj_li<false>;
+            const auto k = media_kind(sc) == kNoMedia ? k_vadj_li<kNoMedia> : k_vadj_li<kAnyMedia>;
             k<<<blocks((long long)n), kBlock, 0, st>>>(sc, rp, qli, (long long)n, dimg, grad, xadj, perm, ctr);
             ++launches;
             DT_VCK(cudaGetLastError());
@@ -170,7 +170,7 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
         tot_edge += ne;
         for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
             const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
-            const auto k = surfaces_only(sc) ? k_vadj_edge<true> : k_vadj_edge<false>;
+            const auto k = media_kind(sc) == kNoMedia ? k_vadj_edge<kNoMedia> : k_vadj_edge<kAnyMedia>;
             k<<<blocks(cnt * rp.sppse), kBlock, 0, st>>>(sc, rp, qe, (long long)r0, cnt, qli, ctr);
             ++launches;
             DT_VCK(cudaGetLastError());
@@ -193,7 +193,7 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
             rp.prim_begin = k0;
             rp.prim_count = std::min(chunk, ns - k0);
             const int *perm = li_sorted ? sort_primary_samples(rp, sb, li_cap, st, launches) : nullptr;
-            const auto k = surfaces_only(sc) ? k_vadj_primary<true> : k_vadj_primary<false>;
+            const auto k = media_kind(sc) == kNoMedia ? k_vadj_primary<kNoMedia> : k_vadj_primary<kAnyMedia>;
             k<<<blocks(rp.prim_count), kBlock, 0, st>>>(sc, rp, qli, perm, ctr);
             ++launches;
             DT_VCK(cudaGetLastError());

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_vadj_chain(DevScene sc, RenderPar
 
 // one thread per (edge record, edge sample): k_edge's geometry, then two VLiTasks carrying
 // the gradient coefficients instead of per-slot scalars
-template <bool kSurf>
+template <int kMedia>
 __global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderParams rp, Queue qe, long long rec_begin,
                                                       long long rec_count, Queue qli, unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderPar
             ok = !is_zero3(val);
         }
         if (ok) {
-            const float tr = eval_transmittance<kSurf>(sc, tof(x0), w1f, true, med1, (float)dist, rng, r.depth, c);
+            const float tr = eval_transmittance<kMedia>(sc, tof(x0), w1f, true, med1, (float)dist, rng, r.depth, c);
             ok = tr > kEps;
         }
         if (ok) {
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_edge(DevScene sc, RenderPar
 }
 
 // one thread per primary-edge sample: k_primary's geometry with the projection Jacobian
-template <bool kSurf>
+template <int kMedia>
 __global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, RenderParams rp, Queue qli, const int *perm,
                                                          unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, Render
             float3 o, d;
             const PrimaryNdc ndc(cam, pp);
             ndc.ray(cam, e, 0, o, d);
-            const float tr = eval_transmittance<kSurf>(sc, o, d, false, cam.med_id, primary_edge_dist(e, u), rng,
+            const float tr = eval_transmittance<kMedia>(sc, o, d, false, cam.med_id, primary_edge_dist(e, u), rng,
                                                        rp.max_bounces - 1, c);
             if (tr > kEps) {
                 // screen velocity of the edge point along the normal, per coordinate of v0 and v1
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(kBlock, 12) k_vadj_primary(DevScene sc, Render
 // one thread per VLiTask: Li, then K = dot(dL/dI, w (x) Li) times the coefficients; the pairs
 // in sorted order (perm, or queue order) as k_li. The two sub-paths of a sample share the
 // coefficients: their lanes add up K first and each scatters half of the nine values.
-template <bool kSurf>
+template <int kMedia>
 __global__ void __launch_bounds__(kBlock, 10) k_vadj_li(DevScene sc, RenderParams rp, Queue qli, long long count,
                                                     const float *dimg, float *grad, float *xadj, const int *perm,
                                                     unsigned long long *ctr) {
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(kBlock, 10) k_vadj_li(DevScene sc, RenderParam
         Rng rng;
         rng.init(rp.seed, t.key);
         n = 1;
-        const float3 L = li_path<kSurf>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
+        const float3 L = li_path<kMedia>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c);
         const float3 gp = mk(__ldg(dimg + 3 * (size_t)t.pixel), __ldg(dimg + 3 * (size_t)t.pixel + 1),
                              __ldg(dimg + 3 * (size_t)t.pixel + 2));
         K = dot(gp, cmul(f3(t.w), L));

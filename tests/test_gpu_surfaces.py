@@ -42,3 +42,21 @@ def test_surface_kernels_equal_the_general_ones(bsdf, w, h, spp, depth):
                 out.append(r)
         for a, b in zip(*out):
             _near(a, b)
+
+
+# Homogeneous media alone: kernels without grid tracking. A 2^3 grid medium that no shape uses
+# selects the general ones.
+@pytest.mark.parametrize("w,h,spp,depth", [(1, 1, 1, 1), (13, 7, 5, 3), (40, 33, 8, 6)])
+def test_homogeneous_kernels_equal_the_general_ones(w, h, spp, depth):
+    kw = dict(seed=4, spp=spp, max_bounces=depth, sppe=32, sppse=3)
+    for nder in (1, 3, 4, 8):
+        out = []
+        for general in (False, True):
+            spec = scenes.config0(w, h, subdiv=2, nder=nder)
+            if general:
+                spec.media.append(scenes.MediumSpec(
+                    _abi.MEDIUM_HETEROGENEOUS, phase_id=0, density=np.ones((2, 2, 2), np.float32),
+                    vol_min=(-1.0,) * 3, vol_max=(1.0,) * 3))
+            with native.NativeScene(spec) as s:
+                out.append(s.render(**kw).copy())
+        _near(*out)
