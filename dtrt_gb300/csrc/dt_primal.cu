@@ -15,8 +15,13 @@
 
 namespace dt {
 
-template <int kMedia>
-__global__ void __launch_bounds__(kBlock, 10) k_primal(DevScene sc, RenderParams rp, double *img_acc,
+// Renders of fewer paths than this wait for their longest path rather than for a free warp: they
+// take the kernels at four blocks per SM, without spills (at ten and eight blocks small clouds
+// and spheres were 10 to 18 % slower); above it the resident warps count.
+constexpr long long kManyPaths = 1 << 19;
+
+template <int kMedia, int kBlocks>
+__global__ void __launch_bounds__(kBlock, kBlocks) k_primal(DevScene sc, RenderParams rp, double *img_acc,
                                                    unsigned long long *ctr) {
     const long long gi = (long long)blockIdx.x * kBlock + threadIdx.x;
     const bool active = gi < rp.path_count;
@@ -72,7 +77,8 @@ __global__ void __launch_bounds__(kBlock) k_primal_start(DevScene sc, RenderPara
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
-__global__ void __launch_bounds__(kBlock, 8) k_primal_level(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
+template <int kBlocks>
+__global__ void __launch_bounds__(kBlock, kBlocks) k_primal_level(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
                                                          const int *q_in, const unsigned long long *cnt_in, int *q_out,
                                                          unsigned long long *cnt_out, unsigned long long *ctr) {
     const long long n = (long long)*cnt_in;
@@ -183,8 +189,10 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     DT_PCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
     DT_PCK(cudaEventRecord(e0, st));
-    launches += (uint64_t)prepare_cells(s, sc, total, false, st);
+    launches += (uint64_t)prepare_cells(s, sc, total / 8, false, st);  // a primal path makes few lookups
+    const bool many = total >= kManyPaths;
     if (wavefront) {
+        const auto level = many ? k_primal_level<8> : k_primal_level<4>;
         const long long nb = (total + B - 1) / B;
         DT_PCK(in_lanes(sb, st, lanes, nb, [&](long long k, int lane, cudaStream_t q) {
             RenderParams r = rp;
@@ -199,8 +207,8 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
             if (e != cudaSuccess) return e;
             k_primal_start<<<blocks(r.path_count), kBlock, 0, q>>>(sc, r, states, rets, qa, lcnt, ctr);
             for (int L = 0; L < levels; ++L)
-                k_primal_level<<<gw, kBlock, 0, q>>>(sc, r, states, rets, (L & 1) ? qb : qa, lcnt + L, (L & 1) ? qa : qb,
-                                                     lcnt + L + 1, ctr);
+                level<<<gw, kBlock, 0, q>>>(sc, r, states, rets, (L & 1) ? qb : qa, lcnt + L, (L & 1) ? qa : qb,
+                                            lcnt + L + 1, ctr);
             k_primal_accum<<<blocks(r.path_count), kBlock, 0, q>>>(r, rets, sb.adj_img);
             return cudaGetLastError();
         }));
@@ -209,7 +217,9 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     for (long long b0 = wavefront ? total : 0; b0 < total; b0 += B) {
         rp.path_begin = b0;
         rp.path_count = std::min(B, total - b0);
-        const auto k = media_kind(sc) == kNoMedia ? k_primal<kNoMedia> : k_primal<kAnyMedia>;
+        const bool none = media_kind(sc) == kNoMedia;
+        const auto k = many ? (none ? k_primal<kNoMedia, 10> : k_primal<kAnyMedia, 10>)
+                            : (none ? k_primal<kNoMedia, 4> : k_primal<kAnyMedia, 4>);
         k<<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, sb.adj_img, ctr);
         ++launches;
         DT_PCK(cudaGetLastError());
