@@ -273,7 +273,7 @@ int upload_wave_layout(dtrt_batch *b, const std::vector<int> &order, long long s
 }
 
 // One replay wavefront over the uploaded numbering, in chunks of a workspace's capacity:
-// pass A (start, one launch per vertex kind and level, totals), then, when an item asks
+// pass A (start, one launch per vertex level, totals), then, when an item asks
 // for a density gradient, pass B. Every level launch covers live paths of all items; a
 // chunk spans item boundaries. Chunks are independent: they are dealt round-robin to the
 // caller's stream and the side streams, each with its own workspace, so that one chunk's
