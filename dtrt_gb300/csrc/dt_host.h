@@ -14,10 +14,14 @@ void set_last_error(const std::string &msg);
 // Wavefront batches in flight at once, each on a stream and a workspace of its own: a batch's
 // last levels hold few paths and take as long as their slowest vertex, and the other batches
 // run in the meantime; small batches read neighbouring voxels. C3 forward (33.6 M paths): one
-// lane of 2^23 paths 68.8 ms, 4 lanes of 2^21 63.7, 8 of 2^20 63.1, 8 of 2^19 66.4; its
-// density adjoint: one lane of 2^24 39.7, 8 of 2^20 36.9, 8 of 2^21 35.5; C1 primal: one of
+// lane of 2^23 paths 68.8 ms, 4 lanes of 2^21 63.7, 8 of 2^20 63.1, 8 of 2^19 66.4; C1 primal: one of
 // 2^22 15.9, 8 of 2^20 14.8, 8 of 2^19 14.1. Eight streams are what the device queues.
 constexpr int kLanes = 8;
+// The density replay keeps 780 B a path, and a program that holds many scenes holds a workspace
+// for each: 2^22 paths in all (3.3 GB). C3 density adjoint: one lane of 2^22 41.4 ms, 2 of
+// 2^21 39.3, 4 of 2^20 38.0, 8 of 2^19 38.7 (8 of 2^21, 13 GB, 35.5).
+constexpr int kReplayLanes = 4;
+constexpr long long kReplayBatchPaths = 1ll << 20;
 
 // Device buffers reused across renders of one scene, grown on demand.
 struct Scratch {
