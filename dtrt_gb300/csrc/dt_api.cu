@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "dt_bvh.h"
+#include "dt_desc.h"
 #include "dt_host.h"
 
 namespace dt {
@@ -519,12 +520,7 @@ int build_scene(dtrt_scene *s, const dtrt_scene_desc *d, Builder &bld, bool rebu
     std::vector<std::vector<HV>> vad(d->num_shapes);  // dual vertices per shape
     bool any_vel = false, any_normals = false;
     for (int i = 0; i < d->num_shapes; ++i) {
-        // all-zero velocities (a SceneManager writes an array for every shape) move nothing
-        const dtrt_shape_desc &sv = d->shapes[i];
-        if (sv.velocities && !any_vel) {
-            const size_t nvel = (size_t)sv.num_vertices * 3 * (N + (sv.normals ? 1 : 0));
-            any_vel = std::any_of(sv.velocities, sv.velocities + nvel, [](float x) { return x != 0.f; });
-        }
+        any_vel = any_vel || shape_moves(d->shapes[i], N);
         any_normals = any_normals || d->shapes[i].normals;
     }
     int vtot = 0, ttot = 0;
