@@ -175,7 +175,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     uint64_t launches = 0;
     float ms_replay = 0.f;
     DT_ACK(cudaEventRecord(e0, st));
-    launches += (uint64_t)prepare_cells(s, sc, total, grad != nullptr && dimg != nullptr, st);
+    launches += (uint64_t)prepare_cells(s, sc, total, 16, grad != nullptr && dimg != nullptr, st);
     // schedule: the wavefront (pass A and pass B each one launch per vertex over the live
     // paths) for large renders, as dtrt_render_fwd's camera schedule
     const long long B = 1ll << 24;  // paths per megakernel launch

@@ -55,13 +55,19 @@ __global__ void k_cells_gather(const float4 *cells, int rx, int ry, int rz, floa
     grad[v] = sum;
 }
 
-int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, bool with_grad, cudaStream_t st) {
+int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, int per_path, bool with_grad, cudaStream_t st) {
     sc.cells = nullptr;
     sc.grad_cells = nullptr;
     const long long n = s->density_voxels;
     // The copy costs 40 B of traffic per voxel, 14 us for 128^3; a path makes some tens of
-    // lookups. At most 2^27 voxels (4 GiB each copy).
-    if (n <= 0 || paths < n / 16 || n > (1ll << 27)) return 0;
+    // lookups. At most 2^27 voxels (4 GiB each copy). A replay that scatters gains from the first
+    // path for every 16 voxels: its atomics on a small grid collide (16^3, 10^6 paths: 23.7 ms on
+    // voxels, 7.2 on cells; 32^3, 14,400 paths: 1.75, 1.66). A render that only reads takes as
+    // long as its longest path below 2^16 paths, and voxels of a grid below 32^3 stay in L1 where
+    // its cells do not (forward 40^3, 14,400 paths: 0.90 ms on cells, 0.86 on voxels; primal 20^3,
+    // 250,000: 0.91, 0.88; the other side, forward 64^3, 10^6: 1.79, 1.88).
+    if (n <= 0 || n > (1ll << 27) || paths < n / per_path) return 0;
+    if (!with_grad && (n < (1ll << 15) || paths < kWavefrontMinPaths)) return 0;
     Scratch &sb = s->scratch;
     if (!ensure_buffer(&sb.cells, &sb.cells_bytes, (size_t)n * 32 * (with_grad ? 2 : 1))) {
         cudaGetLastError();  // no room: the kernels read the voxels

@@ -762,31 +762,51 @@ DT_D bool grid_cell(const DevGrid &g, float3 p, int &x1, int &y1, int &z1) {
     z1 = (int)floorf(p.z);
     return true;
 }
+// Scenes without media and null BSDFs (kNoMedia) or without density grids (kNoGrids) take the Li,
+// Lins and edge kernels' queries without the code they do not need: without media a shadow
+// ray is one any-hit traversal and an emitter lookup one closest hit; without grids a segment's
+// transmittance is one exponential. Their warps waited for instructions in 3 of 14 cycles per
+// issue (kNoMedia, with the pair sums of k_li: C2 forward 89.4 -> 81.1 ms, vertex adjoint 26.7 ->
+// 24.7, primal mesh 1.72 -> 1.55; kNoGrids: C0 forward 18.1 -> 17.4, render_scene 8.3 -> 8.2).
+// kNoCells: grids are read from their voxels alone (DevScene::cells is not looked at), the primal
+// kernels of small renders: the choice in each loop costs 2 to 3 % where the longest path counts.
+enum { kAnyMedia = 0, kNoMedia = 1, kNoGrids = 2, kNoCells = 3 };
+
 // The 8 corners of a medium's density cell, y then x fastest: lo at z1, hi at z1 + 1. Large
 // renders read them from a copy of the grid with the corners of each cell together
 // (DevScene::cells: two 128-bit loads of one sector instead of 8 loads of 4 or 5).
 struct Corners {
     float4 lo, hi;
 };
-DT_D Corners grid_corners(const DevScene &sc, const DevMedium &m, int x1, int y1, int z1) {
-    const DevGrid &g = m.density;
-    const int sy = g.res[0], sz = g.res[0] * g.res[1];
-    const size_t base = (size_t)z1 * sz + (size_t)y1 * sy + x1;
-    if (sc.cells) {
-        const float4 *q = sc.cells + 2 * ((size_t)m.grad_off + base);
-        return {__ldg(q), __ldg(q + 1)};
+// Where a medium's corners are read: from its cells when the render has them. The tracking loops
+// look this up once: asked at every step, it stood in front of the corners' loads (C3-like cloud,
+// 1.0e6 paths: forward 1.84 -> 1.79 ms, primal 1.93 -> 1.89; 14,400 paths: primal 0.48 -> 0.45).
+struct GridSource {
+    const float4 *cells;
+    const float *data;
+    DT_D Corners corners(const DevGrid &g, int x1, int y1, int z1) const {
+        const int sy = g.res[0], sz = g.res[0] * g.res[1];
+        const size_t base = (size_t)z1 * sz + (size_t)y1 * sy + x1;
+        if (cells) {
+            const float4 *q = cells + 2 * base;
+            return {__ldg(q), __ldg(q + 1)};
+        }
+        const float *d = data + base;
+        return {make_float4(__ldg(d), __ldg(d + 1), __ldg(d + sy), __ldg(d + sy + 1)),
+                make_float4(__ldg(d + sz), __ldg(d + sz + 1), __ldg(d + sz + sy), __ldg(d + sz + sy + 1))};
     }
-    const float *d = g.data + base;
-    return {make_float4(__ldg(d), __ldg(d + 1), __ldg(d + sy), __ldg(d + sy + 1)),
-            make_float4(__ldg(d + sz), __ldg(d + sz + 1), __ldg(d + sz + sy), __ldg(d + sz + sy + 1))};
+};
+template <int kMedia = kAnyMedia>
+DT_D GridSource grid_source(const DevScene &sc, const DevMedium &m) {
+    return {kMedia == kNoCells || !sc.cells ? nullptr : sc.cells + 2 * (size_t)m.grad_off, m.density.data};
 }
-DT_D float grid_lookup(const DevScene &sc, const DevMedium &m, float3 pw, Ctr &c) {  // gridvolume.h:144-171
+DT_D float grid_lookup(const GridSource &src, const DevGrid &g, float3 pw, Ctr &c) {  // gridvolume.h:144-171
     c.lookups++;
-    const float3 p = grid_point(m.density, pw);
+    const float3 p = grid_point(g, pw);
     int x1, y1, z1;
-    if (!grid_cell(m.density, p, x1, y1, z1)) return 0.f;
+    if (!grid_cell(g, p, x1, y1, z1)) return 0.f;
     const float fx = p.x - x1, fy = p.y - y1, fz = p.z - z1, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    const Corners q = grid_corners(sc, m, x1, y1, z1);
+    const Corners q = src.corners(g, x1, y1, z1);
     return ((q.lo.x * gx + q.lo.y * fx) * gy + (q.lo.z * gx + q.lo.w * fx) * fy) * gz +
            ((q.hi.x * gx + q.hi.y * fx) * gy + (q.hi.z * gx + q.hi.w * fx) * fy) * fz;
 }
@@ -795,15 +815,14 @@ DT_D float grid_lookup(const DevScene &sc, const DevMedium &m, float3 pw, Ctr &c
 // the point's velocity in the grid, h . -(rot_j x q + trans_j) = -(rot_j . (q x h) +
 // trans_j . h) with q = p - centre (gridvolume.h:301-326): one gradient serves every slot,
 // and its sums over the samples of a line integral do as well.
-DT_D float grid_lookup_grad(const DevScene &sc, const DevMedium &m, float3 pw, float3 &h, Ctr &c) {
-    const DevGrid &g = m.density;
+DT_D float grid_lookup_grad(const GridSource &src, const DevGrid &g, float3 pw, float3 &h, Ctr &c) {
     c.lookups++;
     h = mk(0.f, 0.f, 0.f);
     const float3 p = grid_point(g, pw);
     int x1, y1, z1;
     if (!grid_cell(g, p, x1, y1, z1)) return 0.f;
     const float fx = p.x - x1, fy = p.y - y1, fz = p.z - z1, gx = 1.f - fx, gy = 1.f - fy, gz = 1.f - fz;
-    const Corners k = grid_corners(sc, m, x1, y1, z1);
+    const Corners k = src.corners(g, x1, y1, z1);
     const float d000 = k.lo.x, d001 = k.lo.y, d010 = k.lo.z, d011 = k.lo.w;
     const float d100 = k.hi.x, d101 = k.hi.y, d110 = k.hi.z, d111 = k.hi.w;
     const float a00 = d000 * gx + d001 * fx, a01 = d010 * gx + d011 * fx, a10 = d100 * gx + d101 * fx,
@@ -821,11 +840,11 @@ DT_D Df<N> grid_lookup_ad(const DevScene &sc, const DevMedium &m, const DV<G> &p
     const bool voxel_dirs = g.dgrid != nullptr && g.dgrid_n == N;
     // A static grid sampled at a point without derivatives has none either: the plain
     // lookup gives the same dual exactly (all slots zero) at a fraction of the cost.
-    if (N == 0 || (!g.moving && !voxel_dirs && pw.der_zero(0.f))) return Df<N>(grid_lookup(sc, m, pw.val(), c));
+    if (N == 0 || (!g.moving && !voxel_dirs && pw.der_zero(0.f))) return Df<N>(grid_lookup(grid_source(sc, m), g, pw.val(), c));
     if constexpr (G == 0) {
         if (!voxel_dirs) {
             float3 h;
-            Df<N> r(grid_lookup_grad(sc, m, pw.val(), h, c));
+            Df<N> r(grid_lookup_grad(grid_source(sc, m), g, pw.val(), h, c));
             const float3 qh = cross(pw.val() - f3(g.center), h);
 #pragma unroll
             for (int j = 0; j < N; ++j) r.d[j] = -(dot(f3(g.rot_vel[j]), qh) + dot(f3(g.trans_vel[j]), h));
@@ -944,18 +963,10 @@ DT_D bool aabb_hit(const DevGrid &g, float3 o, float3 d, float &tn, float &tf) {
     return true;
 }
 
-// Scenes without media and null BSDFs (kNoMedia) or without density grids (kNoGrids) take the Li,
-// Lins and edge kernels' queries without the code they do not need: without media a shadow
-// ray is one any-hit traversal and an emitter lookup one closest hit; without grids a segment's
-// transmittance is one exponential. Their warps waited for instructions in 3 of 14 cycles per
-// issue (kNoMedia, with the pair sums of k_li: C2 forward 89.4 -> 81.1 ms, vertex adjoint 26.7 ->
-// 24.7, primal mesh 1.72 -> 1.55; kNoGrids: C0 forward 18.1 -> 17.4, render_scene 8.3 -> 8.2).
-enum { kAnyMedia = 0, kNoMedia = 1, kNoGrids = 2 };
-
 // ------------------------------------------------------------------ media
 DT_D float3 sig_s(const DevScene &sc, const DevMedium &m, float3 x, Ctr &c) {  // homogeneous.h:57, heterogeneous.h:88-90
     if (m.type == MEDIUM_HOMOGENEOUS) return f3(m.sigma_s);
-    return f3(m.albedo) * (m.scale * grid_lookup(sc, m, x, c));
+    return f3(m.albedo) * (m.scale * grid_lookup(grid_source(sc, m), m.density, x, c));
 }
 
 // homogeneous.cpp:6-24 / heterogeneous.cpp:9-37; moves `o` to the scatter point
@@ -981,6 +992,7 @@ DT_HEAVY bool sample_distance(const DevScene &sc, const DevMedium &m, float3 &o,
     tn = fmaxf(tn, 0.f);
     tf = fminf(tf, tmax);
     float t = tn;
+    const GridSource src = grid_source<kMedia>(sc, m);
     for (int dep = 0;; ++dep) {
         t -= logf(rng.next1()) * m.max_inv_density;
         if (t > tf) break;
@@ -989,7 +1001,7 @@ DT_HEAVY bool sample_distance(const DevScene &sc, const DevMedium &m, float3 &o,
             break;
         }
         const float3 p = o + d * t;
-        const float dens = grid_lookup(sc, m, p, c);
+        const float dens = grid_lookup(src, m.density, p, c);
         if (rng.next1() * m.density.max_value < dens) {
             o = p;
             thr = cmul(thr, m.albedo_vol.valid ? grid_lookup3(m.albedo_vol, p) : f3(m.albedo));
@@ -1031,11 +1043,12 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
         // sample positions without derivatives on a static grid: each sample's derivative is
         // d_scale[j] * density(p), so the integral needs only the sum of ten plain lookups
         const float3 o = ray.o.val(), d = ray.d.val();
+        const GridSource src = grid_source(sc, m);
         float sum = 0.f;
 #pragma unroll 1
         for (int i = 0; i < 10; ++i) {
             const float r = ((float)i + rng.next1()) * 0.1f;
-            sum += grid_lookup(sc, m, o + d * (tmin.v + len * r), c);
+            sum += grid_lookup(src, m.density, o + d * (tmin.v + len * r), c);
         }
 #pragma unroll
         for (int j = 0; j < N; ++j) out[j] = scale.d[j] * sum * (len * 0.1f);
@@ -1044,6 +1057,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
         // q x h over the samples give every slot (grid_lookup_grad): 6 multiply-adds per slot
         // after the loop instead of a dual lookup per sample
         const float3 o = ray.o.val(), d = ray.d.val(), ctr = f3(m.density.center);
+        const GridSource src = grid_source(sc, m);
         float sum = 0.f;
         float3 sh = mk(0.f, 0.f, 0.f), sqh = sh;
 #pragma unroll 1
@@ -1051,7 +1065,7 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
             const float r = ((float)i + rng.next1()) * 0.1f;
             const float3 p = o + d * (tmin.v + len * r);
             float3 h;
-            sum += grid_lookup_grad(sc, m, p, h, c);
+            sum += grid_lookup_grad(src, m.density, p, h, c);
             sh += h;
             sqh += cross(p - ctr, h);
         }
@@ -1076,12 +1090,12 @@ DT_HEAVY void int_sig_t(const DevScene &sc, const DevMedium &m, const RayAD<G> &
     if constexpr (G > 0) {
         const float3 o = ray.o.val(), d = ray.d.val();
         if (!tmax.der_zero(1e-6f)) {
-            const float dv = m.scale * grid_lookup(sc, m, o + d * (tmax.v - kEps), c);
+            const float dv = m.scale * grid_lookup(grid_source(sc, m), m.density, o + d * (tmax.v - kEps), c);
 #pragma unroll
             for (int j = 0; j < N; ++j) out[j] += tmax.d[j] * dv;
         }
         if (!tmin.der_zero(1e-6f)) {
-            const float dv = m.scale * grid_lookup(sc, m, o + d * (tmin.v + kEps), c);
+            const float dv = m.scale * grid_lookup(grid_source(sc, m), m.density, o + d * (tmin.v + kEps), c);
 #pragma unroll
             for (int j = 0; j < N; ++j) out[j] -= tmin.d[j] * dv;
         }
@@ -1122,6 +1136,7 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<G
     tn = fmaxf(tn, 0.f);
     tf = fminf(tf, tmax.v);
     float t = tn;
+    const GridSource src = grid_source(sc, m);
     for (int dep = 0;; ++dep) {
         t -= logf(rng.next1()) * m.max_inv_density;
         if (t > tf) break;
@@ -1132,7 +1147,7 @@ DT_HEAVY bool sample_distance_ad(const DevScene &sc, const DevMedium &m, RayAD<G
         // the acceptance test needs the density value only; a null collision discards the
         // derivative slots, so the dual lookup runs at an accepted collision (same point)
         const DV<G> p = ray.o + ray.d * t;
-        const float dv = grid_lookup(sc, m, p.val(), c);
+        const float dv = grid_lookup(src, m.density, p.val(), c);
         if (rng.next1() * m.density.max_value < dv) {
             Ctr again;  // the lookup just counted, repeated with its derivative slots
             const Df<N> dens = grid_lookup_ad<N>(sc, m, p, again);
@@ -1184,6 +1199,7 @@ DT_HEAVY float medium_transmittance(const DevScene &sc, const DevMedium &m, floa
                                 Rng &rng, Ctr &c) {
     if (kMedia == kNoGrids || m.type == MEDIUM_HOMOGENEOUS) return expf((tmin - tmax) * m.sigma_t);
     float ret = 1.f, t = tmin;
+    const GridSource src = grid_source<kMedia>(sc, m);
     int steps = 0;
     while (ret > kEps) {
         t -= logf(rng.next1()) * m.max_inv_density;
@@ -1192,7 +1208,7 @@ DT_HEAVY float medium_transmittance(const DevScene &sc, const DevMedium &m, floa
             set_error(sc, ERR_TRACK_CAP);
             break;
         }
-        ret *= 1.f - grid_lookup(sc, m, o + d * t, c) / m.density.max_value;
+        ret *= 1.f - grid_lookup(src, m.density, o + d * t, c) / m.density.max_value;
     }
     return ret;
 }
@@ -1294,7 +1310,7 @@ DT_HEAVY float3 look_for_emitter(const DevScene &sc, float3 o, float3 d, bool on
         pdf_nee = sc.light_pmf[s.light_id] / (sc.light_area[s.light_id] * G);
         return le(sc, its, -d);
     }
-    if (kMedia == kAnyMedia && sc.has_grid_media) {  // geometry first: chains that miss every emitter skip transmittance
+    if (kMedia != kNoGrids && sc.has_grid_media) {  // geometry first: chains that miss every emitter skip transmittance
         float3 o1 = o;
         Its n1 = its;
         int p1 = prim;

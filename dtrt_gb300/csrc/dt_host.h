@@ -200,8 +200,9 @@ struct dtrt_scene {
 namespace dt {
 // Density cells of a render of `paths` camera paths (with_grad: and zeroed gradient cells) in
 // sc, from the scene's grids as they are now, on stream st; nothing when the render is too
-// small for them or the device has no room. Returns the kernels launched.
-int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, bool with_grad, cudaStream_t st);
+// small for them (`per_path` voxels for each path: 16, or 2 for a primal path, which makes few
+// lookups) or the device has no room. Returns the kernels launched.
+int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, int per_path, bool with_grad, cudaStream_t st);
 // sc.grad_cells summed into the voxels of `grad` (zeroed before); returns the kernels launched
 int gather_cells(const dtrt_scene *s, const DevScene &sc, float *grad, cudaStream_t st);
 template <int N>

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kBlock) k_primal_start(DevScene sc, RenderPara
     if (ctr) flush_counters(ctr, K_CAMERA, c);
 }
 
-template <int kBlocks>
+template <int kMedia, int kBlocks>
 __global__ void __launch_bounds__(kBlock, kBlocks) k_primal_level(DevScene sc, RenderParams rp, LiState *states, float3 *rets,
                                                          const int *q_in, const unsigned long long *cnt_in, int *q_out,
                                                          unsigned long long *cnt_out, unsigned long long *ctr) {
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kBlock, kBlocks) k_primal_level(DevScene sc, R
     for (long long i = (long long)blockIdx.x * kBlock + threadIdx.x; i < n; i += (long long)gridDim.x * kBlock) {
         const int id = q_in[i];
         LiState st = states[id];
-        const bool alive = li_step(sc, st, c);
+        const bool alive = li_step<kMedia>(sc, st, c);
         if (alive) states[id] = st;
         else rets[id] = st.ret;
         push_path(q_out, cnt_out, id, alive);
@@ -189,10 +189,11 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     DT_PCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
     auto blocks = [](long long n) { return (unsigned)((n + kBlock - 1) / kBlock); };
     DT_PCK(cudaEventRecord(e0, st));
-    launches += (uint64_t)prepare_cells(s, sc, total / 8, false, st);  // a primal path makes few lookups
+    launches += (uint64_t)prepare_cells(s, sc, total, 2, false, st);
     const bool many = total >= kManyPaths;
     if (wavefront) {
-        const auto level = many ? k_primal_level<8> : k_primal_level<4>;
+        const auto level = many ? k_primal_level<kAnyMedia, 8>
+                                : (sc.cells ? k_primal_level<kAnyMedia, 4> : k_primal_level<kNoCells, 4>);
         const long long nb = (total + B - 1) / B;
         DT_PCK(in_lanes(sb, st, lanes, nb, [&](long long k, int lane, cudaStream_t q) {
             RenderParams r = rp;
@@ -219,7 +220,7 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
         rp.path_count = std::min(B, total - b0);
         const bool none = media_kind(sc) == kNoMedia;
         const auto k = many ? (none ? k_primal<kNoMedia, 10> : k_primal<kAnyMedia, 10>)
-                            : (none ? k_primal<kNoMedia, 4> : k_primal<kAnyMedia, 4>);
+                            : (none ? k_primal<kNoMedia, 4> : k_primal<kNoCells, 4>);
         k<<<blocks(rp.path_count), kBlock, 0, st>>>(sc, rp, sb.adj_img, ctr);
         ++launches;
         DT_PCK(cudaGetLastError());

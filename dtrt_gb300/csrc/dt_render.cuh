@@ -211,7 +211,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     bool prim_done = false;
     // ---------------------------------------------------------------- pass 1
     const long long total = (long long)npix * std::max(0, o->spp);
-    launches += (uint64_t)prepare_cells(s, sc, total, false, st);
+    launches += (uint64_t)prepare_cells(s, sc, total, 16, false, st);
     if (total > 0) {
         const long long unit = std::max<long long>(128, (long long)rp.spp % 32 == 0 ? std::max(rp.spp, 128) : 128);
         // without records a batch is bounded by the path states alone
