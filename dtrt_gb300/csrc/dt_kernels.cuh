@@ -471,6 +471,10 @@ __global__ void __launch_bounds__(kBlock) k_camera(DevScene sc, RenderParams rp,
 
 // AUTO schedule: the wavefront from this many camera paths per render batch
 constexpr long long kWavefrontMinPaths = 1 << 16;
+// ... and up to this many vertex levels: a wavefront launches every level that max_bounces allows,
+// 4 us each and batch however few paths are left (cloud 256^2 x 64, max_bounces 250 / 1000 / 4000:
+// 6.9 / 15.1 / 64 ms, megakernel 12.9 at each; glass 200^2 x 128: 9.0 / 18.5 / 84, megakernel 40).
+constexpr int kWavefrontMaxLevels = 1024;
 // Blocks per SM of the camera kernels without ray derivatives: they wait on L1 and L2, so
 // warps count more than spills, up to the point where the slots no longer fit (C1, nder 3:
 // 14.4 / 14.1 / 13.5 / 13.9 ms at 3 / 4 / 5 / 6 blocks; C3, nder 8: 71.0 / 68.0 / 68.3 / 68.8).

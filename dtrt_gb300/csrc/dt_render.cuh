@@ -223,7 +223,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         const long long Bw = std::min<long long>(B, total);
         const int levels = o->max_bounces + 1;  // a continuing vertex always spends one bounce
         bool wavefront = s->camera_schedule == DTRT_CAMERA_WAVEFRONT ||
-                         (s->camera_schedule == DTRT_CAMERA_AUTO && Bw >= kWavefrontMinPaths);
+                         (s->camera_schedule == DTRT_CAMERA_AUTO && Bw >= kWavefrontMinPaths && levels <= kWavefrontMaxLevels);
         const size_t state_size = fixed_rays ? CameraStage<N, 0>::state_bytes : CameraStage<N, N>::state_bytes,
                      hit_size = fixed_rays ? CameraStage<N, 0>::hit_bytes : CameraStage<N, N>::hit_bytes;
         const size_t state_bytes = ((size_t)Bw * state_size + 255) & ~(size_t)255,

@@ -319,11 +319,12 @@ int dtrt_scene_set_tracking_cap(dtrt_scene *scene, int max_steps);
  * the density adjoint's replay and the primal render. MEGAKERNEL: one thread carries its
  * path to the end in one launch; WAVEFRONT: launches per path vertex over the paths still
  * alive, compacted into queues after every vertex (path state in device memory between
- * launches); AUTO picks per render (wavefront from 65,536 paths; for the primal render only
- * in scenes with grid media). Same code and random numbers per path and pixel sums in path
- * order: forward and primal images are identical under both, the density gradient equal up
- * to the order of its FP32 atomic sums. dtrt_render_fwd_noalloc, the vertex adjoint and the
- * batch's persistent schedule always use the megakernel. */
+ * launches); AUTO picks per render (wavefront from 65,536 paths, in forward mode up to 1023
+ * bounces; for the primal render only in scenes with grid media). Same code and random
+ * numbers per path and pixel sums in path order: forward and primal images are identical
+ * under both, the density gradient equal up to the order of its FP32 atomic sums.
+ * dtrt_render_fwd_noalloc, the vertex adjoint and the batch's persistent schedule always use
+ * the megakernel. */
 #define DTRT_CAMERA_AUTO 0
 #define DTRT_CAMERA_MEGAKERNEL 1
 #define DTRT_CAMERA_WAVEFRONT 2
