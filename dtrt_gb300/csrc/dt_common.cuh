@@ -145,6 +145,13 @@ DT_HD double angle_d(double s, double c) {
     return a + fma(s, ca, -(c * sa));
 }
 
+// Both sub-paths' values a s and b s of an edge sample in one derivative slot: each rounded to
+// FP32 as a record is, the sum in FP64 as the accumulators are. The two nearly cancel, so an
+// FP32 sum a + b would drop bits that the accumulators kept when each was added by itself. (It
+// is faster: C2 forward 77.6 ms against 79.3. Conversions by moves of bits in place of the FP64
+// pipe's: 82.5, more registers spilled.)
+DT_HD double pair_value(float a, float b, float s) { return (double)(a * s) + (double)(b * s); }
+
 // ------------------------------------------------------------------ FP32 dual number
 // value + N derivative slots; simpleAD.h:20-245 chain rules
 template <int N>

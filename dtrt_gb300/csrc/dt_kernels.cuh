@@ -929,8 +929,8 @@ __global__ void k_li_keys(DevScene sc, const Task *tasks, long long npairs, unsi
 
 // Eight resident blocks per SM: the kernel issues on half the cycles with 11 of 32 lanes
 // active, and more warps hide more of the traversal's latency than their spills cost. The two
-// sub-paths of a sample share pixel and slot weights: their lanes add up the radiance first
-// and each adds every other slot, half the FP64 atomics.
+// sub-paths of a sample share pixel and slot weights: their lanes exchange the radiance and each
+// adds both values of every other slot, half the FP64 atomics.
 template <int N, int kMedia>
 __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, Queue qli, long long begin, long long count,
                                                double *acc1, double *acc2, const int *perm,
@@ -948,9 +948,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, 
         n = 1;
         wl = cmul(f3(t.w), li_path<kMedia>(sc, rng, f3(t.o), f3(t.d), t.depth, t.med, (t.flags & 1) != 0, c));
     }
-    wl = mk(wl.x + __shfl_xor_sync(0xffffffffu, wl.x, 1), wl.y + __shfl_xor_sync(0xffffffffu, wl.y, 1),
-            wl.z + __shfl_xor_sync(0xffffffffu, wl.z, 1));
-    if (gi < count && !is_zero3(wl, 0.f)) {
+    const float3 wp = mk(__shfl_xor_sync(0xffffffffu, wl.x, 1), __shfl_xor_sync(0xffffffffu, wl.y, 1),
+                         __shfl_xor_sync(0xffffffffu, wl.z, 1));
+    if (gi < count && !(is_zero3(wl, 0.f) && is_zero3(wp, 0.f))) {
         const bool prim = (t.flags & 2) != 0;
         double *acc = prim ? acc2 : acc1 + (size_t)rp.npix * 3;  // slot j of the derivative images
         const bool alone = (gi ^ 1) >= count;
@@ -958,9 +958,9 @@ __global__ void __launch_bounds__(kBlock, 8) k_li(DevScene sc, RenderParams rp, 
         for (int j = 0; j < N; ++j) {
             if (t.s[j] == 0.f || (!alone && ((j ^ (int)gi) & 1))) continue;
             double *a = acc + ((size_t)j * rp.npix + t.pixel) * 3;
-            atomicAdd(a, (double)(wl.x * t.s[j]));
-            atomicAdd(a + 1, (double)(wl.y * t.s[j]));
-            atomicAdd(a + 2, (double)(wl.z * t.s[j]));
+            atomicAdd(a, pair_value(wl.x, wp.x, t.s[j]));
+            atomicAdd(a + 1, pair_value(wl.y, wp.y, t.s[j]));
+            atomicAdd(a + 2, pair_value(wl.z, wp.z, t.s[j]));
         }
     }
     if (ctr) flush_counters(ctr, K_LI, c, CT_LI, n);
