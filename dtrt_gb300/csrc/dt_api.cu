@@ -103,16 +103,6 @@ int gather_cells(const dtrt_scene *s, const DevScene &sc, float *grad, cudaStrea
     return launches;
 }
 
-bool ensure_lanes(Scratch &sb, int lanes) {
-    bool ok = sb.fork_ev || cudaEventCreateWithFlags(&sb.fork_ev, cudaEventDisableTiming) == cudaSuccess;
-    for (int k = 0; k < lanes - 1 && ok; ++k) {
-        ok = sb.side[k] || cudaStreamCreateWithFlags(&sb.side[k], cudaStreamNonBlocking) == cudaSuccess;
-        ok = ok && (sb.side_ev[k] || cudaEventCreateWithFlags(&sb.side_ev[k], cudaEventDisableTiming) == cudaSuccess);
-    }
-    if (!ok) cudaGetLastError();
-    return ok;
-}
-
 bool ensure_buffer(void **ptr, size_t *have, size_t need) {
     if (*have >= need && *ptr) return true;
     if (*ptr) cudaFree(*ptr);
@@ -1160,11 +1150,7 @@ int set_edge_weights(dtrt_scene *s, const float *w) {
 }
 
 void free_scratch(Scratch &b) {
-    for (cudaStream_t q : b.side)
-        if (q) cudaStreamDestroy(q);
-    for (cudaEvent_t e : b.side_ev)
-        if (e) cudaEventDestroy(e);
-    if (b.fork_ev) cudaEventDestroy(b.fork_ev);
+    free_lanes(b);
     void *ptrs[] = {b.acc1,     b.acc2,     b.out,     b.qe,     b.ql,      b.qli,       b.counts,   b.err,
                     b.adj_dimg, b.adj_grad, b.adj_out, b.adj_img, b.cam_state, b.cam_q, b.cam_cnt, b.li_sort, b.cells};
     for (void *p : ptrs)

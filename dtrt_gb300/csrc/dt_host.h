@@ -6,17 +6,12 @@
 #include "../../include/dtrt_gb300.h"
 #include "dt_bvh.h"
 #include "dt_kernels.cuh"
+#include "dt_lanes.h"
 
 namespace dt {
 
 void set_last_error(const std::string &msg);
 
-// Wavefront batches in flight at once, each on a stream and a workspace of its own: a batch's
-// last levels hold few paths and take as long as their slowest vertex, and the other batches
-// run in the meantime; small batches read neighbouring voxels. C3 forward (33.6 M paths): one
-// lane of 2^23 paths 68.8 ms, 4 lanes of 2^21 63.7, 8 of 2^20 63.1, 8 of 2^19 66.4; C1 primal: one of
-// 2^22 15.9, 8 of 2^20 14.8, 8 of 2^19 14.1. Eight streams are what the device queues.
-constexpr int kLanes = 8;
 // The density replay keeps 780 B a path, and a program that holds many scenes holds a workspace
 // for each: 2^22 paths in all (3.3 GB). C3 density adjoint: one lane of 2^22 41.4 ms, 2 of
 // 2^21 39.3, 4 of 2^20 38.0, 8 of 2^19 38.7 (8 of 2^21, 13 GB, 35.5).
@@ -24,7 +19,7 @@ constexpr int kReplayLanes = 4;
 constexpr long long kReplayBatchPaths = 1ll << 20;
 
 // Device buffers reused across renders of one scene, grown on demand.
-struct Scratch {
+struct Scratch : Lanes {
     double *acc1 = nullptr, *acc2 = nullptr;
     size_t acc1_n = 0, acc2_n = 0;
     float *out = nullptr;
@@ -46,35 +41,9 @@ struct Scratch {
     // density cells of a render (DevScene::cells), then the replay's gradient in that layout
     void *cells = nullptr;
     size_t cells_bytes = 0;
-    // side streams of the lanes 1..., the fork and join events (made by the first render of several batches)
-    cudaStream_t side[kLanes - 1] = {};
-    cudaEvent_t fork_ev = nullptr, side_ev[kLanes - 1] = {};
 };
 
 bool ensure_buffer(void **ptr, size_t *have, size_t need);
-// Streams and events of `lanes` lanes: false (and the error cleared) when they cannot be made.
-bool ensure_lanes(Scratch &sb, int lanes);
-
-// f(batch, lane, stream) for each of n batches, dealt in turn to st and lanes - 1 side streams
-// that fork from st and join it again.
-template <class F>
-cudaError_t in_lanes(Scratch &sb, cudaStream_t st, int lanes, long long n, F f) {
-    cudaError_t e = cudaSuccess;
-    auto ck = [&](cudaError_t r) { e = e == cudaSuccess ? r : e; };
-    if (lanes > 1) {
-        ck(cudaEventRecord(sb.fork_ev, st));
-        for (int k = 1; k < lanes; ++k) ck(cudaStreamWaitEvent(sb.side[k - 1], sb.fork_ev, 0));
-    }
-    for (long long k = 0; k < n && e == cudaSuccess; ++k) {
-        const int lane = (int)(k % lanes);
-        ck(f(k, lane, lane ? sb.side[lane - 1] : st));
-    }
-    for (int k = 1; k < lanes; ++k) {
-        ck(cudaEventRecord(sb.side_ev[k - 1], sb.side[k - 1]));
-        ck(cudaStreamWaitEvent(st, sb.side_ev[k - 1], 0));
-    }
-    return e;
-}
 
 // Buffers of the Li pair sort for queues of li_cap tasks (li_cap / 2 pairs): false (and
 // the allocation error cleared) when the device has no room, the Li kernels then read the

@@ -307,13 +307,11 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             tot_edge += ne;
             tot_lins += nl;
             // Lins records run on a side stream beside the edge samples and their Li sub-paths
-            const bool lins_aside = nl && ensure_lanes(sb, 2);
-            if (lins_aside) {
-                DT_CK(cudaEventRecord(sb.fork_ev, st));
-                DT_CK(cudaStreamWaitEvent(sb.side[0], sb.fork_ev, 0));
-                run_lins(sb.side[0], nl);
+            SideWork lins(sb, st);
+            if (nl && ensure_lanes(sb, 2)) {
+                DT_CK(lins.fork());
+                run_lins(lins.stream(), nl);
                 ++launches;
-                DT_CK(cudaEventRecord(sb.side_ev[0], sb.side[0]));
             }
             for (unsigned long long r0 = 0; r0 < ne && rp.sppse > 0; r0 += per_chunk) {
                 const long long cnt = (long long)std::min<unsigned long long>(per_chunk, ne - r0);
@@ -332,7 +330,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
             }
             if (nl)
                 if ((rc = timed(ms_li, [&] {
-                         if (lins_aside) cudaStreamWaitEvent(st, sb.side_ev[0], 0);
+                         if (lins.open()) lins.join();
                          else run_lins(st, nl);
                      })))
                     return rc;
