@@ -691,7 +691,7 @@ DT_D int sample_reuse(const double *cdf, int n, double &u, double &pdf) {
     while (idx < n - 1 && __double_as_longlong(__ldg(cdf + idx + 1)) == __double_as_longlong(__ldg(cdf + idx))) ++idx;
     const double c0 = __ldg(cdf + idx);
     pdf = __ldg(cdf + idx + 1) - c0;
-    u = (u - c0) * rcp_d(pdf);
+    u = (u - c0) / pdf;  // rounded once: times rcp_d(pdf) it was off by 0.6 instead of 0.4 x 2^-53 (rms)
     return idx;
 }
 
