@@ -1,5 +1,7 @@
 """FP64 arithmetic of the edge kernels as the device runs it, in a small program of its own: the reuse
-of a CDF's random number is the correctly rounded quotient."""
+of a CDF's random number is the correctly rounded quotient; reciprocal, square root, sine,
+cosine and angle, whose seeds are the device's FP32 approximations, keep the bounds that the
+host build of the same code has (test_fp64_math.py), also at the ends of the seeds' range."""
 import os
 import shutil
 import subprocess
@@ -25,6 +27,16 @@ static __global__ void k_reuse(const double *cdf, int n, const double *u, int m,
     out[3 * i + 1] = x;
     out[3 * i + 2] = pdf;
 }
+static __global__ void k_math(const double *in, int m, double *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const double x = in[4 * i], t = in[4 * i + 1];
+    double *o = out + 6 * i;
+    o[0] = rcp_d(x);
+    o[1] = rsqrt_d(fabs(x), o[2]);
+    sincos_d(t, o[3], o[4]);
+    o[5] = angle_d(in[4 * i + 2], in[4 * i + 3]);
+}
 static std::vector<double> read(const char *p) {
     std::vector<double> v;
     FILE *f = fopen(p, "rb");
@@ -41,11 +53,13 @@ static double *upload(const std::vector<double> &v) {
 }
 int main(int, char **a) {
     const std::vector<double> cdf = read(a[1]), in = read(a[2]);
-    const int m = (int)in.size();
-    std::vector<double> out(3 * (size_t)m);
+    const bool math = cdf.size() < 2;  // no CDF: the functions
+    const int m = (int)in.size() / (math ? 4 : 1);
+    std::vector<double> out((math ? 6 : 3) * (size_t)m);
     double *dc = upload(cdf), *di = upload(in), *dout = upload(out);
     if (!dc || !di || !dout) return 2;
-    k_reuse<<<(m + 127) / 128, 128>>>(dc, (int)cdf.size() - 1, di, m, dout);
+    if (math) k_math<<<(m + 127) / 128, 128>>>(di, m, dout);
+    else k_reuse<<<(m + 127) / 128, 128>>>(dc, (int)cdf.size() - 1, di, m, dout);
     if (cudaMemcpy(out.data(), dout, out.size() * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return 3;
     FILE *g = fopen(a[3], "wb");
     const bool ok = g && fwrite(out.data(), 8, out.size(), g) == out.size();
@@ -85,3 +99,34 @@ def test_cdf_reuse_rounds_once(program, n):
     assert np.array_equal(o[:, 0].astype(int), idx)
     assert np.array_equal(o[:, 2], pdf)
     assert np.array_equal(o[:, 1], (u - cdf[idx]) / pdf)
+
+
+def test_math_keeps_the_bounds_of_the_host_build(program):
+    rng = np.random.default_rng(3)
+    n = 20000
+    x = np.exp(rng.uniform(-300, 300, n)) * rng.choice([-1.0, 1.0], n)
+    x[: n // 2] = rng.uniform(-4, 4, n // 2)
+    # the ends of the FP32 seeds' range, 2^-125 to 2^125, and the powers beside them
+    ends = [s * 2.0 ** e * m for e in (-127, -126, -125, -124, 124, 125, 126, 127) for s in (1, -1)
+            for m in (1.0, np.nextafter(1.0, 2.0), 1.5, np.nextafter(2.0, 1.0))]
+    x[: len(ends)] = ends
+    t = rng.uniform(0, np.pi, n)
+    t[:11] = [0.0, np.pi, np.pi / 2, np.pi / 4, 3 * np.pi / 4, 1e-7, np.pi - 1e-7, 1e-12, 1e-300, 0.78539816, 2.35619449]
+    o = program([0.0], np.stack([x, t, np.sin(t), np.cos(t)], 1), 6)
+    eps = 2.0 ** -53
+    # a seed off by 2^-21 at most leaves 2^-63 after the third-order step: the roundings remain, as on the host
+    assert np.abs(o[:, 0] * x - 1).max() <= 5 * eps
+    assert np.abs(o[:, 1] * np.sqrt(np.abs(x)) - 1).max() <= 6 * eps
+    assert np.abs(o[:, 2] / np.sqrt(np.abs(x)) - 1).max() <= 6 * eps
+    assert np.abs(o[:, 3] - np.sin(t)).max() <= 4 * eps and np.abs(o[:, 4] - np.cos(t)).max() <= 4 * eps
+    assert np.abs(o[:, 5] - t).max() <= 8 * eps
+
+
+def test_math_of_zero_and_not_finite(program):
+    x = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, 1.7e308])
+    o = program([0.0], np.stack([x, 0 * np.ones(7), np.zeros(7), np.ones(7)], 1), 6)
+    with np.errstate(all="ignore"):
+        np.testing.assert_array_equal(o[:, 0], 1 / x)
+        np.testing.assert_array_equal(o[:, 2], np.sqrt(np.abs(x)))
+        np.testing.assert_array_equal(o[:, 1], 1 / np.sqrt(np.abs(x)))
+    assert (o[:, 5] == 0).all()
