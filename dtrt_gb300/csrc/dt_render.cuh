@@ -141,8 +141,8 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     DT_CK(cudaEventCreate(&e1));
     double ms_camera = 0, ms_edge = 0, ms_li = 0, ms_primary = 0;
     uint64_t launches = 0;
-    auto timed = [&](double &acc, auto &&launch) -> int {
-        ++launches;
+    auto timed = [&](double &acc, auto &&launch, int kernels = 1) -> int {
+        launches += kernels;
         cudaEventRecord(e0, st);
         launch();
         cudaEventRecord(e1, st);
@@ -191,7 +191,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     // primary-edge samples, a chunk at most at once
     uint64_t prim_samples = 0;
     const long long prim_chunk = std::max<long long>(1, (long long)(li_cap / 2));
-    if (o->sppe > 0 && sc.num_pedges > 0) {
+    if (o->sppe > 0 && sc.num_pedges > 0 && !fixed_rays) {  // no edge moves on the screen under fixed rays
         prim_samples = (uint64_t)std::ceil(sc.pedge_sum * o->sppe / 128.0) * 128;
         rp.prim_weight = sc.pedge_sum / (double)prim_samples;
     }
@@ -328,17 +328,15 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                 }
                 if ((rc = drain_li())) return rc;
             }
-            if (nl)
-                if ((rc = timed(ms_li, [&] {
-                         if (lins.open()) lins.join();
-                         else run_lins(st, nl);
-                     })))
-                    return rc;
+            if (lins.open()) {
+                if ((rc = timed(ms_li, [&] { lins.join(); }, 0))) return rc;  // what is left of the Lins kernel
+            } else if (nl && (rc = timed(ms_li, [&] { run_lins(st, nl); }))) {
+                return rc;
+            }
         }
     }
     // ---------------------------------------------------------------- pass 2: primary edges
-    // (no edge moves on the screen under fixed rays)
-    for (long long k0 = 0; k0 < (long long)prim_samples && !fixed_rays && !prim_done; k0 += prim_chunk) {
+    for (long long k0 = 0; k0 < (long long)prim_samples && !prim_done; k0 += prim_chunk) {
         if ((rc = run_primary(k0, std::min(prim_chunk, (long long)prim_samples - k0)))) return rc;
         if ((rc = drain_li())) return rc;
     }

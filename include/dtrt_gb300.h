@@ -173,7 +173,7 @@ typedef struct {
     uint64_t edge_records;    /* secondary-edge vertex records                      */
     uint64_t edge_samples;    /* secondary-edge samples evaluated                   */
     uint64_t lins_records;    /* Lins boundary records                              */
-    uint64_t primary_edge_samples;
+    uint64_t primary_edge_samples; /* samples run: 0 where no edge can move on the screen */
     uint64_t li_tasks;        /* non-AD sub-paths traced (edge, Lins, primary edge) */
     uint64_t rays;            /* closest-hit queries                                */
     uint64_t node_visits;     /* BVH nodes fetched                                  */
@@ -186,7 +186,8 @@ typedef struct {
     double ms_total;
     double ms_camera;         /* camera AD path kernel(s)                           */
     double ms_edge;           /* secondary-edge kernel(s)                           */
-    double ms_li;             /* Li sub-path kernel(s)                              */
+    double ms_li;             /* Li sub-path kernel(s), and what the Lins kernel, which runs
+                               * beside the edge samples and their sub-paths, takes longer than they do */
     double ms_primary;        /* primary-edge kernel(s)                             */
     double ms_setup;          /* scene upload / derived data for this render        */
     int counters_enabled;
