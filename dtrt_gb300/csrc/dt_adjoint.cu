@@ -185,7 +185,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     int lanes = 1;
     if (wavefront) {
         const long long cap = std::min<long long>(kReplayBatchPaths, std::max<long long>(total, 1));
-        lanes = (int)std::min<long long>(kReplayLanes, std::max<long long>(1, (total + cap - 1) / cap));
+        lanes = lanes_for((total + cap - 1) / cap, cap, kReplayLanes, kReplayLanes * kReplayBatchPaths);
         if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
         const size_t bytes = (AdjWave::bytes(cap, o->max_bounces + 1) + 255) & ~(size_t)255;
         if (ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * bytes)) {

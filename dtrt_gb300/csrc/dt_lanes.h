@@ -1,5 +1,7 @@
 // dtrt_gb300 — side streams of a render: batches in flight at once, and work beside the main stream.
 #pragma once
+#include <algorithm>
+
 #include <cuda_runtime_api.h>
 
 namespace dt {
@@ -16,6 +18,12 @@ struct Lanes {
     cudaStream_t side[kLanes - 1] = {};
     cudaEvent_t fork_ev = nullptr, side_ev[kLanes - 1] = {};
 };
+
+// Lanes for n batches of batch_paths paths each: `most`, or fewer where so many workspaces would
+// hold more than most_paths paths (a batch takes whole pixels, and one may have 2^24 samples).
+inline int lanes_for(long long n, long long batch_paths, int most, long long most_paths) {
+    return (int)std::max<long long>(1, std::min({(long long)most, n, most_paths / std::max<long long>(1, batch_paths)}));
+}
 
 // Streams and events of `lanes` lanes: false (and the error cleared) when they cannot be made.
 inline bool ensure_lanes(Lanes &sb, int lanes) {

@@ -172,7 +172,7 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     int lanes = 1;
     if (wavefront) {
         B = std::min<long long>(1ll << 19, std::max<long long>(total, 1));
-        lanes = (int)std::min<long long>(kLanes, std::max<long long>(1, (total + B - 1) / B));
+        lanes = lanes_for((total + B - 1) / B, B, kLanes, kLanes * B);
         if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
         sbytes = ((size_t)B * sizeof(LiState) + 255) & ~(size_t)255;
         wbytes = (sbytes + (size_t)B * sizeof(float3) + 255) & ~(size_t)255;

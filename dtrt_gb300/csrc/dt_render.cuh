@@ -230,7 +230,7 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
                      work_bytes = (state_bytes + (size_t)Bw * sizeof(VertexIn) + 255) & ~(size_t)255;
         const long long nb = (total + B - 1) / B;
         // several batches in flight; the counters read each batch's level counts, so one then
-        int lanes = wavefront && fixed_rays && !ctr ? (int)std::min<long long>(kLanes, nb) : 1;
+        int lanes = wavefront && fixed_rays && !ctr ? lanes_for(nb, Bw, kLanes, kLanes * kStaticBatchPaths) : 1;
         if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
         if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * work_bytes) &&
                            ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * lanes * Bw * sizeof(int)) &&

@@ -93,3 +93,37 @@ def test_forked_streams_join(tmp_path):
                     str(tmp_path / "d.cpp"), "-o", exe], check=True)
     r = subprocess.run([exe], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stderr)
+
+
+LANES = r"""
+#include "dt_lanes.h"
+#include <cstdio>
+using dt::lanes_for;
+int main() {
+    const long long P = 1ll << 20;
+    // as planned: up to 8 batches of 2^20 paths
+    if (lanes_for(1, P, 8, 8 * P) != 1 || lanes_for(3, P, 8, 8 * P) != 3 || lanes_for(99, P, 8, 8 * P) != 8) return 1;
+    if (lanes_for(0, 1, 8, 8 * P) != 1) return 2;  // nothing to render
+    // one pixel with more samples than a batch was meant to hold
+    if (lanes_for(4, 1ll << 24, 8, 8 * P) != 1 || lanes_for(4, 1ll << 22, 8, 8 * P) != 2) return 3;
+    for (long long b = 1; b < (1ll << 26); b = b * 3 + 1)
+        for (long long n : {0ll, 1ll, 2ll, 7ll, 8ll, 1000ll}) {
+            const int k = lanes_for(n, b, 8, 8 * P);
+            if (k < 1 || k > 8 || (k > 1 && (k * b > 8 * P || k > n))) return 4;
+        }
+    puts("ok");
+    return 0;
+}
+"""
+
+
+def test_lanes_are_bounded_by_their_paths(tmp_path):
+    if not shutil.which("g++") or not os.path.isdir(CUDA_INC):
+        pytest.skip("g++ or the CUDA headers are missing")
+    # the functions that call the runtime are linked against nothing: only lanes_for is used
+    (tmp_path / "d.cpp").write_text(LANES)
+    exe = str(tmp_path / "d")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CUDA_INC, "-I", os.path.join(ROOT, "dtrt_gb300", "csrc"),
+                    str(tmp_path / "d.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stderr)
