@@ -145,7 +145,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
         if (on_device) {
             dimg = d_image;
         } else {
-            if (!ensure_buffer((void **)&sb.adj_dimg, &sb.adj_dimg_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
+            if (!ensure_buffer(sb, (void **)&sb.adj_dimg, &sb.adj_dimg_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
             DT_ACK(cudaMemcpyAsync(sb.adj_dimg, d_image, npix * 3 * 4, cudaMemcpyHostToDevice, st));
             dimg = sb.adj_dimg;
         }
@@ -156,14 +156,15 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
         if (on_device) {
             grad = d_density;
         } else {
-            if (!ensure_buffer((void **)&sb.adj_grad, &sb.adj_grad_n, nvox * 4)) return DTRT_ERR_CUDA;
+            if (!ensure_buffer(sb, (void **)&sb.adj_grad, &sb.adj_grad_n, nvox * 4)) return DTRT_ERR_CUDA;
             grad = sb.adj_grad;
         }
         DT_ACK(cudaMemsetAsync(grad, 0, nvox * 4, st));
     }
     double *img_acc = nullptr;
     if (image) {
-        if (!ensure_buffer((void **)&sb.adj_img, &sb.adj_img_n, npix * 3 * 8)) return DTRT_ERR_CUDA;
+        if (!ensure_buffer(sb, (void **)&sb.adj_img, &sb.adj_img_n, npix * 3 * 8)) return DTRT_ERR_CUDA;
+        if (!on_device && !ensure_buffer(sb, (void **)&sb.adj_out, &sb.adj_out_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
         img_acc = sb.adj_img;
         DT_ACK(cudaMemsetAsync(img_acc, 0, npix * 3 * 8, st));
     }
@@ -175,7 +176,6 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     uint64_t launches = 0;
     float ms_replay = 0.f;
     DT_ACK(cudaEventRecord(e0, st));
-    launches += (uint64_t)prepare_cells(s, sc, total, 16, grad != nullptr && dimg != nullptr, st);
     // schedule: the wavefront (pass A and pass B each one launch per vertex over the live
     // paths) for large renders, as dtrt_render_fwd's camera schedule
     const long long B = 1ll << 24;  // paths per megakernel launch
@@ -188,14 +188,13 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
         lanes = lanes_for((total + cap - 1) / cap, cap, kReplayLanes, kReplayLanes * kReplayBatchPaths);
         if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
         const size_t bytes = (AdjWave::bytes(cap, o->max_bounces + 1) + 255) & ~(size_t)255;
-        if (ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * bytes)) {
-            for (int k = 0; k < lanes; ++k) w[k].carve((char *)sb.cam_state + k * bytes, cap, o->max_bounces + 1);
-        } else {
-            if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
-            cudaGetLastError();  // AUTO: no room for the path states, run the megakernel
-            wavefront = false;
-        }
+        lanes = fit_lanes(lanes, [&](int k) { return ensure_buffer(sb, &sb.cam_state, &sb.cam_state_bytes, k * bytes); },
+                          [&] { drop_wavefront(sb); });
+        for (int k = 0; k < lanes; ++k) w[k].carve((char *)sb.cam_state + k * bytes, cap, o->max_bounces + 1);
+        if (!lanes && s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
+        wavefront = lanes > 0;  // AUTO: no room for the path states, run the megakernel
     }
+    launches += (uint64_t)prepare_cells(s, sc, total, 16, grad != nullptr && dimg != nullptr, st);
     if (wavefront) {
         int sms = 0;
         DT_ACK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
@@ -216,11 +215,7 @@ int render_adjoint(dtrt_scene *s, const dtrt_render_options *o, const float *d_i
     if (grad) launches += (uint64_t)gather_cells(s, sc, grad, st);
     DT_ACK(cudaEventRecord(e1, st));
     if (image) {
-        float *dst = image;
-        if (!on_device) {
-            if (!ensure_buffer((void **)&sb.adj_out, &sb.adj_out_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
-            dst = sb.adj_out;
-        }
+        float *dst = on_device ? image : sb.adj_out;
         k_adjoint_image<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(rp.npix, img_acc, dst);
         ++launches;
         DT_ACK(cudaGetLastError());

@@ -69,7 +69,7 @@ int prepare_cells(dtrt_scene *s, DevScene &sc, long long paths, int per_path, bo
     if (n <= 0 || n > (1ll << 27) || paths < n / per_path) return 0;
     if (!with_grad && (n < (1ll << 15) || paths < kWavefrontMinPaths)) return 0;
     Scratch &sb = s->scratch;
-    if (!ensure_buffer(&sb.cells, &sb.cells_bytes, (size_t)n * 32 * (with_grad ? 2 : 1))) {
+    if (!ensure_buffer(sb, &sb.cells, &sb.cells_bytes, (size_t)n * 32 * (with_grad ? 2 : 1))) {
         cudaGetLastError();  // no room: the kernels read the voxels
         return 0;
     }
@@ -103,19 +103,19 @@ int gather_cells(const dtrt_scene *s, const DevScene &sc, float *grad, cudaStrea
     return launches;
 }
 
-bool ensure_buffer(void **ptr, size_t *have, size_t need) {
-    if (*have >= need && *ptr) return true;
-    if (*ptr) cudaFree(*ptr);
-    *ptr = nullptr;
-    *have = 0;
-    cudaError_t e = cudaMalloc(ptr, std::max<size_t>(need, 256));
-    if (e != cudaSuccess) {
-        set_last_error(std::string("cudaMalloc(") + std::to_string(need) + "): " + cudaGetErrorString(e));
-        *ptr = nullptr;
-        return false;
+bool ensure_buffer(Scratch &sb, void **ptr, size_t *have, size_t need) {
+    const cudaError_t e = grow_buffer(ptr, have, need, &sb.cells, &sb.cells_bytes);
+    if (e != cudaSuccess) set_last_error(std::string("cudaMalloc(") + std::to_string(need) + "): " + cudaGetErrorString(e));
+    return e == cudaSuccess;
+}
+
+void drop_wavefront(Scratch &sb) {
+    void **ptrs[] = {&sb.cam_state, &sb.cam_q, &sb.cam_cnt};
+    for (void **p : ptrs) {
+        if (*p) cudaFree(*p);
+        *p = nullptr;
     }
-    *have = std::max<size_t>(need, 256);
-    return true;
+    sb.cam_state_bytes = sb.cam_q_bytes = sb.cam_cnt_bytes = 0;
 }
 
 namespace {

@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "../../include/dtrt_gb300.h"
+#include "dt_buffers.h"
 #include "dt_bvh.h"
 #include "dt_kernels.cuh"
 #include "dt_lanes.h"
@@ -43,14 +44,18 @@ struct Scratch : Lanes {
     size_t cells_bytes = 0;
 };
 
-bool ensure_buffer(void **ptr, size_t *have, size_t need);
+// A buffer of at least `need` bytes at *ptr; a full device gives up the density cells, which no kernel
+// of the render reads yet: prepare_cells comes after every other buffer.
+bool ensure_buffer(Scratch &sb, void **ptr, size_t *have, size_t need);
+// The wavefront workspaces (cam_state, cam_q, cam_cnt) given back
+void drop_wavefront(Scratch &sb);
 
 // Buffers of the Li pair sort for queues of li_cap tasks (li_cap / 2 pairs): false (and
 // the allocation error cleared) when the device has no room, the Li kernels then read the
 // queue in order.
 inline bool ensure_li_sort(Scratch &sb, uint64_t li_cap) {
     const long long cap = (long long)(li_cap / 2);
-    if (ensure_buffer(&sb.li_sort, &sb.li_sort_bytes, (size_t)cap * 16 + radix_hist_entries(cap) * 4)) return true;
+    if (ensure_buffer(sb, &sb.li_sort, &sb.li_sort_bytes, (size_t)cap * 16 + radix_hist_entries(cap) * 4)) return true;
     cudaGetLastError();
     return false;
 }

@@ -154,7 +154,8 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
     DT_PCK(cudaMemsetAsync(sb.err, 0, sizeof(unsigned int), st));
     DT_PCK(cudaMemsetAsync(sb.counts, 0, kCountSlots * sizeof(unsigned long long), st));
     unsigned long long *ctr = s->counters ? sb.counts + 8 : nullptr;
-    if (!ensure_buffer((void **)&sb.adj_img, &sb.adj_img_n, npix * 3 * 8)) return DTRT_ERR_CUDA;
+    if (!ensure_buffer(sb, (void **)&sb.adj_img, &sb.adj_img_n, npix * 3 * 8)) return DTRT_ERR_CUDA;
+    if (!out_on_device && !ensure_buffer(sb, (void **)&sb.adj_out, &sb.adj_out_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
     DT_PCK(cudaMemsetAsync(sb.adj_img, 0, npix * 3 * 8, st));
     cudaEvent_t e0, e1;
     DT_PCK(cudaEventCreate(&e0));
@@ -176,12 +177,14 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
         if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
         sbytes = ((size_t)B * sizeof(LiState) + 255) & ~(size_t)255;
         wbytes = (sbytes + (size_t)B * sizeof(float3) + 255) & ~(size_t)255;
-        if (!(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * wbytes) &&
-              ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)2 * lanes * B * sizeof(int)) &&
-              ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)lanes * (levels + 1) * sizeof(unsigned long long)))) {
+        lanes = fit_lanes(lanes, [&](int k) {
+            return ensure_buffer(sb, &sb.cam_state, &sb.cam_state_bytes, k * wbytes) &&
+                   ensure_buffer(sb, &sb.cam_q, &sb.cam_q_bytes, (size_t)2 * k * B * sizeof(int)) &&
+                   ensure_buffer(sb, &sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)k * (levels + 1) * sizeof(unsigned long long));
+        }, [&] { drop_wavefront(sb); });
+        if (!lanes) {
             if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
-            cudaGetLastError();  // AUTO: no room for the path states, run the megakernel
-            wavefront = false;
+            wavefront = false;  // AUTO: no room for the path states, run the megakernel
             B = 1ll << 26;
         }
     }
@@ -226,11 +229,7 @@ int render_primal(dtrt_scene *s, const dtrt_render_options *o, float *out, int o
         DT_PCK(cudaGetLastError());
     }
     DT_PCK(cudaEventRecord(e1, st));
-    float *dst = out;
-    if (!out_on_device) {
-        if (!ensure_buffer((void **)&sb.adj_out, &sb.adj_out_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
-        dst = sb.adj_out;
-    }
+    float *dst = out_on_device ? out : sb.adj_out;
     k_primal_image<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(rp.npix, sb.adj_img, dst);
     ++launches;
     DT_PCK(cudaGetLastError());

@@ -111,9 +111,9 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     const size_t npix = (size_t)rp.npix;
     // ---------------------------------------------------------------- buffers
     const size_t acc1_n = (N + 1) * npix * 3, acc2_n = (size_t)N * npix * 3, out_n = (N + 1) * npix * 3;
-    if (!ensure_buffer((void **)&sb.acc1, &sb.acc1_n, acc1_n * 8) || !ensure_buffer((void **)&sb.acc2, &sb.acc2_n, acc2_n * 8))
+    if (!ensure_buffer(sb, (void **)&sb.acc1, &sb.acc1_n, acc1_n * 8) || !ensure_buffer(sb, (void **)&sb.acc2, &sb.acc2_n, acc2_n * 8))
         return DTRT_ERR_CUDA;
-    if (!out_on_device && !ensure_buffer((void **)&sb.out, &sb.out_n, out_n * 4)) return DTRT_ERR_CUDA;
+    if (!out_on_device && !ensure_buffer(sb, (void **)&sb.out, &sb.out_n, out_n * 4)) return DTRT_ERR_CUDA;
     const uint64_t li_cap = s->queue_cap ? s->queue_cap : (uint64_t)24 << 20;
     // 16 Mi records bound a camera batch at 16Mi/(max_bounces+1) paths (1.5 M at depth 10):
     // few launches, so the partial last wave of each batch costs little
@@ -122,9 +122,9 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     // no queues, and the camera stage without ray derivatives (C1, C3 and every density or
     // material optimisation)
     const bool fixed_rays = static_rays(sc);
-    if (!fixed_rays && (!ensure_buffer(&sb.qli, &sb.qli_bytes, li_cap * sizeof(LiTask<N>)) ||
-                        !ensure_buffer(&sb.qe, &sb.qe_bytes, rec_cap * sizeof(EdgeRec<N>)) ||
-                        !ensure_buffer(&sb.ql, &sb.ql_bytes, rec_cap * sizeof(LinsRec<N>))))
+    if (!fixed_rays && (!ensure_buffer(sb, &sb.qli, &sb.qli_bytes, li_cap * sizeof(LiTask<N>)) ||
+                        !ensure_buffer(sb, &sb.qe, &sb.qe_bytes, rec_cap * sizeof(EdgeRec<N>)) ||
+                        !ensure_buffer(sb, &sb.ql, &sb.ql_bytes, rec_cap * sizeof(LinsRec<N>))))
         return DTRT_ERR_CUDA;
     if (!sb.counts) DT_CK(cudaMalloc(&sb.counts, kCountSlots * sizeof(unsigned long long)));
     if (!sb.err) DT_CK(cudaMalloc(&sb.err, sizeof(unsigned int)));
@@ -211,7 +211,6 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
     bool prim_done = false;
     // ---------------------------------------------------------------- pass 1
     const long long total = (long long)npix * std::max(0, o->spp);
-    launches += (uint64_t)prepare_cells(s, sc, total, 16, false, st);
     if (total > 0) {
         const long long unit = std::max<long long>(128, (long long)rp.spp % 32 == 0 ? std::max(rp.spp, 128) : 128);
         // without records a batch is bounded by the path states alone
@@ -232,13 +231,16 @@ int render_n(dtrt_scene *s, const dtrt_render_options *o, float *out, int out_on
         // several batches in flight; the counters read each batch's level counts, so one then
         int lanes = wavefront && fixed_rays && !ctr ? lanes_for(nb, Bw, kLanes, kLanes * kStaticBatchPaths) : 1;
         if (lanes > 1 && !ensure_lanes(sb, lanes)) lanes = 1;
-        if (wavefront && !(ensure_buffer(&sb.cam_state, &sb.cam_state_bytes, lanes * work_bytes) &&
-                           ensure_buffer(&sb.cam_q, &sb.cam_q_bytes, (size_t)4 * lanes * Bw * sizeof(int)) &&
-                           ensure_buffer(&sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * lanes * (levels + 1) * sizeof(unsigned long long)))) {
-            if (s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
-            cudaGetLastError();  // AUTO: no room for the path states, run the megakernel
-            wavefront = false;
+        if (wavefront) {
+            lanes = fit_lanes(lanes, [&](int k) {
+                return ensure_buffer(sb, &sb.cam_state, &sb.cam_state_bytes, k * work_bytes) &&
+                       ensure_buffer(sb, &sb.cam_q, &sb.cam_q_bytes, (size_t)4 * k * Bw * sizeof(int)) &&
+                       ensure_buffer(sb, &sb.cam_cnt, &sb.cam_cnt_bytes, (size_t)3 * k * (levels + 1) * sizeof(unsigned long long));
+            }, [&] { drop_wavefront(sb); });
+            if (!lanes && s->camera_schedule == DTRT_CAMERA_WAVEFRONT) return DTRT_ERR_CUDA;
+            wavefront = lanes > 0;  // AUTO: no room for the path states, run the megakernel
         }
+        launches += (uint64_t)prepare_cells(s, sc, total, 16, false, st);
         int sms = 0;
         DT_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device));
         used_wavefront = wavefront;

@@ -95,34 +95,34 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
     // ---------------------------------------------------------------- buffers
     const float *dimg = d_image;
     if (!on_device) {
-        if (!ensure_buffer((void **)&sb.adj_dimg, &sb.adj_dimg_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
+        if (!ensure_buffer(sb, (void **)&sb.adj_dimg, &sb.adj_dimg_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
         DT_VCK(cudaMemcpyAsync(sb.adj_dimg, d_image, npix * 3 * 4, cudaMemcpyHostToDevice, st));
         dimg = sb.adj_dimg;
     }
     const size_t nv3 = (size_t)sc.num_verts * 3;
     float *grad = d_vertices;
     if (!on_device) {
-        if (!ensure_buffer((void **)&sb.adj_grad, &sb.adj_grad_n, std::max<size_t>(nv3, 1) * 4)) return DTRT_ERR_CUDA;
+        if (!ensure_buffer(sb, (void **)&sb.adj_grad, &sb.adj_grad_n, std::max<size_t>(nv3, 1) * 4)) return DTRT_ERR_CUDA;
         grad = sb.adj_grad;
     }
     if (nv3) DT_VCK(cudaMemsetAsync(grad, 0, nv3 * 4, st));
     double *img_acc = nullptr;
     if (image) {
-        if (!ensure_buffer((void **)&sb.adj_img, &sb.adj_img_n, npix * 3 * 8)) return DTRT_ERR_CUDA;
+        if (!ensure_buffer(sb, (void **)&sb.adj_img, &sb.adj_img_n, npix * 3 * 8)) return DTRT_ERR_CUDA;
         img_acc = sb.adj_img;
         DT_VCK(cudaMemsetAsync(img_acc, 0, npix * 3 * 8, st));
     }
     const int levels = o->max_bounces + 1;
     const uint64_t li_cap = s->queue_cap ? s->queue_cap : (uint64_t)24 << 20;
     const uint64_t rec_cap = s->queue_cap ? s->queue_cap : (uint64_t)8 << 20;
-    if (!ensure_buffer(&sb.qli, &sb.qli_bytes, li_cap * sizeof(VLiTask)) ||
-        !ensure_buffer(&sb.qe, &sb.qe_bytes, rec_cap * sizeof(VEdgeRec)))
+    if (!ensure_buffer(sb, &sb.qli, &sb.qli_bytes, li_cap * sizeof(VLiTask)) ||
+        !ensure_buffer(sb, &sb.qe, &sb.qe_bytes, rec_cap * sizeof(VEdgeRec)))
         return DTRT_ERR_CUDA;
     const long long total = (long long)npix * std::max(0, o->spp);
     long long B = std::max<long long>(128, (long long)(rec_cap / (uint64_t)levels));
     B = std::min<long long>(B, std::max<long long>(total, 1));
     float *xadj = nullptr;  // x0 gradient slots of one batch (held in the Lins queue buffer)
-    if (!ensure_buffer(&sb.ql, &sb.ql_bytes, (size_t)B * levels * 3 * 4)) return DTRT_ERR_CUDA;
+    if (!ensure_buffer(sb, &sb.ql, &sb.ql_bytes, (size_t)B * levels * 3 * 4)) return DTRT_ERR_CUDA;
     xadj = (float *)sb.ql;
     Queue qe{sb.qe, sb.counts + 0, rec_cap}, qli{sb.qli, sb.counts + 2, li_cap};
     cudaEvent_t e0, e1;
@@ -204,7 +204,7 @@ int render_vertex_adjoint(dtrt_scene *s, const dtrt_render_options *o, const flo
     if (image) {
         float *dst = image;
         if (!on_device) {
-            if (!ensure_buffer((void **)&sb.adj_out, &sb.adj_out_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
+            if (!ensure_buffer(sb, (void **)&sb.adj_out, &sb.adj_out_n, npix * 3 * 4)) return DTRT_ERR_CUDA;
             dst = sb.adj_out;
         }
         k_adjoint_image<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(rp.npix, img_acc, dst);
