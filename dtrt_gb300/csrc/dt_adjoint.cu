@@ -2,9 +2,11 @@
 //
 // The replay runs with derivative width 0 whatever the scene's nder: the adjoint needs the
 // path values only, and the per-voxel gradient replaces the derivative slots. The scene
-// copy given to the kernel drops every velocity input; values and random decisions are
-// those of dtrt_render_fwd. (At width 1, with a slot that was always zero, an AdjState took
-// 208 B instead of 144 B.)
+// copy given to the kernel drops every velocity input; values and random decisions are those of
+// dtrt_render_fwd at nder 1. (At nder 3 and more the forward kernels round a Henyey-Greenstein
+// direction in another order, frame_to_world: the same image to 2e-8, behind a dielectric of alpha
+// 1e-4 to 4e-5, in 2-norm. At width 1, with a slot that was always zero, an AdjState took 208 B
+// instead of 144 B.)
 #include <algorithm>
 #include <chrono>
 #include <cstring>

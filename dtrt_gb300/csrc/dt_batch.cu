@@ -150,7 +150,7 @@ struct dtrt_batch {
 namespace dt {
 namespace {
 
-// paths per workspace of the batch wavefront (about 780 B of replay state per path)
+// paths per workspace of the batch wavefront (684 B of replay state per path)
 constexpr long long kBatchWaveCap = 1ll << 23;
 
 #define DT_BCK(call)                                                                 \

@@ -70,7 +70,12 @@ DT_HD double3_ crossd(double3_ a, double3_ b) { return mkd(a.y * b.z - a.z * b.y
 // The FP64 pipe issues two lanes a cycle per SM (1/64 of FP32), and the edge kernels are bound
 // by it: a library division or square root takes about ten of its instructions, acos or sincos
 // about forty. These take 3 (reciprocal), 6 (square root with its reciprocal) and 19 (sine and
-// cosine on [0, pi]), to the last two bits. Seeds are FP32, moved by shifts of the bits.
+// cosine on [0, pi]), to the last two bits. Seeds are FP32, moved by shifts of the bits. Each is
+// off by up to 2.5 x 2^-53 where the library's are off by 0.5 to 1; the edge-point solve and the
+// primary-edge distance made of them are, against 200-bit values, as exact as with the library
+// functions or more in every output (the angle from its sine and cosine loses nothing where
+// acos did: edges of 320 to 20,480 triangles, angle 31 to 1.5e6 -> 1.2 to 75 x 2^-53 rms,
+// direction 3 to 321 -> 0.8, distance 3 to 4850 -> 1, normal equal; primary distance 0.93 -> 0.79).
 #ifdef __CUDA_ARCH__
 DT_HD uint64_t bits_of(double x) { return (uint64_t)__double_as_longlong(x); }
 DT_HD double of_bits(uint64_t b) { return __longlong_as_double((long long)b); }
@@ -263,9 +268,7 @@ struct Frame {
     DT_D Frame() {}
     DT_D explicit Frame(float3 nn) : n(nn) {
         const float R[9] = DT_PREROT_INIT;
-        from_rotated(R, rot_apply(R, nn));
-    }
-    DT_D void from_rotated(const float *R, float3 q) {
+        const float3 q = rot_apply(R, nn);
         float3 tt;
         if (fabsf(q.x) > fabsf(q.y)) {
             float il = 1.0f / sqrtf(q.x * q.x + q.z * q.z);

@@ -13,9 +13,10 @@ namespace dt {
 
 void set_last_error(const std::string &msg);
 
-// The density replay keeps 780 B a path, and a program that holds many scenes holds a workspace
-// for each: 2^22 paths in all (3.3 GB). C3 density adjoint: one lane of 2^22 41.4 ms, 2 of
-// 2^21 39.3, 4 of 2^20 38.0, 8 of 2^19 38.7 (8 of 2^21, 13 GB, 35.5).
+// The density replay keeps 684 B a path (144 B of state, 32 of inputs, 16 of queues, 12 of values,
+// 480 of events), and a program that holds many scenes holds a workspace for each: 2^22 paths in
+// all (2.9 GB). C3 density adjoint: one lane of 2^22 40.7 ms, 2 of 2^21 38.5, 4 of 2^20 37.2, 8 of
+// 2^19 38.0 (8 of 2^21, 11.5 GB, 34.7).
 constexpr int kReplayLanes = 4;
 constexpr long long kReplayBatchPaths = 1ll << 20;
 
@@ -61,8 +62,9 @@ inline bool ensure_li_sort(Scratch &sb, uint64_t li_cap) {
 }
 
 // Fewer pairs or samples than this run in queue order: the sort's 13 launches take about 60 us,
-// more than it saves them (preview of 3,300 pairs: Li 0.25 -> 0.19 ms; render_scene, some
-// 2^17 samples a stage: 8.7 -> 8.4 ms with 2^18 here against 2^12).
+// more than it saves them (2^12 / 2^17 / 2^18 here: preview of 3,300 pairs 0.66 / 0.64 / 0.67 ms,
+// the last two the same code there; render_scene, some 2^17 samples a stage, 8.6 / 8.3 / 8.3; C0
+// forward, 10^7, equal).
 constexpr long long kSortMin = 1 << 17;
 
 // The n queued Li tasks' pairs (slots 2m, 2m + 1) in key order (k_li_keys) on stream st;
@@ -97,9 +99,11 @@ inline const int *sort_primary_samples(const RenderParams &rp, Scratch &sb, uint
 }
 
 
-// Rays and hits of the scene carry no derivatives: nothing moves but materials and media
-// (vertex, normal and camera velocities all absent or exactly zero). Continuation rays then
-// have none either: a scatter point lies on its ray, a new direction is sampled from values.
+// Rays and hits of the scene carry no derivatives: nothing moves but materials and media (vertex
+// and camera velocities all absent or exactly zero, and no shape has vertex normals: their
+// derivative array is there with them, velocities or not, and the general kernels read it).
+// Continuation rays then have none either: a scatter point lies on its ray, a new direction is
+// sampled from values.
 inline bool static_rays(const DevScene &sc) {
     if (sc.vert_der || sc.face_n_der || sc.normal_der || sc.moving_geometry) return false;
     for (int j = 0; j < sc.nder; ++j)
@@ -118,7 +122,8 @@ inline int media_kind(const DevScene &sc) {
 }
 
 // Camera paths per batch of a scene of static_rays(): its batches hold no records, only path
-// states (256 MB at nder 8), and kLanes of them run at once
+// states, vertex inputs and queues (224 to 384 B a path from nder 1 to 8: 0.24 to 0.40 GB a
+// batch), and up to kLanes of them run at once (1.9 to 3.2 GB)
 constexpr long long kStaticBatchPaths = 1ll << 20;
 
 // Buffers of the camera wavefront for `cap` paths: path states, vertex inputs, four

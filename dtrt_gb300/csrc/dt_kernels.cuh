@@ -480,8 +480,9 @@ constexpr int kWavefrontMaxLevels = 1024;
 // 14.4 / 14.1 / 13.5 / 13.9 ms at 3 / 4 / 5 / 6 blocks; C3, nder 8: 71.0 / 68.0 / 68.3 / 68.8).
 template <int N>
 constexpr int kCamBlocks = N > 4 ? 4 : 5;
-// With ray derivatives (camera stage of C0, nder 1: 3.03 / 2.39 / 2.19 / 2.09 ms at 2 / 3 / 4 /
-// 5 blocks; C2, nder 8: 10.90 / 10.46 / 10.71 / 10.78).
+// With ray derivatives (camera stage of C0, nder 1: 3.03 / 2.39 / 2.18 / 2.09 ms at 2 / 3 / 4 /
+// 5 blocks; nder 3 and 4: 3.10 and 3.54 at 4, 3.07 and 3.49 at 5; C2, nder 8: 10.90 / 10.46 /
+// 10.71 / 10.78 at 2 to 5). Up to nder 4 the step from 4 to 5 is less than 0.6 % of a render.
 template <int N>
 constexpr int kCamBlocksAd = N > 4 ? 3 : 4;
 

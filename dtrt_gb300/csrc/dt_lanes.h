@@ -8,9 +8,10 @@ namespace dt {
 
 // Wavefront batches in flight at once, each on a stream and a workspace of its own: a batch's
 // last levels hold few paths and take as long as their slowest vertex, and the other batches
-// run in the meantime; small batches read neighbouring voxels. C3 forward (33.6 M paths): one
-// lane of 2^23 paths 68.8 ms, 4 lanes of 2^21 63.7, 8 of 2^20 63.1, 8 of 2^19 66.4; C1 primal: one of
-// 2^22 15.9, 8 of 2^20 14.8, 8 of 2^19 14.1. Eight streams are what the device queues.
+// run in the meantime; small batches read neighbouring voxels. C3 forward (33.6 M paths) / C1
+// forward (16.8 M): 2 lanes of 2^23 paths 64.8 / 12.2 ms, 4 of 2^21 61.4 / 11.2, 8 of 2^20 60.8 /
+// 11.1, 8 of 2^21 61.2 / 11.2, 8 of 2^19 64.0 / 11.6; C1 primal: 2 lanes of 2^22 15.3, 4 of 2^21
+// 14.9, 8 of 2^20 14.7, 8 of 2^19 14.0, 8 of 2^18 14.7. Eight streams are what the device queues.
 constexpr int kLanes = 8;
 
 // Streams of the lanes 1..., the fork and join events (made by the first render that needs them)
